@@ -37,18 +37,6 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
     return total;
 }
 
-__device__ __forceinline__ float block_max(float v, float* scratch) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    __syncthreads();
-    if (lane == 0) scratch[warp] = v;
-    __syncthreads();
-    float best = scratch[0];
-    for (int w = 1; w < warps; ++w) best = fmaxf(best, scratch[w]);
-    return best;
-}
-
 // stream_out = half(stream_in + delta) (or stream_in when delta is null); normed = weight * half(s * rsqrt(mean(s^2) + eps))
 __global__ void __launch_bounds__(256)
 add_rmsnorm_kernel(const __half* __restrict__ stream_in, const __half* __restrict__ delta, const __half* __restrict__ weight,
@@ -144,155 +132,301 @@ struct AttentionParams {
     unsigned* status;         // set to 1 when the position does not fit the cache
 };
 
-// One CTA per query head, 128 threads.  D/8 consecutive lanes share a cached position: each reads 16
-// bytes of its K (then V) row, so a row is one coalesced 128- or 256-byte read, and the 128 threads
-// cover 16 (D = 64) or 8 (D = 128) positions per pass with independent loads in flight.
+// A cluster of CTAs per query head; each CTA takes a contiguous part of the cached positions, and every group of D/8 lanes
+// walks its own positions with a running maximum, sum and weighted V row, so nothing is exchanged before the end.  Then
+// the warps of a CTA are added up in shared memory, each CTA's result is written into the first CTA's shared memory
+// (distributed shared memory), one cluster barrier, and the first CTA adds those up.
+//
+// Bound: latency of a dependent kernel at short contexts, loads in flight at long ones.  One CTA per head left 116 SMs idle
+// and took 47.6 us a layer at 1500 positions (TinyLlama: 32 heads of 64); eight take 5.9 us.  Two or four heads of a KV
+// head in one CTA would read each K and V row fewer times out of L2; it was 0.4 us faster there and 0.5 us slower at 4
+// positions, where the extra arithmetic is all latency.  Rows are requested two passes ahead (two register buffers of
+// kAttnBatch rows of K and V).  Contexts of one part's worth use one CTA per cluster and no cluster barrier: the other
+// CTAs leave at once.
+constexpr int kAttnThreads = 256;
+constexpr int kAttnWarps = kAttnThreads / 32;
+constexpr int kAttnMaxParts = 8;                      // CTAs per cluster: the portable limit
+constexpr int kAttnBatch = 2;                         // passes requested together
+constexpr float kNoScore = -1.0e30f;
+
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_acquire() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// The address of `local` in the shared memory of the cluster's first CTA.
+__device__ __forceinline__ uint32_t in_first_cta(const void* local) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote)
+                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(local))));
+    return remote;
+}
+__device__ __forceinline__ void store_cluster(uint32_t address, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(address), "f"(v) : "memory");
+}
+
+// Eight FP16 values of the token's qkv row, which need not start on a 16-byte boundary.
+__device__ __forceinline__ uint4 load8_any(const __half* src) {
+    if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) return *reinterpret_cast<const uint4*>(src);
+    uint4 q;
+    __half* h = reinterpret_cast<__half*>(&q);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) h[i] = src[i];
+    return q;
+}
+
+// Rotary embedding of eight dims, rounded as the framework rounds it: cos/sin in FP16, two FP16 products, one FP16 sum
+// (the _rn forms are never contracted into one fused multiply-add).  `own` holds the dims, `other` the ones half a head away.
+__device__ __forceinline__ uint4 rotate8(const uint4& own, const uint4& other, bool first_half, const __half2* c, const __half2* s) {
+    uint4 out;
+    const __half2* a = reinterpret_cast<const __half2*>(&own);
+    const __half2* b = reinterpret_cast<const __half2*>(&other);
+    __half2* o = reinterpret_cast<__half2*>(&out);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __half2 turned = first_half ? __hneg2(b[i]) : b[i];
+        o[i] = __hadd2_rn(__hmul2_rn(a[i], c[i]), __hmul2_rn(turned, s[i]));
+    }
+    return out;
+}
+
 template <int D>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kAttnThreads)
 attention_decode_kernel(const AttentionParams p) {
     constexpr int kLanesPerPos = D / 8;
-    constexpr int kPosPerPass = 128 / kLanesPerPos;
-    extern __shared__ float scores[];                 // max_len floats
-    __shared__ float scratch[4];
-    __shared__ float q[D];
-    __shared__ __align__(16) __half k_new[D];
-    __shared__ __align__(16) __half v_new[D];
-    __shared__ float partial[kPosPerPass][D];
-    constexpr int kEarlyPasses = 2;                   // passes whose cache rows are requested before anything else
-    const int head = blockIdx.x;
+    constexpr int kPosPerPass = kAttnThreads / kLanesPerPos;   // 32 (D = 64) or 16 (D = 128)
+    constexpr int kPosPerBatch = kPosPerPass * kAttnBatch;
+    // A part is at least what one CTA requests before it needs any of it: less is not worth the cluster barrier.
+    constexpr int kPosPerPart = 2 * kPosPerBatch;
     constexpr int half_d = D / 2;
-    const int kv_head = head / (p.q_heads / p.kv_heads);
-    const int sub = threadIdx.x % kLanesPerPos;       // which 8 of the D dims
-    const int slot = threadIdx.x / kLanesPerPos;      // which position of a pass
-    const uint4* k_rows = reinterpret_cast<const uint4*>(p.k_cache + static_cast<size_t>(kv_head) * p.max_len * D) + sub;
-    const uint4* v_rows = reinterpret_cast<const uint4*>(p.v_cache + static_cast<size_t>(kv_head) * p.max_len * D) + sub;
+    __shared__ __align__(16) __half cos_table[half_d];
+    __shared__ __align__(16) __half sin_table[half_d];
+    static_assert(D <= kAttnThreads);
+    __shared__ __align__(16) float warp_acc[kAttnWarps][D];
+    __shared__ float warp_max[kAttnWarps], warp_sum[kAttnWarps];
+    __shared__ float part_acc[kAttnMaxParts][D];               // the first CTA's are written by the whole cluster
+    __shared__ float part_max[kAttnMaxParts], part_sum[kAttnMaxParts];
+
+    uint32_t part, max_parts;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(part));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(max_parts));
+    const int head = blockIdx.x / max_parts;
+    const int group_heads = p.q_heads / p.kv_heads;
+    const int kv_head = head / group_heads;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int sub = tid % kLanesPerPos;               // which 8 of the D dims
+    const int slot = tid / kLanesPerPos;              // which position of a pass
     pdl_release_downstream();
-    // Nothing below depends on the kernel just before this one (it produces qkv): the position was set
-    // and the older cache rows were written by earlier steps.  So the first rows of K and V, the position
-    // and the rotary frequencies are requested before waiting for that kernel.  Rows at or past the
-    // position hold stale data; they are fetched (inside the cache) and never used.
-    uint4 k_early[kEarlyPasses], v_early[kEarlyPasses];
-#pragma unroll
-    for (int e = 0; e < kEarlyPasses; ++e) {
-        const int t = min(e * kPosPerPass + slot, p.max_len - 1);
-        k_early[e] = k_rows[static_cast<size_t>(t) * kLanesPerPos];
-        v_early[e] = v_rows[static_cast<size_t>(t) * kLanesPerPos];
-    }
+    // Nothing up to the wait depends on the kernel just before this one (it produces qkv): the position was set and the
+    // older cache rows were written by earlier steps.  The first part starts at position 0 whatever the context, so its
+    // first rows are requested without waiting for the position; rows past it hold stale data and are never used.
     const long long pos = *p.position;
-    const float freq = p.inv_freq[threadIdx.x % half_d];
-    pdl_wait_for_upstream();
+    const float freq = p.inv_freq[tid % half_d];
+    const size_t head_base = static_cast<size_t>(kv_head) * p.max_len * kLanesPerPos + sub;
+    const uint4* k_rows = reinterpret_cast<const uint4*>(p.k_cache) + head_base;
+    const uint4* v_rows = reinterpret_cast<const uint4*>(p.v_cache) + head_base;
+    struct Rows {
+        uint4 k[kAttnBatch], v[kAttnBatch];
+    };
+    Rows even, odd;
+    if (part == 0) {
+        const size_t t = static_cast<size_t>(min(slot, p.max_len - 1));
+        even.k[0] = k_rows[t * kLanesPerPos];
+        even.v[0] = v_rows[t * kLanesPerPos];
+    }
     if (pos < 0 || pos >= p.max_len) {
-        if (threadIdx.x == 0) atomicMax(p.status, 1u);
+        if (tid == 0 && part == 0) atomicMax(p.status, 1u);
+        pdl_wait_for_upstream();
         return;
     }
+    const int newest = static_cast<int>(pos);         // positions [0, newest) come from the cache, the newest from qkv
+    const int parts = min(static_cast<int>(max_parts), newest / kPosPerPart + 1);
+    if (parts == 1 && part > 0) return;
+    if (parts > 1) cluster_arrive_relaxed();          // "this CTA runs": waited for before its memory is written to
+    if (static_cast<int>(part) >= parts) {            // no positions for this CTA: it only takes part in the barriers
+        cluster_wait_acquire();
+        cluster_arrive_release();
+        cluster_wait_acquire();
+        return;
+    }
+    const int per_part = newest / parts + 1;
+    const int begin = static_cast<int>(part) * per_part;
+    const int end = min(newest + 1, begin + per_part);
+    auto fetch = [&](Rows& rows, int base) {
+#pragma unroll
+        for (int e = 0; e < kAttnBatch; ++e) {
+            const int t = base + e * kPosPerPass + slot;
+            if (t < min(end, newest) && (e > 0 || base > 0)) {
+                rows.k[e] = k_rows[static_cast<size_t>(t) * kLanesPerPos];
+                rows.v[e] = v_rows[static_cast<size_t>(t) * kLanesPerPos];
+            }
+        }
+    };
+    fetch(even, begin);
+    fetch(odd, begin + kPosPerBatch);
+    if (tid < half_d) {
+        float sn, cs;
+        sincosf(static_cast<float>(pos) * freq, &sn, &cs);
+        cos_table[tid] = __float2half_rn(cs * p.rope_scale);
+        sin_table[tid] = __float2half_rn(sn * p.rope_scale);
+    }
+    __syncthreads();
+    const bool first_half = sub < kLanesPerPos / 2;
+    const int pair_sub = sub ^ (kLanesPerPos / 2);    // the lane whose dims are half a head away
+    const __half2* my_cos = reinterpret_cast<const __half2*>(cos_table + (sub * 8) % half_d);
+    const __half2* my_sin = reinterpret_cast<const __half2*>(sin_table + (sub * 8) % half_d);
+
+    pdl_wait_for_upstream();
     const __half* q_in = p.qkv + head * D;
     const __half* k_in = p.qkv + p.q_heads * D + kv_head * D;
     const __half* v_in = p.qkv + (p.q_heads + p.kv_heads) * D + kv_head * D;
-    // rotary embedding, rounded as the framework rounds it: cos/sin to FP16, two FP16 products, one FP16 sum
-    if (threadIdx.x < D) {
-        const int i = threadIdx.x;
-        const float angle = static_cast<float>(pos) * freq;
-        float sn, cs;
-        sincosf(angle, &sn, &cs);
-        const __half c = __float2half_rn(cs * p.rope_scale);
-        const __half s = __float2half_rn(sn * p.rope_scale);
-        const __half q_rot = i < half_d ? __hneg(q_in[i + half_d]) : q_in[i - half_d];
-        const __half k_rot = i < half_d ? __hneg(k_in[i + half_d]) : k_in[i - half_d];
-        // the _rn forms are never contracted into one fused multiply-add: two roundings, then a third
-        q[i] = __half2float(__hadd_rn(__hmul_rn(q_in[i], c), __hmul_rn(q_rot, s)));
-        const __half k_val = __hadd_rn(__hmul_rn(k_in[i], c), __hmul_rn(k_rot, s));
-        k_new[i] = k_val;
-        v_new[i] = v_in[i];
-        if (head % (p.q_heads / p.kv_heads) == 0) {   // one CTA per KV head appends to the cache
-            p.k_cache[(static_cast<size_t>(kv_head) * p.max_len + pos) * D + i] = k_val;
-            p.v_cache[(static_cast<size_t>(kv_head) * p.max_len + pos) * D + i] = v_in[i];
+    const uint4 q_own = load8_any(q_in + sub * 8), q_other = load8_any(q_in + pair_sub * 8);
+    uint4 k_new = make_uint4(0u, 0u, 0u, 0u), v_new = k_new;
+    if (end > newest) {                               // the CTA whose part ends with the newest position
+        const uint4 k_own = load8_any(k_in + sub * 8), k_other = load8_any(k_in + pair_sub * 8);
+        v_new = load8_any(v_in + sub * 8);
+        k_new = rotate8(k_own, k_other, first_half, my_cos, my_sin);
+        if (slot == 0 && head % group_heads == 0) {   // one cluster of the KV head appends to the cache
+            const size_t row = head_base + static_cast<size_t>(newest) * kLanesPerPos;
+            reinterpret_cast<uint4*>(p.k_cache)[row] = k_new;
+            reinterpret_cast<uint4*>(p.v_cache)[row] = v_new;
         }
     }
-    __syncthreads();
-
-    const int length = static_cast<int>(pos) + 1;
-    // The newest position comes from shared memory, not from the cache: another CTA writes it there.
-    auto row_piece = [&](const uint4* rows, const __half* newest, const uint4 (&early)[kEarlyPasses], int base, int t) {
-        if (t == length - 1) return reinterpret_cast<const uint4*>(newest)[sub];
-        if (base == 0) return early[0];
-        if (base == kPosPerPass) return early[1];
-        return rows[static_cast<size_t>(t) * kLanesPerPos];
+    auto widen8 = [](const uint4& piece, float (&f)[8]) {
+        const __half2* pairs = reinterpret_cast<const __half2*>(&piece);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 two = __half22float2(pairs[i]);
+            f[2 * i] = two.x;
+            f[2 * i + 1] = two.y;
+        }
     };
-    float qf[8];
+    float q[8], acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    float top = kNoScore, sum = 0.0f;
+    widen8(rotate8(q_own, q_other, first_half, my_cos, my_sin), q);
+    auto use = [&](Rows& rows, int base) {
+        if (base + warp * (32 / kLanesPerPos) >= end) return;   // nothing for this warp
+        float dot[kAttnBatch];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) qf[i] = q[sub * 8 + i];
-
-    float local_max = -INFINITY;
-#pragma unroll 4
-    for (int base = 0; base < length; base += kPosPerPass) {
-        const int t = base + slot;
-        float dot = 0.0f;
-        if (t < length) {
-            const uint4 piece = row_piece(k_rows, k_new, k_early, base, t);
-            const __half2* h = reinterpret_cast<const __half2*>(&piece);
+        for (int e = 0; e < kAttnBatch; ++e) {
+            float k[8];
+            widen8(base + e * kPosPerPass + slot == newest ? k_new : rows.k[e], k);
+            dot[e] = 0.0f;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2 kk = __half22float2(h[i]);
-                dot += qf[2 * i] * kk.x + qf[2 * i + 1] * kk.y;
+            for (int i = 0; i < 8; ++i) dot[e] += q[i] * k[i];
+        }
+#pragma unroll
+        for (int o = kLanesPerPos / 2; o > 0; o >>= 1) {
+#pragma unroll
+            for (int e = 0; e < kAttnBatch; ++e) dot[e] += __shfl_xor_sync(0xffffffffu, dot[e], o);
+        }
+        // a new maximum: what has been summed so far shrinks by e^(old - new)
+        float next = top;
+#pragma unroll
+        for (int e = 0; e < kAttnBatch; ++e) {
+            dot[e] *= p.softmax_scale;
+            if (base + e * kPosPerPass + slot < end) next = fmaxf(next, dot[e]);
+        }
+        const float shrink = expf(top - next);
+        top = next;
+        sum *= shrink;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] *= shrink;
+#pragma unroll
+        for (int e = 0; e < kAttnBatch; ++e) {
+            const int t = base + e * kPosPerPass + slot;
+            if (t < end) {
+                float v[8];
+                widen8(t == newest ? v_new : rows.v[e], v);
+                const float w = expf(dot[e] - top);
+                sum += w;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[i] += w * v[i];
             }
         }
+    };
+    for (int base = begin; base < end; base += 2 * kPosPerBatch) {
+        use(even, base);
+        fetch(even, base + 2 * kPosPerBatch);
+        use(odd, base + kPosPerBatch);
+        fetch(odd, base + 3 * kPosPerBatch);
+    }
+    // lane groups of a warp, then the warps, then the CTAs of the cluster
 #pragma unroll
-        for (int o = kLanesPerPos / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        if (t < length) {
-            dot *= p.softmax_scale;
-            if (sub == 0) scores[t] = dot;
-            local_max = fmaxf(local_max, dot);
+    for (int o = kLanesPerPos; o < 32; o <<= 1) {
+        const float other_top = __shfl_xor_sync(0xffffffffu, top, o);
+        const float next = fmaxf(top, other_top);
+        const float mine = expf(top - next), theirs = expf(other_top - next);
+        top = next;
+        sum = sum * mine + __shfl_xor_sync(0xffffffffu, sum, o) * theirs;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] = acc[i] * mine + __shfl_xor_sync(0xffffffffu, acc[i], o) * theirs;
+    }
+    if (lane < kLanesPerPos) {
+        float4* to = reinterpret_cast<float4*>(&warp_acc[warp][lane * 8]);
+        to[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        to[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+        if (lane == 0) {
+            warp_max[warp] = top;
+            warp_sum[warp] = sum;
         }
     }
-    const float top = block_max(local_max, scratch);  // its barriers also publish the scores
-    float local_sum = 0.0f;
-    for (int t = threadIdx.x; t < length; t += blockDim.x) {
-        const float e = expf(scores[t] - top);
-        scores[t] = e;
-        local_sum += e;
-    }
-    const float denom = block_sum(local_sum, scratch);
-
-    float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 4
-    for (int base = 0; base < length; base += kPosPerPass) {
-        const int t = base + slot;
-        if (t < length) {
-            const float w = scores[t];
-            const uint4 piece = row_piece(v_rows, v_new, v_early, base, t);
-            const __half2* h = reinterpret_cast<const __half2*>(&piece);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2 vv = __half22float2(h[i]);
-                acc[2 * i] += w * vv.x;
-                acc[2 * i + 1] += w * vv.y;
-            }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) partial[slot][sub * 8 + i] = acc[i];
     __syncthreads();
-    if (threadIdx.x < D) {
-        float total = 0.0f;
-#pragma unroll
-        for (int g = 0; g < kPosPerPass; ++g) total += partial[g][threadIdx.x];
-        p.out[head * D + threadIdx.x] = __float2half_rn(total / denom);
+    // one element of the head's output: its weighted sum, the sum of the weights, and the maximum both refer to
+    auto merge = [&](int count, const float* maxima, const float* sums, const float (*rows)[D], float& best, float& total,
+                     float& weight) {
+        best = kNoScore;
+        total = weight = 0.0f;
+        for (int r = 0; r < count; ++r) best = fmaxf(best, maxima[r]);
+        for (int r = 0; r < count; ++r) {
+            const float w = expf(maxima[r] - best);
+            weight += w * sums[r];
+            total += w * rows[r][tid];
+        }
+    };
+    float best, total, weight;
+    if (parts > 1) cluster_wait_acquire();            // every CTA of the cluster has started
+    if (tid < D) {
+        merge(kAttnWarps, warp_max, warp_sum, warp_acc, best, total, weight);
+        if (parts == 1) {
+            p.out[head * D + tid] = __float2half_rn(total / weight);
+        } else {
+            store_cluster(in_first_cta(&part_acc[part][tid]), total);
+            if (tid == 0) {
+                store_cluster(in_first_cta(&part_max[part]), best);
+                store_cluster(in_first_cta(&part_sum[part]), weight);
+            }
+        }
+    }
+    if (parts == 1) return;
+    __syncwarp();
+    cluster_arrive_release();
+    cluster_wait_acquire();
+    if (part == 0 && tid < D) {
+        merge(parts, part_max, part_sum, part_acc, best, total, weight);
+        p.out[head * D + tid] = __float2half_rn(total / weight);
     }
 }
 
 template <typename... Params, typename... Args>
-int launch_kernel(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, bool programmatic, cudaStream_t stream,
-                  Args... args) {
+int launch_kernel(void (*kernel)(Params...), dim3 grid, dim3 block, int cluster, size_t smem, bool programmatic,
+                  cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t launch = {};
     launch.gridDim = grid;
     launch.blockDim = block;
     launch.dynamicSmemBytes = smem;
     launch.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
     launch.attrs = attr;
-    launch.numAttrs = programmatic ? 1 : 0;
+    if (programmatic) {
+        attr[launch.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[launch.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[launch.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[launch.numAttrs].val.clusterDim.x = static_cast<unsigned>(cluster);
+        attr[launch.numAttrs].val.clusterDim.y = 1;
+        attr[launch.numAttrs++].val.clusterDim.z = 1;
+    }
     if (cudaLaunchKernelEx(&launch, kernel, static_cast<Params>(args)...) != cudaSuccess) return W4A16_ERR_LAUNCH;
     g_launch_count.fetch_add(1, std::memory_order_relaxed);
     return W4A16_OK;
@@ -302,17 +436,17 @@ int launch_kernel(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
 
 int launch_add_rmsnorm(const __half* stream_in, const __half* delta, const __half* weight, __half* stream_out,
                        __half* normed, int hidden, float eps, bool programmatic, cudaStream_t stream) {
-    return launch_kernel(add_rmsnorm_kernel, dim3(1), dim3(256), static_cast<size_t>(hidden) * sizeof(__half), programmatic,
+    return launch_kernel(add_rmsnorm_kernel, dim3(1), dim3(256), 1, static_cast<size_t>(hidden) * sizeof(__half), programmatic,
                          stream, stream_in, delta, weight, stream_out, normed, hidden, eps);
 }
 
 int launch_silu_mul(const __half* gate_up, __half* out, int inter, bool programmatic, cudaStream_t stream) {
-    return launch_kernel(silu_mul_kernel, dim3((inter + 255) / 256), dim3(256), 0, programmatic, stream, gate_up, out, inter);
+    return launch_kernel(silu_mul_kernel, dim3((inter + 255) / 256), dim3(256), 1, 0, programmatic, stream, gate_up, out, inter);
 }
 
 int launch_argmax_advance(const __half* logits, int count, long long* token, long long* position, bool programmatic,
                           cudaStream_t stream) {
-    return launch_kernel(argmax_advance_kernel, dim3(1), dim3(1024), 0, programmatic, stream, logits, count, token, position);
+    return launch_kernel(argmax_advance_kernel, dim3(1), dim3(1024), 1, 0, programmatic, stream, logits, count, token, position);
 }
 
 int launch_attention_decode(const __half* qkv, __half* k_cache, __half* v_cache, __half* out, const long long* position,
@@ -320,22 +454,13 @@ int launch_attention_decode(const __half* qkv, __half* k_cache, __half* v_cache,
                             float softmax_scale, unsigned* status, bool programmatic, cudaStream_t stream) {
     AttentionParams params{qkv, k_cache, v_cache, out, position, inv_freq, q_heads, kv_heads, head_dim, max_len,
                            rope_scale, softmax_scale, status};
-    const size_t smem = static_cast<size_t>(max_len) * sizeof(float);      // the scores; the rest is static
     auto kernel = head_dim == 64 ? attention_decode_kernel<64> : attention_decode_kernel<128>;
-    if (smem > 32 * 1024) {
-        if (smem > 160 * 1024) return W4A16_ERR_TOO_LARGE;
-        static bool raised[64][2] = {};
-        int device = 0;
-        if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return W4A16_ERR_LAUNCH;
-        const int which = head_dim == 64 ? 0 : 1;
-        if (!raised[device][which]) {
-            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess) {
-                return W4A16_ERR_LAUNCH;
-            }
-            raised[device][which] = true;
-        }
-    }
-    return launch_kernel(kernel, dim3(q_heads), dim3(128), smem, programmatic, stream, params);
+    // CTAs per head: as many as the cache can give a part's worth of positions each, and no more than two per SM in all.
+    const int positions = kAttnThreads / (head_dim / 8) * kAttnBatch * 2;
+    int parts = 1;
+    while (parts < kAttnMaxParts && parts * positions < max_len && 2 * parts * q_heads <= 2 * 148) parts *= 2;
+    return launch_kernel(kernel, dim3(static_cast<unsigned>(q_heads) * parts), dim3(kAttnThreads), parts, 0, programmatic,
+                         stream, params);
 }
 
 }  // namespace w4a16

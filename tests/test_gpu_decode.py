@@ -92,6 +92,31 @@ def test_attention_decode_matches_rope_plus_sdpa(q_heads, kv_heads, head_dim):
     assert status.item() == 1
 
 
+@pytest.mark.parametrize(("q_heads", "kv_heads", "head_dim", "max_len"), [(8, 2, 64, 2048), (6, 6, 128, 1100), (160, 8, 64, 300)])
+def test_attention_decode_splits_long_contexts(q_heads, kv_heads, head_dim, max_len):
+    """Positions around the edges of passes, batches and parts, on a cache that is already full of other rows."""
+    from nibble_b200.decode import attention_decode
+
+    g = torch.Generator(device="cuda").manual_seed(max_len)
+    draw = lambda *shape: torch.randn(shape, generator=g, device="cuda").half()  # noqa: E731
+    k_cache, v_cache = draw(kv_heads, max_len, head_dim), draw(kv_heads, max_len, head_dim)
+    inv_freq = torch.zeros((head_dim // 2,), device="cuda")           # no rotation: the caches are the reference's rows
+    status = torch.zeros((1,), dtype=torch.int32, device="cuda")
+    out = torch.empty((1, q_heads * head_dim), dtype=torch.float16, device="cuda")
+    edges = (0, 1, 15, 16, 31, 32, 63, 64, 127, 128, 129, 255, 256, 257, 511, 513, 1000, 1023, 1024, 1025, 2046)
+    for pos in [e for e in edges if e < max_len - 1] + [max_len - 1]:
+        qkv = draw(1, (q_heads + 2 * kv_heads) * head_dim) * 2
+        position = torch.full((1,), pos, dtype=torch.long, device="cuda")
+        attention_decode(qkv, k_cache, v_cache, out, position, inv_freq, q_heads, kv_heads, head_dim, 1.0, status)
+        q, k, v = (part.view(-1, head_dim) for part in qkv[0].split([q_heads * head_dim] + [kv_heads * head_dim] * 2))
+        assert torch.equal(k_cache[:, pos], k) and torch.equal(v_cache[:, pos], v)
+        keys, values = (c[:, : pos + 1].float().repeat_interleave(q_heads // kv_heads, 0) for c in (k_cache, v_cache))
+        scores = torch.einsum("hd,htd->ht", q.float(), keys) * head_dim ** -0.5
+        want = torch.einsum("ht,htd->hd", scores.softmax(-1), values).reshape(1, -1)
+        torch.testing.assert_close(out.float(), want, rtol=2e-3, atol=1e-3)
+    assert status.item() == 0
+
+
 def test_argmax_advance_picks_the_first_maximum():
     from nibble_b200.decode import argmax_advance
 
