@@ -96,6 +96,13 @@ int w4a16_linear_f16(const void* x, const void* packed, const void* scales, void
                      void* workspace, size_t workspace_bytes,
                      uint32_t flags, w4a16_stream_t stream);
 
+/* Same as w4a16_linear_f16, with `bias` (FP16 [N], may be NULL) added to the rounded FP16 result -- the bits of a separate
+ * FP16 addition, without its launch.  A bias with W4A16_FLAG_OUTPUT_F32 or K == 0 returns W4A16_ERR_BAD_CONFIG. */
+int w4a16_linear_f16_bias(const void* x, const void* packed, const void* scales, const void* bias, void* y,
+                          int64_t M, int64_t N, int64_t K, int64_t group_size,
+                          void* workspace, size_t workspace_bytes,
+                          uint32_t flags, w4a16_stream_t stream);
+
 /* Same as w4a16_linear_f16 with an explicit launch shape for the fast path (tuning, tests).
  * Returns W4A16_ERR_BAD_CONFIG when the fast path does not apply or the shape is not built. */
 int w4a16_linear_f16_config(const void* x, const void* packed, const void* scales, void* y,

@@ -4,8 +4,9 @@ Two shared objects are produced next to this file:
 
 * ``libw4a16_b200.so`` -- the CUDA kernels behind a plain C ABI (``include/w4a16_b200.h``),
   compiled by nvcc for ``sm_100a`` only; it does not link against torch.
-* ``_C.so`` -- the torch operator shim (``csrc/int4_linear.cpp``) that registers
-  ``torch.ops.w4a16.linear`` / ``dequantize`` and forwards to the C ABI.
+* ``_C.so`` -- the torch side: the operators (``csrc/int4_linear.cpp`` registers ``torch.ops.w4a16.linear`` /
+  ``dequantize`` and forwards to the C ABI) and, as a Python module, the native forward of ``QuantizedLinear``
+  (``csrc/linear_module.cpp``).
 
 ``python nibble_b200/_build.py`` builds both; nothing is rebuilt while the outputs are newer than
 every source.
@@ -100,15 +101,17 @@ def build_checked(force: bool = False) -> pathlib.Path:
 
 
 def build_torch_shim(force: bool = False) -> pathlib.Path:
-    """Compile ``csrc/int4_linear.cpp`` against the installed torch and link it to the core library."""
+    """Compile the C++ sources against the installed torch and Python and link them to the core library."""
     build_core(force)
     if (not force and TORCH_LIB.exists()
             and TORCH_LIB.stat().st_mtime >= max(_sources_mtime(), CORE_LIB.stat().st_mtime)):
         return TORCH_LIB
+    import sysconfig
+
     import torch
     from torch.utils import cpp_extension
 
-    includes = []
+    includes = ["-isystem", sysconfig.get_paths()["include"]]
     for path in cpp_extension.include_paths("cuda"):
         includes += ["-isystem", path]
     torch_lib_dir = pathlib.Path(torch.__file__).resolve().parent / "lib"
@@ -117,8 +120,8 @@ def build_torch_shim(force: bool = False) -> pathlib.Path:
         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
         "-DTORCH_EXTENSION_NAME=_C",
         *includes, "-I", str(INCLUDE),
-        str(CSRC / "int4_linear.cpp"), "-o", str(TORCH_LIB),
-        f"-L{torch_lib_dir}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch",
+        str(CSRC / "int4_linear.cpp"), str(CSRC / "linear_module.cpp"), "-o", str(TORCH_LIB),
+        f"-L{torch_lib_dir}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python",
         f"-L{PKG}", "-l:libw4a16_b200.so",
         "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib_dir}",
     ]

@@ -95,6 +95,7 @@ _I = ctypes.c_int64
 # name -> (restype, argtypes): the complete exported surface of include/w4a16_b200.h
 C_API = {
     "w4a16_linear_f16": (ctypes.c_int, [_P, _P, _P, _P, _I, _I, _I, _I, _P, ctypes.c_size_t, ctypes.c_uint32, _P]),
+    "w4a16_linear_f16_bias": (ctypes.c_int, [_P, _P, _P, _P, _P, _I, _I, _I, _I, _P, ctypes.c_size_t, ctypes.c_uint32, _P]),
     "w4a16_linear_f16_config": (
         ctypes.c_int,
         [_P, _P, _P, _P, _I, _I, _I, _I, _P, ctypes.c_size_t, ctypes.c_uint32, ctypes.POINTER(LinearConfig), _P],
@@ -174,9 +175,12 @@ def status_string(status: int) -> str:
 
 
 @functools.lru_cache(maxsize=None)
-def load_torch_ops() -> None:
+def load_torch_ops():
+    """Registers ``torch.ops.w4a16.*`` and returns the extension module."""
     if not TORCH_LIB.exists():
         raise ImportError(f"{TORCH_LIB.name} is not built; run `python nibble_b200/_build.py`")
-    import torch
+    import importlib
 
-    torch.ops.load_library(str(TORCH_LIB))
+    import torch  # noqa: F401  (its libraries first)
+
+    return importlib.import_module(__package__ + "._C")

@@ -109,6 +109,12 @@ size_t w4a16_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
 int w4a16_linear_f16(const void* x, const void* packed, const void* scales, void* y, int64_t M, int64_t N,
                      int64_t K, int64_t group_size, void* workspace, size_t workspace_bytes, uint32_t flags,
                      w4a16_stream_t stream) {
+    return w4a16_linear_f16_bias(x, packed, scales, nullptr, y, M, N, K, group_size, workspace, workspace_bytes, flags, stream);
+}
+
+int w4a16_linear_f16_bias(const void* x, const void* packed, const void* scales, const void* bias, void* y, int64_t M, int64_t N,
+                          int64_t K, int64_t group_size, void* workspace, size_t workspace_bytes, uint32_t flags,
+                          w4a16_stream_t stream) {
     const int status = validate_linear(x, packed, scales, y, M, N, K, group_size);
     if (status != W4A16_OK || M == 0 || N == 0) return status;
     w4a16::LinearProblem p{static_cast<const __half*>(x), static_cast<const uint8_t*>(packed),
@@ -116,6 +122,8 @@ int w4a16_linear_f16(const void* x, const void* packed, const void* scales, void
                            workspace, workspace_bytes};
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const bool out_f32 = (flags & W4A16_FLAG_OUTPUT_F32) != 0;
+    p.bias = static_cast<const __half*>(bias);
+    if (bias != nullptr && (out_f32 || K == 0)) return W4A16_ERR_BAD_CONFIG;
     if (K == 0) {
         const size_t element = out_f32 ? sizeof(float) : sizeof(__half);
         return cudaMemsetAsync(y, 0, static_cast<size_t>(M) * N * element, s) == cudaSuccess

@@ -109,6 +109,7 @@ struct GridSync {
 struct StepHooks {
     GridSync& sync;
     __device__ __forceinline__ void at_start() {}
+    __device__ __forceinline__ bool weights_wait(const MmaParams&) const { return false; }
     __device__ __forceinline__ void before_activations() { sync.wait_for_previous(); }
     __device__ __forceinline__ void after_outputs() { sync.arrive(); }
 };

@@ -3,8 +3,9 @@
 // int4_linear_cuda / int4_dequantize_cuda do (csrc/int4_linear_kernel.cu:646-691, 809-841: every
 // violation is a TORCH_CHECK, i.e. a Python RuntimeError), allocates the output from the caching
 // allocator and hands raw pointers plus the current stream to the C ABI in include/w4a16_b200.h.
-// No kernel lives here.
+// No kernel lives here.  linear_module.cpp, the native side of QuantizedLinear.forward, calls these operators.
 #include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/library.h>
@@ -13,6 +14,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <optional>
 #include <utility>
 
 #include "../../include/w4a16_b200.h"
@@ -60,8 +62,9 @@ void check_status(int status, const char* what) {
     TORCH_CHECK(status == W4A16_OK, what, " failed: ", w4a16_status_string(status));
 }
 
+// `activations` is [..., K] when `any_rank`, else [M, K]; the result keeps its leading dimensions.
 at::Tensor linear_impl(const at::Tensor& activations, const at::Tensor& packed_weights, const at::Tensor& scales,
-                       int64_t group_size, bool out_f32) {
+                       const at::Tensor* bias, int64_t group_size, bool out_f32, bool any_rank) {
     TORCH_CHECK(activations.is_cuda(), "activations must be a CUDA tensor");
     TORCH_CHECK(packed_weights.is_cuda(), "packed_weights must be a CUDA tensor");
     TORCH_CHECK(scales.is_cuda(), "scales must be a CUDA tensor");
@@ -70,7 +73,11 @@ at::Tensor linear_impl(const at::Tensor& activations, const at::Tensor& packed_w
     TORCH_CHECK(activations.scalar_type() == at::kHalf, "activations must have dtype torch.float16");
     TORCH_CHECK(packed_weights.scalar_type() == at::kByte, "packed_weights must have dtype torch.uint8");
     TORCH_CHECK(scales.scalar_type() == at::kHalf, "scales must have dtype torch.float16");
-    TORCH_CHECK(activations.dim() == 2, "activations must have shape [M, K]");
+    if (any_rank) {
+        TORCH_CHECK(activations.dim() >= 1, "activations must have shape [..., K]");
+    } else {
+        TORCH_CHECK(activations.dim() == 2, "activations must have shape [M, K]");
+    }
     TORCH_CHECK(packed_weights.dim() == 2, "packed_weights must have shape [N, K / 2]");
     TORCH_CHECK(scales.dim() == 2, "scales must have shape [N, K / group_size]");
     TORCH_CHECK(activations.is_contiguous(), "activations must be contiguous");
@@ -79,16 +86,24 @@ at::Tensor linear_impl(const at::Tensor& activations, const at::Tensor& packed_w
     TORCH_CHECK(group_size > 0, "group_size must be greater than zero");
     TORCH_CHECK(group_size % 2 == 0, "group_size must be even because each byte contains two weights");
 
-    const int64_t m = activations.size(0);
-    const int64_t k = activations.size(1);
+    const int64_t k = activations.size(-1);
     const int64_t n = packed_weights.size(0);
     TORCH_CHECK(packed_weights.size(1) * 2 == k, "packed_weights and activations must describe the same K dimension");
     TORCH_CHECK(k % group_size == 0, "K must be divisible by group_size");
     TORCH_CHECK(scales.size(0) == n && scales.size(1) == k / group_size,
                 "scales must have shape [N, K / group_size]");
+    if (bias != nullptr) {
+        TORCH_CHECK(bias->device() == activations.device() && bias->scalar_type() == at::kHalf && bias->is_contiguous() &&
+                        bias->dim() == 1 && bias->size(0) == n,
+                    "bias must be a contiguous float16 tensor with shape [N] on the activations' device");
+    }
 
     const c10::cuda::CUDAGuard guard(activations.device());
-    at::Tensor output = at::empty({m, n}, out_f32 ? activations.options().dtype(at::kFloat) : activations.options());
+    c10::SmallVector<int64_t, 5> shape(activations.sizes().begin(), activations.sizes().end());
+    int64_t m = 1;
+    for (size_t i = 0; i + 1 < shape.size(); ++i) m *= shape[i];
+    shape.back() = n;
+    at::Tensor output = at::detail::empty_cuda(shape, out_f32 ? at::kFloat : at::kHalf, activations.device(), c10::nullopt);
     if (m == 0 || n == 0) return output;
 
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
@@ -105,7 +120,7 @@ at::Tensor linear_impl(const at::Tensor& activations, const at::Tensor& packed_w
     }
 
     int status;
-    if (forced_tiles != 0 && !(flags & W4A16_FLAG_FORCE_GENERIC) && group_size == 128 &&
+    if (forced_tiles != 0 && bias == nullptr && !(flags & W4A16_FLAG_FORCE_GENERIC) && group_size == 128 &&
         reinterpret_cast<uintptr_t>(activations.data_ptr()) % 16 == 0 &&
         reinterpret_cast<uintptr_t>(packed_weights.data_ptr()) % 16 == 0) {
         w4a16_linear_config config = {forced_tiles, 0, 0, 0, 0};
@@ -113,9 +128,12 @@ at::Tensor linear_impl(const at::Tensor& activations, const at::Tensor& packed_w
                                          output.data_ptr(), m, n, k, group_size, workspace, workspace_bytes,
                                          flags, &config, reinterpret_cast<w4a16_stream_t>(stream));
     } else {
-        status = w4a16_linear_f16(activations.data_ptr(), packed_weights.data_ptr(), scales.data_ptr(),
-                                  output.data_ptr(), m, n, k, group_size, workspace, workspace_bytes, flags,
-                                  reinterpret_cast<w4a16_stream_t>(stream));
+        // (an empty K leaves zeros, which the C entry point does not add a bias to)
+        const bool fold = bias != nullptr && k > 0;
+        status = w4a16_linear_f16_bias(activations.data_ptr(), packed_weights.data_ptr(), scales.data_ptr(),
+                                       fold ? bias->data_ptr() : nullptr, output.data_ptr(), m, n, k, group_size, workspace,
+                                       workspace_bytes, flags, reinterpret_cast<w4a16_stream_t>(stream));
+        if (bias != nullptr && !fold) output.add_(*bias);
     }
     check_status(status, "w4a16::linear");
     return output;
@@ -123,13 +141,19 @@ at::Tensor linear_impl(const at::Tensor& activations, const at::Tensor& packed_w
 
 at::Tensor linear_cuda_impl(const at::Tensor& activations, const at::Tensor& packed_weights,
                             const at::Tensor& scales, int64_t group_size) {
-    return linear_impl(activations, packed_weights, scales, group_size, false);
+    return linear_impl(activations, packed_weights, scales, nullptr, group_size, false, false);
 }
 
 // Same product with the unrounded FP32 sums as output: the per-device partial of a K-sharded layer.
 at::Tensor linear_partial_cuda_impl(const at::Tensor& activations, const at::Tensor& packed_weights,
                                     const at::Tensor& scales, int64_t group_size) {
-    return linear_impl(activations, packed_weights, scales, group_size, true);
+    return linear_impl(activations, packed_weights, scales, nullptr, group_size, true, false);
+}
+
+// The module's whole fused call: activations of any rank, and the bias inside the kernel.
+at::Tensor linear_bias_cuda_impl(const at::Tensor& activations, const at::Tensor& packed_weights, const at::Tensor& scales,
+                                 const std::optional<at::Tensor>& bias, int64_t group_size) {
+    return linear_impl(activations, packed_weights, scales, bias.has_value() ? &*bias : nullptr, group_size, false, true);
 }
 
 at::Tensor dequantize_cuda_impl(const at::Tensor& packed_weights, const at::Tensor& scales, int64_t group_size) {
@@ -191,6 +215,8 @@ std::tuple<at::Tensor, at::Tensor> quantize_pack_cuda_impl(const at::Tensor& wei
 
 TORCH_LIBRARY(w4a16, m) {
     m.def("linear(Tensor activations, Tensor packed_weights, Tensor scales, int group_size) -> Tensor");
+    // not in the reference: any rank, bias added in the kernel
+    m.def("linear_bias(Tensor activations, Tensor packed_weights, Tensor scales, Tensor? bias, int group_size) -> Tensor");
     m.def("dequantize(Tensor packed_weights, Tensor scales, int group_size) -> Tensor");
     // not in the reference: FP32 partial sums for layers sharded along K
     m.def("linear_partial(Tensor activations, Tensor packed_weights, Tensor scales, int group_size) -> Tensor");
@@ -200,6 +226,7 @@ TORCH_LIBRARY(w4a16, m) {
 
 TORCH_LIBRARY_IMPL(w4a16, CUDA, m) {
     m.impl("linear", &linear_cuda_impl);
+    m.impl("linear_bias", &linear_bias_cuda_impl);
     m.impl("dequantize", &dequantize_cuda_impl);
     m.impl("linear_partial", &linear_partial_cuda_impl);
     m.impl("quantize_pack", &quantize_pack_cuda_impl);

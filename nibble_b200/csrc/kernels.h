@@ -31,6 +31,7 @@ struct LinearProblem {
     const w4a16_input_transform* input = nullptr;   // x is derived from other buffers while it is staged
     const w4a16_peer_source* source = nullptr;  // x is another sharded layer's published result
     int64_t x_ld = 0;                           // elements between batch rows of x (0: K)
+    const __half* bias = nullptr;               // [N], added to the FP16 result (FP16 output only)
 };
 
 // Workspace layout for split-K: arrival counters first, FP32 partials after them.
@@ -41,8 +42,9 @@ size_t linear_workspace_bytes_for(int64_t M, int64_t N, int splits);
 w4a16_linear_config choose_linear_config(int64_t M, int64_t N, int64_t K, int max_splits);
 
 // Tensor-core path: requires group == 128 and 16-byte aligned x / packed.  Returns a W4A16_* code.
-// `out_f32` makes y an FP32 [M, N] matrix (unrounded sums, for partial results that are added up).
-int launch_linear_mma(const LinearProblem& p, const w4a16_linear_config& cfg, bool programmatic,
+// `out_f32` makes y an FP32 [M, N] matrix (unrounded sums, for partial results that are added up).  `early_weights`:
+// the caller vouches that no kernel still running writes the weights (W4A16_FLAG_PROGRAMMATIC_LAUNCH).
+int launch_linear_mma(const LinearProblem& p, const w4a16_linear_config& cfg, bool early_weights,
                       bool out_f32, cudaStream_t stream);
 
 // Bounds-check word of the streaming kernel; W4A16_ERR_BAD_CONFIG in builds without -DW4A16_BOUNDS_CHECK.

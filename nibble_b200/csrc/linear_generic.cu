@@ -15,10 +15,11 @@ namespace {
 constexpr int kGenericBatch = 8;
 constexpr int kGenericWarps = 4;
 
+template <bool BIAS>
 __global__ void __launch_bounds__(kGenericWarps * 32)
 linear_generic_kernel(const __half* __restrict__ x, const uint8_t* __restrict__ packed,
                       const __half* __restrict__ scales, void* __restrict__ y, int64_t M, int64_t N,
-                      int64_t K, int64_t group, int out_f32) {
+                      int64_t K, int64_t group, int out_f32, const __half* __restrict__ bias) {
     const int lane = threadIdx.x & 31;
     const int64_t row = static_cast<int64_t>(blockIdx.x) * kGenericWarps + (threadIdx.x >> 5);
     if (row >= N) return;
@@ -56,7 +57,9 @@ linear_generic_kernel(const __half* __restrict__ x, const uint8_t* __restrict__ 
             if (out_f32) {
                 static_cast<float*>(y)[(m0 + m) * N + row] = v;
             } else {
-                static_cast<__half*>(y)[(m0 + m) * N + row] = __float2half_rn(v);
+                __half out = __float2half_rn(v);
+                if (BIAS) out = __hadd(out, bias[row]);
+                static_cast<__half*>(y)[(m0 + m) * N + row] = out;
             }
         }
     }
@@ -69,8 +72,9 @@ int launch_linear_generic(const LinearProblem& p, bool out_f32, cudaStream_t str
     const int64_t batch_blocks = (p.M + kGenericBatch - 1) / kGenericBatch;
     if (row_blocks > INT32_MAX || batch_blocks > 65535) return W4A16_ERR_TOO_LARGE;
     const dim3 grid(static_cast<unsigned>(row_blocks), static_cast<unsigned>(batch_blocks), 1);
-    linear_generic_kernel<<<grid, kGenericWarps * 32, 0, stream>>>(p.x, p.packed, p.scales, p.y, p.M, p.N,
-                                                                   p.K, p.group, out_f32 ? 1 : 0);
+    const auto kernel = p.bias != nullptr ? linear_generic_kernel<true> : linear_generic_kernel<false>;
+    kernel<<<grid, kGenericWarps * 32, 0, stream>>>(p.x, p.packed, p.scales, p.y, p.M, p.N,
+                                                                   p.K, p.group, out_f32 ? 1 : 0, p.bias);
     if (cudaGetLastError() != cudaSuccess) return W4A16_ERR_LAUNCH;
     g_launch_count.fetch_add(1, std::memory_order_relaxed);
     return W4A16_OK;

@@ -54,6 +54,7 @@ struct KernelHooks {
     // The successor is released with the very first instruction: its CTAs only take SM resources this grid does not
     // use, and the earlier they are resident the more of their prologue and weight prefetch hides under this grid.
     __device__ __forceinline__ void at_start() { pdl_release_downstream(); }
+    __device__ __forceinline__ bool weights_wait(const MmaParams& p) const { return p.early_weights == 0; }
     __device__ __forceinline__ void before_activations() { pdl_wait_for_upstream(); }
     __device__ __forceinline__ void after_outputs() {}
 };
@@ -448,7 +449,7 @@ int read_bounds_check(unsigned* site, unsigned* count) {
 #endif
 }
 
-int launch_linear_mma(const LinearProblem& prob, const w4a16_linear_config& cfg_in, bool programmatic,
+int launch_linear_mma(const LinearProblem& prob, const w4a16_linear_config& cfg_in, bool early_weights,
                       bool out_f32, cudaStream_t stream) {
     if (prob.group != kGroup || prob.K % kGroup != 0) return W4A16_ERR_BAD_CONFIG;
     if (prob.M > INT32_MAX || prob.N > INT32_MAX || prob.K > INT32_MAX) return W4A16_ERR_TOO_LARGE;
@@ -520,6 +521,8 @@ int launch_linear_mma(const LinearProblem& prob, const w4a16_linear_config& cfg_
     params.norm_weight = nullptr;
     params.stream_out = nullptr;
     params.eps = 0.0f;
+    params.early_weights = early_weights ? 1 : 0;
+    params.bias = prob.bias;
     if (prob.input != nullptr && prob.input->kind != W4A16_INPUT_PLAIN) {
         const w4a16_input_transform& in = *prob.input;
         auto aligned = [](const void* q) { return reinterpret_cast<uintptr_t>(q) % 16 == 0; };
@@ -656,7 +659,10 @@ int launch_linear_mma(const LinearProblem& prob, const w4a16_linear_config& cfg_
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     launch.attrs = attr;
-    launch.numAttrs = programmatic ? 1 : 0;
+    // Always programmatic: with the weights waited for (early_weights false) the kernel still starts, and its first weights
+    // travel to L2, while the one before it drains; a kernel of another kind in front completes before this one starts.
+    // Not so the tensor-parallel launches, whose CTAs would hold SMs while they wait for other GPUs.
+    launch.numAttrs = early_weights || kernel == variant.fn ? 1 : 0;
     void* args[] = {const_cast<MmaParams*>(&params)};
     if (cudaLaunchKernelExC(&launch, kernel, args) != cudaSuccess) return W4A16_ERR_LAUNCH;
     g_launch_count.fetch_add(1, std::memory_order_relaxed);

@@ -1,0 +1,96 @@
+// QuantizedLinear.forward in one native call.
+//
+// The module's Python forward checks its arguments, flattens them, goes through torch.ops and reshapes: about 8 us of
+// interpreter and binding time around a 2 us kernel at M = 1.  linear_forward() makes the same checks and calls the same
+// operators through their dispatcher handles (so profilers, dispatch modes and fake tensors see them as before) in a
+// quarter of that.  It takes only the ordinary case -- a plain, contiguous FP16 CUDA tensor outside tracing, autocast and
+// function modes -- and returns NotImplemented for everything else, including every invalid call: the Python code then
+// decides, and raises what it always raised.
+#include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/autocast_mode.h>
+#include <ATen/core/dispatch/Dispatcher.h>
+#include <c10/core/InferenceMode.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
+
+#include <optional>
+
+namespace {
+
+using LinearBias = at::Tensor(const at::Tensor&, const at::Tensor&, const at::Tensor&, const std::optional<at::Tensor>&, int64_t);
+using Dequantize = at::Tensor(const at::Tensor&, const at::Tensor&, int64_t);
+
+template <typename Signature>
+c10::TypedOperatorHandle<Signature> operator_handle(const char* name) {
+    return c10::Dispatcher::singleton().findSchemaOrThrow(name, "").typed<Signature>();
+}
+
+// nibble_b200/linear.py: uses_fused_kernel, which states the reasons.
+bool uses_fused_kernel(int64_t rows, int64_t out_features, int64_t group_size) {
+    if (rows <= 64) return true;
+    if (group_size % 32 != 0) return true;
+    if (group_size != 128) return false;
+    return rows <= 1024 && (out_features + 127) / 128 >= 40;
+}
+
+// A tensor nobody has subclassed, wrapped or asked to track gradients of.
+bool plain(PyObject* object) {
+    if (!THPVariable_CheckExact(object)) return false;
+    const at::Tensor& t = THPVariable_Unpack(object);
+    return t.is_cuda() && !t.requires_grad() && t.is_contiguous() &&
+           !t.key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched,
+                                                     c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Batched}));
+}
+
+// linear_forward(activations, packed_weights, scales, bias or None, group_size, fused) -> Tensor or NotImplemented
+PyObject* linear_forward(PyObject*, PyObject* const* args, Py_ssize_t count) {
+    HANDLE_TH_ERRORS
+    if (count != 6 || !plain(args[0]) || !plain(args[1]) || !plain(args[2]) || (args[3] != Py_None && !plain(args[3])) ||
+        at::impl::torch_function_mode_enabled() || c10::impl::TorchDispatchModeTLS::any_modes_set() ||
+        torch::jit::tracer::isTracing() || at::autocast::is_autocast_enabled(at::kCUDA)) {
+        Py_RETURN_NOTIMPLEMENTED;
+    }
+    const at::Tensor& x = THPVariable_Unpack(args[0]);
+    const at::Tensor& packed = THPVariable_Unpack(args[1]);
+    const at::Tensor& scales = THPVariable_Unpack(args[2]);
+    std::optional<at::Tensor> bias;
+    if (args[3] != Py_None) bias = THPVariable_Unpack(args[3]);
+    const int64_t group_size = PyLong_AsLongLong(args[4]);
+    const int fused = PyObject_IsTrue(args[5]);
+    if (PyErr_Occurred() != nullptr) return nullptr;
+    if (x.dim() < 1 || x.scalar_type() != at::kHalf || packed.dim() != 2 || x.size(-1) != packed.size(1) * 2 || x.size(-1) == 0 ||
+        group_size <= 0 || x.device() != packed.device() || x.device() != scales.device()) {
+        Py_RETURN_NOTIMPLEMENTED;
+    }
+    const int64_t rows = x.numel() / x.size(-1);
+    at::Tensor out;
+    {
+        pybind11::gil_scoped_release unlocked;             // a launch may block when the stream's queue is full
+        const at::AutoDispatchBelowADInplaceOrView below;  // nothing here takes part in autograd
+        if ((fused != 0 || group_size % 32 != 0) && uses_fused_kernel(rows, packed.size(0), group_size)) {
+            static const auto op = operator_handle<LinearBias>("w4a16::linear_bias");
+            out = op.call(x, packed, scales, bias, group_size);
+        } else {
+            static const auto op = operator_handle<Dequantize>("w4a16::dequantize");
+            out = at::linear(x, op.call(packed, scales, group_size));
+            if (bias.has_value()) out.add_(*bias);
+        }
+    }
+    return THPVariable_Wrap(std::move(out));
+    END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef methods[] = {
+    {"linear_forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(linear_forward)), METH_FASTCALL,
+     "linear_forward(activations, packed_weights, scales, bias, group_size, fused) -> Tensor or NotImplemented"},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_C", "Native side of nibble_b200: torch operators and QuantizedLinear.forward.", -1,
+                          methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__C() { return PyModule_Create(&module_def); }

@@ -140,6 +140,7 @@ struct TcParams {
     int k_splits;         // CTAs that share one output tile, each taking a range of K (1: none)
     int split_k;          // K of one such range: a multiple of 256 (whole copies of codes)
     float* partial;       // [k_splits, M, N] FP32 sums of the ranges when k_splits > 1, else null
+    const __half* bias;   // [N] or null: added to the rounded result
 };
 
 // A position in a ring of `size` slots together with the parity of the mbarrier phase it is in.
@@ -168,7 +169,8 @@ __device__ __forceinline__ void tile_coords(int tile, const TcParams& p, int& m_
     m_tile = first + (local - n_tile * gm);
 }
 
-template <int SUB>
+// BIAS is a template parameter because the test for it inside the store loop cost the unbiased kernel 40 % at K = 1024.
+template <int SUB, bool BIAS>
 __global__ void __launch_bounds__(kThreadsTc, 1)
 linear_tcgen05_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_map,
                       const __grid_constant__ CUtensorMap w_map) {
@@ -245,6 +247,9 @@ linear_tcgen05_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_ma
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     unsigned tmem_base;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+    // Set-up is over: the next kernel may take the SMs this one leaves, and this one may touch global memory.
+    pdl_release_downstream();
+    pdl_wait_for_upstream();
 
     bool healthy = true;
     if (warp == 0) {
@@ -342,6 +347,7 @@ linear_tcgen05_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_ma
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const unsigned taddr = tmem_base + (static_cast<unsigned>(quarter * 32) << 16) + buf * kMaxBN;
             __half* out = p.y + static_cast<size_t>(m0) * p.N + n;
+            const __half bias = BIAS && n < p.N ? p.bias[n] : __half();
             // a K range leaves its unrounded sums; a small kernel adds the ranges in order and rounds once
             float* out_partial = p.partial == nullptr ? nullptr
                 : p.partial + (static_cast<size_t>(item.split) * p.M + m0) * static_cast<size_t>(p.N) + n;
@@ -366,7 +372,9 @@ linear_tcgen05_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_ma
                             if (out_partial != nullptr) {
                                 out_partial[static_cast<size_t>(col + j) * p.N] = __uint_as_float(v[j]);
                             } else {
-                                out[static_cast<size_t>(col + j) * p.N] = __float2half_rn(__uint_as_float(v[j]));
+                                __half value = __float2half_rn(__uint_as_float(v[j]));
+                                if (BIAS) value = __hadd(value, bias);
+                                out[static_cast<size_t>(col + j) * p.N] = value;
                             }
                         }
                     }
@@ -486,10 +494,23 @@ linear_tcgen05_kernel(const TcParams p, const __grid_constant__ CUtensorMap x_ma
     }
 }
 
-// y = half(sum of the K ranges' partial sums, in range order): four outputs per thread, 16-byte loads.
-__global__ void sum_ranges_kernel(const float* __restrict__ partial, __half* __restrict__ y, long long count, int ranges) {
-    const long long i = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
+// y = half(sum of the K ranges' partial sums, in range order) (+ bias): VECTOR (4 or 1) outputs per thread.
+template <int VECTOR>
+__global__ void sum_ranges_kernel(const float* __restrict__ partial, __half* __restrict__ y, long long count, int ranges,
+                                  const __half* __restrict__ bias, int N) {
+    const long long i = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * VECTOR;
+    pdl_wait_for_upstream();
     if (i >= count) return;
+    auto finish = [&](float v, int j) {
+        const __half h = __float2half_rn(v);
+        return bias == nullptr ? h : __hadd(h, bias[(i + j) % N]);
+    };
+    if constexpr (VECTOR == 1) {
+        float sum = __ldcg(partial + i);
+        for (int r = 1; r < ranges; ++r) sum += __ldcg(partial + static_cast<long long>(r) * count + i);
+        y[i] = finish(sum, 0);
+        return;
+    }
     float4 sum = __ldcg(reinterpret_cast<const float4*>(partial + i));
     for (int r = 1; r < ranges; ++r) {
         const float4 v = __ldcg(reinterpret_cast<const float4*>(partial + static_cast<long long>(r) * count + i));
@@ -498,8 +519,8 @@ __global__ void sum_ranges_kernel(const float* __restrict__ partial, __half* __r
         sum.z += v.z;
         sum.w += v.w;
     }
-    const __half2 lo = __floats2half2_rn(sum.x, sum.y);
-    const __half2 hi = __floats2half2_rn(sum.z, sum.w);
+    const __half2 lo = __halves2half2(finish(sum.x, 0), finish(sum.y, 1));
+    const __half2 hi = __halves2half2(finish(sum.z, 2), finish(sum.w, 3));
     uint2 out;
     out.x = *reinterpret_cast<const uint32_t*>(&lo);
     out.y = *reinterpret_cast<const uint32_t*>(&hi);
@@ -598,6 +619,7 @@ int launch_linear_tcgen05(const LinearProblem& prob, cudaStream_t stream) {
     params.split_k = static_cast<int>(split_k);
     params.partial = splits > 1 ? reinterpret_cast<float*>(static_cast<char*>(prob.workspace) + linear_counter_bytes(prob.M, prob.N))
                                 : nullptr;
+    params.bias = prob.bias;
     params.total_tiles *= splits;
     // as many operand stages as fit beside the code ring: 4 with a 256-row batch tile, 8 up to 80 rows
     const size_t fixed = static_cast<size_t>(kCodeSlots) * kPackedTileBytes + 1024 /* alignment slack */ + kBarrierBytes;
@@ -612,37 +634,55 @@ int launch_linear_tcgen05(const LinearProblem& prob, cudaStream_t stream) {
     params.dequant_groups = params.stages == 8 ? 4 : params.stages == 6 ? 3 : params.stages;
     if (fit < 2) return W4A16_ERR_TOO_LARGE;
     const size_t smem = params.stages * stage_bytes + fixed;
-    const void* kernel = sub_tiles == 2 ? reinterpret_cast<const void*>(linear_tcgen05_kernel<2>)
-                                        : reinterpret_cast<const void*>(linear_tcgen05_kernel<1>);
+    static const void* const kernels[2][2] = {
+        {reinterpret_cast<const void*>(linear_tcgen05_kernel<1, false>), reinterpret_cast<const void*>(linear_tcgen05_kernel<1, true>)},
+        {reinterpret_cast<const void*>(linear_tcgen05_kernel<2, false>), reinterpret_cast<const void*>(linear_tcgen05_kernel<2, true>)}};
+    const void* kernel = kernels[sub_tiles - 1][prob.bias != nullptr];
     // the shared-memory attribute and the SM count are kept per device
     static int sm_count[64] = {};
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return W4A16_ERR_LAUNCH;
     if (sm_count[device] == 0) {
         int sms = 0;
-        if (cudaFuncSetAttribute(linear_tcgen05_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kSmemLimitTc) != cudaSuccess ||
-            cudaFuncSetAttribute(linear_tcgen05_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kSmemLimitTc) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0) {
+        for (int k = 0; k < 4; ++k) {
+            if (cudaFuncSetAttribute(kernels[k >> 1][k & 1], cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimitTc) != cudaSuccess) {
+                return W4A16_ERR_LAUNCH;
+            }
+        }
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0) {
             return W4A16_ERR_LAUNCH;
         }
         sm_count[device] = sms;
     }
     const int grid = static_cast<int>(std::min<int64_t>(params.total_tiles, sm_count[device]));
+    cudaLaunchConfig_t launch = {};
+    launch.gridDim = dim3(static_cast<unsigned>(grid));
+    launch.blockDim = dim3(kThreadsTc);
+    launch.dynamicSmemBytes = smem;
+    launch.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    launch.attrs = attr;
+    launch.numAttrs = 1;      // sets up under the kernel in front (83 rows, 512 -> 28928, back to back: 14.0 -> 11.8 us)
     void* args[] = {&params, &x_map, &w_map};
-    if (cudaLaunchKernel(kernel, dim3(grid), dim3(kThreadsTc), args, smem, stream) != cudaSuccess) return W4A16_ERR_LAUNCH;
+    if (cudaLaunchKernelExC(&launch, kernel, args) != cudaSuccess) return W4A16_ERR_LAUNCH;
     g_launch_count.fetch_add(1, std::memory_order_relaxed);
     if (splits > 1) {
         // y = half(sum of the ranges, in order)
         const long long count = static_cast<long long>(prob.M) * prob.N;
-        if (count % 4 != 0 || reinterpret_cast<uintptr_t>(prob.y) % 8 != 0) {
-            return launch_sum_partials(params.partial, static_cast<__half*>(prob.y), count, splits, nullptr, false, stream);
-        }
-        const long long blocks = (count / 4 + 255) / 256;
+        const int vector = count % 4 == 0 && reinterpret_cast<uintptr_t>(prob.y) % 8 == 0 ? 4 : 1;
+        const long long blocks = (count / vector + 255) / 256;
         if (blocks > INT32_MAX) return W4A16_ERR_TOO_LARGE;
-        sum_ranges_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(params.partial, static_cast<__half*>(prob.y), count, splits);
-        if (cudaGetLastError() != cudaSuccess) return W4A16_ERR_LAUNCH;
+        launch.gridDim = dim3(static_cast<unsigned>(blocks));
+        launch.blockDim = dim3(256);
+        launch.dynamicSmemBytes = 0;
+        launch.numAttrs = 1;
+        if (cudaLaunchKernelEx(&launch, vector == 4 ? sum_ranges_kernel<4> : sum_ranges_kernel<1>,
+                               static_cast<const float*>(params.partial), static_cast<__half*>(prob.y), count, splits, prob.bias,
+                               static_cast<int>(prob.N)) != cudaSuccess) {
+            return W4A16_ERR_LAUNCH;
+        }
         g_launch_count.fetch_add(1, std::memory_order_relaxed);
     }
     return W4A16_OK;

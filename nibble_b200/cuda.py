@@ -23,6 +23,10 @@ def _register_fakes() -> None:
     def _linear_partial_fake(activations, packed_weights, scales, group_size):
         return activations.new_empty((activations.shape[0], packed_weights.shape[0]), dtype=torch.float32)
 
+    @torch.library.register_fake("w4a16::linear_bias")
+    def _linear_bias_fake(activations, packed_weights, scales, bias, group_size):
+        return activations.new_empty((*activations.shape[:-1], packed_weights.shape[0]))
+
     @torch.library.register_fake("w4a16::dequantize")
     def _dequantize_fake(packed_weights, scales, group_size):
         # [N, K/2] -> FP16 [N, K]
@@ -37,8 +41,13 @@ def _register_fakes() -> None:
                 weights.new_empty((rows, cols // group_size), dtype=torch.float16))
 
 
+def linear_forward(*arguments):
+    """Stands in for the native forward where the extension did not load: every call is left to the Python code."""
+    return NotImplemented
+
+
 try:
-    _native.load_torch_ops()
+    linear_forward = _native.load_torch_ops().linear_forward
     _register_fakes()
 except (ImportError, OSError, RuntimeError) as error:  # not built, stale, or built against another torch
     _EXTENSION_LOAD_ERROR: Exception | None = error

@@ -11,7 +11,7 @@ from __future__ import annotations
 import torch
 import torch.nn.functional as F
 
-from .cuda import dequantize_cuda, linear_cuda
+from .cuda import dequantize_cuda, linear_cuda, linear_forward
 from .quantization import quantize_and_pack_weights
 
 # Largest flattened batch M sent to the streaming (mma.sync) fused kernel.  The reference stops at 8
@@ -133,6 +133,14 @@ class QuantizedLinear(torch.nn.Module):
 
     # ------------------------------------------------------------------ forward
     def forward(self, activations: torch.Tensor) -> torch.Tensor:
+        # The ordinary call is one native function (csrc/linear_module.cpp); what it does not take -- and every invalid
+        # call -- it leaves to the code below, which computes the same.
+        if not torch.compiler.is_compiling():
+            buffers = self._buffers
+            out = linear_forward(activations, buffers["packed_weights"], buffers["scales"], buffers["bias"], self.group_size,
+                                 self.fused)
+            if out is not NotImplemented:
+                return out
         if activations.ndim < 1:
             raise ValueError("activations must have at least one dimension")
         if activations.shape[-1] != self.in_features:

@@ -179,3 +179,29 @@ def test_model_checkpoint_loads_straight_onto_the_device(tmp_path):
     q = target.q_proj
     check_against_oracle(q(x) - q.bias, x, q.packed_weights, q.scales)
     assert target(x).shape == (2, 1024) and not torch.isnan(target(x)).any()
+
+
+@pytest.mark.parametrize(("k", "n"), [(1024, 77), (8192, 1024), (4096, 5248)])
+@pytest.mark.parametrize("rows", [1, 7, 13, 48, 100, 300])
+def test_native_forward_equals_the_python_forward(rows, k, n):
+    """Same bits through the native call (bias added inside the kernel) and through the operators plus a separate
+    addition, for streaming, split and GEMM launches, with any leading dimensions."""
+    from nibble_b200 import linear as linear_module
+
+    g = torch.Generator().manual_seed(rows + n)
+    packed, scales = quantize_and_pack_weights((torch.randn((n, k), generator=g) * 0.02).cuda(), 128)
+    x = torch.randn((1, rows, k), generator=g).half().cuda()
+    for bias in (None, torch.randn((n,), generator=g).half().cuda()):
+        layer = QuantizedLinear(packed, scales, 128, bias=bias)
+        native = linear_module.linear_forward(x, packed, scales, bias, 128, True)
+        assert native is not NotImplemented and native.shape == (1, rows, n)
+        use_fused = linear_module.uses_fused_kernel(rows, n, 128)
+        run = linear_module._run_fused if use_fused else linear_module._run_dequant_matmul
+        want = run(x.view(rows, k), packed, scales, 128).view(1, rows, n)
+        assert torch.equal(native, want if bias is None else want + bias)
+        assert torch.equal(layer(x), native)
+    # what the native call does not take, the module still does
+    wide = torch.zeros((rows + 1, 2 * k), dtype=torch.float16, device="cuda")[:rows]
+    wide[:, :k] = x[0]
+    assert rows == 1 or linear_module.linear_forward(wide[:, :k], packed, scales, None, 128, True) is NotImplemented
+    torch.testing.assert_close(QuantizedLinear(packed, scales, 128)(wide[:, :k]), want[0])
