@@ -79,7 +79,8 @@ typedef struct w4a16_linear_config {
  * favours it) a tcgen05 GEMM whose producer warps dequantise into the operand tiles
  * (no FP16 weight matrix in memory; weights enter the product as half(code * scale), the arithmetic of
  * the reference's dequantise-then-matmul prefill route, w4a16/linear.py:132-152).
- * Otherwise a generic kernel that accepts any even group_size and any alignment.
+ * group_size 64 and 32 run the streaming kernel at every M when K is a multiple of 128 and x, packed and scales are
+ * 16-byte aligned.  Otherwise a generic kernel that accepts any even group_size and any alignment.
  * The GEMM shares the K of an output tile between up to four CTAs when a layer has too few 128-row tiles for the
  * SMs (FP32 partial sums in the workspace, added in order and rounded once by a second small kernel); without
  * enough workspace it runs unsplit.

@@ -28,6 +28,12 @@ bool fast_path_applies(const void* x, const void* packed, int64_t K, int64_t gro
     return group == w4a16::kGroupFast && K > 0 && aligned16(x) && aligned16(packed);
 }
 
+// Groups below 128 stream like 128-wide ones while K still comes in whole 128-wide chunks.
+bool small_group_streams(const void* x, const void* packed, const void* scales, int64_t K, int64_t group) {
+    return group != w4a16::kGroupFast && w4a16::is_stream_group(group) && K > 0 && K % w4a16::kGroupFast == 0 && aligned16(x) &&
+           aligned16(packed) && aligned16(scales);
+}
+
 }  // namespace
 
 namespace {
@@ -130,11 +136,12 @@ int w4a16_linear_f16_bias(const void* x, const void* packed, const void* scales,
                    ? W4A16_OK
                    : W4A16_ERR_LAUNCH;
     }
-    if ((flags & W4A16_FLAG_FORCE_GENERIC) || !fast_path_applies(x, packed, K, group_size)) {
+    const bool small_group = small_group_streams(x, packed, scales, K, group_size);
+    if ((flags & W4A16_FLAG_FORCE_GENERIC) || (!small_group && !fast_path_applies(x, packed, K, group_size))) {
         return w4a16::launch_linear_generic(p, out_f32, s);
     }
     // Prefill-sized batches, and medium ones on large layers: dense enough for the tcgen05 tensor cores.
-    if (routes_to_tcgen05(M, N, K, flags)) return w4a16::launch_linear_tcgen05(p, s);
+    if (!small_group && routes_to_tcgen05(M, N, K, flags)) return w4a16::launch_linear_tcgen05(p, s);
     // Split K across CTAs only as far as the caller's workspace allows.
     int max_splits = 1;
     if (workspace != nullptr && aligned16(workspace)) {
@@ -152,7 +159,7 @@ int w4a16_linear_f16_bias(const void* x, const void* packed, const void* scales,
     // Too much activation data for one CTA's shared memory and no workspace to split K further: the tcgen05 GEMM
     // has no such limit (nor has the generic kernel, for FP32 output or when the GEMM is switched off).
     if (launched == W4A16_ERR_WORKSPACE) {
-        if (!out_f32 && !(flags & W4A16_FLAG_NO_TCGEN05)) return w4a16::launch_linear_tcgen05(p, s);
+        if (!out_f32 && !small_group && !(flags & W4A16_FLAG_NO_TCGEN05)) return w4a16::launch_linear_tcgen05(p, s);
         return w4a16::launch_linear_generic(p, out_f32, s);
     }
     return launched;

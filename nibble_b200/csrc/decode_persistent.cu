@@ -323,7 +323,7 @@ decode_step_kernel(const StepParams s, const int head_dim) {
         if (kind == kOpLinear) {
             const MmaParams p = s.ops[i].linear;
             StepHooks hooks{sync};
-            linear_mma_body<1, 1, 1, kStepKW, 2, kStepStages, kFeatRowIndex>(p, smem, hooks);
+            linear_mma_body<1, 1, 1, kStepKW, 2, kStepStages, kGroup, kFeatRowIndex>(p, smem, hooks);
         } else if (kind == kOpAttention) {
             const AttentionOp p = s.ops[i].attention;
             if (static_cast<int>(blockIdx.x) < p.q_heads) {
@@ -421,7 +421,7 @@ MmaParams step_linear(const void* x, const void* packed, const void* scales, voi
 
 size_t step_smem_bytes(const w4a16_decode_model& m) {
     const int max_k = std::max(std::max(m.hidden, m.intermediate), m.q_heads * m.head_dim);
-    const size_t linear = kFlagBytes + sizeof(float) * 2 * kStepKW * 4 * 32 + static_cast<size_t>(kStepStages) * stage_bytes<1, 2>() +
+    const size_t linear = kFlagBytes + sizeof(float) * 2 * kStepKW * 4 * 32 + static_cast<size_t>(kStepStages) * stage_bytes<1, 2, kGroup>() +
                           static_cast<size_t>(max_k) * sizeof(__half);
     const int lanes_per_pos = m.head_dim / 8;
     const size_t attention = sizeof(float) * (((m.max_len + 3) & ~3) + 8 + m.head_dim + (kThreads / lanes_per_pos) * m.head_dim) +

@@ -112,7 +112,8 @@ at::Tensor linear_impl(const at::Tensor& activations, const at::Tensor& packed_w
 
     void* workspace = nullptr;
     size_t workspace_bytes = 0;
-    const size_t wanted = w4a16_linear_workspace_bytes_flags(m, n, k, flags);
+    // (the GEMM, which has its own wish for scratch, is built for 128-wide groups)
+    const size_t wanted = w4a16_linear_workspace_bytes_flags(m, n, k, group_size == 128 ? flags : flags | W4A16_FLAG_NO_TCGEN05);
     if (wanted > 0 && wanted <= static_cast<size_t>(kWorkspaceBytes)) {
         at::Tensor& ws = workspace_for(activations.device(), stream);
         workspace = ws.data_ptr();

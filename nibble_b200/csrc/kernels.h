@@ -34,6 +34,9 @@ struct LinearProblem {
     const __half* bias = nullptr;               // [N], added to the FP16 result (FP16 output only)
 };
 
+// Scale groups the streaming kernel is built for (K a multiple of 128 all the same).
+constexpr bool is_stream_group(int64_t group) { return group == 128 || group == 64 || group == 32; }
+
 // Workspace layout for split-K: arrival counters first, FP32 partials after them.
 size_t linear_counter_bytes(int64_t M, int64_t N);
 size_t linear_workspace_bytes_for(int64_t M, int64_t N, int splits);
@@ -41,7 +44,7 @@ size_t linear_workspace_bytes_for(int64_t M, int64_t N, int splits);
 // Picks a launch shape for the tensor-core kernel.  `max_splits` caps k_splits (1 = no workspace).
 w4a16_linear_config choose_linear_config(int64_t M, int64_t N, int64_t K, int max_splits);
 
-// Tensor-core path: requires group == 128 and 16-byte aligned x / packed.  Returns a W4A16_* code.
+// Tensor-core path: requires is_stream_group(group) and 16-byte aligned x / packed (and scales, for groups below 128).  Returns a W4A16_* code.
 // `out_f32` makes y an FP32 [M, N] matrix (unrounded sums, for partial results that are added up).  `early_weights`:
 // the caller vouches that no kernel still running writes the weights (W4A16_FLAG_PROGRAMMATIC_LAUNCH).
 int launch_linear_mma(const LinearProblem& p, const w4a16_linear_config& cfg, bool early_weights,

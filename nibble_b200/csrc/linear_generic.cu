@@ -1,6 +1,6 @@
 // Generic W4A16 linear: any even group size, any pointer alignment, any batch size.
-// Correctness path for the cases the tensor-core kernel declines (group_size != 128 or x / packed
-// not 16-byte aligned), like the reference's one-thread-per-output kernel
+// Correctness path for the cases the tensor-core kernels decline (group_size other than 128, 64 and 32, K not a multiple
+// of 128, pointers not 16-byte aligned), like the reference's one-thread-per-output kernel
 // (csrc/int4_linear_kernel.cu:20-69) -- but a warp walks one output row with byte-wide coalesced
 // loads and keeps up to eight batch rows in registers, so the packed row is read once per eight.
 #include <cuda_fp16.h>

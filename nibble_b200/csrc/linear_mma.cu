@@ -44,39 +44,11 @@
 
 #include "kernels.h"
 #include "linear_mma_body.cuh"
+#include "linear_mma_variants.cuh"
 #include "unpack.cuh"
 
 namespace w4a16 {
 namespace {
-
-// Hooks of the stand-alone kernel: programmatic dependent launch on the way in, nothing on the way out.
-struct KernelHooks {
-    // The successor is released with the very first instruction: its CTAs only take SM resources this grid does not
-    // use, and the earlier they are resident the more of their prologue and weight prefetch hides under this grid.
-    __device__ __forceinline__ void at_start() { pdl_release_downstream(); }
-    __device__ __forceinline__ bool weights_wait(const MmaParams& p) const { return p.early_weights == 0; }
-    __device__ __forceinline__ void before_activations() { pdl_wait_for_upstream(); }
-    __device__ __forceinline__ void after_outputs() {}
-};
-
-template <int NT, int XB, int TILES, int KW, int U, int STAGES>
-__global__ void __launch_bounds__(kThreads, min_ctas_per_sm<NT, TILES>())
-linear_mma_kernel(const MmaParams p) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    KernelHooks hooks;
-    linear_mma_body<NT, XB, TILES, KW, U, STAGES, 0>(p, smem, hooks);
-}
-
-// The same kernel with the tensor-parallel sender and reader paths compiled in (launches that carry a
-// w4a16_peer_target or a w4a16_peer_source).
-template <int NT, int XB, int TILES, int KW, int U, int STAGES>
-__global__ void __launch_bounds__(kThreads, min_ctas_per_sm<NT, TILES>())
-linear_mma_exchange_kernel(const MmaParams p) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    KernelHooks hooks;
-    linear_mma_body<NT, XB, TILES, KW, U, STAGES, kFeatExchange>(p, smem, hooks);
-}
-
 
 // What a kernel needs to be the reader of a sharded layer's publication.
 struct ReaderParams {
@@ -175,41 +147,20 @@ __global__ void sum_partials_kernel(const void* __restrict__ partials, __half* _
 }
 
 // ------------------------------------------------------------------------------------------------
-struct Variant {
-    const void* fn;
-    const void* fn_exchange;   // the build with the tensor-parallel paths; null where it is not instantiated
-    int red_bytes;     // shared memory for the cross-warp reduction
-    int stage_bytes;   // shared memory of one pipeline stage
-    int stages;
-    int x_rows;        // batch rows stored per chunk of x (XB)
-};
-
-template <int NT, int XB, int TILES, int KW, int U, int STAGES>
-Variant variant_of() {
-    constexpr int RW = kWarpsPerCta / KW;
-    constexpr int red = KW > 1 ? 2 * KW * TILES * NT * 4 * 32 * RW * static_cast<int>(sizeof(float)) : 0;
-    const void* exchange = nullptr;
-    if constexpr (TILES == 1) {   // sharded layers always run one 16-row tile per warp
-        exchange = reinterpret_cast<const void*>(&linear_mma_exchange_kernel<NT, XB, TILES, KW, U, STAGES>);
-    }
-    return {reinterpret_cast<const void*>(&linear_mma_kernel<NT, XB, TILES, KW, U, STAGES>), exchange, red,
-            stage_bytes<TILES, U>(), STAGES, XB};
-}
-
 template <int NT, int XB, int TILES, int KW>
 bool pick_pipeline(int unroll, int stages, Variant* v) {
     if (unroll == 1) {   // odd K/128: the slow-scale path, one tile per warp and one ring depth only
         if constexpr (TILES == 1) {
             if (stages != 3) return false;
-            *v = variant_of<NT, XB, 1, KW, 1, 3>();
+            *v = variant_of<NT, XB, 1, KW, 1, 3, kGroup>();
             return true;
         } else {
             return false;
         }
     }
     if (unroll != 2) return false;
-    if (stages == 3) { *v = variant_of<NT, XB, TILES, KW, 2, 3>(); return true; }
-    if (stages == 4) { *v = variant_of<NT, XB, TILES, KW, 2, 4>(); return true; }
+    if (stages == 3) { *v = variant_of<NT, XB, TILES, KW, 2, 3, kGroup>(); return true; }
+    if (stages == 4) { *v = variant_of<NT, XB, TILES, KW, 2, 4, kGroup>(); return true; }
     return false;
 }
 
@@ -238,7 +189,8 @@ bool pick_tiles(const w4a16_linear_config& c, Variant* v) {
     }
 }
 
-bool pick_variant(int nt, bool single_row, const w4a16_linear_config& c, Variant* v) {
+bool pick_variant(int64_t group, int nt, bool single_row, const w4a16_linear_config& c, Variant* v) {
+    if (group != kGroup) return pick_group_variant(static_cast<int>(group), nt, single_row, c, v);
     switch (nt) {
         case 1: return single_row ? pick_tiles<1, 1>(c, v) : pick_tiles<1, 8>(c, v);
         case 2: return pick_tiles<2, 16>(c, v);
@@ -451,7 +403,7 @@ int read_bounds_check(unsigned* site, unsigned* count) {
 
 int launch_linear_mma(const LinearProblem& prob, const w4a16_linear_config& cfg_in, bool early_weights,
                       bool out_f32, cudaStream_t stream) {
-    if (prob.group != kGroup || prob.K % kGroup != 0) return W4A16_ERR_BAD_CONFIG;
+    if (!is_stream_group(prob.group) || prob.K % kGroup != 0) return W4A16_ERR_BAD_CONFIG;
     if (prob.M > INT32_MAX || prob.N > INT32_MAX || prob.K > INT32_MAX) return W4A16_ERR_TOO_LARGE;
     w4a16_linear_config cfg = cfg_in;
     const int nt = batch_tiles_for(prob.M);
@@ -465,6 +417,12 @@ int launch_linear_mma(const LinearProblem& prob, const w4a16_linear_config& cfg_
         return W4A16_ERR_BAD_CONFIG;
     }
     if (cfg.unroll != 1 && cfg.unroll != 2) return W4A16_ERR_BAD_CONFIG;
+    if (prob.group != kGroup) {
+        // several scales of a row travel together: 16-byte copies at most
+        if (reinterpret_cast<uintptr_t>(prob.scales) % 16 != 0) return W4A16_ERR_BAD_CONFIG;
+        cfg.row_tiles = 1;
+        cfg.k_warps = cfg.k_warps <= 2 ? 2 : 8;
+    }
     if (cfg.stages != 0 && cfg.stages != 3 && cfg.stages != 4) return W4A16_ERR_BAD_CONFIG;
 
     const int per_split = (chunks + splits - 1) / splits;
@@ -479,7 +437,7 @@ int launch_linear_mma(const LinearProblem& prob, const w4a16_linear_config& cfg_
     if (cfg.stages == 0) {
         cfg.stages = cfg.unroll == 1 ? 3 : 4;
         if (cfg.unroll == 2) {
-            if (!pick_variant(nt, prob.M == 1, cfg, &variant)) return W4A16_ERR_BAD_CONFIG;
+            if (!pick_variant(prob.group, nt, prob.M == 1, cfg, &variant)) return W4A16_ERR_BAD_CONFIG;
             const size_t fixed = kFlagBytes + variant.red_bytes + x_slice_bytes(x_rows, chunks_per_split);
             const size_t half_sm = static_cast<size_t>(kSmemPerSm / 2 - 1024);
             const bool two_with_four = fixed + 4u * variant.stage_bytes <= half_sm;
@@ -488,7 +446,7 @@ int launch_linear_mma(const LinearProblem& prob, const w4a16_linear_config& cfg_
             if (!two_with_four && (two_with_three || !four_fit)) cfg.stages = 3;
         }
     }
-    if (!pick_variant(nt, prob.M == 1, cfg, &variant)) return W4A16_ERR_BAD_CONFIG;
+    if (!pick_variant(prob.group, nt, prob.M == 1, cfg, &variant)) return W4A16_ERR_BAD_CONFIG;
 
     MmaParams params;
     params.x = prob.x;

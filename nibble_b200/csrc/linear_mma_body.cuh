@@ -217,6 +217,17 @@ __device__ __forceinline__ uint4 lds16(unsigned addr) {
     return v;
 }
 
+// Four 8x8 matrices of 16-bit elements: lane L points at row L % 8 of matrix L / 8, and lane (g, t) receives the t-th word of
+// row g of each.
+template <int OFFSET>
+__device__ __forceinline__ uint4 ldmatrix4(unsigned addr) {
+    uint4 v;
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4+%5];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(addr), "n"(OFFSET));
+    return v;
+}
+
 template <int OFFSET>
 __device__ __forceinline__ uint32_t lds4(unsigned addr) {
     uint32_t v;
@@ -231,10 +242,10 @@ __device__ __forceinline__ void cp_async16(unsigned dst, const void* src) {
                  "n"(SRC_OFFSET)
                  : "memory");
 }
-template <int DST_OFFSET, int SRC_OFFSET>
-__device__ __forceinline__ void cp_async4(unsigned dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0+%1], [%2+%3], 4;" ::"r"(dst), "n"(DST_OFFSET), "l"(src),
-                 "n"(SRC_OFFSET)
+template <int BYTES, int DST_OFFSET, int SRC_OFFSET>
+__device__ __forceinline__ void cp_async_small(unsigned dst, const void* src) {   // 4, 8 or 16 bytes
+    asm volatile("cp.async.ca.shared.global [%0+%1], [%2+%3], %4;" ::"r"(dst), "n"(DST_OFFSET), "l"(src),
+                 "n"(SRC_OFFSET), "n"(BYTES)
                  : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
@@ -246,10 +257,11 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // Bytes one pipeline stage occupies per CTA: per thread U chunks x 2*TILES rows x 16 bytes of
-// packed weights, plus (U == 2) per warp one 4-byte scale pair for each of its 16*TILES rows.
-template <int TILES, int U>
+// packed weights, plus (U == 2) per warp the two chunks' scales (one 4-byte pair with 128-wide groups) for each of its
+// 16*TILES rows.
+template <int TILES, int U, int GROUP>
 __host__ __device__ constexpr int stage_bytes() {
-    return kThreads * (2 * TILES * U * 16) + (U == 2 ? kWarpsPerCta * 16 * TILES * 4 : 0);
+    return kThreads * (2 * TILES * U * 16) + (U == 2 ? kWarpsPerCta * 16 * TILES * 4 * (kGroup / GROUP) : 0);
 }
 
 // Resident CTAs per SM the register allocation aims for.
@@ -304,6 +316,11 @@ __device__ __noinline__ void stage_tagged(const uint4* base, size_t row_units, i
 // XB     batch rows stored per chunk in the shared copy of x: 1 (M == 1) or 8*NT (padded)
 // TILES  16-row tiles per warp           KW  warps splitting K of one row tile
 // U      chunks per pipeline step        STAGES  ring depth
+// GROUP  K elements per scale: 128, 64 or 32.  An MMA may only add up products of one scale group.  With 128-wide groups
+//        lane t of a quad unpacks bytes 16t..16t+15 of a chunk (k = 32t..32t+31), so every MMA spans the chunk; with
+//        smaller ones the quad has to work on one 32-wide run of k at a time: lane t unpacks word t of 16-byte piece i.
+//        ldmatrix does that distribution (the pieces are stored with a XOR swizzle so that it is free of bank conflicts),
+//        x is stored for the same order, and the accumulator is scaled once per group.
 // `smem` is the CTA's dynamic shared memory (128-byte aligned).  `hooks.before_activations()` runs once the
 // whole weight ring has been requested and must return only when x may be read and y written;
 // `hooks.after_outputs()` runs when this CTA has written its last output.  The function may be called
@@ -315,13 +332,17 @@ __device__ __noinline__ void stage_tagged(const uint4* base, size_t row_units, i
 constexpr int kFeatExchange = 1;
 constexpr int kFeatRowIndex = 2;
 
-template <int NT, int XB, int TILES, int KW, int U, int STAGES, int FEATURES, typename Hooks>
+template <int NT, int XB, int TILES, int KW, int U, int STAGES, int GROUP, int FEATURES, typename Hooks>
 __device__ __forceinline__ void linear_mma_body(const MmaParams& p, unsigned char* smem, Hooks& hooks) {
     constexpr int RW = kWarpsPerCta / KW;
     constexpr int kRowsPerTile = 16 * TILES;
     constexpr int kAccPerLane = TILES * NT * 4;
     constexpr int kRedFloats = KW > 1 ? 2 * KW * kAccPerLane * 32 : 0;   // per group, double buffered
-    constexpr int kStageBytes = stage_bytes<TILES, U>();
+    constexpr int kStageBytes = stage_bytes<TILES, U, GROUP>();
+    constexpr int kScalesPerChunk = kGroup / GROUP;
+    constexpr int kStepScaleBytes = 4 * kScalesPerChunk;                 // of one row, U == 2
+    constexpr int kWordsPerScale = 4 / kScalesPerChunk;                  // words of a lane's 16 bytes that share a scale
+    static_assert(GROUP == 128 || GROUP == 64 || GROUP == 32);
     constexpr int kItemBytes = kThreads * 16;                            // one 16-byte item of every thread
     constexpr int kScaleOffset = 2 * TILES * U * kItemBytes;             // scales follow the weights
     constexpr int kPeriod = (STAGES % 2 == 0) ? STAGES : 2 * STAGES;     // steps per unrolled loop body
@@ -372,11 +393,16 @@ __device__ __forceinline__ void linear_mma_body(const MmaParams& p, unsigned cha
     // one __syncwarp after the wait publishes them, and orders the refill after everyone's reads.
     // U == 1: a step is 64 bytes per row and every lane copies exactly what it consumes itself.
     constexpr int kCopies = U == 2 ? 4 * TILES : 2 * TILES;   // 16-byte copies per lane per step
-    const unsigned ring_w = ring + tid * 16;                  // consumer view: this lane's entry of item 0
-    const unsigned ring_s = ring + kScaleOffset + warp * (16 * TILES * 4);   // this warp's scale pairs
+    // Groups below 128: piece p of row r (of 8) is stored as entry 4r + (p ^ (r / 2)), see GROUP above.
+    const unsigned ring_w = GROUP == 128
+        ? ring + tid * 16                                     // consumer view: this lane's entry of item 0
+        : ring + (warp * 32 + (lane & 7) * 4 + ((lane >> 3) ^ ((lane & 7) >> 1))) * 16;   // ... the row it names to ldmatrix
+    const unsigned ring_s = ring + kScaleOffset + warp * (16 * TILES * kStepScaleBytes);   // this warp's scales
+    const unsigned copy_piece = GROUP == 128 ? (lane & 3) : U == 2 ? (lane & 3) ^ (lane >> 4) : (lane & 3) ^ (lane >> 3);
     const unsigned copy_dst = U == 2
-        ? ring + ((lane >> 2) & 1) * kItemBytes + (warp * 32 + (lane >> 3) * 4 + (lane & 3)) * 16
-        : ring_w;
+        ? ring + ((lane >> 2) & 1) * kItemBytes + (warp * 32 + (lane >> 3) * 4 + copy_piece) * 16
+        : ring + (warp * 32 + (lane & 28) + copy_piece) * 16;
+    const unsigned copy_dst_odd = GROUP == 128 ? copy_dst : copy_dst ^ 32u;   // U == 2: rows 4..7 of a row half
     // Source pointers are kept "as of position 0 of the unrolled period": the copy issued at
     // position POS reads p_src + POS * (bytes per step), an immediate, so the pointers move once per
     // period instead of once per step.
@@ -399,7 +425,7 @@ __device__ __forceinline__ void linear_mma_body(const MmaParams& p, unsigned cha
         }
         if constexpr (U == 2) {
             const int r = min(row0 + (lane & (16 * TILES - 1)), p.N - 1);
-            p_scl = p.scales + static_cast<size_t>(r) * p.chunks + w_begin - pos * U;
+            p_scl = p.scales + (static_cast<size_t>(r) * p.chunks + w_begin - pos * U) * kScalesPerChunk;
         }
         p_left = steps_per_tile;
     };
@@ -420,7 +446,7 @@ __device__ __forceinline__ void linear_mma_body(const MmaParams& p, unsigned cha
                                      copy_dst + OFFSET + 16 <= ring + STAGES * kStageBytes, 4)) {
                 return;
             }
-            cp_async16<OFFSET, POS * kStepBytes>(copy_dst, p_src[j]);
+            cp_async16<OFFSET, POS * kStepBytes>(U == 2 && (j & 1) ? copy_dst_odd : copy_dst, p_src[j]);
         }
     };
     // Requests the next step of this warp's stream into the ring slot of period position POS and
@@ -440,9 +466,10 @@ __device__ __forceinline__ void linear_mma_body(const MmaParams& p, unsigned cha
             copy_at(pos_tag, std::integral_constant<int, 6>{});
             copy_at(pos_tag, std::integral_constant<int, 7>{});
             if constexpr (U == 2) {
-                if (scale_lane && W4A16_IN_BOUNDS(p_scl + POS * U >= p.scales &&
-                                                      p_scl + POS * U + 2 <= p.scales + static_cast<size_t>(p.N) * p.chunks, 5)) {
-                    cp_async4<SLOT * kStageBytes, POS * U * 2>(ring_s + lane * 4, p_scl);
+                if (scale_lane && W4A16_IN_BOUNDS(p_scl + POS * U * kScalesPerChunk >= p.scales &&
+                                                      p_scl + (POS + 1) * U * kScalesPerChunk <=
+                                                          p.scales + static_cast<size_t>(p.N) * p.chunks * kScalesPerChunk, 5)) {
+                    cp_async_small<kStepScaleBytes, SLOT * kStageBytes, POS * kStepScaleBytes>(ring_s + lane * kStepScaleBytes, p_scl);
                 }
             }
             if (--p_left == 0) {
@@ -451,7 +478,7 @@ __device__ __forceinline__ void linear_mma_body(const MmaParams& p, unsigned cha
             } else if constexpr (NEXT_POS == 0) {
 #pragma unroll
                 for (int j = 0; j < kCopies; ++j) p_src[j] += kPeriod * kStepBytes;
-                if constexpr (U == 2) p_scl += kPeriod * U;
+                if constexpr (U == 2) p_scl += kPeriod * U * kScalesPerChunk;
             }
         }
         cp_async_commit();
@@ -470,7 +497,8 @@ __device__ __forceinline__ void linear_mma_body(const MmaParams& p, unsigned cha
             const unsigned bytes = static_cast<unsigned>(min(steps_per_tile, STAGES)) * kStepBytes;
             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
                          ::"l"(p.packed + static_cast<size_t>(r) * row_bytes + static_cast<size_t>(w_begin) * kChunkBytes), "r"(bytes));
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.scales + static_cast<size_t>(r) * p.chunks + w_begin));
+            asm volatile("prefetch.global.L2 [%0];"
+                         ::"l"(p.scales + (static_cast<size_t>(r) * p.chunks + w_begin) * kScalesPerChunk));
         }
         hooks.before_activations();
     }
@@ -502,14 +530,15 @@ __device__ __forceinline__ void linear_mma_body(const MmaParams& p, unsigned cha
 
     // ---- stage this CTA's slice of x in shared memory, in B-fragment order --------------------
     // 16-byte unit ((c * 4 + i) * XB + n) * 4 + t holds, for batch row n, the eight activations
-    // k = c*128 + t*32 + i*8 .. +8 re-paired as (x0,x4)(x1,x5)(x2,x6)(x3,x7).
+    // k = c*128 + t*32 + i*8 .. +8 (groups below 128: c*128 + i*32 + t*8 .. +8) re-paired as (x0,x4)(x1,x5)(x2,x6)(x3,x7).
     // With p.x_mode set, the activations are computed here from what produced them: silu(gate) * up of
     // a fused gate/up output, or the RMSNorm of the residual stream plus the last block's output (one
     // CTA also writes the summed stream back).
     {
         const int units_per_row = span * 16;   // 16-byte pieces of one batch row in this K slice
         auto put = [&](const uint4& q, int j, int n) {
-            const int c = j >> 4, tt = (j >> 2) & 3, i = j & 3;
+            const int c = j >> 4, high = (j >> 2) & 3, low = j & 3;
+            const int tt = GROUP == 128 ? high : low, i = GROUP == 128 ? low : high;
             const unsigned dst = xs + (((c * 4 + i) * XB + n) * 4 + tt) * 16;
             if (!W4A16_IN_BOUNDS(n >= 0 && n < XB && j >= 0 && dst + 16 <= xs + static_cast<unsigned>(span) * (XB * 256), 1)) return;
             asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(prmt(q.x, q.z, 0x5410u)),
@@ -645,7 +674,7 @@ __device__ __forceinline__ void linear_mma_body(const MmaParams& p, unsigned cha
     // Registers of one step: U chunks of packed words for 2*TILES rows, and their scale pairs.
     struct StepRegs {
         uint4 w[U][TILES][2];
-        uint32_t s[TILES][2];
+        uint32_t s[TILES][2][kScalesPerChunk];   // U == 2: two chunks' scales; U == 1: one chunk's, half of the words
     };
     StepRegs buf[2];
 
@@ -656,10 +685,25 @@ __device__ __forceinline__ void linear_mma_body(const MmaParams& p, unsigned cha
     auto load_step = [&](StepRegs& regs, auto slot_tag) {
         constexpr int SLOT = decltype(slot_tag)::value;
         auto item = [&](auto index_tag) -> uint4 {
-            return lds16<SLOT * kStageBytes + decltype(index_tag)::value * kItemBytes>(ring_w);
+            constexpr int OFFSET = SLOT * kStageBytes + decltype(index_tag)::value * kItemBytes;
+            if constexpr (GROUP == 128) {
+                return lds16<OFFSET>(ring_w);
+            } else {
+                return ldmatrix4<OFFSET>(ring_w);
+            }
         };
-        auto scale = [&](auto index_tag) -> uint32_t {
-            return lds4<SLOT * kStageBytes + decltype(index_tag)::value * 32>(ring_s + g * 4);
+        auto scale = [&](uint32_t* out, auto index_tag) {
+            constexpr int OFFSET = SLOT * kStageBytes + decltype(index_tag)::value * 8 * kStepScaleBytes;
+            if constexpr (GROUP == 32) {
+                const uint4 four = lds16<OFFSET>(ring_s + g * kStepScaleBytes);
+                out[0] = four.x;
+                out[1] = four.y;
+                out[2] = four.z;
+                out[3] = four.w;
+            } else {
+                out[0] = lds4<OFFSET>(ring_s + g * kStepScaleBytes);
+                if constexpr (GROUP == 64) out[1] = lds4<OFFSET + 4>(ring_s + g * kStepScaleBytes);
+            }
         };
         if constexpr (U == 2) {
             // item (tile, half, chunk) = ((tile*2 + half) * 2 + chunk); scale pair of row tile*16 + half*8 + g
@@ -667,15 +711,15 @@ __device__ __forceinline__ void linear_mma_body(const MmaParams& p, unsigned cha
             regs.w[1][0][0] = item(std::integral_constant<int, 1>{});
             regs.w[0][0][1] = item(std::integral_constant<int, 2>{});
             regs.w[1][0][1] = item(std::integral_constant<int, 3>{});
-            regs.s[0][0] = scale(std::integral_constant<int, 0>{});
-            regs.s[0][1] = scale(std::integral_constant<int, 1>{});
+            scale(regs.s[0][0], std::integral_constant<int, 0>{});
+            scale(regs.s[0][1], std::integral_constant<int, 1>{});
             if constexpr (TILES == 2) {
                 regs.w[0][1][0] = item(std::integral_constant<int, 4>{});
                 regs.w[1][1][0] = item(std::integral_constant<int, 5>{});
                 regs.w[0][1][1] = item(std::integral_constant<int, 6>{});
                 regs.w[1][1][1] = item(std::integral_constant<int, 7>{});
-                regs.s[1][0] = scale(std::integral_constant<int, 2>{});
-                regs.s[1][1] = scale(std::integral_constant<int, 3>{});
+                scale(regs.s[1][0], std::integral_constant<int, 2>{});
+                scale(regs.s[1][1], std::integral_constant<int, 3>{});
             }
         } else {
             regs.w[0][0][0] = item(std::integral_constant<int, 0>{});
@@ -683,7 +727,15 @@ __device__ __forceinline__ void linear_mma_body(const MmaParams& p, unsigned cha
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int r = min(scale_row0 + h * 8 + g, p.N - 1);
-                regs.s[0][h] = ldg_nc_u16(p.scales + static_cast<size_t>(r) * p.chunks + w_begin + scale_step);
+                const __half* src = p.scales + (static_cast<size_t>(r) * p.chunks + w_begin + scale_step) * kScalesPerChunk;
+                if constexpr (GROUP == 128) {
+                    regs.s[0][h][0] = ldg_nc_u16(src);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < kScalesPerChunk / 2; ++q) {
+                        regs.s[0][h][q] = __ldg(reinterpret_cast<const unsigned*>(src) + q);
+                    }
+                }
             }
             if (++scale_step == steps_per_tile) {
                 scale_step = 0;
@@ -732,7 +784,7 @@ __device__ __forceinline__ void linear_mma_body(const MmaParams& p, unsigned cha
                 unpack8(word_hi, a_hi);
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt) {
-                    if constexpr (i == 0) {   // the chunk's first product starts from the zero registers
+                    if constexpr (i % kWordsPerScale == 0) {   // a scale group's first product starts from the zero registers
                         mma_m16n8k16_from(acc[tl][nt], zero, a_lo[0], a_hi[0], a_lo[1], a_hi[1], b[nt].x, b[nt].y);
                     } else {
                         mma_m16n8k16(acc[tl][nt], a_lo[0], a_hi[0], a_lo[1], a_hi[1], b[nt].x, b[nt].y);
@@ -741,24 +793,33 @@ __device__ __forceinline__ void linear_mma_body(const MmaParams& p, unsigned cha
                 }
             }
         };
-        word_step(std::integral_constant<int, 0>{});
-        word_step(std::integral_constant<int, 1>{});
-        word_step(std::integral_constant<int, 2>{});
-        word_step(std::integral_constant<int, 3>{});
+        // adds what one scale group has accumulated, times its scale
+        auto apply_scale = [&](auto sub_tag) {
+            constexpr int index = u * kScalesPerChunk + decltype(sub_tag)::value;   // of the step's scales of a row
 #pragma unroll
-        for (int tl = 0; tl < TILES; ++tl) {
-            const __half2 pair_lo = *reinterpret_cast<const __half2*>(&regs.s[tl][0]);
-            const __half2 pair_hi = *reinterpret_cast<const __half2*>(&regs.s[tl][1]);
-            const float s_lo = u == 0 ? __low2float(pair_lo) : __high2float(pair_lo);
-            const float s_hi = u == 0 ? __low2float(pair_hi) : __high2float(pair_hi);
+            for (int tl = 0; tl < TILES; ++tl) {
+                const __half2 pair_lo = *reinterpret_cast<const __half2*>(&regs.s[tl][0][index >> 1]);
+                const __half2 pair_hi = *reinterpret_cast<const __half2*>(&regs.s[tl][1][index >> 1]);
+                const float s_lo = index % 2 == 0 ? __low2float(pair_lo) : __high2float(pair_lo);
+                const float s_hi = index % 2 == 0 ? __low2float(pair_hi) : __high2float(pair_hi);
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-                total[tl][nt][0] = fmaf(acc[tl][nt][0], s_lo, total[tl][nt][0]);
-                total[tl][nt][1] = fmaf(acc[tl][nt][1], s_lo, total[tl][nt][1]);
-                total[tl][nt][2] = fmaf(acc[tl][nt][2], s_hi, total[tl][nt][2]);
-                total[tl][nt][3] = fmaf(acc[tl][nt][3], s_hi, total[tl][nt][3]);
+                for (int nt = 0; nt < NT; ++nt) {
+                    total[tl][nt][0] = fmaf(acc[tl][nt][0], s_lo, total[tl][nt][0]);
+                    total[tl][nt][1] = fmaf(acc[tl][nt][1], s_lo, total[tl][nt][1]);
+                    total[tl][nt][2] = fmaf(acc[tl][nt][2], s_hi, total[tl][nt][2]);
+                    total[tl][nt][3] = fmaf(acc[tl][nt][3], s_hi, total[tl][nt][3]);
+                }
             }
-        }
+        };
+        word_step(std::integral_constant<int, 0>{});
+        if constexpr (GROUP == 32) apply_scale(std::integral_constant<int, 0>{});
+        word_step(std::integral_constant<int, 1>{});
+        if constexpr (GROUP == 32) apply_scale(std::integral_constant<int, 1>{});
+        if constexpr (GROUP == 64) apply_scale(std::integral_constant<int, 0>{});
+        word_step(std::integral_constant<int, 2>{});
+        if constexpr (GROUP == 32) apply_scale(std::integral_constant<int, 2>{});
+        word_step(std::integral_constant<int, 3>{});
+        apply_scale(std::integral_constant<int, kScalesPerChunk - 1>{});
     };
     auto compute_step = [&](const StepRegs& regs) {
         compute_chunk(regs, std::integral_constant<int, 0>{});

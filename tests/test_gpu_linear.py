@@ -282,3 +282,20 @@ def test_graph_capture_and_replay():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, eager * 0.5)
+
+
+# ---------------------------------------------------------------- scale groups below 128
+@pytest.mark.parametrize("gs", [64, 32])
+@pytest.mark.parametrize(("k", "n"), [(128, 16), (384, 77), (1024, 130), (2688, 41), (8192, 96), (28672, 24)])
+def test_small_scale_groups_stream(k, n, gs):
+    """Odd and even chunk counts, ragged rows, every batch tile, with and without K split across CTAs."""
+    rng = np.random.default_rng(k + gs)
+    packed = torch.from_numpy(rng.integers(0, 256, size=(n, k // 2), dtype=np.uint8)).cuda()
+    scales = torch.from_numpy((rng.random((n, k // gs)) * 0.02 + 1e-3).astype(np.float16)).cuda()
+    for m in (1, 2, 8, 9, 16, 17, 33, 65):
+        x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float16)).cuda()
+        check_against_oracle(capi_linear(x, packed, scales, gs), x, packed, scales, gs)
+        check_against_oracle(linear_cuda(x, packed, scales, gs), x, packed, scales, gs)
+    # scales that are not 16-byte aligned take the generic kernel
+    shifted = torch.empty((scales.numel() + 1,), dtype=torch.float16, device="cuda")[1:].view_as(scales).copy_(scales)
+    check_against_oracle(linear_cuda(x[:3], packed, shifted, gs), x[:3], packed, shifted, gs)
