@@ -72,6 +72,10 @@ bool routes_to_tcgen05(int64_t M, int64_t N, int64_t K, uint32_t flags) {
     return gemm_us < (M <= 16 ? 0.85 : 1.0) * streaming_us;
 }
 
+int launch_gemm(const w4a16::LinearProblem& p, cudaStream_t stream) {
+    return p.M <= w4a16::kGemmMaxRows ? w4a16::launch_linear_gemm(p, stream) : w4a16::launch_linear_tcgen05(p, stream);
+}
+
 }  // namespace
 
 bool w4a16::linear_routes_to_tcgen05(int64_t M, int64_t N, int64_t K, uint32_t flags) {
@@ -103,7 +107,9 @@ size_t w4a16_linear_workspace_bytes_flags(int64_t M, int64_t N, int64_t K, uint3
     if (M <= 0 || N <= 0 || K <= 0 || K % w4a16::kGroupFast != 0) return 0;
     // The generic kernel uses no scratch; the tcgen05 GEMM wants some only for layers with few tiles.
     if (flags & W4A16_FLAG_FORCE_GENERIC) return 0;
-    if (routes_to_tcgen05(M, N, K, flags)) return w4a16::tcgen05_workspace_bytes(M, N, K);
+    if (routes_to_tcgen05(M, N, K, flags)) {
+        return M <= w4a16::kGemmMaxRows ? w4a16::gemm_workspace_bytes(M, N, K) : w4a16::tcgen05_workspace_bytes(M, N, K);
+    }
     const w4a16_linear_config c = w4a16::choose_linear_config(M, N, K, w4a16::kMaxKSplits);
     return w4a16::linear_workspace_bytes_for(M, N, c.k_splits);
 }
@@ -141,7 +147,7 @@ int w4a16_linear_f16_bias(const void* x, const void* packed, const void* scales,
         return w4a16::launch_linear_generic(p, out_f32, s);
     }
     // Prefill-sized batches, and medium ones on large layers: dense enough for the tcgen05 tensor cores.
-    if (!small_group && routes_to_tcgen05(M, N, K, flags)) return w4a16::launch_linear_tcgen05(p, s);
+    if (!small_group && routes_to_tcgen05(M, N, K, flags)) return launch_gemm(p, s);
     // Split K across CTAs only as far as the caller's workspace allows.
     int max_splits = 1;
     if (workspace != nullptr && aligned16(workspace)) {
@@ -159,7 +165,7 @@ int w4a16_linear_f16_bias(const void* x, const void* packed, const void* scales,
     // Too much activation data for one CTA's shared memory and no workspace to split K further: the tcgen05 GEMM
     // has no such limit (nor has the generic kernel, for FP32 output or when the GEMM is switched off).
     if (launched == W4A16_ERR_WORKSPACE) {
-        if (!out_f32 && !small_group && !(flags & W4A16_FLAG_NO_TCGEN05)) return w4a16::launch_linear_tcgen05(p, s);
+        if (!out_f32 && !small_group && !(flags & W4A16_FLAG_NO_TCGEN05)) return launch_gemm(p, s);
         return w4a16::launch_linear_generic(p, out_f32, s);
     }
     return launched;

@@ -55,7 +55,11 @@ int read_bounds_check(unsigned* site, unsigned* count);
 
 // Prefill-sized batches: dequantisation fused into a tcgen05 GEMM (group == 128, aligned x / packed).
 int launch_linear_tcgen05(const LinearProblem& p, cudaStream_t stream);
-// Status word of that kernel (non-zero: a bounded barrier wait gave up); reading clears it and synchronises.
+// The same for batches of up to kGemmMaxRows rows with the weights in tensor memory (linear_gemm.cu); groups of 64 and 32 too.
+int launch_linear_gemm(const LinearProblem& p, cudaStream_t stream);
+size_t gemm_workspace_bytes(int64_t M, int64_t N, int64_t K);
+constexpr int kGemmMaxRows = 128;
+// Status word of these kernels (non-zero: a bounded barrier wait gave up); reading clears it and synchronises.
 int read_tcgen05_status(unsigned* value);
 constexpr int kTcgen05MinRows = 65;     // from here on every fast-path call with FP16 output takes the GEMM
 // Scratch the GEMM wants (FP32 partial sums of K ranges, for layers with few tiles); it runs unsplit without.

@@ -43,6 +43,7 @@
 #include <algorithm>
 
 #include "kernels.h"
+#include "tcgen05.cuh"
 #include "unpack.cuh"
 
 namespace w4a16 {
@@ -69,63 +70,11 @@ constexpr int kBarrierBytes = 512;
 constexpr int kSmemLimitTc = 227 * 1024;
 constexpr int kTmemColumns = 2 * kMaxBN;
 constexpr int kGroupM = 4;        // batch tiles walked together before moving along N
-constexpr unsigned kSpinLimit = 1u << 20;
-
-// Set when a bounded wait inside the tensor-core kernel gives up (which barrier: low byte).
+// Set when a bounded wait inside a tensor-core kernel gives up (which barrier: low byte).
 __device__ unsigned g_tcgen05_status = 0;
 
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-    return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(unsigned bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// Bounded wait for the phase with the given parity to complete.  False (and a status code) on give-up.
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, unsigned code) {
-    for (unsigned spin = 0; spin < kSpinLimit; ++spin) {
-        unsigned done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    atomicMax(&g_tcgen05_status, code);
-    return false;
-}
-
-// Shared-memory operand descriptor: K-major tile, 128-byte swizzle, rows 128 bytes apart, 8-row
-// groups 1024 bytes apart, descriptor version 1 (sm_100).
-__device__ __forceinline__ uint64_t operand_desc(unsigned smem_address) {
-    uint64_t desc = (smem_address & 0x3FFFFu) >> 4;   // start address, 16-byte units
-    desc |= static_cast<uint64_t>(1) << 16;           // leading byte offset (unused with swizzle): 1
-    desc |= static_cast<uint64_t>(1024 >> 4) << 32;   // stride byte offset between 8-row groups
-    desc |= static_cast<uint64_t>(1) << 46;           // version
-    desc |= static_cast<uint64_t>(2) << 61;           // SWIZZLE_128B
-    return desc;
-}
-
-__device__ __forceinline__ void umma_f16(unsigned tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t instr_desc,
-                                         uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(instr_desc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void umma_commit(unsigned bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    return mbar_wait(bar, parity, code, &g_tcgen05_status);
 }
 
 struct TcParams {
@@ -527,25 +476,22 @@ __global__ void sum_ranges_kernel(const float* __restrict__ partial, __half* __r
     *reinterpret_cast<uint2*>(y + i) = out;
 }
 
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// The driver's tensor-map encoder, looked up through the runtime so that libcuda is not a link dependency.
-EncodeTiledFn tensor_map_encoder() {
-    static EncodeTiledFn fn = [] {
-        void* entry = nullptr;
-        cudaDriverEntryPointQueryResult found;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &entry, cudaEnableDefault, &found) != cudaSuccess ||
-            found != cudaDriverEntryPointSuccess) {
-            entry = nullptr;
-        }
-        return reinterpret_cast<EncodeTiledFn>(entry);
-    }();
-    return fn;
-}
-
 }  // namespace
+
+// The status word's device address, looked up once per device.
+unsigned* tcgen05_status_address() {
+    static std::atomic<unsigned*> cached[64] = {};
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return nullptr;
+    unsigned* address = cached[device].load(std::memory_order_relaxed);
+    if (address == nullptr) {
+        void* found = nullptr;
+        if (cudaGetSymbolAddress(&found, g_tcgen05_status) != cudaSuccess) return nullptr;
+        address = static_cast<unsigned*>(found);
+        cached[device].store(address, std::memory_order_relaxed);
+    }
+    return address;
+}
 
 // K ranges per output tile that the GEMM wants for a problem: more than one when the layer has so few tiles that
 // half the SMs or more would idle and K is long enough to share (ranges of 1024 or more, a multiple of 256, and
