@@ -164,8 +164,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 linear_gemm_kernel(const GemmParams p, const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map) {
     constexpr int kScales = kBlockK / GROUP;                               // per row and K block
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    __shared__ int verdict;                                                // all parts of a tile are in place
-    __shared__ TileParts shared_parts;
+    // Whether all parts of a tile are in place: for the drain warps, and for all warps at the end (both may be at it at once).
+    __shared__ int drain_verdict, verdict;
+    __shared__ TileParts drain_parts, shared_parts;
     const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;           // swizzle patterns are a function of the address
     const unsigned x_half_bytes = static_cast<unsigned>(p.bn) * 128;       // 64 K of every batch row, 128-byte swizzled
     auto x_slot = [&](int s) { return base + s * 2 * x_half_bytes; };
@@ -500,16 +501,16 @@ linear_gemm_kernel(const GemmParams p, const __grid_constant__ CUtensorMap x_map
                 __threadfence();
                 drain_barrier();
                 if (tid == kFirstDrainWarp * 32) {
-                    shared_parts = parts_of(p, seg.tile);
-                    verdict = atomicAdd(p.counters + seg.tile, 1u) == static_cast<unsigned>(shared_parts.last - shared_parts.first);
-                    if (verdict) p.counters[seg.tile] = 0u;                // ready for the next call
+                    drain_parts = parts_of(p, seg.tile);
+                    drain_verdict = atomicAdd(p.counters + seg.tile, 1u) == static_cast<unsigned>(drain_parts.last - drain_parts.first);
+                    if (drain_verdict) p.counters[seg.tile] = 0u;                // ready for the next call
                 }
                 drain_barrier();
-                if (verdict != 0) {
+                if (drain_verdict != 0) {
                     __threadfence();
                     for (int i = 0; i < 2 * p.bn; i += 16) {
                         float sum[16];
-                        add_parts(shared_parts, false, chunk_at(i), sum);
+                        add_parts(drain_parts, false, chunk_at(i), sum);
                         emit(seg.tile, sum, chunk_at(i));
                     }
                 }
