@@ -251,16 +251,32 @@ linear_gemm_kernel(const GemmParams p, const __grid_constant__ CUtensorMap x_map
 #pragma unroll
         for (int j = 0; j < 16; ++j) sum[j] = __uint_as_float(v[j]);
     };
-    auto emit = [&](int tile, const float (&sum)[16], const Chunk& at) {   // rounded, to the output
+    // Rounded, to the output.  Few instructions per element: the drain warps share their schedulers with 24 dequantisers.
+    auto emit = [&](int tile, const float (&sum)[16], const Chunk& at) {
         const int n = tile / p.m_tiles * kRows + at.row, m = tile % p.m_tiles * p.bn + at.col;
         if (n >= p.N) return;
-        __half* out = p.y + static_cast<size_t>(m) * p.N + n;
-        const __half bias = p.bias != nullptr ? p.bias[n] : __half();
+        char* out = reinterpret_cast<char*>(p.y + static_cast<size_t>(m) * p.N + n);
+        const unsigned stride = static_cast<unsigned>(p.N) * 2u;
+        __half2 pair[8];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            __half value = __float2half_rn(sum[j]);
-            if (p.bias != nullptr) value = __hadd(value, bias);
-            if (m + j < p.M) out[static_cast<size_t>(j) * p.N] = value;
+        for (int j = 0; j < 8; ++j) pair[j] = __floats2half2_rn(sum[2 * j], sum[2 * j + 1]);
+        if (p.bias != nullptr) {
+            const __half2 bias = __half2half2(p.bias[n]);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) pair[j] = __hadd2(pair[j], bias);
+        }
+        if (m + 16 <= p.M) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                *reinterpret_cast<__half*>(out) = j % 2 == 0 ? __low2half(pair[j / 2]) : __high2half(pair[j / 2]);
+                out += stride;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                if (m + j < p.M) *reinterpret_cast<__half*>(out) = j % 2 == 0 ? __low2half(pair[j / 2]) : __high2half(pair[j / 2]);
+                out += stride;
+            }
         }
     };
     auto store_part = [&](int which, const float (&sum)[16], const Chunk& at) {
