@@ -79,11 +79,11 @@ typedef struct w4a16_linear_config {
  * favours it) a tcgen05 GEMM whose producer warps dequantise into the operand tiles
  * (no FP16 weight matrix in memory; weights enter the product as half(code * scale), the arithmetic of
  * the reference's dequantise-then-matmul prefill route, w4a16/linear.py:132-152).
- * group_size 64 and 32 run the streaming kernel at every M when K is a multiple of 128 and x, packed and scales are
- * 16-byte aligned.  Otherwise a generic kernel that accepts any even group_size and any alignment.
- * The GEMM shares the K of an output tile between up to four CTAs when a layer has too few 128-row tiles for the
- * SMs (FP32 partial sums in the workspace, added in order and rounded once by a second small kernel); without
- * enough workspace it runs unsplit.
+ * group_size 64 and 32 run the streaming kernel up to M = 64 and the GEMM above when K is a multiple of 128 and x, packed
+ * and scales are 16-byte aligned.  Otherwise a generic kernel that accepts any even group_size and any alignment.
+ * The GEMM shares the K of an output tile between CTAs when a layer has too few tiles for the SMs: inside a thread-block
+ * cluster, or through FP32 partial sums in the workspace that are added in a fixed order and rounded once; without enough
+ * workspace the second does not happen.
  * `workspace` may be NULL (then K is never split across CTAs); if given it must be 16-byte aligned,
  * hold at least w4a16_linear_workspace_bytes(M, N, K) bytes, be zero-filled before its first use
  * and not be shared by calls that may run concurrently.  The library leaves it ready for re-use, by calls

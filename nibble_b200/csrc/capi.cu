@@ -73,10 +73,20 @@ bool routes_to_tcgen05(int64_t M, int64_t N, int64_t K, uint32_t flags) {
 }
 
 int launch_gemm(const w4a16::LinearProblem& p, cudaStream_t stream) {
-    return p.M <= w4a16::kGemmMaxRows ? w4a16::launch_linear_gemm(p, stream) : w4a16::launch_linear_tcgen05(p, stream);
+    const bool tensor_memory = p.group != w4a16::kGroupFast || w4a16::gemm_from_tensor_memory(p.M, p.N, p.K);
+    return tensor_memory ? w4a16::launch_linear_gemm(p, stream) : w4a16::launch_linear_tcgen05(p, stream);
 }
 
 }  // namespace
+
+// Measured on 16 layers at 65 to 2048 rows: weights in tensor memory are faster up to 512 rows (8192 -> 28672: 128 rows 64 against
+// 88 us, 384 rows 167 against 219) and level or up to 15 % slower above, where 256-row batch tiles read x half as often.  A layer whose
+// 128-row tiles just fit one round of SMs has nothing to share, and with a short K the other kernel's shorter start shows
+// (1024 -> 12928, 128 rows: 12.1 against 11.1 us).
+bool w4a16::gemm_from_tensor_memory(int64_t M, int64_t N, int64_t K) {
+    const int64_t tiles = (N + 127) / 128;
+    return M <= 512 && !(M <= 128 && K <= 1024 && tiles > 74 && tiles <= 148);
+}
 
 bool w4a16::linear_routes_to_tcgen05(int64_t M, int64_t N, int64_t K, uint32_t flags) {
     return routes_to_tcgen05(M, N, K, flags);
@@ -108,7 +118,7 @@ size_t w4a16_linear_workspace_bytes_flags(int64_t M, int64_t N, int64_t K, uint3
     // The generic kernel uses no scratch; the tcgen05 GEMM wants some only for layers with few tiles.
     if (flags & W4A16_FLAG_FORCE_GENERIC) return 0;
     if (routes_to_tcgen05(M, N, K, flags)) {
-        return M <= w4a16::kGemmMaxRows ? w4a16::gemm_workspace_bytes(M, N, K) : w4a16::tcgen05_workspace_bytes(M, N, K);
+        return w4a16::gemm_from_tensor_memory(M, N, K) ? w4a16::gemm_workspace_bytes(M, N, K) : w4a16::tcgen05_workspace_bytes(M, N, K);
     }
     const w4a16_linear_config c = w4a16::choose_linear_config(M, N, K, w4a16::kMaxKSplits);
     return w4a16::linear_workspace_bytes_for(M, N, c.k_splits);
@@ -146,8 +156,12 @@ int w4a16_linear_f16_bias(const void* x, const void* packed, const void* scales,
     if ((flags & W4A16_FLAG_FORCE_GENERIC) || (!small_group && !fast_path_applies(x, packed, K, group_size))) {
         return w4a16::launch_linear_generic(p, out_f32, s);
     }
-    // Prefill-sized batches, and medium ones on large layers: dense enough for the tcgen05 tensor cores.
-    if (!small_group && routes_to_tcgen05(M, N, K, flags)) return launch_gemm(p, s);
+    // Prefill-sized batches, and medium ones on large layers: dense enough for the tcgen05 tensor cores.  (Small groups only
+    // from 65 rows on: the streaming kernel does not round their weights, and no batch below has been rounded before.)
+    const bool to_gemm = small_group ? M >= w4a16::kTcgen05MinRows && !out_f32 && !(flags & W4A16_FLAG_NO_TCGEN05) ||
+                                           (flags & W4A16_FLAG_FORCE_TCGEN05) && !out_f32
+                                     : routes_to_tcgen05(M, N, K, flags);
+    if (to_gemm) return launch_gemm(p, s);
     // Split K across CTAs only as far as the caller's workspace allows.
     int max_splits = 1;
     if (workspace != nullptr && aligned16(workspace)) {

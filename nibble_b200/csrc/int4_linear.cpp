@@ -24,7 +24,7 @@ namespace {
 // Split-K scratch, one buffer per (device, stream) so calls on different streams never share it.
 // Allocated zero-filled on first use and kept for the life of the process; the first call on a
 // stream should therefore happen before that stream is captured into a CUDA graph.
-constexpr int64_t kWorkspaceBytes = 40 << 20;   // largest request of the shapes in the bench tables: 33 MiB (M = 512 on 8192 x 8192 takes none; M = 256 does)
+constexpr int64_t kWorkspaceBytes = 40 << 20;   // largest request: 38 MiB (the GEMM's parts, two of 256 x 128 sums for each of 148 CTAs)
 
 at::Tensor& workspace_for(const at::Device& device, cudaStream_t stream) {
     static std::mutex mutex;
@@ -112,8 +112,10 @@ at::Tensor linear_impl(const at::Tensor& activations, const at::Tensor& packed_w
 
     void* workspace = nullptr;
     size_t workspace_bytes = 0;
-    // (the GEMM, which has its own wish for scratch, is built for 128-wide groups)
-    const size_t wanted = w4a16_linear_workspace_bytes_flags(m, n, k, group_size == 128 ? flags : flags | W4A16_FLAG_NO_TCGEN05);
+    // (the query answers for 128-wide groups; small ones stay on the streaming kernel up to 64 rows)
+    const size_t wanted = group_size == 128 ? w4a16_linear_workspace_bytes_flags(m, n, k, flags)
+                          : m > 64          ? static_cast<size_t>(kWorkspaceBytes)
+                                            : w4a16_linear_workspace_bytes_flags(m, n, k, flags | W4A16_FLAG_NO_TCGEN05);
     if (wanted > 0 && wanted <= static_cast<size_t>(kWorkspaceBytes)) {
         at::Tensor& ws = workspace_for(activations.device(), stream);
         workspace = ws.data_ptr();

@@ -644,6 +644,12 @@ struct GemmPlan {
     bool cut;                // runs may hold parts of tiles
 };
 
+// Runs of at least four K blocks, on all SMs where there is that much work.
+constexpr int64_t kMinCutK = 2048, kMaxCutTiles = 65536;
+int cut_grid(long long tiles, int k_blocks, int sms) {
+    return static_cast<int>(std::min<long long>(sms, std::max<long long>(tiles, tiles * k_blocks / 4)));
+}
+
 // `clusters[s]`: clusters of s CTAs that run at once (0 where unknown or none).
 GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, const int* clusters) {
     GemmPlan g;
@@ -651,16 +657,18 @@ GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, const int* clusters
     g.bn = static_cast<int>(((M + g.m_tiles - 1) / g.m_tiles + 15) / 16 * 16);
     g.k_blocks = static_cast<int>(K / kBlockK);
     g.tiles = (N + kRows - 1) / kRows * g.m_tiles;
-    // Times in us, from measurements at 8192 x 8192 and 8192 -> 28672: a K block, a CTA's start and end, the exchange inside a
-    // cluster (13 bytes a clock), the exchange through the workspace (parts of 256 x bn sums written and read back).
-    const double block = 0.62 + 0.003 * std::max(0, g.bn - 64), ends = 4.5;
+    // Times in us, fitted to 65..512 rows on sixteen layers from 1024 x 1024 to 8192 -> 28672 (mostly within 15 %): a K block, a
+    // CTA's start and end, going on to another tile, the exchange inside a cluster (13 bytes a clock), the exchange through
+    // the workspace (parts of 256 x bn sums written and read back).
+    const double block = 0.62 + 0.0045 * std::max(0, g.bn - 64), ends = 4.5, next_tile = 1.0 + 0.012 * g.bn;
     auto by_cluster = [&](int s) { return 1.2 + 0.043 * g.bn * (s - 1) / s; };
     const double by_workspace = 1.5 + 0.025 * g.bn;
     const long long units = g.tiles * g.k_blocks;
     g.cluster = 1;
     g.cut = false;
     g.grid = static_cast<int>(std::min<long long>(sms, g.tiles));
-    double best = static_cast<double>((g.tiles + sms - 1) / sms) * g.k_blocks * block + ends;
+    const double rounds = static_cast<double>((g.tiles + sms - 1) / sms);
+    double best = rounds * g.k_blocks * block + ends + (rounds - 1.0) * next_tile;
     for (int s = 2; s <= kMaxCluster && s <= g.k_blocks; ++s) {
         if (clusters == nullptr || clusters[s] <= 0 || g.tiles * s > INT32_MAX) continue;
         const long long waves = (g.tiles + clusters[s] - 1) / clusters[s];
@@ -670,9 +678,10 @@ GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, const int* clusters
             g.cluster = s;
         }
     }
-    if (K >= 2048 && g.tiles <= 65536) {
-        const long long grid = std::min<long long>(sms, std::max<long long>(g.tiles, units / 4));
-        const double time = static_cast<double>((units + grid - 1) / grid) * block + ends + by_workspace * ((g.k_blocks * grid + units - 1) / units);
+    if (K >= kMinCutK && g.tiles <= kMaxCutTiles) {
+        const long long grid = cut_grid(g.tiles, g.k_blocks, sms);
+        const double time = static_cast<double>((units + grid - 1) / grid) * block + ends + static_cast<double>(g.tiles) / sms * next_tile +
+                            by_workspace * ((g.k_blocks * grid + units - 1) / units);
         if (time < best && grid != g.tiles) {
             g.cluster = 1;
             g.cut = true;
@@ -686,9 +695,12 @@ size_t gemm_partial_bytes(const GemmPlan& g) { return g.cut ? static_cast<size_t
 
 }  // namespace
 
-// What the runs want where K is shared; a device that runs the clusters instead leaves it unused.
+// What runs that cut tiles would take.  (A device that can run the clusters may leave it unused, and plan_gemm() decides
+// whether cutting pays; the answer does not depend on either.)
 size_t gemm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
-    const GemmPlan g = plan_gemm(M, N, K, 148, nullptr);
+    GemmPlan g = plan_gemm(M, N, K, 148, nullptr);
+    g.grid = cut_grid(g.tiles, g.k_blocks, 148);
+    g.cut = K >= kMinCutK && g.tiles <= kMaxCutTiles && g.grid != g.tiles;
     return g.cut ? linear_counter_bytes(M, N) + gemm_partial_bytes(g) : 0;
 }
 

@@ -28,12 +28,24 @@ c10::TypedOperatorHandle<Signature> operator_handle(const char* name) {
     return c10::Dispatcher::singleton().findSchemaOrThrow(name, "").typed<Signature>();
 }
 
-// nibble_b200/linear.py: uses_fused_kernel, which states the reasons.
-bool uses_fused_kernel(int64_t rows, int64_t out_features, int64_t group_size) {
+// Whether a batch goes to the fused operator, or is multiplied by dequantised FP16 weights (same arithmetic from 65 rows
+// on: weights rounded to FP16, FP32 sums).  The lines come from times of both on 16 layers at 65 to 2048 rows:
+//   - dequantising and cuBLAS cost about 6 us + 2.5 bytes a weight + the matrix product at its full rate, and 14 us of host
+//     time: unbeaten above 1024 rows, and on mid-sized layers above 256 (2048 -> 5632, 512 rows: 17.7 against 20.5 us), but not on
+//     small ones, where the host sets the pace (1024 -> 1920, 89 rows: 15.8 against 9 us);
+//   - cuBLAS falls off its fast kernels where an output row is no multiple of 16 bytes (9216 -> 2575, 128 rows: 125 against 20 us);
+//   - from 513 rows on the operator has 256-row batch tiles, and is ahead only where the last one is nearly full
+//     (8192 -> 28672, 1024 rows: 451 against 494 us; 777 rows: 442 against 362).
+bool uses_fused_kernel(int64_t rows, int64_t out_features, int64_t in_features, int64_t group_size) {
     if (rows <= 64) return true;
     if (group_size % 32 != 0) return true;
-    if (group_size != 128) return false;
-    return rows <= 1024 && (out_features + 127) / 128 >= 40;
+    if (group_size > 128 || in_features % 128 != 0) return false;      // the operator has no tensor-core kernel for these
+    if (out_features % 8 != 0) return true;
+    const int64_t weights = out_features * in_features;
+    const bool shallow = in_features < 1024 && out_features >= 8192;   // many tiles of a few K blocks each
+    if (rows <= 256) return rows <= 128 || !shallow;
+    if (rows <= 512) return weights <= 9 << 19 || (weights >= 32 << 20 && !shallow);
+    return group_size == 128 && rows <= 1024 && (256 - rows % 256) % 256 < 64 && weights >= 64 << 20;
 }
 
 // A tensor nobody has subclassed, wrapped or asked to track gradients of.
@@ -70,13 +82,20 @@ PyObject* linear_forward(PyObject*, PyObject* const* args, Py_ssize_t count) {
     {
         pybind11::gil_scoped_release unlocked;             // a launch may block when the stream's queue is full
         const at::AutoDispatchBelowADInplaceOrView below;  // nothing here takes part in autograd
-        if ((fused != 0 || group_size % 32 != 0) && uses_fused_kernel(rows, packed.size(0), group_size)) {
+        if ((fused != 0 || group_size % 32 != 0) && uses_fused_kernel(rows, packed.size(0), x.size(-1), group_size)) {
             static const auto op = operator_handle<LinearBias>("w4a16::linear_bias");
             out = op.call(x, packed, scales, bias, group_size);
         } else {
             static const auto op = operator_handle<Dequantize>("w4a16::dequantize");
-            out = at::linear(x, op.call(packed, scales, group_size));
+            // (at::mm on two dimensions rather than at::linear, which takes 2 us longer to get there)
+            const at::Tensor weights = op.call(packed, scales, group_size);
+            out = at::mm(x.view({rows, x.size(-1)}), weights.t());
             if (bias.has_value()) out.add_(*bias);
+            if (x.dim() != 2) {
+                c10::SmallVector<int64_t, 5> shape(x.sizes().begin(), x.sizes().end());
+                shape.back() = weights.size(0);
+                out = out.view(shape);
+            }
         }
     }
     return THPVariable_Wrap(std::move(out));

@@ -17,7 +17,8 @@ from .quantization import quantize_and_pack_weights
 # Largest flattened batch M sent to the streaming (mma.sync) fused kernel.  The reference stops at 8
 # and dequantises to FP16 + cuBLAS above that (w4a16/linear.py:9,179-187).
 FUSED_MAX_ROWS = 64
-# Above FUSED_MAX_ROWS the operator runs the tcgen05 kernel that dequantises inside the GEMM.  It beats
+# Above FUSED_MAX_ROWS the operator runs the tcgen05 kernels that dequantise inside the GEMM.  (This is the rule of the
+# Python forward; the native one, which takes nearly every call, draws finer lines: csrc/linear_module.cpp.)  It beats
 # dequantise-then-cuBLAS while the FP16 weight matrix's round trip through HBM is a large share of the
 # cuBLAS time (batches up to about a thousand rows) and there are enough 128-channel weight tiles to
 # occupy the GPU; outside that window the module does what the reference does.

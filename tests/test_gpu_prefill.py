@@ -169,3 +169,31 @@ def test_all_nibble_values_and_repeatability(golden):
     assert torch.equal(first, second)
     assert _device_status() == 0
     check_against_oracle(first, x, packed, scales, fp16_weights=True)
+
+
+@pytest.mark.parametrize(("m", "k", "n", "gs"), [
+    (40, 1024, 1000, 128),     # few tiles: a cluster per tile
+    (65, 4096, 1900, 128),     # batch tile above 64 rows: two weight slots
+    (128, 8192, 28672, 128),   # equal runs that cut tiles, two segments each
+    (40, 8192, 28672, 128),    # ... with three weight slots
+    (100, 5632, 12345, 128),   # ... on ragged channels
+    (130, 512, 40000, 128),    # runs of several whole tiles, two batch tiles
+    (512, 1024, 5000, 128),
+    (128, 4096, 3000, 64), (300, 8192, 1000, 32), (77, 2048, 32000, 32),
+])
+def test_gemm_from_tensor_memory(m, k, n, gs):
+    """Every way the GEMM shares tiles, with and without a workspace, against the product with the same FP16 weights."""
+    from nibble_b200 import dequantize_cuda
+
+    _device_status()
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    packed, scales = quantize_and_pack_weights(torch.randn((n, k), generator=g, device="cuda") * 0.02, gs)
+    x = torch.randn((m, k), generator=g, device="cuda").half()
+    want = x.float() @ dequantize_cuda(packed, scales, gs).float().t()
+    ws = torch.zeros(40 << 20, dtype=torch.uint8, device="cuda")
+    for workspace in (ws, ws, None):
+        y = capi_linear(x, packed, scales, gs, workspace=workspace, flags=_native.FLAG_FORCE_TCGEN05)
+        torch.testing.assert_close(y.float(), want, rtol=2e-3, atol=2e-3)
+        assert torch.equal(y, capi_linear(x, packed, scales, gs, workspace=workspace, flags=_native.FLAG_FORCE_TCGEN05))
+    assert int(ws[: 256 * 1024].sum()) == 0
+    assert _device_status() == 0, "a barrier wait gave up"
