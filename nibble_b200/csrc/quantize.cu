@@ -6,10 +6,7 @@
 //   scale = half(step)                                     (rounded after the codes are made)
 // byte j of a row holds code 2j in its low nibble and code 2j+1 in its high nibble.
 //
-// 128-wide groups (the format's default): half a warp per group, a lane keeps its eight consecutive
-// weights in registers (one 16-byte load for FP16, two for FP32), the group maximum is a four-step
-// shuffle reduction inside the half warp, and the eight codes leave as one 4-byte store.  Bound: HBM,
-// 2.5 (FP16 input) or 4.5 (FP32) bytes per weight; the IEEE divisions keep it near the issue limit.
+// Groups of 128, 64 and 32: quantize_pack_group_kernel below, weights read once.
 // Other group sizes: one warp per group, weights read twice (maximum, then codes).
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -66,76 +63,123 @@ quantize_pack_kernel(const T* __restrict__ weights, uint8_t* __restrict__ packed
     }
 }
 
-__device__ __forceinline__ void load8(const __half* p, float (&w)[8]) {
-    const uint4 q = *reinterpret_cast<const uint4*>(p);
-    const __half2* h = reinterpret_cast<const __half2*>(&q);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float2 f = __half22float2(h[i]);
-        w[2 * i] = f.x;
-        w[2 * i + 1] = f.y;
+// Eight consecutive weights, as loaded and as floats.
+template <typename T>
+struct Eight;
+template <>
+struct Eight<__half> {
+    uint4 raw;
+    __device__ __forceinline__ void load(const __half* p) { raw = __ldcs(reinterpret_cast<const uint4*>(p)); }
+    // largest magnitude: in FP16, two at a time
+    __device__ __forceinline__ float amax() const {
+        const __half2* h = reinterpret_cast<const __half2*>(&raw);
+        const __half2 m = __hmax2(__hmax2(__habs2(h[0]), __habs2(h[1])), __hmax2(__habs2(h[2]), __habs2(h[3])));
+        return fmaxf(__low2float(m), __high2float(m));
     }
-}
-__device__ __forceinline__ void load8(const float* p, float (&w)[8]) {
-    const float4 a = reinterpret_cast<const float4*>(p)[0];
-    const float4 b = reinterpret_cast<const float4*>(p)[1];
-    w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
-    w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+    __device__ __forceinline__ void floats(float (&w)[8]) const {
+        const __half2* h = reinterpret_cast<const __half2*>(&raw);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 f = __half22float2(h[i]);
+            w[2 * i] = f.x;
+            w[2 * i + 1] = f.y;
+        }
+    }
+};
+template <>
+struct Eight<float> {
+    float4 lo, hi;
+    __device__ __forceinline__ void load(const float* p) {
+        lo = __ldcs(reinterpret_cast<const float4*>(p));
+        hi = __ldcs(reinterpret_cast<const float4*>(p) + 1);
+    }
+    __device__ __forceinline__ float amax() const {
+        return fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(lo.y)), fmaxf(fabsf(lo.z), fabsf(lo.w))),
+                     fmaxf(fmaxf(fabsf(hi.x), fabsf(hi.y)), fmaxf(fabsf(hi.z), fabsf(hi.w))));
+    }
+    __device__ __forceinline__ void floats(float (&w)[8]) const {
+        w[0] = lo.x; w[1] = lo.y; w[2] = lo.z; w[3] = lo.w;
+        w[4] = hi.x; w[5] = hi.y; w[6] = hi.z; w[7] = hi.w;
+    }
+};
+
+// Eight codes as one word.
+//
+// Fast route: t = w * (1/step) + 1.5 * 2^23 in one FMA rounds the exact product to the nearest even integer; r = t - 1.5 * 2^23
+// is that integer.  The product and the reference's fl(w / step) differ by a few ulp at most, so both round to the same
+// integer unless the quotient sits within 1e-4 of a tie k + 0.5; a lane that sees such a weight (about one in 600), or whose
+// 1/step is not finite, redoes its codes with the IEEE division.
+//
+// Packing in floats: four codes are a number of at most 16 bits, r0 + 16 r1 + 256 r2 + 4096 r3 + 0x8888, exact in FP32 and read
+// off the mantissa after adding 2^23; the 8 added to each nibble is its sign bit flipped.
+__device__ __forceinline__ uint32_t pack_codes(const float (&w)[8], float step, float inv_step) {
+    constexpr float kMagic = 12582912.0f;
+    float r[8], off = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        r[i] = fmaf(w[i], inv_step, kMagic) - kMagic;
+        off = fmaxf(off, fabsf(fmaf(w[i], inv_step, -r[i])));
+    }
+    float lo = fmaf(fmaf(fmaf(r[3], 16.0f, r[2]), 16.0f, r[1]), 16.0f, r[0]) + (8388608.0f + 34952.0f);
+    float hi = fmaf(fmaf(fmaf(r[7], 16.0f, r[6]), 16.0f, r[5]), 16.0f, r[4]) + (8388608.0f + 34952.0f);
+    uint32_t word = __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x5410) ^ 0x88888888u;
+    // fmaxf drops a NaN, so infinity and NaN are looked for where they come from
+    if (off > 0.4999f || !(inv_step <= 3.0e38f)) {
+        word = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) word |= code_of(w[i], step) << (4 * i);
+    }
+    return word;
 }
 
-// group == 128 and 16-byte aligned weights: sixteen lanes per group, eight weights per lane
-template <typename T>
+// GROUP 128, 64 or 32 and 16-byte aligned weights: GROUP / 16 lanes share a group, a lane holds weights 8l..8l+7 of each half
+// of it, so both loads of the lanes are contiguous, and what a group costs once (two IEEE divisions, the shuffles) is
+// shared by 16 weights.  Bound: HBM at 2.5 bytes (FP16) or 4.5 (FP32) a weight, with about nine instructions a weight close behind.
+// 28672 x 8192 from FP16, 128-wide groups: 148 -> 115 us (5.1 TB/s);
+// from FP32 164 us (6.4 TB/s); with 64- and 32-wide groups, which read the weights twice before, 803 and 1406 -> 115 us.
+template <typename T, int GROUP>
 __global__ void __launch_bounds__(256)
-quantize_pack_128_kernel(const T* __restrict__ weights, uint8_t* __restrict__ packed, __half* __restrict__ scales,
-                         int64_t total_groups) {
-    const int lane16 = threadIdx.x & 15;
-    const int64_t halves = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 4);
-    // every lane of a warp runs the same number of rounds: the shuffles below name the whole warp
-    const int64_t rounds = (total_groups + halves - 1) / halves;
-    int64_t g = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 4) + (threadIdx.x >> 4);
-    for (int64_t r = 0; r < rounds; ++r, g += halves) {
+quantize_pack_group_kernel(const T* __restrict__ weights, uint8_t* __restrict__ packed, __half* __restrict__ scales,
+                           int64_t total_groups) {
+    constexpr int kLanes = GROUP / 16;
+    constexpr int kGroupsPerBlock = 256 / kLanes;
+    const int l = threadIdx.x % kLanes;
+    for (int64_t block = blockIdx.x; block * kGroupsPerBlock < total_groups; block += gridDim.x) {
+        const int64_t g = block * kGroupsPerBlock + threadIdx.x / kLanes;
         const bool live = g < total_groups;
-        float w[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        if (live) load8(weights + g * 128 + lane16 * 8, w);
-        float amax = 0.0f;
+        Eight<T> a, b;
+        const T* src = weights + (live ? g : total_groups - 1) * GROUP + l * 8;
+        a.load(src);
+        b.load(src + GROUP / 2);
+        float amax = fmaxf(a.amax(), b.amax());
 #pragma unroll
-        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(w[i]));
-#pragma unroll
-        for (int offset = 8; offset > 0; offset >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, offset));
-        if (!live) continue;
+        for (int offset = kLanes / 2; offset > 0; offset >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, offset));
         const float step = amax == 0.0f ? 1.0f : __fdiv_rn(amax, 7.0f);
         const float inv_step = __fdiv_rn(1.0f, step);
-        // Fast route for all eight codes: t = w * (1/step) + 1.5 * 2^23 in one FMA leaves round-half-even of the
-        // exact product in the low mantissa bits of t (|w / step| <= 7, so the low nibble of t's bit pattern IS the
-        // two's-complement code).  The product and the reference's fl(w / step) differ by a few ulp at most, so
-        // both round to the same integer unless the quotient sits within 1e-4 of a tie k + 0.5; a lane that sees
-        // such a weight redoes its eight codes with the IEEE division (about one lane in 600).
-        constexpr float kMagic = 12582912.0f;
-        unsigned word = 0;
-        bool near_tie = false;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float t = fmaf(w[i], inv_step, kMagic);
-            const float q = w[i] * inv_step;
-            near_tie |= fabsf(q - (t - kMagic)) > 0.4999f;
-            word |= (__float_as_uint(t) & 0xFu) << (4 * i);
+        float w[8];
+        uint32_t* out = reinterpret_cast<uint32_t*>(packed + g * (GROUP / 2)) + l;
+        a.floats(w);
+        const uint32_t first = pack_codes(w, step, inv_step);
+        b.floats(w);
+        const uint32_t second = pack_codes(w, step, inv_step);
+        if (live) {
+            out[0] = first;
+            out[GROUP / 16] = second;
+            if (l == 0) scales[g] = __float2half_rn(step);
         }
-        if (near_tie) {
-            word = 0;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) word |= code_of(w[i], step) << (4 * i);
-        }
-        reinterpret_cast<uint32_t*>(packed + g * 64)[lane16] = word;
-        if (lane16 == 0) scales[g] = __float2half_rn(step);
     }
 }
 
 template <typename T>
 int launch(const T* weights, uint8_t* packed, __half* scales, int64_t N, int64_t K, int64_t group, cudaStream_t stream) {
     const int64_t total_groups = N * (K / group);
-    if (group == 128 && reinterpret_cast<uintptr_t>(weights) % 16 == 0 && reinterpret_cast<uintptr_t>(packed) % 4 == 0) {
-        const int64_t fast_blocks = std::min<int64_t>((total_groups + 15) / 16, 148 * 32);
-        quantize_pack_128_kernel<T><<<static_cast<unsigned>(fast_blocks), 256, 0, stream>>>(weights, packed, scales, total_groups);
+    if ((group == 128 || group == 64 || group == 32) && reinterpret_cast<uintptr_t>(weights) % 16 == 0 &&
+        reinterpret_cast<uintptr_t>(packed) % 4 == 0) {
+        const int64_t groups_per_block = 256 / (group / 16);
+        const int64_t fast_blocks = std::min<int64_t>((total_groups + groups_per_block - 1) / groups_per_block, 148 * 64);
+        const auto kernel = group == 128 ? quantize_pack_group_kernel<T, 128>
+                            : group == 64 ? quantize_pack_group_kernel<T, 64> : quantize_pack_group_kernel<T, 32>;
+        kernel<<<static_cast<unsigned>(fast_blocks), 256, 0, stream>>>(weights, packed, scales, total_groups);
         if (cudaGetLastError() != cudaSuccess) return W4A16_ERR_LAUNCH;
         g_launch_count.fetch_add(1, std::memory_order_relaxed);
         return W4A16_OK;
