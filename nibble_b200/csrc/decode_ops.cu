@@ -138,15 +138,16 @@ struct AttentionParams {
 // (distributed shared memory), one cluster barrier, and the first CTA adds those up.
 //
 // Bound: latency of a dependent kernel at short contexts, loads in flight at long ones.  One CTA per head left 116 SMs idle
-// and took 47.6 us a layer at 1500 positions (TinyLlama: 32 heads of 64); eight take 5.9 us.  Two or four heads of a KV
+// and took 47.6 us a layer at 1500 positions (TinyLlama: 32 heads of 64); four take 5.4 us.  Two or four heads of a KV
 // head in one CTA would read each K and V row fewer times out of L2; it was 0.4 us faster there and 0.5 us slower at 4
-// positions, where the extra arithmetic is all latency.  Rows are requested two passes ahead (two register buffers of
-// kAttnBatch rows of K and V).  Contexts of one part's worth use one CTA per cluster and no cluster barrier: the other
+// positions, where the extra arithmetic is all latency.  Eight passes are requested ahead (two register buffers of
+// kAttnBatch rows of K and V), and the grid stays at one CTA per SM: with four passes and twice the CTAs a TinyLlama token
+// took 530 us at 1500 positions, 504 at 500 and 454 at 4, against 518, 470 and 444.  Contexts of one part's worth use one CTA per cluster and no cluster barrier: the other
 // CTAs leave at once.
 constexpr int kAttnThreads = 256;
 constexpr int kAttnWarps = kAttnThreads / 32;
 constexpr int kAttnMaxParts = 8;                      // CTAs per cluster: the portable limit
-constexpr int kAttnBatch = 2;                         // passes requested together
+constexpr int kAttnBatch = 4;                         // passes requested together
 constexpr float kNoScore = -1.0e30f;
 
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
@@ -195,8 +196,7 @@ attention_decode_kernel(const AttentionParams p) {
     constexpr int kLanesPerPos = D / 8;
     constexpr int kPosPerPass = kAttnThreads / kLanesPerPos;   // 32 (D = 64) or 16 (D = 128)
     constexpr int kPosPerBatch = kPosPerPass * kAttnBatch;
-    // A part is at least what one CTA requests before it needs any of it: less is not worth the cluster barrier.
-    constexpr int kPosPerPart = 2 * kPosPerBatch;
+    constexpr int kPosPerPart = 4 * kPosPerPass;               // at least: less is not worth the cluster barrier
     constexpr int half_d = D / 2;
     __shared__ __align__(16) __half cos_table[half_d];
     __shared__ __align__(16) __half sin_table[half_d];
@@ -455,10 +455,10 @@ int launch_attention_decode(const __half* qkv, __half* k_cache, __half* v_cache,
     AttentionParams params{qkv, k_cache, v_cache, out, position, inv_freq, q_heads, kv_heads, head_dim, max_len,
                            rope_scale, softmax_scale, status};
     auto kernel = head_dim == 64 ? attention_decode_kernel<64> : attention_decode_kernel<128>;
-    // CTAs per head: as many as the cache can give a part's worth of positions each, and no more than two per SM in all.
-    const int positions = kAttnThreads / (head_dim / 8) * kAttnBatch * 2;
+    // CTAs per head: as many as the cache can give a part's worth of positions each, and no more than one per SM in all.
+    const int positions = kAttnThreads / (head_dim / 8) * 4;
     int parts = 1;
-    while (parts < kAttnMaxParts && parts * positions < max_len && 2 * parts * q_heads <= 2 * 148) parts *= 2;
+    while (parts < kAttnMaxParts && parts * positions < max_len && 2 * parts * q_heads <= 148) parts *= 2;
     return launch_kernel(kernel, dim3(static_cast<unsigned>(q_heads) * parts), dim3(kAttnThreads), parts, 0, programmatic,
                          stream, params);
 }
