@@ -83,7 +83,7 @@ typedef struct w4a16_linear_config {
  * and scales are 16-byte aligned.  Otherwise a generic kernel that accepts any even group_size and any alignment.
  * The GEMM shares the K of an output tile between CTAs when a layer has too few tiles for the SMs: inside a thread-block
  * cluster, or through FP32 partial sums in the workspace that are added in a fixed order and rounded once; without enough
- * workspace the second does not happen.
+ * workspace (up to 39 MB, more than the query below asks for) the second does not happen.
  * `workspace` may be NULL (then K is never split across CTAs); if given it must be 16-byte aligned,
  * hold at least w4a16_linear_workspace_bytes(M, N, K) bytes, be zero-filled before its first use
  * and not be shared by calls that may run concurrently.  The library leaves it ready for re-use, by calls

@@ -117,9 +117,8 @@ size_t w4a16_linear_workspace_bytes_flags(int64_t M, int64_t N, int64_t K, uint3
     if (M <= 0 || N <= 0 || K <= 0 || K % w4a16::kGroupFast != 0) return 0;
     // The generic kernel uses no scratch; the tcgen05 GEMM wants some only for layers with few tiles.
     if (flags & W4A16_FLAG_FORCE_GENERIC) return 0;
-    if (routes_to_tcgen05(M, N, K, flags)) {
-        return w4a16::gemm_from_tensor_memory(M, N, K) ? w4a16::gemm_workspace_bytes(M, N, K) : w4a16::tcgen05_workspace_bytes(M, N, K);
-    }
+    // (With weights in tensor memory a larger one, up to 39 MB, lets equal runs cut tiles; it does without.)
+    if (routes_to_tcgen05(M, N, K, flags)) return w4a16::tcgen05_workspace_bytes(M, N, K);
     const w4a16_linear_config c = w4a16::choose_linear_config(M, N, K, w4a16::kMaxKSplits);
     return w4a16::linear_workspace_bytes_for(M, N, c.k_splits);
 }

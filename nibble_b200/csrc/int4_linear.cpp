@@ -112,10 +112,8 @@ at::Tensor linear_impl(const at::Tensor& activations, const at::Tensor& packed_w
 
     void* workspace = nullptr;
     size_t workspace_bytes = 0;
-    // (the query answers for 128-wide groups; small ones stay on the streaming kernel up to 64 rows)
-    const size_t wanted = group_size == 128 ? w4a16_linear_workspace_bytes_flags(m, n, k, flags)
-                          : m > 64          ? static_cast<size_t>(kWorkspaceBytes)
-                                            : w4a16_linear_workspace_bytes_flags(m, n, k, flags | W4A16_FLAG_NO_TCGEN05);
+    // From nine rows on the GEMM may run, which uses as much as there is.  (The query answers for 128-wide groups.)
+    const size_t wanted = m > 8 && !out_f32 ? static_cast<size_t>(kWorkspaceBytes) : w4a16_linear_workspace_bytes_flags(m, n, k, flags);
     if (wanted > 0 && wanted <= static_cast<size_t>(kWorkspaceBytes)) {
         at::Tensor& ws = workspace_for(activations.device(), stream);
         workspace = ws.data_ptr();

@@ -644,12 +644,6 @@ struct GemmPlan {
     bool cut;                // runs may hold parts of tiles
 };
 
-// Runs of at least four K blocks, on all SMs where there is that much work.
-constexpr int64_t kMinCutK = 2048, kMaxCutTiles = 65536;
-int cut_grid(long long tiles, int k_blocks, int sms) {
-    return static_cast<int>(std::min<long long>(sms, std::max<long long>(tiles, tiles * k_blocks / 4)));
-}
-
 // `clusters[s]`: clusters of s CTAs that run at once (0 where unknown or none).
 GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, const int* clusters) {
     GemmPlan g;
@@ -678,8 +672,9 @@ GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, const int* clusters
             g.cluster = s;
         }
     }
-    if (K >= kMinCutK && g.tiles <= kMaxCutTiles) {
-        const long long grid = cut_grid(g.tiles, g.k_blocks, sms);
+    if (K >= 2048 && g.tiles <= 65536) {
+        // runs of at least four K blocks, on all SMs where there is that much work
+        const long long grid = std::min<long long>(sms, std::max<long long>(g.tiles, units / 4));
         const double time = static_cast<double>((units + grid - 1) / grid) * block + ends + static_cast<double>(g.tiles) / sms * next_tile +
                             by_workspace * ((g.k_blocks * grid + units - 1) / units);
         if (time < best && grid != g.tiles) {
@@ -691,18 +686,10 @@ GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, const int* clusters
     return g;
 }
 
+// At most 38 MB: two parts of 256 x 128 sums for each SM.
 size_t gemm_partial_bytes(const GemmPlan& g) { return g.cut ? static_cast<size_t>(g.grid) * 2 * kRows * g.bn * sizeof(float) : 0; }
 
 }  // namespace
-
-// What runs that cut tiles would take.  (A device that can run the clusters may leave it unused, and plan_gemm() decides
-// whether cutting pays; the answer does not depend on either.)
-size_t gemm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
-    GemmPlan g = plan_gemm(M, N, K, 148, nullptr);
-    g.grid = cut_grid(g.tiles, g.k_blocks, 148);
-    g.cut = K >= kMinCutK && g.tiles <= kMaxCutTiles && g.grid != g.tiles;
-    return g.cut ? linear_counter_bytes(M, N) + gemm_partial_bytes(g) : 0;
-}
 
 int launch_linear_gemm(const LinearProblem& prob, cudaStream_t stream) {
     if (prob.K % kBlockK != 0 || prob.K <= 0 || !is_stream_group(prob.group)) return W4A16_ERR_BAD_CONFIG;

@@ -1,4 +1,4 @@
-// QuantizedLinear.forward in one native call.
+// The Python entry points' native side: QuantizedLinear.forward in one call, and the operators without torch.ops.
 //
 // The module's Python forward checks its arguments, flattens them, goes through torch.ops and reshapes: about 8 us of
 // interpreter and binding time around a 2 us kernel at M = 1.  linear_forward() makes the same checks and calls the same
@@ -17,9 +17,12 @@
 #include <torch/csrc/jit/frontend/tracer.h>
 
 #include <optional>
+#include <tuple>
 
 namespace {
 
+using QuantizePack = std::tuple<at::Tensor, at::Tensor>(const at::Tensor&, int64_t);
+using Linear = at::Tensor(const at::Tensor&, const at::Tensor&, const at::Tensor&, int64_t);
 using LinearBias = at::Tensor(const at::Tensor&, const at::Tensor&, const at::Tensor&, const std::optional<at::Tensor>&, int64_t);
 using Dequantize = at::Tensor(const at::Tensor&, const at::Tensor&, int64_t);
 
@@ -57,12 +60,75 @@ bool plain(PyObject* object) {
                                                      c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Batched}));
 }
 
+// Nothing that wants to see or change calls made from Python is active.
+bool ordinary_context() {
+    return !at::impl::torch_function_mode_enabled() && !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
+           !torch::jit::tracer::isTracing() && !at::autocast::is_autocast_enabled(at::kCUDA);
+}
+
+// linear(activations, packed_weights, scales, group_size) -> Tensor or NotImplemented
+PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t count) {
+    HANDLE_TH_ERRORS
+    if (count != 4 || !plain(args[0]) || !plain(args[1]) || !plain(args[2]) || !PyLong_Check(args[3]) || !ordinary_context()) {
+        Py_RETURN_NOTIMPLEMENTED;
+    }
+    const int64_t group_size = PyLong_AsLongLong(args[3]);
+    if (PyErr_Occurred() != nullptr) return nullptr;
+    at::Tensor out;
+    {
+        pybind11::gil_scoped_release unlocked;
+        const at::AutoDispatchBelowADInplaceOrView below;
+        static const auto op = operator_handle<Linear>("w4a16::linear");
+        out = op.call(THPVariable_Unpack(args[0]), THPVariable_Unpack(args[1]), THPVariable_Unpack(args[2]), group_size);
+    }
+    return THPVariable_Wrap(std::move(out));
+    END_HANDLE_TH_ERRORS
+}
+
+// dequantize(packed_weights, scales, group_size) -> Tensor or NotImplemented
+PyObject* dequantize(PyObject*, PyObject* const* args, Py_ssize_t count) {
+    HANDLE_TH_ERRORS
+    if (count != 3 || !plain(args[0]) || !plain(args[1]) || !PyLong_Check(args[2]) || !ordinary_context()) Py_RETURN_NOTIMPLEMENTED;
+    const int64_t group_size = PyLong_AsLongLong(args[2]);
+    if (PyErr_Occurred() != nullptr) return nullptr;
+    at::Tensor out;
+    {
+        pybind11::gil_scoped_release unlocked;
+        const at::AutoDispatchBelowADInplaceOrView below;
+        static const auto op = operator_handle<Dequantize>("w4a16::dequantize");
+        out = op.call(THPVariable_Unpack(args[0]), THPVariable_Unpack(args[1]), group_size);
+    }
+    return THPVariable_Wrap(std::move(out));
+    END_HANDLE_TH_ERRORS
+}
+
+// quantize_pack(weights, group_size) -> (packed, scales) or NotImplemented
+PyObject* quantize_pack(PyObject*, PyObject* const* args, Py_ssize_t count) {
+    HANDLE_TH_ERRORS
+    if (count != 2 || !plain(args[0]) || !PyLong_Check(args[1]) || !ordinary_context()) Py_RETURN_NOTIMPLEMENTED;
+    const int64_t group_size = PyLong_AsLongLong(args[1]);
+    if (PyErr_Occurred() != nullptr) return nullptr;
+    std::tuple<at::Tensor, at::Tensor> out;
+    {
+        pybind11::gil_scoped_release unlocked;
+        const at::AutoDispatchBelowADInplaceOrView below;
+        static const auto op = operator_handle<QuantizePack>("w4a16::quantize_pack");
+        out = op.call(THPVariable_Unpack(args[0]), group_size);
+    }
+    PyObject* packed = THPVariable_Wrap(std::move(std::get<0>(out)));
+    PyObject* scales = packed == nullptr ? nullptr : THPVariable_Wrap(std::move(std::get<1>(out)));
+    PyObject* pair = scales == nullptr ? nullptr : PyTuple_Pack(2, packed, scales);
+    Py_XDECREF(packed);
+    Py_XDECREF(scales);
+    return pair;
+    END_HANDLE_TH_ERRORS
+}
+
 // linear_forward(activations, packed_weights, scales, bias or None, group_size, fused) -> Tensor or NotImplemented
 PyObject* linear_forward(PyObject*, PyObject* const* args, Py_ssize_t count) {
     HANDLE_TH_ERRORS
     if (count != 6 || !plain(args[0]) || !plain(args[1]) || !plain(args[2]) || (args[3] != Py_None && !plain(args[3])) ||
-        at::impl::torch_function_mode_enabled() || c10::impl::TorchDispatchModeTLS::any_modes_set() ||
-        torch::jit::tracer::isTracing() || at::autocast::is_autocast_enabled(at::kCUDA)) {
+        !ordinary_context()) {
         Py_RETURN_NOTIMPLEMENTED;
     }
     const at::Tensor& x = THPVariable_Unpack(args[0]);
@@ -102,9 +168,15 @@ PyObject* linear_forward(PyObject*, PyObject* const* args, Py_ssize_t count) {
     END_HANDLE_TH_ERRORS
 }
 
+using FastCall = PyObject* (*)(PyObject*, PyObject* const*, Py_ssize_t);
+PyCFunction method(FastCall f) { return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)); }
+
 PyMethodDef methods[] = {
-    {"linear_forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(linear_forward)), METH_FASTCALL,
+    {"linear_forward", method(linear_forward), METH_FASTCALL,
      "linear_forward(activations, packed_weights, scales, bias, group_size, fused) -> Tensor or NotImplemented"},
+    {"linear", method(linear), METH_FASTCALL, "linear(activations, packed_weights, scales, group_size) -> Tensor or NotImplemented"},
+    {"dequantize", method(dequantize), METH_FASTCALL, "dequantize(packed_weights, scales, group_size) -> Tensor or NotImplemented"},
+    {"quantize_pack", method(quantize_pack), METH_FASTCALL, "quantize_pack(weights, group_size) -> (Tensor, Tensor) or NotImplemented"},
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_C", "Native side of nibble_b200: torch operators and QuantizedLinear.forward.", -1,

@@ -41,13 +41,18 @@ def _register_fakes() -> None:
                 weights.new_empty((rows, cols // group_size), dtype=torch.float16))
 
 
-def linear_forward(*arguments):
-    """Stands in for the native forward where the extension did not load: every call is left to the Python code."""
+def _left_to_python(*arguments):
+    """Stands in for a native entry point where the extension did not load: every call is left to the Python code."""
     return NotImplemented
 
 
+linear_forward = _native_linear = _native_dequantize = _native_quantize_pack = _left_to_python
 try:
-    linear_forward = _native.load_torch_ops().linear_forward
+    # csrc/linear_module.cpp: the ordinary case of the functions below (and of the module's forward) without torch.ops.
+    # NotImplemented, for anything out of the ordinary or wrong, means: go through the operator.
+    _extension = _native.load_torch_ops()
+    linear_forward, _native_linear = _extension.linear_forward, _extension.linear
+    _native_dequantize, _native_quantize_pack = _extension.dequantize, _extension.quantize_pack
     _register_fakes()
 except (ImportError, OSError, RuntimeError) as error:  # not built, stale, or built against another torch
     _EXTENSION_LOAD_ERROR: Exception | None = error
@@ -123,6 +128,10 @@ def linear_cuda(
     Invalid arguments raise ``RuntimeError``.
     """
     _require_extension()
+    if not torch.compiler.is_compiling():
+        out = _native_linear(activations, packed_weights, scales, group_size)
+        if out is not NotImplemented:
+            return out
     return torch.ops.w4a16.linear(activations, packed_weights, scales, group_size)
 
 
@@ -136,6 +145,10 @@ def dequantize_cuda(
     Needs ``group_size`` to be a positive multiple of 32 and 16-byte aligned packed weights.
     """
     _require_extension()
+    if not torch.compiler.is_compiling():
+        out = _native_dequantize(packed_weights, scales, group_size)
+        if out is not NotImplemented:
+            return out
     return torch.ops.w4a16.dequantize(packed_weights, scales, group_size)
 
 
@@ -159,4 +172,8 @@ def quantize_and_pack_cuda(weights: torch.Tensor, group_size: int = 128) -> tupl
     in one kernel, bit-identical to ``quantize_and_pack_weights`` (the reference's host routine,
     w4a16/quantization.py:65-113).  Not part of the reference's surface."""
     _require_extension()
+    if not torch.compiler.is_compiling():
+        out = _native_quantize_pack(weights, group_size)
+        if out is not NotImplemented:
+            return out
     return torch.ops.w4a16.quantize_pack(weights, group_size)

@@ -17,6 +17,7 @@ from __future__ import annotations
 import torch
 
 _NIBBLE = 0x0F
+_cuda = None      # the sibling module, once it is needed
 
 
 def _require_2d(tensor: torch.Tensor, what: str) -> None:
@@ -89,7 +90,9 @@ def quantize_and_pack_weights(
     """
     if weights.is_cuda and weights.ndim == 2 and weights.dtype in (torch.float16, torch.float32) \
             and group_size > 0 and group_size % 2 == 0 and weights.shape[1] % group_size == 0:
-        from . import cuda as _cuda   # late: this module must import without the extension
+        global _cuda
+        if _cuda is None:
+            from . import cuda as _cuda   # late: this module must import without the extension
 
         if _cuda.cuda_extension_available():
             return _cuda.quantize_and_pack_cuda(weights, group_size)
