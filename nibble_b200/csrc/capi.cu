@@ -53,12 +53,11 @@ bool routes_to_tcgen05(int64_t M, int64_t N, int64_t K, uint32_t flags) {
         // Narrow layers: the fits below do not hold (few row tiles, so the streaming kernel leans on K splits whose
         // partial sums and repeated activation staging grow with the batch).  Measured: with K = 5632, N = 2048 the
         // GEMM, sharing K between CTAs, takes 14-15 us at 24..64 rows where the streaming kernel takes 22-42 us;
-        // with K = 2048 the streaming kernel wins throughout.  So: from 17 rows on, when the streaming kernel
-        // would split K four ways or more and the layer has at least eight weight tiles.
+        // with K = 2048 the streaming kernel wins throughout.  So: from 17 rows on, when a fourth of K is what fits the
+        // streaming kernel's shared memory (K of 4992 and more) and the layer has at least eight weight tiles.
         // (with N = 1024 and K = 8192 the streaming kernel is still ahead at 17..32 rows, 14-15 us against 18 us,
         // and behind from 33 on, 24 us against 19 us)
-        if (M <= 16 || N < 1024 || K < 4096 || (N < 2048 && M <= 32)) return false;
-        return w4a16::choose_linear_config(M, N, K, w4a16::kMaxKSplits).k_splits >= 4;
+        return M > 16 && N >= 1024 && K >= 4992 && (N >= 2048 || M > 32);
     }
     const double padded = M <= 16 ? 16.0 : M <= 32 ? 32.0 : 64.0;
     const double giga_macs = padded * static_cast<double>(K) * static_cast<double>(N) * 1e-9;
@@ -120,7 +119,9 @@ size_t w4a16_linear_workspace_bytes_flags(int64_t M, int64_t N, int64_t K, uint3
     // (With weights in tensor memory a larger one, up to 39 MB, lets equal runs cut tiles; it does without.)
     if (routes_to_tcgen05(M, N, K, flags)) return w4a16::tcgen05_workspace_bytes(M, N, K);
     const w4a16_linear_config c = w4a16::choose_linear_config(M, N, K, w4a16::kMaxKSplits);
-    return w4a16::linear_workspace_bytes_for(M, N, c.k_splits);
+    // (A layer of few row tiles and long K may always be split, if only by w4a16_linear_f16_config.)
+    const bool may_split = N < 4096 && K >= 4096;
+    return w4a16::linear_workspace_bytes_for(M, N, may_split && c.k_splits < 2 ? 2 : c.k_splits);
 }
 
 size_t w4a16_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
@@ -171,7 +172,7 @@ int w4a16_linear_f16_bias(const void* x, const void* packed, const void* scales,
             }
         }
     }
-    w4a16_linear_config cfg = w4a16::choose_linear_config(M, N, K, max_splits);
+    w4a16_linear_config cfg = w4a16::choose_linear_config(M, N, K, max_splits, small_group);
     if (reinterpret_cast<uintptr_t>(scales) % 4 != 0) cfg.unroll = 1;
     const int launched =
         w4a16::launch_linear_mma(p, cfg, (flags & W4A16_FLAG_PROGRAMMATIC_LAUNCH) != 0, out_f32, s);

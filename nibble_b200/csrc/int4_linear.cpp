@@ -10,6 +10,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/library.h>
 
+#include <unistd.h>
+
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -22,9 +24,12 @@
 namespace {
 
 // Split-K scratch, one buffer per (device, stream) so calls on different streams never share it.
-// Allocated zero-filled on first use and kept for the life of the process; the first call on a
+// Allocated on first use, its counters zeroed, and kept for the life of the process; the first call on a
 // stream should therefore happen before that stream is captured into a CUDA graph.
 constexpr int64_t kWorkspaceBytes = 40 << 20;   // largest request: 38 MiB (the GEMM's parts, two of 256 x 128 sums for each of 148 CTAs)
+
+// The arrival counters of any problem whose scratch fits: the fixed 256 KB prefix, and then some.
+constexpr int64_t kCounterBytes = 1 << 20;
 
 at::Tensor& workspace_for(const at::Device& device, cudaStream_t stream) {
     static std::mutex mutex;
@@ -33,29 +38,39 @@ at::Tensor& workspace_for(const at::Device& device, cudaStream_t stream) {
     auto key = std::make_pair(static_cast<int>(device.index()), stream);
     auto it = cache->find(key);
     if (it == cache->end()) {
-        it = cache->emplace(key, at::zeros({kWorkspaceBytes}, at::TensorOptions().dtype(at::kByte).device(device))).first;
+        it = cache->emplace(key, at::empty({kWorkspaceBytes}, at::TensorOptions().dtype(at::kByte).device(device))).first;
+        it->second.narrow(0, 0, kCounterBytes).zero_();
     }
     return it->second;
 }
 
-// W4A16_ROWS_PER_WARP selects how many output rows one lane owns: 2 (one 16-row tile per warp) or
-// 4 (two tiles); 1 is accepted for compatibility and means 2.  Anything else is an error, as in
-// the reference (csrc/int4_linear_kernel.cu:481-491).
-int row_tiles_from_env() {
-    const char* choice = std::getenv("W4A16_ROWS_PER_WARP");
-    if (choice == nullptr) return 0;
-    const int rows = std::atoi(choice);
-    TORCH_CHECK(rows == 1 || rows == 2 || rows == 4, "W4A16_ROWS_PER_WARP must be 1, 2, or 4");
-    return rows == 4 ? 2 : 1;
-}
-
-uint32_t flags_from_env() {
+// The W4A16_* environment variables, read on every call (they may change between calls) in one pass over the environment.
+//   W4A16_ROWS_PER_WARP  how many output rows one lane owns: 2 (one 16-row tile per warp) or 4 (two tiles); 1 is accepted
+//                        for compatibility and means 2.  Anything else is an error, as in the reference
+//                        (csrc/int4_linear_kernel.cu:481-491).
+//   W4A16_DECODE         "generic" forces the generic kernel
+//   W4A16_PDL            "1": weights may be read before the kernel in front has finished
+struct EnvironmentChoices {
+    int row_tiles = 0;      // 0: not forced
     uint32_t flags = 0;
-    const char* decode = std::getenv("W4A16_DECODE");
-    if (decode != nullptr && std::strcmp(decode, "generic") == 0) flags |= W4A16_FLAG_FORCE_GENERIC;
-    const char* pdl = std::getenv("W4A16_PDL");
-    if (pdl != nullptr && std::strcmp(pdl, "1") == 0) flags |= W4A16_FLAG_PROGRAMMATIC_LAUNCH;
-    return flags;
+};
+EnvironmentChoices environment_choices() {
+    EnvironmentChoices choices;
+    for (char** entry = environ; entry != nullptr && *entry != nullptr; ++entry) {
+        const char* text = *entry;
+        if (text[0] != 'W' || std::strncmp(text, "W4A16_", 6) != 0) continue;
+        text += 6;
+        if (std::strncmp(text, "ROWS_PER_WARP=", 14) == 0) {
+            const int rows = std::atoi(text + 14);
+            TORCH_CHECK(rows == 1 || rows == 2 || rows == 4, "W4A16_ROWS_PER_WARP must be 1, 2, or 4");
+            choices.row_tiles = rows == 4 ? 2 : 1;
+        } else if (std::strcmp(text, "DECODE=generic") == 0) {
+            choices.flags |= W4A16_FLAG_FORCE_GENERIC;
+        } else if (std::strcmp(text, "PDL=1") == 0) {
+            choices.flags |= W4A16_FLAG_PROGRAMMATIC_LAUNCH;
+        }
+    }
+    return choices;
 }
 
 void check_status(int status, const char* what) {
@@ -107,8 +122,9 @@ at::Tensor linear_impl(const at::Tensor& activations, const at::Tensor& packed_w
     if (m == 0 || n == 0) return output;
 
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
-    const uint32_t flags = flags_from_env() | (out_f32 ? W4A16_FLAG_OUTPUT_F32 : 0u);
-    const int forced_tiles = row_tiles_from_env();
+    const EnvironmentChoices choices = environment_choices();
+    const uint32_t flags = choices.flags | (out_f32 ? W4A16_FLAG_OUTPUT_F32 : 0u);
+    const int forced_tiles = choices.row_tiles;
 
     void* workspace = nullptr;
     size_t workspace_bytes = 0;

@@ -42,7 +42,8 @@ size_t linear_counter_bytes(int64_t M, int64_t N);
 size_t linear_workspace_bytes_for(int64_t M, int64_t N, int splits);
 
 // Picks a launch shape for the tensor-core kernel.  `max_splits` caps k_splits (1 = no workspace).
-w4a16_linear_config choose_linear_config(int64_t M, int64_t N, int64_t K, int max_splits);
+// `small_group`: for scale groups below 128.
+w4a16_linear_config choose_linear_config(int64_t M, int64_t N, int64_t K, int max_splits, bool small_group = false);
 
 // Tensor-core path: requires is_stream_group(group) and 16-byte aligned x / packed (and scales, for groups below 128).  Returns a W4A16_* code.
 // `out_f32` makes y an FP32 [M, N] matrix (unrounded sums, for partial results that are added up).  `early_weights`:

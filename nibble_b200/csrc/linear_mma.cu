@@ -242,71 +242,121 @@ size_t linear_workspace_bytes_for(int64_t M, int64_t N, int splits) {
     return linear_counter_bytes(M, N) + static_cast<size_t>(splits) * M * N * sizeof(float);
 }
 
-w4a16_linear_config choose_linear_config(int64_t M, int64_t N, int64_t K, int max_splits) {
-    const int sms = 148;
-    w4a16_linear_config c;
-    const int nt = batch_tiles_for(M);
-    const int x_rows = x_rows_for(M);
-    const int64_t batch_blocks = (M + 8 * nt - 1) / (8 * nt);
-    const int chunks = static_cast<int>(K / kGroup);
-    const int64_t tiles16 = (N + 15) / 16;
+namespace {
 
-    c.row_tiles = 1;
-    c.unroll = chunks % 2 == 0 ? 2 : 1;
-    // Warps of a CTA that share one row tile: the fewest that still give about 12 streaming warps
-    // per SM (more only shortens each warp's share of a tile and multiplies the per-tile epilogue).
-    const int64_t want_warps = static_cast<int64_t>(sms) * 12;
-    int kw = 1;
-    while (kw < 8 && tiles16 * batch_blocks * kw < want_warps && chunks >= kw * 2 * c.unroll) kw *= 2;
-    // Single-row launches with at most ~3 row tiles per resident CTA: all eight warps on each tile.  In a
-    // chain of dependent layers the whole share of a CTA is then prefetched before its activations
-    // arrive, and what remains after the wait is at most three short steps per warp instead of four
-    // (measured inside a decode step: 2 us per launch on the fused gate/up layer; within 2 % either
-    // way for independent launches).
-    if (M == 1 && tiles16 <= 1024) {
-        while (kw < 8 && chunks >= kw * 2 * c.unroll) kw *= 2;
+// Launch shape of a single row.
+//   - Up to about three row tiles per resident CTA: all eight warps on each tile.  In a chain of dependent layers the whole share
+//     of a CTA is then prefetched before its activations arrive, and at most three short steps per warp remain after
+//     the wait (2 us per launch on a fused gate/up layer inside a decode step).
+//   - More tiles: as many warps per tile as leave each of them four steps (3072 -> 16000: two warps 8.5 us, eight 10.2;
+//     8192 -> 28672: eight 25.6, one 29.3).
+//   - An activation slice above 32 KB would crowd the copy ring out of shared memory at two CTAs per SM: K is split four ways, and
+//     the fewest warps that still give 12 streaming ones per SM share a tile (28672 -> 8192: 28.2 us, 30.5 split two ways).
+//   - Fewer tiles than a quarter of the SMs and K to spare: K is split until two CTAs per SM have work (16384 -> 512: 5.0 us, 6.6
+//     unsplit).  With 64 tiles unsplit is already faster (8192 -> 1024: 4.6 against 5.2 us).
+w4a16_linear_config choose_single_row(int64_t tiles, int chunks, int sms, int max_splits) {
+    w4a16_linear_config c{};
+    int kw = 1, splits = 1;
+    if (x_slice_bytes(1, chunks) > 32u * 1024 && max_splits > 1) {
+        splits = std::min(4, max_splits);
+        while (kw < 8 && tiles * kw * splits < static_cast<int64_t>(sms) * 12) kw *= 2;
+    } else if (tiles <= 6 * sms) {
+        while (kw < 8 && chunks >= kw * 4) kw *= 2;
+        while (4 * tiles <= sms && splits * 2 <= max_splits && tiles * splits * 2 <= 2 * sms && chunks >= splits * 32) splits *= 2;
+    } else {
+        while (kw < 8 && chunks >= kw * 16 + (kw == 1 ? 8 : 0)) kw *= 2;
     }
-    // Shapes measured on B200 where a different split of the same work is clearly faster (sweeps over
-    // every k_warps x k_splits combination; Llama-70B gate/up and down projections).
-    struct Tuned { int64_t n, k; int k_warps, k_splits; };
-    static const Tuned tuned[] = {
-        {28672, 8192, 8, 1},   // 1792 row tiles: eight warps per tile halve the quarter-full last wave
-        {8192, 28672, 1, 4},   // long K: split across CTAs so the activation slice stays small
+    c.k_warps = kw;
+    c.k_splits = splits;
+    return c;
+}
+
+// Launch shape of a batch: the cheapest by a model fitted to measurements (25 layers from 1024 x 1024 to 28672 -> 8192, batches of 2
+// to 64 rows, every k_warps x k_splits; the pick is on average within 2 % of the fastest).  What the model knows: a CTA's
+// start; the batch rows it stages; its steps, each as long as the step's own chain or the SM's issue slots allow,
+// whichever is longer; the end of a tile; the hand-over of a tile between CTAs that split its K.
+// (28672 -> 8192 at 13 rows: 95 -> 62 us against the rule it replaces; 11008 -> 4096 at 2 rows: 18.8 -> 10.7.)
+w4a16_linear_config choose_batch(int64_t M, int64_t tiles, int chunks, int unroll, int sms, int max_splits, bool small_group) {
+    struct Costs {   // us; steps of 256 K
+        double start, stage_per_kb, stage_per_8_rows, step_issue, step_chain, tile_end, split, split_per_row, split_per_cta;
     };
-    int tuned_splits = 0;
-    if (M <= 8) {
-        for (const Tuned& entry : tuned) {
-            if (entry.n == N && entry.k == K && entry.k_splits <= max_splits) {
-                kw = entry.k_warps;
-                tuned_splits = entry.k_splits;
+    static const Costs costs[3] = {{1.13, 0.0133, 2.19, 0.382, 0.672, 0.132, 5.34, 0.0021, 0.083},
+                                   {1.74, 0.0010, 2.09, 0.414, 0.488, 0.216, 2.52, 0.0006, 0.0},
+                                   {0.07, 0.0006, 1.67, 0.841, 0.306, 1.195, 1.10, 0.0031, 0.0}};
+    const int nt = batch_tiles_for(M), x_rows = x_rows_for(M);
+    const Costs& cost = costs[nt == 1 ? 0 : nt == 2 ? 1 : 2];
+    const int64_t batch_blocks = (M + 8 * nt - 1) / (8 * nt);
+    const int rows = static_cast<int>(std::min<int64_t>(M, 8 * nt));
+    const size_t slot = unroll == 1 ? 8192 : small_group ? 18432 : 16896;
+    const size_t reduction = static_cast<size_t>(nt) * 8192;
+    w4a16_linear_config best{};
+    double best_time = 1e30;
+    best.k_warps = 8;
+    best.k_splits = 1;
+    for (int splits = 1; splits <= std::min(max_splits, kMaxKSplits) && splits <= chunks; splits *= 2) {
+        const int per_split = ((chunks + splits - 1) / splits + unroll - 1) / unroll * unroll;
+        if ((splits - 1) * per_split >= chunks) break;                    // an empty split
+        const size_t slice = x_slice_bytes(x_rows, per_split);
+        // (smaller scale groups are built for two and eight warps)
+        for (int kw = small_group ? 2 : 1; kw <= 8; kw *= small_group ? 4 : 2) {
+            const size_t smem = kFlagBytes + (kw > 1 ? reduction : 0) + slice + 3 * slot;
+            if (smem > static_cast<size_t>(kSmemBudget)) continue;
+            const int per_sm = nt <= 2 && smem <= static_cast<size_t>(kSmemPerSm / 2 - 1024) ? 2 : 1;
+            const int64_t tile_ctas = (tiles * kw + 7) / 8;
+            const int64_t resident = std::max<int64_t>(1, static_cast<int64_t>(sms) * per_sm / (splits * batch_blocks));
+            const int64_t grid_x = std::min(tile_ctas, resident);
+            const int64_t ctas = grid_x * splits * batch_blocks;
+            const double rounds = static_cast<double>((tile_ctas + grid_x - 1) / grid_x);
+            const double active = static_cast<double>(std::min<int64_t>(per_sm, (ctas + sms - 1) / sms));
+            const double waves = static_cast<double>((ctas + static_cast<int64_t>(sms) * per_sm - 1) / (static_cast<int64_t>(sms) * per_sm));
+            const double steps = 0.5 * (((per_split + kw - 1) / kw + unroll - 1) / unroll * unroll);
+            double tile = steps * std::max(cost.step_chain, cost.step_issue * active) + cost.tile_end;
+            if (splits > 1) tile += cost.split + cost.split_per_row * rows * splits + cost.split_per_cta * splits;
+            const double time = waves * (cost.start + cost.stage_per_8_rows * rows / 8.0 +
+                                         cost.stage_per_kb * rows * per_split * 0.25 * active + rounds * tile);
+            if (time < best_time) {
+                best_time = time;
+                best.k_warps = kw;
+                best.k_splits = splits;
             }
         }
     }
-    c.k_warps = kw;
-    // Splitting K across CTAs costs a round trip through the workspace; do it when the row tiles
-    // alone cannot fill the machine ...
-    int splits = tuned_splits > 0 ? tuned_splits : 1;
-    if (M <= 32 && tuned_splits == 0) {
-        while (splits * 2 <= max_splits && splits * 2 <= kMaxKSplits &&
-               tiles16 * batch_blocks * kw * splits < want_warps && chunks >= splits * 2 * kw * 2 * c.unroll) {
-            splits *= 2;
-        }
+    // Nothing fits shared memory: the most splits, for the launch to refuse (and its caller to take another kernel).
+    if (best_time == 1e30) {
+        while (best.k_splits * 2 <= std::min(max_splits, kMaxKSplits) && chunks >= best.k_splits * 2) best.k_splits *= 2;
     }
-    // ... or, for the single-row case, when the activation slice would crowd the copy ring out of
-    // shared memory (two CTAs per SM want it at or below 32 KB) ...
-    if (M == 1 && tuned_splits == 0) {
-        while (x_slice_bytes(x_rows, (chunks + splits - 1) / splits) > 32u * 1024 && splits * 2 <= max_splits &&
-               splits * 2 <= kMaxKSplits && chunks >= splits * 2 * kw * c.unroll) {
-            splits *= 2;
-        }
+    return best;
+}
+
+}  // namespace
+
+w4a16_linear_config choose_linear_config(int64_t M, int64_t N, int64_t K, int max_splits, bool small_group) {
+    // A model calls with a few dozen shapes over and over: each thread keeps its recent answers.
+    struct Answer {
+        int64_t M = -1, N = 0, K = 0;
+        int max_splits = 0;
+        bool small_group = false;
+        w4a16_linear_config config{};
+    };
+    static thread_local Answer answers[64];
+    const uint64_t mixed = (static_cast<uint64_t>(M) * 31 + static_cast<uint64_t>(N)) * 0x9E3779B97F4A7C15ull ^
+                           (static_cast<uint64_t>(K) * 0xC2B2AE3D27D4EB4Full + static_cast<uint64_t>(max_splits * 2 + small_group));
+    Answer& answer = answers[mixed >> 58];
+    if (answer.M == M && answer.N == N && answer.K == K && answer.max_splits == max_splits &&
+        answer.small_group == small_group) {
+        return answer.config;
     }
-    // ... and always when the slice would not fit next to a three-slot ring at all.
-    while (x_slice_bytes(x_rows, (chunks + splits - 1) / splits) > static_cast<size_t>(kSmemBudget - 64 * 1024) &&
-           splits * 2 <= max_splits && splits * 2 <= kMaxKSplits && chunks >= splits * 2) {
-        splits *= 2;
-    }
-    c.k_splits = splits;
-    c.stages = 0;   // chosen at launch from the shared memory left over
+
+    const int sms = 148;
+    const int chunks = static_cast<int>(K / kGroup);
+    const int64_t tiles = (N + 15) / 16;
+    const int unroll = chunks % 2 == 0 ? 2 : 1;
+    w4a16_linear_config c = M == 1 ? choose_single_row(tiles, chunks, sms, max_splits)
+                                   : choose_batch(M, tiles, chunks, unroll, sms, max_splits, small_group);
+    c.row_tiles = 1;     // (two 16-row tiles per warp were never the fastest)
+    c.unroll = unroll;
+    c.stages = 0;        // chosen at launch from the shared memory left over
+    answer = {M, N, K, max_splits, small_group, c};
     return c;
 }
 
