@@ -320,6 +320,9 @@ w4a16_linear_config choose_batch(int64_t M, int64_t tiles, int chunks, int unrol
                 best.k_splits = splits;
             }
         }
+        // With three row tiles per SM the stream of weights is what bounds a batch of up to eight rows, which the model does not
+        // know: K is then split only as far as it takes to fit (28672 -> 8192, 8 rows: four ways 40 us, eight 43).
+        if (nt == 1 && tiles >= 3 * sms && best_time < 1e30) break;
     }
     // Nothing fits shared memory: the most splits, for the launch to refuse (and its caller to take another kernel).
     if (best_time == 1e30) {
