@@ -79,12 +79,14 @@ int launch_gemm(const w4a16::LinearProblem& p, cudaStream_t stream) {
 }  // namespace
 
 // Measured on 16 layers at 65 to 2048 rows: weights in tensor memory are faster up to 512 rows (8192 -> 28672: 128 rows 64 against
-// 88 us, 384 rows 167 against 219) and level or up to 15 % slower above, where 256-row batch tiles read x half as often.  A layer whose
+// 88 us, 384 rows 167 against 219), and up to 1024 on deep layers that are not wide (5632 -> 2048, 777 rows: 27 against 32 us);
+// elsewhere level or up to 15 % slower above 512, where 256-row batch tiles read x half as often.  A layer whose
 // 128-row tiles just fit one round of SMs has nothing to share, and with a short K the other kernel's shorter start shows
 // (1024 -> 12928, 128 rows: 12.1 against 11.1 us).
 bool w4a16::gemm_from_tensor_memory(int64_t M, int64_t N, int64_t K) {
     const int64_t tiles = (N + 127) / 128;
-    return M <= 512 && !(M <= 128 && K <= 1024 && tiles > 74 && tiles <= 148);
+    if (M > 512) return M <= 1024 && K >= 5120 && N * K <= (64 << 20);
+    return !(M <= 128 && K <= 1024 && tiles > 74 && tiles <= 148);
 }
 
 bool w4a16::linear_routes_to_tcgen05(int64_t M, int64_t N, int64_t K, uint32_t flags) {

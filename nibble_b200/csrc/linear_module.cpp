@@ -37,7 +37,9 @@ c10::TypedOperatorHandle<Signature> operator_handle(const char* name) {
 //     time: unbeaten above 1024 rows, and on mid-sized layers above 256 (2048 -> 5632, 512 rows: 17.7 against 20.5 us), but not on
 //     small ones, where the host sets the pace (1024 -> 1920, 89 rows: 15.8 against 9 us);
 //   - cuBLAS falls off its fast kernels where an output row is no multiple of 16 bytes (9216 -> 2575, 128 rows: 125 against 20 us);
-//   - from 513 rows on the operator has 256-row batch tiles, and is ahead only where the last one is nearly full
+//   - from 513 to 1024 rows the operator is ahead on deep layers that are not wide (one launch, and the FP16 weights are a large
+//     share of the work: 11008 -> 4096, 777 rows: 83 against 91 us) and on small ones (5120 -> 1000: 18 against 25); elsewhere it
+//     has 256-row batch tiles and is ahead only where the last one is nearly full
 //     (8192 -> 28672, 1024 rows: 451 against 494 us; 777 rows: 442 against 362).
 bool uses_fused_kernel(int64_t rows, int64_t out_features, int64_t in_features, int64_t group_size) {
     if (rows <= 64) return true;
@@ -48,6 +50,7 @@ bool uses_fused_kernel(int64_t rows, int64_t out_features, int64_t in_features, 
     const bool shallow = in_features < 1024 && out_features >= 8192;   // many tiles of a few K blocks each
     if (rows <= 256) return rows <= 128 || !shallow;
     if (rows <= 512) return weights <= 9 << 19 || (weights >= 32 << 20 && !shallow);
+    if (rows <= 1024 && in_features >= 5120 && (weights <= 6 << 20 || (in_features >= 8192 && weights <= 48 << 20))) return true;
     return group_size == 128 && rows <= 1024 && (256 - rows % 256) % 256 < 64 && weights >= 64 << 20;
 }
 

@@ -135,10 +135,11 @@ __device__ __forceinline__ uint32_t pack_codes(const float (&w)[8], float step, 
 // GROUP 128, 64 or 32 and 16-byte aligned weights: GROUP / 16 lanes share a group, a lane holds weights 8l..8l+7 of each half
 // of it, so both loads of the lanes are contiguous, and what a group costs once (two IEEE divisions, the shuffles) is
 // shared by 16 weights.  Bound: HBM at 2.5 bytes (FP16) or 4.5 (FP32) a weight, with about nine instructions a weight close behind.
-// 28672 x 8192 from FP16, 128-wide groups: 148 -> 115 us (5.1 TB/s);
-// from FP32 164 us (6.4 TB/s); with 64- and 32-wide groups, which read the weights twice before, 803 and 1406 -> 115 us.
+// 28672 x 8192 from FP16, 128-wide groups: 148 -> 109 us (5.4 TB/s);
+// from FP32 155 us (6.8 TB/s); with 64- and 32-wide groups, which read the weights twice before, 803 and 1406 -> 115 us.
+// Eight blocks per SM for FP16 (32 registers) and as many blocks as there are groups for FP32: 114 -> 109 us and 164 -> 155.
 template <typename T, int GROUP>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, sizeof(T) == 2 ? 8 : 6)
 quantize_pack_group_kernel(const T* __restrict__ weights, uint8_t* __restrict__ packed, __half* __restrict__ scales,
                            int64_t total_groups) {
     constexpr int kLanes = GROUP / 16;
@@ -176,7 +177,8 @@ int launch(const T* weights, uint8_t* packed, __half* scales, int64_t N, int64_t
     if ((group == 128 || group == 64 || group == 32) && reinterpret_cast<uintptr_t>(weights) % 16 == 0 &&
         reinterpret_cast<uintptr_t>(packed) % 4 == 0) {
         const int64_t groups_per_block = 256 / (group / 16);
-        const int64_t fast_blocks = std::min<int64_t>((total_groups + groups_per_block - 1) / groups_per_block, 148 * 64);
+        const int64_t fast_blocks = std::min<int64_t>((total_groups + groups_per_block - 1) / groups_per_block,
+                                                           sizeof(T) == 2 ? 148 * 64 : INT32_MAX);
         const auto kernel = group == 128 ? quantize_pack_group_kernel<T, 128>
                             : group == 64 ? quantize_pack_group_kernel<T, 64> : quantize_pack_group_kernel<T, 32>;
         kernel<<<static_cast<unsigned>(fast_blocks), 256, 0, stream>>>(weights, packed, scales, total_groups);
