@@ -273,7 +273,8 @@ int w4a16_linear_f16_input(const void* x, const void* packed, const void* scales
  *   scalar); applies RoPE (cos, sin of position * inv_freq[j], times rope_scale, rounded to FP16) to
  *   q and k, writes k and v into caches laid out [kv_heads][max_len][d], and writes
  *   softmax(q k^T * softmax_scale) v over positions 0..*position to out [q_heads*d].  d is 64 or
- *   128.  A position outside [0, max_len) sets *status to 1 and nothing is written.
+ *   128; both caches must be 16-byte aligned (qkv need not be).  A position outside [0, max_len) sets *status
+ *   to 1 and nothing is written.
  * flags: W4A16_FLAG_PROGRAMMATIC_LAUNCH as for the linear (each kernel waits for its predecessor before
  *   it reads or writes memory).  One exception, for latency: attention_decode reads *position, inv_freq and
  *   the cache rows below the position BEFORE that wait.  A programmatic chain only orders a kernel after its

@@ -388,7 +388,7 @@ int w4a16_attention_decode_f16(const void* qkv, void* k_cache, void* v_cache, vo
         inv_freq == nullptr || status == nullptr) {
         return W4A16_ERR_NULL_POINTER;
     }
-    if (reinterpret_cast<uintptr_t>(k_cache) % 4 != 0 || reinterpret_cast<uintptr_t>(v_cache) % 4 != 0) return W4A16_ERR_MISALIGNED;
+    if (!aligned16(k_cache) || !aligned16(v_cache)) return W4A16_ERR_MISALIGNED;    // rows are read 16 bytes at a time
     return w4a16::launch_attention_decode(static_cast<const __half*>(qkv), static_cast<__half*>(k_cache),
                                           static_cast<__half*>(v_cache), static_cast<__half*>(out),
                                           reinterpret_cast<const long long*>(position), inv_freq, q_heads, kv_heads, head_dim,

@@ -88,6 +88,18 @@ def test_workspace_size_query():
     assert lib.w4a16_linear_workspace_bytes_flags(128, 256, 2048, _native.FLAG_FORCE_TCGEN05) == 0    # K below 4096 is not shared
 
 
+def test_attention_refuses_caches_it_cannot_read_sixteen_bytes_at_a_time():
+    lib = _native.core()
+    before = lib.w4a16_launch_count()
+    one, odd = ctypes.c_void_p(16), ctypes.c_void_p(24)     # 8-byte aligned: enough for FP16 pairs, not for whole pieces of a row
+
+    def attention(k_cache, v_cache):
+        return lib.w4a16_attention_decode_f16(one, k_cache, v_cache, one, one, one, 8, 2, 64, 128, 1.0, 0.125, one, 0, None)
+
+    assert attention(odd, one) == -4 and attention(one, odd) == -4
+    assert lib.w4a16_launch_count() == before
+
+
 def test_missing_library_is_an_error(monkeypatch, tmp_path):
     monkeypatch.setattr(_native, "CORE_LIB", tmp_path / "absent.so")
     _native.core.cache_clear()
