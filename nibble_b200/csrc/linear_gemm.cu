@@ -37,9 +37,9 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include "kernels.h"
+#include "per_device.h"
 #include "tcgen05.cuh"
 #include "unpack.cuh"
 
@@ -701,22 +701,20 @@ int launch_linear_gemm(const LinearProblem& prob, cudaStream_t stream) {
                                            reinterpret_cast<const void*>(linear_gemm_kernel<64>),
                                            reinterpret_cast<const void*>(linear_gemm_kernel<32>)};
     constexpr int kSmem = 225 * 1024;
-    // SM count and resident clusters, learnt once per device
+    // SM count and resident clusters
     struct Device {
-        std::once_flag once;
-        int status = W4A16_OK, sms = 0;
+        int sms = 0;
         int clusters[kMaxCluster + 1] = {};
     };
-    static Device devices[64];
+    static PerDevice<Device> devices;
     int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return W4A16_ERR_LAUNCH;
-    Device& dev = devices[device];
-    std::call_once(dev.once, [&] {
-        dev.status = W4A16_ERR_LAUNCH;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices) return W4A16_ERR_LAUNCH;
+    const Device* dev = nullptr;
+    const int known = devices.get(device, [&](Device& d) -> int {
         for (const void* kernel : kernels) {
-            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) return;
+            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) return W4A16_ERR_LAUNCH;
         }
-        if (cudaDeviceGetAttribute(&dev.sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || dev.sms <= 0) return;
+        if (cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || d.sms <= 0) return W4A16_ERR_LAUNCH;
         for (int s = 2; s <= kMaxCluster; ++s) {
             cudaLaunchConfig_t shape = {};
             shape.gridDim = dim3(static_cast<unsigned>(s));
@@ -728,21 +726,21 @@ int launch_linear_gemm(const LinearProblem& prob, cudaStream_t stream) {
             attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
             shape.attrs = attr;
             shape.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&dev.clusters[s], kernels[0], &shape) != cudaSuccess) {
-                dev.clusters[s] = 0;
+            if (cudaOccupancyMaxActiveClusters(&d.clusters[s], kernels[0], &shape) != cudaSuccess) {
+                d.clusters[s] = 0;
                 (void)cudaGetLastError();
             }
         }
-        dev.status = W4A16_OK;
-    });
-    if (dev.status != W4A16_OK) return dev.status;
-    GemmPlan g = plan_gemm(prob.M, prob.N, prob.K, std::min(dev.sms, 148), dev.clusters);
+        return W4A16_OK;
+    }, &dev);
+    if (known != W4A16_OK) return known;
+    GemmPlan g = plan_gemm(prob.M, prob.N, prob.K, std::min(dev->sms, 148), dev->clusters);
     if (g.tiles * g.k_blocks > INT32_MAX) return W4A16_ERR_TOO_LARGE;
     const size_t counters = linear_counter_bytes(prob.M, prob.N);
     if (g.cut && (prob.workspace == nullptr || reinterpret_cast<uintptr_t>(prob.workspace) % 16 != 0 ||
                   prob.workspace_bytes < counters + gemm_partial_bytes(g))) {
         g.cut = false;
-        g.grid = static_cast<int>(std::min<long long>(dev.sms, g.tiles));
+        g.grid = static_cast<int>(std::min<long long>(dev->sms, g.tiles));
     }
     CUtensorMap x_map, w_map;
     if (!encode_rows(&x_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, prob.x, prob.M, prob.K * 2, 128, g.bn, CU_TENSOR_MAP_SWIZZLE_128B,

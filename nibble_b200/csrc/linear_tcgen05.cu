@@ -43,6 +43,7 @@
 #include <algorithm>
 
 #include "kernels.h"
+#include "per_device.h"
 #include "tcgen05.cuh"
 #include "unpack.cuh"
 
@@ -584,23 +585,21 @@ int launch_linear_tcgen05(const LinearProblem& prob, cudaStream_t stream) {
         {reinterpret_cast<const void*>(linear_tcgen05_kernel<1, false>), reinterpret_cast<const void*>(linear_tcgen05_kernel<1, true>)},
         {reinterpret_cast<const void*>(linear_tcgen05_kernel<2, false>), reinterpret_cast<const void*>(linear_tcgen05_kernel<2, true>)}};
     const void* kernel = kernels[sub_tiles - 1][prob.bias != nullptr];
-    // the shared-memory attribute and the SM count are kept per device
-    static int sm_count[64] = {};
+    static PerDevice<int> sm_counts;
     int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return W4A16_ERR_LAUNCH;
-    if (sm_count[device] == 0) {
-        int sms = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices) return W4A16_ERR_LAUNCH;
+    const int* sms = nullptr;
+    const int known = sm_counts.get(device, [&](int& count) -> int {
         for (int k = 0; k < 4; ++k) {
             if (cudaFuncSetAttribute(kernels[k >> 1][k & 1], cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimitTc) != cudaSuccess) {
                 return W4A16_ERR_LAUNCH;
             }
         }
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0) {
-            return W4A16_ERR_LAUNCH;
-        }
-        sm_count[device] = sms;
-    }
-    const int grid = static_cast<int>(std::min<int64_t>(params.total_tiles, sm_count[device]));
+        return cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && count > 0 ? W4A16_OK
+                                                                                                                   : W4A16_ERR_LAUNCH;
+    }, &sms);
+    if (known != W4A16_OK) return known;
+    const int grid = static_cast<int>(std::min<int64_t>(params.total_tiles, *sms));
     cudaLaunchConfig_t launch = {};
     launch.gridDim = dim3(static_cast<unsigned>(grid));
     launch.blockDim = dim3(kThreadsTc);
