@@ -4,6 +4,8 @@
 //   step  = amax(|w| over the group) / 7 in FP32, 1 for an all-zero group
 //   code  = clamp(round_half_even(w / step), -7, 7)        (FP32 IEEE division, rint)
 //   scale = half(step)                                     (rounded after the codes are made)
+// Weights that are not finite, whatever the group size: a NaN does not count for the maximum and gets code -7, the other weights
+// of its group their own codes; an infinity makes the scale infinite, its own code -7 and those of finite weights 0.
 // byte j of a row holds code 2j in its low nibble and code 2j+1 in its high nibble.
 //
 // Groups of 128, 64 and 32: quantize_pack_group_kernel below, weights read once.
@@ -103,28 +105,37 @@ struct Eight<float> {
     }
 };
 
+// The larger of two numbers; NaN if either is.
+__device__ __forceinline__ float max_or_nan(float a, float b) {
+    float m;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+    return m;
+}
+
 // Eight codes as one word.
 //
 // Fast route: t = w * (1/step) + 1.5 * 2^23 in one FMA rounds the exact product to the nearest even integer; r = t - 1.5 * 2^23
 // is that integer.  The product and the reference's fl(w / step) differ by a few ulp at most, so both round to the same
-// integer unless the quotient sits within 1e-4 of a tie k + 0.5; a lane that sees such a weight (about one in 600), or whose
-// 1/step is not finite, redoes its codes with the IEEE division.
+// integer unless the quotient sits within 1e-4 of a tie k + 0.5; a lane that sees such a weight (about one in 600) redoes its
+// codes with the IEEE division.
 //
 // Packing in floats: four codes are a number of at most 16 bits, r0 + 16 r1 + 256 r2 + 4096 r3 + 0x8888, exact in FP32 and read
-// off the mantissa after adding 2^23; the 8 added to each nibble is its sign bit flipped.
+// off the mantissa after adding 2^23; the 8 added to each nibble is its sign bit flipped.  A weight that is infinite or NaN, or
+// a 1/step that is infinite, would spoil all four codes; it makes its distance from r NaN, which the maximum passes on (fmaxf
+// would drop it), and the division gives each weight its own code.  (Looking at the packed sums
+// instead, 28672 x 8192 from FP16: 122 -> 126 us; this way no change.)
 __device__ __forceinline__ uint32_t pack_codes(const float (&w)[8], float step, float inv_step) {
     constexpr float kMagic = 12582912.0f;
     float r[8], off = 0.0f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         r[i] = fmaf(w[i], inv_step, kMagic) - kMagic;
-        off = fmaxf(off, fabsf(fmaf(w[i], inv_step, -r[i])));
+        off = max_or_nan(off, fabsf(fmaf(w[i], inv_step, -r[i])));
     }
-    float lo = fmaf(fmaf(fmaf(r[3], 16.0f, r[2]), 16.0f, r[1]), 16.0f, r[0]) + (8388608.0f + 34952.0f);
-    float hi = fmaf(fmaf(fmaf(r[7], 16.0f, r[6]), 16.0f, r[5]), 16.0f, r[4]) + (8388608.0f + 34952.0f);
+    const float lo = fmaf(fmaf(fmaf(r[3], 16.0f, r[2]), 16.0f, r[1]), 16.0f, r[0]) + (8388608.0f + 34952.0f);
+    const float hi = fmaf(fmaf(fmaf(r[7], 16.0f, r[6]), 16.0f, r[5]), 16.0f, r[4]) + (8388608.0f + 34952.0f);
     uint32_t word = __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x5410) ^ 0x88888888u;
-    // fmaxf drops a NaN, so infinity and NaN are looked for where they come from
-    if (off > 0.4999f || !(inv_step <= 3.0e38f)) {
+    if (!(off <= 0.4999f)) {
         word = 0;
 #pragma unroll
         for (int i = 0; i < 8; ++i) word |= code_of(w[i], step) << (4 * i);
@@ -152,7 +163,7 @@ quantize_pack_group_kernel(const T* __restrict__ weights, uint8_t* __restrict__ 
         const T* src = weights + (live ? g : total_groups - 1) * GROUP + l * 8;
         a.load(src);
         b.load(src + GROUP / 2);
-        float amax = fmaxf(a.amax(), b.amax());
+        float amax = fmaxf(fmaxf(a.amax(), b.amax()), 0.0f);     // 0 where every weight is NaN
 #pragma unroll
         for (int offset = kLanes / 2; offset > 0; offset >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, offset));
         const float step = amax == 0.0f ? 1.0f : __fdiv_rn(amax, 7.0f);

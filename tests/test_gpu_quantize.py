@@ -94,3 +94,27 @@ def test_near_tie_quotients_match_the_host_division():
     packed, scales = quantize_and_pack_cuda(w.cuda(), 128)
     want_packed, want_scales = _host(w, 128)
     assert torch.equal(packed.cpu(), want_packed) and torch.equal(scales.cpu(), want_scales)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("group", [128, 64, 32, 16, 6])
+def test_weights_that_are_not_finite_spoil_no_other_code(dtype, group):
+    """A NaN or an infinity in every position of a group in turn, several in one group, and groups of nothing else."""
+    rng = np.random.default_rng(group)
+    w = (rng.standard_normal((3 * group + 4, group)) * 0.02).astype(np.float32)
+    for i, value in enumerate((np.nan, np.inf, -np.inf)):
+        w[np.arange(group) + i * group, np.arange(group)] = value
+    w[-4] = np.nan
+    w[-3, ::2] = np.nan
+    w[-2, : group // 2], w[-2, -1] = np.nan, np.inf
+    w[-1] = np.where(rng.random(group) < 0.3, np.nan, 0.0)
+    w = torch.from_numpy(w).to(dtype)
+    exact = w.float().numpy()
+    with np.errstate(invalid="ignore"):
+        amax = np.fmax.reduce(np.abs(exact), axis=1, initial=0.0).astype(np.float32)
+        step = np.where(amax == 0, np.float32(1), amax / np.float32(7)).astype(np.float32)
+        codes = np.rint(exact / step[:, None])
+        codes = np.where(np.isnan(codes), -7, np.clip(codes, -7, 7)).astype(np.int8)
+    packed, scales = quantize_and_pack_cuda(w.cuda(), group)
+    assert np.array_equal(oracle.unpack_int4(packed.cpu().numpy()), codes)
+    assert np.array_equal(scales.cpu().numpy()[:, 0], step.astype(np.float16))
