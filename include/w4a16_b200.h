@@ -56,7 +56,10 @@ enum {
     /* Keep batches of 65 rows and more on the mma.sync kernel instead of the tcgen05 GEMM (A/B, tests). */
     W4A16_FLAG_NO_TCGEN05 = 1u << 3,
     /* Route to the tcgen05 GEMM whatever the batch size, when the fast path applies and y is FP16 (A/B, tests). */
-    W4A16_FLAG_FORCE_TCGEN05 = 1u << 4
+    W4A16_FLAG_FORCE_TCGEN05 = 1u << 4,
+    /* Weights may enter the product as half(code * scale) from 65 rows on with group_size 64 and 32 too (with 128 they do
+     * anyway): such batches then take the tcgen05 GEMM.  Without it their codes and scales stay exact. */
+    W4A16_FLAG_FP16_WEIGHTS = 1u << 5
 };
 
 /* Explicit launch shape of the fused tensor-core kernel; zero fields mean "choose for me". */
@@ -79,8 +82,9 @@ typedef struct w4a16_linear_config {
  * favours it) a tcgen05 GEMM whose producer warps dequantise into the operand tiles
  * (no FP16 weight matrix in memory; weights enter the product as half(code * scale), the arithmetic of
  * the reference's dequantise-then-matmul prefill route, w4a16/linear.py:132-152).
- * group_size 64 and 32 run the streaming kernel up to M = 64 and the GEMM above when K is a multiple of 128 and x, packed
- * and scales are 16-byte aligned.  Otherwise a generic kernel that accepts any even group_size and any alignment.
+ * group_size 64 and 32 run the streaming kernel (from 65 rows on in launches of 64 rows, or as the GEMM with
+ * W4A16_FLAG_FP16_WEIGHTS) when K is a multiple of 128 and x, packed and scales are 16-byte aligned.  Otherwise a generic kernel
+ * that accepts any even group_size and any alignment.
  * The GEMM shares the K of an output tile between CTAs when a layer has too few tiles for the SMs: inside a thread-block
  * cluster, or through FP32 partial sums in the workspace that are added in a fixed order and rounded once; without enough
  * workspace (up to 39 MB, more than the query below asks for) the second does not happen.

@@ -76,6 +76,40 @@ int launch_gemm(const w4a16::LinearProblem& p, cudaStream_t stream) {
     return tensor_memory ? w4a16::launch_linear_gemm(p, stream) : w4a16::launch_linear_tcgen05(p, stream);
 }
 
+// Whether a call with 64- or 32-wide groups goes to the GEMM, which rounds each weight to FP16.  Only where the caller has said
+// that this will do (as the module does, which dequantises to FP16 above 64 rows in any case): the operator's contract for these
+// groups is exact codes and FP32 scales whatever the batch.
+bool small_group_routes_to_gemm(int64_t M, uint32_t flags) {
+    if (flags & W4A16_FLAG_OUTPUT_F32) return false;
+    if (flags & W4A16_FLAG_FORCE_TCGEN05) return true;
+    return (flags & W4A16_FLAG_FP16_WEIGHTS) && !(flags & W4A16_FLAG_NO_TCGEN05) && M >= w4a16::kTcgen05MinRows;
+}
+
+// Batch rows of one launch where a larger batch of small groups streams: two passes of the kernel, side by side.
+constexpr int64_t kSmallGroupRows = 64;
+
+// The streaming kernel, with K split across CTAs only as far as the caller's workspace allows.
+int launch_streaming(const w4a16::LinearProblem& p, bool small_group, uint32_t flags, cudaStream_t stream) {
+    const bool out_f32 = (flags & W4A16_FLAG_OUTPUT_F32) != 0;
+    int max_splits = 1;
+    if (p.workspace != nullptr && aligned16(p.workspace)) {
+        for (int splits = w4a16::kMaxKSplits; splits > 1; splits >>= 1) {
+            if (p.workspace_bytes >= w4a16::linear_workspace_bytes_for(p.M, p.N, splits)) {
+                max_splits = splits;
+                break;
+            }
+        }
+    }
+    w4a16_linear_config cfg = w4a16::choose_linear_config(p.M, p.N, p.K, max_splits, small_group);
+    if (reinterpret_cast<uintptr_t>(p.scales) % 4 != 0) cfg.unroll = 1;
+    const int launched = w4a16::launch_linear_mma(p, cfg, (flags & W4A16_FLAG_PROGRAMMATIC_LAUNCH) != 0, out_f32, stream);
+    // Too much activation data for one CTA's shared memory and no workspace to split K further: the tcgen05 GEMM
+    // has no such limit (nor has the generic kernel, for FP32 output, small groups or when the GEMM is switched off).
+    if (launched != W4A16_ERR_WORKSPACE) return launched;
+    if (!out_f32 && !small_group && !(flags & W4A16_FLAG_NO_TCGEN05)) return launch_gemm(p, stream);
+    return w4a16::launch_linear_generic(p, out_f32, stream);
+}
+
 }  // namespace
 
 // Measured on 16 layers at 65 to 2048 rows: weights in tensor memory are faster up to 512 rows (8192 -> 28672: 128 rows 64 against
@@ -158,33 +192,20 @@ int w4a16_linear_f16_bias(const void* x, const void* packed, const void* scales,
     if ((flags & W4A16_FLAG_FORCE_GENERIC) || (!small_group && !fast_path_applies(x, packed, K, group_size))) {
         return w4a16::launch_linear_generic(p, out_f32, s);
     }
-    // Prefill-sized batches, and medium ones on large layers: dense enough for the tcgen05 tensor cores.  (Small groups only
-    // from 65 rows on: the streaming kernel does not round their weights, and no batch below has been rounded before.)
-    const bool to_gemm = small_group ? M >= w4a16::kTcgen05MinRows && !out_f32 && !(flags & W4A16_FLAG_NO_TCGEN05) ||
-                                           (flags & W4A16_FLAG_FORCE_TCGEN05) && !out_f32
-                                     : routes_to_tcgen05(M, N, K, flags);
-    if (to_gemm) return launch_gemm(p, s);
-    // Split K across CTAs only as far as the caller's workspace allows.
-    int max_splits = 1;
-    if (workspace != nullptr && aligned16(workspace)) {
-        for (int splits = w4a16::kMaxKSplits; splits > 1; splits >>= 1) {
-            if (workspace_bytes >= w4a16::linear_workspace_bytes_for(M, N, splits)) {
-                max_splits = splits;
-                break;
-            }
-        }
+    if (small_group ? small_group_routes_to_gemm(M, flags) : routes_to_tcgen05(M, N, K, flags)) return launch_gemm(p, s);
+    if (!small_group || M <= kSmallGroupRows) return launch_streaming(p, small_group, flags, s);
+    // Large batches of small groups whose weights may not be rounded: 64 rows after the other, each with the whole workspace to
+    // split K into.  (8192 x 8192, 64-wide groups, 65 / 512 rows: 110 / 766 us; the generic kernel 1585 / 11268; the GEMM, with
+    // rounded weights, 26 / 68.)
+    for (int64_t m = 0; m < M; m += kSmallGroupRows) {
+        w4a16::LinearProblem rows = p;
+        rows.x += m * K;
+        rows.y = static_cast<char*>(p.y) + static_cast<size_t>(m) * N * (out_f32 ? sizeof(float) : sizeof(__half));
+        rows.M = M - m < kSmallGroupRows ? M - m : kSmallGroupRows;
+        const int launched = launch_streaming(rows, small_group, flags, s);
+        if (launched != W4A16_OK) return launched;
     }
-    w4a16_linear_config cfg = w4a16::choose_linear_config(M, N, K, max_splits, small_group);
-    if (reinterpret_cast<uintptr_t>(scales) % 4 != 0) cfg.unroll = 1;
-    const int launched =
-        w4a16::launch_linear_mma(p, cfg, (flags & W4A16_FLAG_PROGRAMMATIC_LAUNCH) != 0, out_f32, s);
-    // Too much activation data for one CTA's shared memory and no workspace to split K further: the tcgen05 GEMM
-    // has no such limit (nor has the generic kernel, for FP32 output or when the GEMM is switched off).
-    if (launched == W4A16_ERR_WORKSPACE) {
-        if (!out_f32 && !small_group && !(flags & W4A16_FLAG_NO_TCGEN05)) return launch_gemm(p, s);
-        return w4a16::launch_linear_generic(p, out_f32, s);
-    }
-    return launched;
+    return W4A16_OK;
 }
 
 int w4a16_linear_f16_input(const void* x, const void* packed, const void* scales, void* y, int64_t M, int64_t N,

@@ -77,7 +77,7 @@ void check_status(int status, const char* what) {
     TORCH_CHECK(status == W4A16_OK, what, " failed: ", w4a16_status_string(status));
 }
 
-// `activations` is [..., K] when `any_rank`, else [M, K]; the result keeps its leading dimensions.
+// `activations` is [..., K] when `any_rank` (the module's call), else [M, K]; the result keeps its leading dimensions.
 at::Tensor linear_impl(const at::Tensor& activations, const at::Tensor& packed_weights, const at::Tensor& scales,
                        const at::Tensor* bias, int64_t group_size, bool out_f32, bool any_rank) {
     TORCH_CHECK(activations.is_cuda(), "activations must be a CUDA tensor");
@@ -123,7 +123,8 @@ at::Tensor linear_impl(const at::Tensor& activations, const at::Tensor& packed_w
 
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
     const EnvironmentChoices choices = environment_choices();
-    const uint32_t flags = choices.flags | (out_f32 ? W4A16_FLAG_OUTPUT_F32 : 0u);
+    // (the module's large batches are the product with dequantised FP16 weights, whichever kernel forms it)
+    const uint32_t flags = choices.flags | (out_f32 ? W4A16_FLAG_OUTPUT_F32 : 0u) | (any_rank ? W4A16_FLAG_FP16_WEIGHTS : 0u);
     const int forced_tiles = choices.row_tiles;
 
     void* workspace = nullptr;

@@ -123,8 +123,8 @@ def linear_cuda(
     """FP16 ``[M, K]`` x packed INT4 ``[N, K/2]`` -> FP16 ``[M, N]`` on the current CUDA stream.
 
     ``group_size == 128`` with 16-byte aligned activations and weights runs the fused tensor-core
-    kernel for every M, and so do 64 and 32 with K a multiple of 128; other even group sizes or misaligned tensors run the
-    generic kernel.
+    kernel for every M, and so do 64 and 32 with K a multiple of 128 (codes and scales stay exact whatever the batch);
+    other even group sizes or misaligned tensors run the generic kernel.
     Invalid arguments raise ``RuntimeError``.
     """
     _require_extension()

@@ -299,3 +299,24 @@ def test_small_scale_groups_stream(k, n, gs):
     # scales that are not 16-byte aligned take the generic kernel
     shifted = torch.empty((scales.numel() + 1,), dtype=torch.float16, device="cuda")[1:].view_as(scales).copy_(scales)
     check_against_oracle(linear_cuda(x[:3], packed, shifted, gs), x[:3], packed, shifted, gs)
+
+
+@pytest.mark.parametrize("gs", [64, 32])
+@pytest.mark.parametrize(("m", "k", "n"), [(64, 128, 40), (65, 128, 40), (130, 4096, 24), (200, 1152, 17), (65, 8192, 130)])
+def test_small_scale_groups_keep_exact_weights_whatever_the_batch(m, k, n, gs):
+    """Half of each chunk is 5 s * 4, half 4 s * -5 with s = 1 + 2^-10: every partial sum is exact in FP32 and the total 0.  As
+    FP16 weights, 5 s rounds down to 5 + 2^-8 (4 s is exact) and the total is -1/4 per chunk."""
+    five_then_four = torch.cat([torch.full((32,), 0x55), torch.full((32,), 0x44)]).to(torch.uint8).repeat(k // 128)
+    packed = five_then_four.repeat(n, 1).cuda()
+    scales = torch.full((n, k // gs), 1.0 + 2.0 ** -10, dtype=torch.float16, device="cuda")
+    x = torch.cat([torch.full((64,), 4.0), torch.full((64,), -5.0)]).half().repeat(k // 128).repeat(m, 1).cuda()
+    zero = torch.zeros((m, n), dtype=torch.float16, device="cuda")
+    assert torch.equal(linear_cuda(x, packed, scales, gs), zero)
+    assert torch.equal(torch.ops.w4a16.linear(x, packed, scales, gs), zero)
+    assert torch.equal(capi_linear(x, packed, scales, gs), zero)
+    assert torch.equal(capi_linear(x, packed, scales, gs, workspace=new_workspace(m, n, k)), zero)
+    assert torch.equal(torch.ops.w4a16.linear_partial(x, packed, scales, gs), zero.float())
+    rounded = capi_linear(x, packed, scales, gs, flags=_native.FLAG_FP16_WEIGHTS)     # what the module's large batches are
+    assert torch.equal(rounded, zero if m <= 64 else torch.full_like(zero, -0.25 * (k // 128)))
+    bias = torch.arange(n, dtype=torch.float16, device="cuda")
+    assert torch.equal(torch.ops.w4a16.linear_bias(x, packed, scales, bias, gs), rounded + bias)
