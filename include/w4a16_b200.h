@@ -87,7 +87,7 @@ typedef struct w4a16_linear_config {
  * that accepts any even group_size and any alignment.
  * The GEMM shares the K of an output tile between CTAs when a layer has too few tiles for the SMs: inside a thread-block
  * cluster, or through FP32 partial sums in the workspace that are added in a fixed order and rounded once; without enough
- * workspace (up to 39 MB, more than the query below asks for) the second does not happen.
+ * workspace (up to 39 MB; w4a16_linear_scratch_bytes says how much) the second does not happen.
  * `workspace` may be NULL (then K is never split across CTAs); if given it must be 16-byte aligned,
  * hold at least w4a16_linear_workspace_bytes(M, N, K) bytes, be zero-filled before its first use
  * and not be shared by calls that may run concurrently.  The library leaves it ready for re-use, by calls
@@ -116,13 +116,16 @@ int w4a16_linear_f16_config(const void* x, const void* packed, const void* scale
                             uint32_t flags, const w4a16_linear_config* config,
                             w4a16_stream_t stream);
 
-/* Bytes of workspace that let w4a16_linear_f16 split K across CTAs for this problem
- * (FP32 partial sums plus arrival counters).  Never fails; returns 0 for empty problems. */
+/* Bytes of workspace with which K can be split across CTAs for this problem (FP32 partial sums plus arrival counters), by
+ * w4a16_linear_f16 or by an explicit launch shape: an allocation that serves a layer.  Never fails; returns 0 for empty problems. */
 size_t w4a16_linear_workspace_bytes(int64_t M, int64_t N, int64_t K);
 /* The same for a call made with `flags`: batches that w4a16_linear_f16 sends to the tcgen05 GEMM
  * (M >= 65 without W4A16_FLAG_OUTPUT_F32 / W4A16_FLAG_NO_TCGEN05) or to the generic kernel need none.
  * w4a16_linear_workspace_bytes(M, N, K) is this function with flags == 0. */
 size_t w4a16_linear_workspace_bytes_flags(int64_t M, int64_t N, int64_t K, uint32_t flags);
+/* Exactly what w4a16_linear_f16 uses of a workspace for this call (aligned pointers) on the current device: 0 when nothing is
+ * shared through one, so that none need be passed; with fewer bytes it shares less, with more it does the same. */
+size_t w4a16_linear_scratch_bytes(int64_t M, int64_t N, int64_t K, int64_t group_size, uint32_t flags);
 
 /*
  * Tensor-parallel exchange (no counterpart in the reference, which is single-GPU).  A layer sharded over

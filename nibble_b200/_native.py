@@ -102,6 +102,7 @@ C_API = {
     ),
     "w4a16_linear_workspace_bytes": (ctypes.c_size_t, [_I, _I, _I]),
     "w4a16_linear_workspace_bytes_flags": (ctypes.c_size_t, [_I, _I, _I, ctypes.c_uint32]),
+    "w4a16_linear_scratch_bytes": (ctypes.c_size_t, [_I, _I, _I, _I, ctypes.c_uint32]),
     "w4a16_linear_f16_static_scratch": (ctypes.c_int, [_P, _P, _P, _P, _I, _I, _I, _I, ctypes.c_uint32, _P]),
     "w4a16_static_scratch_bytes": (ctypes.c_size_t, []),
     "w4a16_linear_f16_peers": (

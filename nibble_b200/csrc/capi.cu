@@ -164,6 +164,23 @@ size_t w4a16_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
     return w4a16_linear_workspace_bytes_flags(M, N, K, 0);
 }
 
+size_t w4a16_linear_scratch_bytes(int64_t M, int64_t N, int64_t K, int64_t group_size, uint32_t flags) {
+    if (M <= 0 || N <= 0 || K <= 0 || K % w4a16::kGroupFast != 0 || !w4a16::is_stream_group(group_size)) return 0;
+    if (flags & W4A16_FLAG_FORCE_GENERIC) return 0;
+    const bool small_group = group_size != w4a16::kGroupFast;
+    if (small_group ? small_group_routes_to_gemm(M, flags) : routes_to_tcgen05(M, N, K, flags)) {
+        return small_group || w4a16::gemm_from_tensor_memory(M, N, K) ? w4a16::gemm_scratch_bytes(M, N, K)
+                                                                      : w4a16::tcgen05_workspace_bytes(M, N, K);
+    }
+    auto streaming = [&](int64_t rows) {
+        return w4a16::linear_workspace_bytes_for(
+            rows, N, w4a16::choose_linear_config(rows, N, K, w4a16::kMaxKSplits, small_group).k_splits);
+    };
+    if (!small_group || M <= kSmallGroupRows) return streaming(M);
+    const size_t whole = streaming(kSmallGroupRows), rest = M % kSmallGroupRows > 0 ? streaming(M % kSmallGroupRows) : 0;
+    return whole > rest ? whole : rest;
+}
+
 int w4a16_linear_f16(const void* x, const void* packed, const void* scales, void* y, int64_t M, int64_t N,
                      int64_t K, int64_t group_size, void* workspace, size_t workspace_bytes, uint32_t flags,
                      w4a16_stream_t stream) {

@@ -12,6 +12,7 @@
 
 #include <unistd.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -23,25 +24,28 @@
 
 namespace {
 
-// Split-K scratch, one buffer per (device, stream) so calls on different streams never share it.
-// Allocated on first use, its counters zeroed, and kept for the life of the process; the first call on a
-// stream should therefore happen before that stream is captured into a CUDA graph.
-constexpr int64_t kWorkspaceBytes = 40 << 20;   // largest request: 38 MiB (the GEMM's parts, two of 256 x 128 sums for each of 148 CTAs)
+// Scratch of calls that share K between CTAs, one buffer per (device, stream) so that calls on different streams never share it.
+// Allocated by the first such call on a stream, its counters zeroed, and kept: the kernels leave the counters at zero.  A call
+// that needs more replaces it; the caching allocator hands the old one out again on the same stream only, behind the calls that
+// used it.
+constexpr int64_t kWorkspaceBytes = 40 << 20;   // the most: 38 MiB are the GEMM's parts, two of 256 x 128 sums for each of 148 CTAs
 
 // The arrival counters of any problem whose scratch fits: the fixed 256 KB prefix, and then some.
 constexpr int64_t kCounterBytes = 1 << 20;
 
-at::Tensor& workspace_for(const at::Device& device, cudaStream_t stream) {
+at::Tensor workspace_for(const at::Device& device, cudaStream_t stream, int64_t bytes) {
     static std::mutex mutex;
     static auto* cache = new std::map<std::pair<int, cudaStream_t>, at::Tensor>();
     std::lock_guard<std::mutex> lock(mutex);
-    auto key = std::make_pair(static_cast<int>(device.index()), stream);
-    auto it = cache->find(key);
-    if (it == cache->end()) {
-        it = cache->emplace(key, at::empty({kWorkspaceBytes}, at::TensorOptions().dtype(at::kByte).device(device))).first;
-        it->second.narrow(0, 0, kCounterBytes).zero_();
+    at::Tensor& kept = (*cache)[std::make_pair(static_cast<int>(device.index()), stream)];
+    if (!kept.defined() || kept.numel() < bytes) {
+        int64_t size = 1 << 20;
+        while (size < bytes) size *= 2;
+        kept = at::Tensor();
+        kept = at::detail::empty_cuda({std::min(size, kWorkspaceBytes)}, at::kByte, device, c10::nullopt);
+        C10_CUDA_CHECK(cudaMemsetAsync(kept.data_ptr(), 0, static_cast<size_t>(std::min<int64_t>(kept.numel(), kCounterBytes)), stream));
     }
-    return it->second;
+    return kept;
 }
 
 // The W4A16_* environment variables, read on every call (they may change between calls) in one pass over the environment.
@@ -127,14 +131,14 @@ at::Tensor linear_impl(const at::Tensor& activations, const at::Tensor& packed_w
     const uint32_t flags = choices.flags | (out_f32 ? W4A16_FLAG_OUTPUT_F32 : 0u) | (any_rank ? W4A16_FLAG_FP16_WEIGHTS : 0u);
     const int forced_tiles = choices.row_tiles;
 
+    at::Tensor scratch;      // held until the call is enqueued, whatever other threads do with the stream's buffer
     void* workspace = nullptr;
     size_t workspace_bytes = 0;
-    // From nine rows on the GEMM may run, which uses as much as there is.  (The query answers for 128-wide groups.)
-    const size_t wanted = m > 8 && !out_f32 ? static_cast<size_t>(kWorkspaceBytes) : w4a16_linear_workspace_bytes_flags(m, n, k, flags);
-    if (wanted > 0 && wanted <= static_cast<size_t>(kWorkspaceBytes)) {
-        at::Tensor& ws = workspace_for(activations.device(), stream);
-        workspace = ws.data_ptr();
-        workspace_bytes = static_cast<size_t>(ws.numel());
+    const size_t wanted = w4a16_linear_scratch_bytes(m, n, k, group_size, flags);
+    if (wanted > 0) {
+        scratch = workspace_for(activations.device(), stream, std::min<int64_t>(static_cast<int64_t>(wanted), kWorkspaceBytes));
+        workspace = scratch.data_ptr();
+        workspace_bytes = static_cast<size_t>(scratch.numel());
     }
 
     int status;

@@ -58,6 +58,8 @@ int read_bounds_check(unsigned* site, unsigned* count);
 int launch_linear_tcgen05(const LinearProblem& p, cudaStream_t stream);
 // The same with the weights in tensor memory (linear_gemm.cu); groups of 64 and 32 too, aligned x / packed.
 int launch_linear_gemm(const LinearProblem& p, cudaStream_t stream);
+// Bytes of workspace that launch_linear_gemm uses on the current device: counters and parts of tiles that equal runs cut, or 0.
+size_t gemm_scratch_bytes(int64_t M, int64_t N, int64_t K);
 // Which of the two takes a call with 128-wide groups.
 bool gemm_from_tensor_memory(int64_t M, int64_t N, int64_t K);
 // Status word of these kernels (non-zero: a bounded barrier wait gave up); reading clears it and synchronises.

@@ -689,7 +689,71 @@ GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, const int* clusters
 // At most 38 MB: two parts of 256 x 128 sums for each SM.
 size_t gemm_partial_bytes(const GemmPlan& g) { return g.cut ? static_cast<size_t>(g.grid) * 2 * kRows * g.bn * sizeof(float) : 0; }
 
+constexpr int kSmem = 225 * 1024;
+
+const void* gemm_kernel(int64_t group) {
+    static const void* const kernels[3] = {reinterpret_cast<const void*>(linear_gemm_kernel<128>),
+                                           reinterpret_cast<const void*>(linear_gemm_kernel<64>),
+                                           reinterpret_cast<const void*>(linear_gemm_kernel<32>)};
+    return kernels[group == 128 ? 0 : group == 64 ? 1 : 2];
+}
+
+// SM count and resident clusters of each size.  As initialised: a B200.
+struct GemmDevice {
+    int sms = 148;
+    int clusters[kMaxCluster + 1] = {0, 0, 74, 45, 33, 26, 22, 15, 15};
+};
+
+int learn_device(int device, GemmDevice& d) {
+    for (const int group : {128, 64, 32}) {
+        if (cudaFuncSetAttribute(gemm_kernel(group), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) {
+            return W4A16_ERR_LAUNCH;
+        }
+    }
+    if (cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || d.sms <= 0) return W4A16_ERR_LAUNCH;
+    for (int s = 2; s <= kMaxCluster; ++s) {
+        cudaLaunchConfig_t shape = {};
+        shape.gridDim = dim3(static_cast<unsigned>(s));
+        shape.blockDim = dim3(kGemmThreads);
+        shape.dynamicSmemBytes = kSmem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = static_cast<unsigned>(s);
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        shape.attrs = attr;
+        shape.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&d.clusters[s], gemm_kernel(128), &shape) != cudaSuccess) {
+            d.clusters[s] = 0;
+            (void)cudaGetLastError();
+        }
+    }
+    return W4A16_OK;
+}
+
+int current_device(const GemmDevice** dev) {
+    static PerDevice<GemmDevice> devices;
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices) return W4A16_ERR_LAUNCH;
+    return devices.get(device, [device](GemmDevice& d) { return learn_device(device, d); }, dev);
+}
+
+GemmPlan plan_on(const GemmDevice& dev, int64_t M, int64_t N, int64_t K) {
+    return plan_gemm(M, N, K, std::min(dev.sms, 148), dev.clusters);
+}
+
 }  // namespace
+
+size_t gemm_scratch_bytes(int64_t M, int64_t N, int64_t K) {
+    if (M > INT32_MAX || N > INT32_MAX || K > INT32_MAX) return 0;
+    static const GemmDevice b200;
+    const GemmDevice* dev = nullptr;
+    if (current_device(&dev) != W4A16_OK) {            // asked where there is no device: the answer for a B200
+        (void)cudaGetLastError();
+        dev = &b200;
+    }
+    const GemmPlan g = plan_on(*dev, M, N, K);
+    return g.cut ? linear_counter_bytes(M, N) + gemm_partial_bytes(g) : 0;
+}
 
 int launch_linear_gemm(const LinearProblem& prob, cudaStream_t stream) {
     if (prob.K % kBlockK != 0 || prob.K <= 0 || !is_stream_group(prob.group)) return W4A16_ERR_BAD_CONFIG;
@@ -697,44 +761,10 @@ int launch_linear_gemm(const LinearProblem& prob, cudaStream_t stream) {
     if (reinterpret_cast<uintptr_t>(prob.x) % 16 != 0 || reinterpret_cast<uintptr_t>(prob.packed) % 16 != 0) {
         return W4A16_ERR_MISALIGNED;
     }
-    static const void* const kernels[3] = {reinterpret_cast<const void*>(linear_gemm_kernel<128>),
-                                           reinterpret_cast<const void*>(linear_gemm_kernel<64>),
-                                           reinterpret_cast<const void*>(linear_gemm_kernel<32>)};
-    constexpr int kSmem = 225 * 1024;
-    // SM count and resident clusters
-    struct Device {
-        int sms = 0;
-        int clusters[kMaxCluster + 1] = {};
-    };
-    static PerDevice<Device> devices;
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices) return W4A16_ERR_LAUNCH;
-    const Device* dev = nullptr;
-    const int known = devices.get(device, [&](Device& d) -> int {
-        for (const void* kernel : kernels) {
-            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) return W4A16_ERR_LAUNCH;
-        }
-        if (cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || d.sms <= 0) return W4A16_ERR_LAUNCH;
-        for (int s = 2; s <= kMaxCluster; ++s) {
-            cudaLaunchConfig_t shape = {};
-            shape.gridDim = dim3(static_cast<unsigned>(s));
-            shape.blockDim = dim3(kGemmThreads);
-            shape.dynamicSmemBytes = kSmem;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = static_cast<unsigned>(s);
-            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-            shape.attrs = attr;
-            shape.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&d.clusters[s], kernels[0], &shape) != cudaSuccess) {
-                d.clusters[s] = 0;
-                (void)cudaGetLastError();
-            }
-        }
-        return W4A16_OK;
-    }, &dev);
+    const GemmDevice* dev = nullptr;
+    const int known = current_device(&dev);
     if (known != W4A16_OK) return known;
-    GemmPlan g = plan_gemm(prob.M, prob.N, prob.K, std::min(dev->sms, 148), dev->clusters);
+    GemmPlan g = plan_on(*dev, prob.M, prob.N, prob.K);
     if (g.tiles * g.k_blocks > INT32_MAX) return W4A16_ERR_TOO_LARGE;
     const size_t counters = linear_counter_bytes(prob.M, prob.N);
     if (g.cut && (prob.workspace == nullptr || reinterpret_cast<uintptr_t>(prob.workspace) % 16 != 0 ||
@@ -773,7 +803,7 @@ int launch_linear_gemm(const LinearProblem& prob, cudaStream_t stream) {
     params.tiles = static_cast<int>(g.tiles);
     params.units = static_cast<int>(g.tiles) * g.k_blocks;
 
-    const void* kernel = kernels[prob.group == 128 ? 0 : prob.group == 64 ? 1 : 2];
+    const void* kernel = gemm_kernel(prob.group);
     cudaLaunchConfig_t launch = {};
     launch.gridDim = dim3(static_cast<unsigned>(g.cluster > 1 ? g.tiles * g.cluster : g.grid));
     launch.blockDim = dim3(kGemmThreads);

@@ -71,9 +71,8 @@ int w4a16_linear_f16_static_scratch(const void* x, const void* packed, const voi
     if (!fast || (flags & W4A16_FLAG_FORCE_GENERIC)) {
         return w4a16_linear_f16(x, packed, scales, y, M, N, K, group_size, nullptr, 0, flags, stream);
     }
-    // The split the library wants for this problem, on the route this call will take, decides how
-    // much scratch is needed (none when the batch goes to the tcgen05 GEMM).
-    const size_t needed = w4a16_linear_workspace_bytes_flags(M, N, K, flags);
+    // What the call will share through scratch, on the route it will take (most calls: nothing).
+    const size_t needed = w4a16_linear_scratch_bytes(M, N, K, group_size, flags);
     if (needed > kStaticScratchBytes) {
         // the GEMM runs without scratch too (K not split across CTAs); the streaming kernel's split is not optional
         if (w4a16::linear_routes_to_tcgen05(M, N, K, flags)) {

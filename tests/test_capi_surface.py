@@ -88,6 +88,34 @@ def test_workspace_size_query():
     assert lib.w4a16_linear_workspace_bytes_flags(128, 256, 2048, _native.FLAG_FORCE_TCGEN05) == 0    # K below 4096 is not shared
 
 
+def test_scratch_query_names_only_what_the_call_uses():
+    """The exact query: 0 for calls that share nothing through memory, the parts of their tiles for those that do (without a
+    device, the answers for a B200)."""
+    lib = _native.core()
+    scratch = lib.w4a16_linear_scratch_bytes
+    counters = 256 * 1024
+    # one row: split only where the activations or the few row tiles ask for it
+    for n, k in ((2048, 2048), (2048, 5632), (1024, 8192), (28672, 8192), (4096, 14336)):
+        assert scratch(1, n, k, 128, 0) == 0
+    assert scratch(1, 8192, 28672, 128, 0) == counters + 4 * 8192 * 4
+    assert scratch(1, 512, 16384, 128, 0) > 0 and scratch(1, 512, 16384, 64, 0) > 0
+    # the GEMM: clusters and whole tiles use none, equal runs two parts of 256 x batch sums for each SM
+    assert scratch(48, 8192, 8192, 128, 0) == 0
+    assert scratch(128, 28672, 8192, 128, 0) == counters + 148 * 2 * 256 * 128 * 4
+    assert scratch(512, 8192, 8192, 128, 0) == 0
+    # groups of 64 and 32: launches of at most 64 rows, unless the weights may be rounded
+    assert scratch(512, 8192, 8192, 64, 0) == scratch(64, 8192, 8192, 64, 0) > 0
+    assert scratch(128, 28672, 8192, 32, _native.FLAG_FP16_WEIGHTS) == scratch(128, 28672, 8192, 128, 0)
+    # nothing for the generic kernel, other groups, empty or invalid problems
+    assert scratch(1, 8192, 28672, 128, _native.FLAG_FORCE_GENERIC) == 0
+    assert scratch(1, 8192, 28672, 256, 0) == scratch(1, 8192, 28688, 16, 0) == 0
+    assert scratch(0, 8, 128, 128, 0) == scratch(4, 0, 128, 128, 0) == scratch(-1, 8, 128, 128, 0) == scratch(1, 8, 100, 128, 0) == 0
+    # never more than the query that an allocation for a layer goes by, where that one is asked about the same route
+    for m in (1, 2, 8, 16):
+        for n, k in ((256, 2048), (1024, 8192), (8192, 28672), (11008, 4096)):
+            assert scratch(m, n, k, 128, _native.FLAG_NO_TCGEN05) <= lib.w4a16_linear_workspace_bytes_flags(m, n, k, _native.FLAG_NO_TCGEN05)
+
+
 def test_attention_refuses_caches_it_cannot_read_sixteen_bytes_at_a_time():
     lib = _native.core()
     before = lib.w4a16_launch_count()

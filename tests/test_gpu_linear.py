@@ -320,3 +320,33 @@ def test_small_scale_groups_keep_exact_weights_whatever_the_batch(m, k, n, gs):
     assert torch.equal(rounded, zero if m <= 64 else torch.full_like(zero, -0.25 * (k // 128)))
     bias = torch.arange(n, dtype=torch.float16, device="cuda")
     assert torch.equal(torch.ops.w4a16.linear_bias(x, packed, scales, bias, gs), rounded + bias)
+
+
+def test_operator_takes_no_more_scratch_than_the_call_uses():
+    """On a stream of its own: calls that share no tile through memory allocate nothing beside their output, whatever the
+    batch; one that does keeps a buffer of its own size, not of the largest there is."""
+    lib = _native.core()
+    plain = [(1, 5632, 2048), (1, 8192, 1024), (48, 8192, 8192), (13, 4864, 5003), (128, 2048, 5632), (100, 8192, 1024)]
+    split = (1, 28672, 8192)
+    data = {}
+    for m, k, n in plain + [split]:
+        packed = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda")
+        scales = torch.full((n, k // 128), 0.01, dtype=torch.float16, device="cuda")
+        data[(m, k, n)] = (torch.randn((m, k), device="cuda").half(), packed, scales)
+        linear_cuda(*data[(m, k, n)], 128)               # first launches (module loading) out of the way
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        for case in plain:
+            assert lib.w4a16_linear_scratch_bytes(case[0], case[2], case[1], 128, 0) == 0
+            before = torch.cuda.memory_allocated()
+            y = linear_cuda(*data[case], 128)
+            torch.cuda.synchronize()
+            del y
+            assert torch.cuda.memory_allocated() == before, case
+        before = torch.cuda.memory_allocated()
+        for _ in range(3):
+            linear_cuda(*data[split], 128)
+        torch.cuda.synchronize()
+        kept = torch.cuda.memory_allocated() - before
+        need = lib.w4a16_linear_scratch_bytes(split[0], split[2], split[1], 128, 0)
+        assert need <= kept <= 2 << 20

@@ -197,3 +197,26 @@ def test_gemm_from_tensor_memory(m, k, n, gs):
         assert torch.equal(y, capi_linear(x, packed, scales, gs, workspace=workspace, flags=_native.FLAG_FORCE_TCGEN05))
     assert int(ws[: 256 * 1024].sum()) == 0
     assert _device_status() == 0, "a barrier wait gave up"
+
+
+@pytest.mark.parametrize(("m", "k", "n", "gs"), [(128, 8192, 28672, 128), (40, 8192, 28672, 128), (100, 5632, 12345, 128),
+                                                 (128, 8192, 28672, 64)])
+def test_scratch_query_is_exact_for_equal_runs(m, k, n, gs):
+    """With the bytes the query names the GEMM does what it does with any more; with one less, what it does without."""
+    lib = _native.core()
+    flags = _native.FLAG_FP16_WEIGHTS
+    need = lib.w4a16_linear_scratch_bytes(m, n, k, gs, flags)
+    assert need > 256 * 1024
+    torch.manual_seed(m + n)
+    packed = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda")
+    scales = (torch.rand((n, k // gs), device="cuda") * 0.01 + 1e-3).half()
+    x = torch.randn((m, k), device="cuda").half()
+
+    def run(size):
+        workspace = None if size is None else torch.zeros(size, dtype=torch.uint8, device="cuda")
+        return capi_linear(x, packed, scales, gs, workspace=workspace, flags=flags)
+
+    shared, whole = run(need), run(None)
+    assert torch.equal(run(40 << 20), shared) and torch.equal(run(need - 1), whole)
+    torch.testing.assert_close(shared, whole, rtol=2e-3, atol=2e-3)
+    assert _device_status() == 0
