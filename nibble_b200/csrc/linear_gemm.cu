@@ -463,6 +463,9 @@ linear_gemm_kernel(const GemmParams p, const __grid_constant__ CUtensorMap x_map
             };
             uint32_t v[16];
             weights_of(0, v);
+            // The slot is next written by a TMA copy, through another proxy: the arrival alone does not order this lane's reads
+            // before it.  (Without the fence a few rows of a call in some ten were read after the refill; it costs 0 to 0.6 %.)
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();                                                  // every lane has its codes
             if (lane == 0) mbar_arrive(codes_free_bar(c));
             if ((c += kDequantGroups) >= static_cast<unsigned>(p.code_slots)) {
