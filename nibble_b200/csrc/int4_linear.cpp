@@ -24,16 +24,29 @@
 
 namespace {
 
-// Scratch of calls that share K between CTAs, one buffer per (device, stream) so that calls on different streams never share it.
-// Allocated by the first such call on a stream, its counters zeroed, and kept: the kernels leave the counters at zero.  A call
-// that needs more replaces it; the caching allocator hands the old one out again on the same stream only, behind the calls that
-// used it.
+// Scratch of calls that share K between CTAs: arrival counters, zero between calls, and FP32 parts.
 constexpr int64_t kWorkspaceBytes = 40 << 20;   // the most: 38 MiB are the GEMM's parts, two of 256 x 128 sums for each of 148 CTAs
 
 // The arrival counters of any problem whose scratch fits: the fixed 256 KB prefix, and then some.
 constexpr int64_t kCounterBytes = 1 << 20;
 
+at::Tensor zeroed_scratch(const at::Device& device, cudaStream_t stream, int64_t bytes) {
+    at::Tensor scratch = at::detail::empty_cuda({bytes}, at::kByte, device, c10::nullopt);
+    C10_CUDA_CHECK(cudaMemsetAsync(scratch.data_ptr(), 0, static_cast<size_t>(std::min(bytes, kCounterBytes)), stream));
+    return scratch;
+}
+
+// Outside of graph capture: one buffer per (device, stream), so that calls on different streams never share it, allocated and
+// zeroed by the first call that needs it and kept, since the kernels leave the counters at zero.  A call that needs more replaces
+// it; the caching allocator hands the old one out again on the same stream only, behind the calls that used it.
+//
+// During capture: memory of the graph's own for each call, zeroed by a node of that graph in front of its kernel.  A kept buffer
+// would tie the graph to counters that another graph or an eager call may not have cleared yet (its zeroing would be a node of
+// whichever graph was captured first) or is using at the time of the replay.  (One zeroing costs a replay 1 to 2 us.)
 at::Tensor workspace_for(const at::Device& device, cudaStream_t stream, int64_t bytes) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    C10_CUDA_CHECK(cudaStreamIsCapturing(stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone) return zeroed_scratch(device, stream, bytes);
     static std::mutex mutex;
     static auto* cache = new std::map<std::pair<int, cudaStream_t>, at::Tensor>();
     std::lock_guard<std::mutex> lock(mutex);
@@ -42,8 +55,7 @@ at::Tensor workspace_for(const at::Device& device, cudaStream_t stream, int64_t 
         int64_t size = 1 << 20;
         while (size < bytes) size *= 2;
         kept = at::Tensor();
-        kept = at::detail::empty_cuda({std::min(size, kWorkspaceBytes)}, at::kByte, device, c10::nullopt);
-        C10_CUDA_CHECK(cudaMemsetAsync(kept.data_ptr(), 0, static_cast<size_t>(std::min<int64_t>(kept.numel(), kCounterBytes)), stream));
+        kept = zeroed_scratch(device, stream, std::min(size, kWorkspaceBytes));
     }
     return kept;
 }

@@ -350,3 +350,39 @@ def test_operator_takes_no_more_scratch_than_the_call_uses():
         kept = torch.cuda.memory_allocated() - before
         need = lib.w4a16_linear_scratch_bytes(split[0], split[2], split[1], 128, 0)
         assert need <= kept <= 2 << 20
+
+
+@pytest.mark.parametrize(("m", "k", "n"), [(1, 28672, 8192), (6, 14336, 4096), (12, 8192, 4096), (128, 8192, 28672), (40, 8192, 28672)])
+def test_captured_graphs_do_not_depend_on_each_others_replays(m, k, n):
+    """Two graphs captured on a stream whose first sharing calls are these, in memory that holds garbage; the second replayed
+    first, eager calls in between.  Every replay and call gives the bits of an ordinary one."""
+    assert _native.core().w4a16_linear_scratch_bytes(m, n, k, 128, 0) > 0
+    torch.manual_seed(m + k)
+    packed = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda")
+    scales = (torch.rand((n, k // 128), device="cuda") * 0.01 + 1e-3).half()
+    x = torch.randn((m, k), device="cuda").half()
+    want = linear_cuda(x, packed, scales, 128)
+    torch.cuda.synchronize()
+    pool, stream = torch.cuda.graph_pool_handle(), torch.cuda.Stream()
+    litter = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(litter, pool=pool, stream=stream):
+        garbage = torch.full((96 << 20,), 255, dtype=torch.uint8, device="cuda")
+    litter.replay()
+    torch.cuda.synchronize()
+    del garbage
+    graphs, outputs = [], []
+    for _ in range(2):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, pool=pool, stream=stream):
+            outputs.append([linear_cuda(x, packed, scales, 128) for _ in range(2)])
+        graphs.append(graph)
+    for which in (1, 0, 1, 1, 0):
+        for y in outputs[which]:
+            y.fill_(float("nan"))
+        graphs[which].replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, want) for y in outputs[which])
+        with torch.cuda.stream(stream):
+            assert torch.equal(linear_cuda(x, packed, scales, 128), want)
+        torch.cuda.synchronize()
+    assert torch.equal(linear_cuda(x, packed, scales, 128), want)
