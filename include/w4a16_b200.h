@@ -117,11 +117,11 @@ int w4a16_linear_f16_config(const void* x, const void* packed, const void* scale
                             w4a16_stream_t stream);
 
 /* Bytes of workspace with which K can be split across CTAs for this problem (FP32 partial sums plus arrival counters), by
- * w4a16_linear_f16 or by an explicit launch shape: an allocation that serves a layer.  Never fails; returns 0 for empty problems. */
+ * w4a16_linear_f16 or by an explicit launch shape: an allocation that serves a layer, up to 39 MB where the GEMM cuts tiles into
+ * equal runs.  Never fails; returns 0 for empty problems. */
 size_t w4a16_linear_workspace_bytes(int64_t M, int64_t N, int64_t K);
-/* The same for a call made with `flags`: batches that w4a16_linear_f16 sends to the tcgen05 GEMM
- * (M >= 65 without W4A16_FLAG_OUTPUT_F32 / W4A16_FLAG_NO_TCGEN05) or to the generic kernel need none.
- * w4a16_linear_workspace_bytes(M, N, K) is this function with flags == 0. */
+/* The same for a call made with `flags`; w4a16_linear_workspace_bytes(M, N, K) is this function with flags == 0.  (What equal
+ * runs need is left out for batches that only W4A16_FLAG_FORCE_TCGEN05 sends to the GEMM.) */
 size_t w4a16_linear_workspace_bytes_flags(int64_t M, int64_t N, int64_t K, uint32_t flags);
 /* Exactly what w4a16_linear_f16 uses of a workspace for this call (aligned pointers) on the current device: 0 when nothing is
  * shared through one, so that none need be passed; with fewer bytes it shares less, with more it does the same. */

@@ -149,15 +149,17 @@ const char* w4a16_status_string(int status) {
 }
 
 size_t w4a16_linear_workspace_bytes_flags(int64_t M, int64_t N, int64_t K, uint32_t flags) {
-    if (M <= 0 || N <= 0 || K <= 0 || K % w4a16::kGroupFast != 0) return 0;
-    // The generic kernel uses no scratch; the tcgen05 GEMM wants some only for layers with few tiles.
-    if (flags & W4A16_FLAG_FORCE_GENERIC) return 0;
-    // (With weights in tensor memory a larger one, up to 39 MB, lets equal runs cut tiles; it does without.)
-    if (routes_to_tcgen05(M, N, K, flags)) return w4a16::tcgen05_workspace_bytes(M, N, K);
-    const w4a16_linear_config c = w4a16::choose_linear_config(M, N, K, w4a16::kMaxKSplits);
-    // (A layer of few row tiles and long K may always be split, if only by w4a16_linear_f16_config.)
-    const bool may_split = N < 4096 && K >= 4096;
-    return w4a16::linear_workspace_bytes_for(M, N, may_split && c.k_splits < 2 ? 2 : c.k_splits);
+    if (M <= 0 || N <= 0 || K <= 0 || K % w4a16::kGroupFast != 0 || (flags & W4A16_FLAG_FORCE_GENERIC)) return 0;
+    size_t wanted;
+    if (routes_to_tcgen05(M, N, K, flags)) {
+        wanted = w4a16::tcgen05_workspace_bytes(M, N, K);     // K of layers of few tiles, in the kernel that has it from memory
+    } else {
+        // a layer of few row tiles and long K may always be split, if only by w4a16_linear_f16_config
+        const int splits = w4a16::choose_linear_config(M, N, K, w4a16::kMaxKSplits).k_splits;
+        wanted = w4a16::linear_workspace_bytes_for(M, N, N < 4096 && K >= 4096 && splits < 2 ? 2 : splits);
+    }
+    const size_t used = flags & W4A16_FLAG_FORCE_TCGEN05 ? 0 : w4a16_linear_scratch_bytes(M, N, K, w4a16::kGroupFast, flags);
+    return used > wanted ? used : wanted;
 }
 
 size_t w4a16_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {

@@ -281,7 +281,8 @@ class PeerView:
 
 
 def _workspace(m: int, n: int, k: int, device) -> torch.Tensor | None:
-    need = _native.core().w4a16_linear_workspace_bytes(m, n, k)
+    # (the peer entry point streams whatever the batch; other batches of 9..64 rows may go to the GEMM)
+    need = _native.core().w4a16_linear_scratch_bytes(m, n, k, 128, _native.FLAG_NO_TCGEN05)
     return torch.zeros(need, dtype=torch.uint8, device=device) if need else None
 
 

@@ -116,6 +116,27 @@ def test_scratch_query_names_only_what_the_call_uses():
             assert scratch(m, n, k, 128, _native.FLAG_NO_TCGEN05) <= lib.w4a16_linear_workspace_bytes_flags(m, n, k, _native.FLAG_NO_TCGEN05)
 
 
+def test_workspace_query_covers_what_the_call_uses():
+    """A caller who allocates by the query gets every way of sharing that the call's own route has, equal runs included."""
+    lib = _native.core()
+    assert lib.w4a16_linear_workspace_bytes(128, 28672, 8192) == lib.w4a16_linear_scratch_bytes(128, 28672, 8192, 128, 0) > 37 << 20
+    for m in (1, 2, 7, 8, 9, 16, 17, 33, 64, 65, 128, 200, 512, 777, 1024, 2048):
+        for n, k in ((256, 2048), (2048, 5632), (5632, 2048), (1024, 8192), (8192, 8192), (28672, 8192), (8192, 28672), (5003, 4864), (12345, 5632)):
+            for flags in (0, _native.FLAG_NO_TCGEN05, _native.FLAG_OUTPUT_F32):
+                assert lib.w4a16_linear_workspace_bytes_flags(m, n, k, flags) >= lib.w4a16_linear_scratch_bytes(m, n, k, 128, flags)
+
+
+def test_peer_layers_allocate_for_the_kernel_that_runs_them():
+    """Their launches stream at any batch, so a batch that would otherwise go to the GEMM needs the streaming kernel's scratch:
+    32 rows of K = 8192 do not fit a CTA's shared memory unsplit."""
+    from nibble_b200 import sharded
+
+    need = _native.core().w4a16_linear_scratch_bytes(32, 4096, 8192, 128, _native.FLAG_NO_TCGEN05)
+    assert need > 256 * 1024 + 32 * 4096 * 4
+    assert sharded._workspace(32, 4096, 8192, "cpu").numel() == need
+    assert sharded._workspace(1, 2048, 2048, "cpu") is None
+
+
 def test_attention_refuses_caches_it_cannot_read_sixteen_bytes_at_a_time():
     lib = _native.core()
     before = lib.w4a16_launch_count()

@@ -146,3 +146,17 @@ def test_plain_sum_of_partials():
     assert status == 0
     expect = ((parts[0] + parts[1]) + parts[2]).half()
     assert torch.equal(out, expect)
+
+
+@pytest.mark.parametrize("rows", [17, 32, 64])
+def test_medium_batches_split_long_k_on_the_streaming_kernel(rows):
+    """The peer entry point streams at any batch: K = 8192 at 17 rows and more fits shared memory only when it is split, with
+    the scratch of the streaming kernel (the ordinary entry point sends these calls to the GEMM)."""
+    torch.manual_seed(rows)
+    packed = torch.randint(0, 256, (10240, 4096), dtype=torch.uint8, device="cuda")
+    scales = (torch.rand((10240, 64), device="cuda") * 0.01 + 1e-3).half()
+    layer = PeerColumnParallelQuantizedLinear(packed, scales, local=LocalRanks(1), rank=0, name="wide", max_rows=rows)
+    x = torch.randn((rows, 8192), generator=torch.Generator().manual_seed(rows)).half().cuda()
+    out = layer(x)
+    columns = np.sort(np.random.default_rng(rows).choice(10240, size=64, replace=False))
+    check_against_oracle(out, x, packed, scales, rows=columns)
