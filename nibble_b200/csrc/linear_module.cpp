@@ -32,7 +32,8 @@ c10::TypedOperatorHandle<Signature> operator_handle(const char* name) {
 }
 
 // Whether a batch goes to the fused operator, or is multiplied by dequantised FP16 weights (same arithmetic from 65 rows
-// on: weights rounded to FP16, FP32 sums).  The lines come from times of both on 16 layers at 65 to 2048 rows:
+// on: weights rounded to FP16, FP32 sums).  linear.py states the same rule (takes_operator) for the calls that stay in Python; a
+// test holds the two together.  The lines come from times of both on 16 layers at 65 to 2048 rows:
 //   - dequantising and cuBLAS cost about 6 us + 2.5 bytes a weight + the matrix product at its full rate, and 14 us of host
 //     time: unbeaten above 1024 rows, and on mid-sized layers above 256 (2048 -> 5632, 512 rows: 17.7 against 20.5 us), but not on
 //     small ones, where the host sets the pace (1024 -> 1920, 89 rows: 15.8 against 9 us);
@@ -171,6 +172,23 @@ PyObject* linear_forward(PyObject*, PyObject* const* args, Py_ssize_t count) {
     END_HANDLE_TH_ERRORS
 }
 
+// uses_fused_kernel(rows, out_features, in_features, group_size) -> bool
+PyObject* rule(PyObject*, PyObject* const* args, Py_ssize_t count) {
+    HANDLE_TH_ERRORS
+    int64_t value[4] = {};
+    if (count != 4) {
+        PyErr_SetString(PyExc_TypeError, "uses_fused_kernel takes four integers");
+        return nullptr;
+    }
+    for (int i = 0; i < 4; ++i) {
+        value[i] = PyLong_AsLongLong(args[i]);
+        if (PyErr_Occurred() != nullptr) return nullptr;
+    }
+    if (uses_fused_kernel(value[0], value[1], value[2], value[3])) Py_RETURN_TRUE;
+    Py_RETURN_FALSE;
+    END_HANDLE_TH_ERRORS
+}
+
 using FastCall = PyObject* (*)(PyObject*, PyObject* const*, Py_ssize_t);
 PyCFunction method(FastCall f) { return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)); }
 
@@ -180,6 +198,7 @@ PyMethodDef methods[] = {
     {"linear", method(linear), METH_FASTCALL, "linear(activations, packed_weights, scales, group_size) -> Tensor or NotImplemented"},
     {"dequantize", method(dequantize), METH_FASTCALL, "dequantize(packed_weights, scales, group_size) -> Tensor or NotImplemented"},
     {"quantize_pack", method(quantize_pack), METH_FASTCALL, "quantize_pack(weights, group_size) -> (Tensor, Tensor) or NotImplemented"},
+    {"uses_fused_kernel", method(rule), METH_FASTCALL, "uses_fused_kernel(rows, out_features, in_features, group_size) -> bool"},
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_C", "Native side of nibble_b200: torch operators and QuantizedLinear.forward.", -1,

@@ -135,6 +135,22 @@ def linear_cuda(
     return torch.ops.w4a16.linear(activations, packed_weights, scales, group_size)
 
 
+def linear_bias_cuda(
+    activations: torch.Tensor,
+    packed_weights: torch.Tensor,
+    scales: torch.Tensor,
+    bias: torch.Tensor | None,
+    group_size: int = 128,
+) -> torch.Tensor:
+    """What ``QuantizedLinear`` calls: activations of any rank ``[..., K]``, the FP16 bias added inside the kernel.
+
+    Not part of the reference's surface.  Unlike ``linear_cuda`` it lets batches of 65 rows and more round each weight to FP16
+    whatever the group size, as the product with dequantised weights does.
+    """
+    _require_extension()
+    return torch.ops.w4a16.linear_bias(activations, packed_weights, scales, bias, group_size)
+
+
 def dequantize_cuda(
     packed_weights: torch.Tensor,
     scales: torch.Tensor,

@@ -10,31 +10,60 @@ from __future__ import annotations
 
 import torch
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
-from .cuda import dequantize_cuda, linear_cuda, linear_forward
+from .cuda import dequantize_cuda, linear_bias_cuda, linear_cuda, linear_forward
 from .quantization import quantize_and_pack_weights
 
 # Largest flattened batch M sent to the streaming (mma.sync) fused kernel.  The reference stops at 8
 # and dequantises to FP16 + cuBLAS above that (w4a16/linear.py:9,179-187).
 FUSED_MAX_ROWS = 64
-# Above FUSED_MAX_ROWS the operator runs the tcgen05 kernels that dequantise inside the GEMM.  (This is the rule of the
-# Python forward; the native one, which takes nearly every call, draws finer lines: csrc/linear_module.cpp.)  It beats
-# dequantise-then-cuBLAS while the FP16 weight matrix's round trip through HBM is a large share of the
-# cuBLAS time (batches up to about a thousand rows) and there are enough 128-channel weight tiles to
-# occupy the GPU; outside that window the module does what the reference does.
+
+
+def takes_operator(rows: int, out_features: int, in_features: int, group_size: int) -> bool:
+    """Whether ``forward`` sends a flattened batch of ``rows`` to the fused operator, or multiplies it by dequantised weights.
+
+    The native forward has the same rule (csrc/linear_module.cpp: uses_fused_kernel, with the measurements it was drawn from);
+    this statement of it is for calls that the native one leaves to Python, where tracing has to see what is compared.
+    """
+    if rows <= FUSED_MAX_ROWS or group_size % 32:
+        return True      # (the dequantise operator needs group_size % 32 == 0; the fused one does not)
+    if group_size > 128 or in_features % 128:
+        return False     # the operator has no tensor-core kernel for these
+    if out_features % 8:
+        return True
+    weights = out_features * in_features
+    shallow = in_features < 1024 and out_features >= 8192
+    if rows <= 256:
+        return rows <= 128 or not shallow
+    if rows <= 512:
+        return weights <= 9 << 19 or (weights >= 32 << 20 and not shallow)
+    if rows <= 1024 and in_features >= 5120 and (weights <= 6 << 20 or (in_features >= 8192 and weights <= 48 << 20)):
+        return True
+    return group_size == 128 and rows <= 1024 and (256 - rows % 256) % 256 < 64 and weights >= 64 << 20
+
+
+# The coarse rule for activations whose arithmetic has to stay visible as torch operators (below), where speed is not the point:
+# the operator up to FUSED_MAX_ROWS, and up to PREFILL_FUSED_MAX_ROWS on layers of PREFILL_MIN_WEIGHT_TILES 128-channel tiles.
 PREFILL_FUSED_MAX_ROWS = 1024
 PREFILL_MIN_WEIGHT_TILES = 40
 
 
 def uses_fused_kernel(rows: int, out_features: int, group_size: int) -> bool:
-    """Whether ``forward`` sends a flattened batch of ``rows`` to the fused operator."""
+    """The coarse rule: whether such a batch of ``rows`` goes to the fused operator."""
     if rows <= FUSED_MAX_ROWS:
         return True
     if group_size % 32:
         return True  # the dequantise operator needs group_size % 32 == 0; the fused one does not
     if group_size != 128:
-        return False  # the tcgen05 kernel is built for 128-wide groups
+        return False
     return rows <= PREFILL_FUSED_MAX_ROWS and -(-out_features // 128) >= PREFILL_MIN_WEIGHT_TILES
+
+
+def _transformed(tensor: torch.Tensor) -> bool:
+    """Whether a function transform (vmap, forward-mode differentiation) follows what is computed from ``tensor``: it can follow
+    the product with dequantised weights, and not the fused operator."""
+    return torch._C._functorch.is_functorch_wrapped_tensor(tensor) or forward_ad.unpack_dual(tensor).tangent is not None
 
 
 def _run_fused(flat, packed_weights, scales, group_size):
@@ -135,7 +164,7 @@ class QuantizedLinear(torch.nn.Module):
     # ------------------------------------------------------------------ forward
     def forward(self, activations: torch.Tensor) -> torch.Tensor:
         # The ordinary call is one native function (csrc/linear_module.cpp); what it does not take -- and every invalid
-        # call -- it leaves to the code below, which computes the same.
+        # call -- it leaves to the code below, which computes the same, by the same kernels.
         if not torch.compiler.is_compiling():
             buffers = self._buffers
             out = linear_forward(activations, buffers["packed_weights"], buffers["scales"], buffers["bias"], self.group_size,
@@ -158,11 +187,17 @@ class QuantizedLinear(torch.nn.Module):
         if not self.scales.is_contiguous():
             raise ValueError("scales must be contiguous")
 
-        # The operator wants a dense [M, K]; views handed over by generation loops often are not.
-        flat = activations.contiguous().reshape(-1, self.in_features)
-        use_fused = (self.fused or self.group_size % 32 != 0) and uses_fused_kernel(
-            flat.shape[0], self.out_features, self.group_size)
-        run = _run_fused if use_fused else _run_dequant_matmul
+        # The operator wants dense activations; views handed over by generation loops often are not.
+        dense = activations.contiguous()
+        flat = dense.reshape(-1, self.in_features)
+        fusable = self.fused or self.group_size % 32 != 0
+        if dense.is_cuda and (torch.compiler.is_compiling() or not _transformed(dense)):
+            if fusable and takes_operator(flat.shape[0], self.out_features, self.in_features, self.group_size):
+                return linear_bias_cuda(dense, self.packed_weights, self.scales, self.bias, self.group_size)
+            run = _run_dequant_matmul
+        else:
+            use_fused = fusable and uses_fused_kernel(flat.shape[0], self.out_features, self.group_size)
+            run = _run_fused if use_fused else _run_dequant_matmul
         flat_out = run(flat, self.packed_weights, self.scales, self.group_size)
         out = flat_out.reshape(*activations.shape[:-1], self.out_features)
         return out if self.bias is None else out + self.bias

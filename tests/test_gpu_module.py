@@ -206,3 +206,40 @@ def test_native_forward_equals_the_python_forward(rows, k, n):
     wide[:, :k] = x[0]
     assert rows == 1 or linear_module.linear_forward(wide[:, :k], packed, scales, None, 128, True) is NotImplemented
     torch.testing.assert_close(QuantizedLinear(packed, scales, 128)(wide[:, :k]), want[0], rtol=2e-3, atol=2e-3)
+
+
+class _Passing(torch.overrides.TorchFunctionMode):
+    def __torch_function__(self, func, types, args=(), kwargs=None):
+        return func(*args, **(kwargs or {}))
+
+
+@pytest.mark.parametrize(("n", "k", "gs"), [(1000, 1152, 128), (2048, 5632, 128), (520, 1024, 64), (5003, 512, 32), (8192, 512, 128)])
+@pytest.mark.parametrize("rows", [1, 48, 65, 130, 300, 600, 777, 1024, 1100])
+def test_every_way_into_the_module_takes_the_native_route(rows, n, k, gs):
+    """Autocast, a function mode, non-contiguous activations and compiled code: the bits and the launches of the plain call."""
+    from nibble_b200 import _native
+
+    count = _native.core().w4a16_launch_count
+    torch.manual_seed(rows + n)
+    packed = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda")
+    scales = (torch.rand((n, k // gs), device="cuda") * 0.01 + 1e-3).half()
+    x = torch.randn((rows, k), device="cuda").half()
+    spaced = torch.zeros((rows, 2 * k), dtype=torch.float16, device="cuda")[:, :k].copy_(x)
+    for bias in (None, torch.randn((n,), device="cuda").half()):
+        layer = QuantizedLinear(packed, scales, gs, bias=bias)
+        before = count()
+        want = layer(x)
+        launches = count() - before
+        w16 = torch.ops.w4a16.dequantize(packed, scales, gs).float()
+        exact = x.float() @ w16.t() + (0 if bias is None else bias.float())
+        torch.testing.assert_close(want.float(), exact, rtol=2e-3, atol=2e-2)
+        before = count()
+        with _Passing():
+            assert torch.equal(layer(x), want)
+        with torch.autocast("cuda", dtype=torch.float16):
+            assert torch.equal(layer(x), want)
+        if rows > 1:
+            assert not spaced.is_contiguous() and torch.equal(layer(spaced), want)
+        assert count() - before == (3 if rows > 1 else 2) * launches
+    torch._dynamo.reset()
+    assert torch.equal(torch.compile(layer, backend="aot_eager", fullgraph=True, dynamic=False)(x), want)

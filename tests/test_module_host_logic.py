@@ -98,6 +98,22 @@ def test_prefill_window_routes_wide_layers_to_the_fused_operator(oracle_backend)
     assert oracle_backend == ["fused", "dequant", "dequant"]
 
 
+def test_python_and_native_forward_state_one_rule():
+    """Every line of the rule and both sides of it, over the sizes a layer can have."""
+    from nibble_b200 import _native
+    from nibble_b200.linear import takes_operator
+
+    native = _native.load_torch_ops().uses_fused_kernel
+    rows = [1, 64, 65, 128, 129, 192, 193, 255, 256, 257, 448, 449, 511, 512, 513, 640, 704, 705, 768, 769, 960, 961, 1023, 1024,
+            1025, 1216, 2048, 5000]
+    sizes = [8, 100, 256, 1000, 1024, 1152, 2048, 2304, 3072, 4096, 5003, 5120, 5632, 6144, 8064, 8192, 11008, 12928, 16384, 28672, 32000]
+    inner = [64, 96, 128, 384, 512, 896, 1024, 1152, 2048, 3072, 4096, 4992, 5120, 5632, 8064, 8192, 11008, 14336, 16384, 28672]
+    verdicts = {(r, n, k, g): takes_operator(r, n, k, g)
+                for r in rows for n in sizes for k in inner for g in (32, 64, 128, 256, 48, 6)}
+    assert all(native(*case) == verdict for case, verdict in verdicts.items())
+    assert {True, False} == set(verdicts.values())
+
+
 def test_group_size_without_dequantize_kernel_stays_fused(oracle_backend):
     layer = _layer(fused=False)  # group_size 4 is not a multiple of 32
     layer(ACTIVATIONS)
