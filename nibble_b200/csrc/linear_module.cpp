@@ -55,11 +55,11 @@ bool uses_fused_kernel(int64_t rows, int64_t out_features, int64_t in_features, 
     return group_size == 128 && rows <= 1024 && (256 - rows % 256) % 256 < 64 && weights >= 64 << 20;
 }
 
-// A tensor nobody has subclassed, wrapped or asked to track gradients of.
+// A tensor nobody has subclassed, wrapped or asked to track gradients of, backward or forward.
 bool plain(PyObject* object) {
     if (!THPVariable_CheckExact(object)) return false;
     const at::Tensor& t = THPVariable_Unpack(object);
-    return t.is_cuda() && !t.requires_grad() && t.is_contiguous() &&
+    return t.is_cuda() && !t.requires_grad() && !t._fw_grad(/*level=*/0).defined() && t.is_contiguous() &&
            !t.key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched,
                                                      c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Batched}));
 }

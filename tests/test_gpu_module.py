@@ -243,3 +243,21 @@ def test_every_way_into_the_module_takes_the_native_route(rows, n, k, gs):
         assert count() - before == (3 if rows > 1 else 2) * launches
     torch._dynamo.reset()
     assert torch.equal(torch.compile(layer, backend="aot_eager", fullgraph=True, dynamic=False)(x), want)
+
+
+@pytest.mark.parametrize("rows", [4, 100])
+def test_transforms_follow_the_product_with_dequantised_weights(rows):
+    """Forward-mode differentiation and vmap see the matrix product where the module forms one."""
+    from torch.autograd import forward_ad
+
+    layer = _layer(n=64, k=256, seed=5)
+    layer.fused = False
+    w16 = torch.ops.w4a16.dequantize(layer.packed_weights, layer.scales, 128)
+    x, direction = torch.randn((2, rows, 256), device="cuda").half()
+    with forward_ad.dual_level():
+        out = forward_ad.unpack_dual(layer(forward_ad.make_dual(x, direction)))
+        assert out.tangent is not None
+        torch.testing.assert_close(out.primal, F.linear(x, w16), rtol=1e-3, atol=1e-3)
+        torch.testing.assert_close(out.tangent, F.linear(direction, w16), rtol=1e-3, atol=1e-3)
+    batched = torch.vmap(layer)(torch.stack([x, direction]))
+    torch.testing.assert_close(batched, torch.stack([layer(x), layer(direction)]), rtol=1e-3, atol=1e-3)
