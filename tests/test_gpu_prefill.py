@@ -243,3 +243,28 @@ def test_gemm_results_do_not_depend_on_timing(m, k, n, gs):
     from nibble_b200 import dequantize_cuda
     torch.testing.assert_close(first.float(), x.float() @ dequantize_cuda(packed, scales, gs).float().t(), rtol=2e-3, atol=1e-2)
     assert _device_status() == 0
+
+
+@pytest.mark.parametrize(("m", "k", "n"), [
+    (512, 1024, 9600), (513, 1024, 9600),      # 4 and 5 batch tiles; from 513 rows on the tiles of one round decide: 5 x 38
+    (777, 1024, 5376), (777, 1024, 5377),      # 147 and 154 tiles
+    (1024, 2048, 8192), (1025, 2048, 8192), (1024, 1920, 8192),
+    (2048, 3968, 4000), (2048, 4096, 4000),
+    (5000, 4096, 1000), (3000, 256, 130),
+])
+def test_both_gemms_beyond_512_rows(m, k, n):
+    """Either side of every line between the two GEMMs: the product with the same FP16 weights, the same bits again, and
+    nothing outside the output."""
+    from nibble_b200 import dequantize_cuda
+
+    _device_status()
+    torch.manual_seed(m + n)
+    packed, scales = quantize_and_pack_weights(torch.randn((n, k), device="cuda") * 0.02, 128)
+    x = torch.randn((m, k), device="cuda").half()
+    want = x.float() @ dequantize_cuda(packed, scales, 128).float().t()
+    need = _native.core().w4a16_linear_scratch_bytes(m, n, k, 128, 0)
+    for workspace in (None, torch.zeros(max(need, 16), dtype=torch.uint8, device="cuda")):
+        y = capi_linear(x, packed, scales, workspace=workspace)
+        torch.testing.assert_close(y.float(), want, rtol=2e-3, atol=2e-3)
+        assert torch.equal(y, capi_linear(x, packed, scales, workspace=workspace))
+    assert _device_status() == 0
