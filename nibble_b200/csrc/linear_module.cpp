@@ -33,26 +33,23 @@ c10::TypedOperatorHandle<Signature> operator_handle(const char* name) {
 
 // Whether a batch goes to the fused operator, or is multiplied by dequantised FP16 weights (same arithmetic from 65 rows
 // on: weights rounded to FP16, FP32 sums).  linear.py states the same rule (takes_operator) for the calls that stay in Python; a
-// test holds the two together.  The lines come from times of both on 16 layers at 65 to 2048 rows:
-//   - dequantising and cuBLAS cost about 6 us + 2.5 bytes a weight + the matrix product at its full rate, and 14 us of host
-//     time: unbeaten above 1024 rows, and on mid-sized layers above 256 (2048 -> 5632, 512 rows: 17.7 against 20.5 us), but not on
-//     small ones, where the host sets the pace (1024 -> 1920, 89 rows: 15.8 against 9 us);
-//   - cuBLAS falls off its fast kernels where an output row is no multiple of 16 bytes (9216 -> 2575, 128 rows: 125 against 20 us);
-//   - from 513 to 1024 rows the operator is ahead on deep layers that are not wide (one launch, and the FP16 weights are a large
-//     share of the work: 11008 -> 4096, 777 rows: 83 against 91 us) and on small ones (5120 -> 1000: 18 against 25); elsewhere it
-//     has 256-row batch tiles and is ahead only where the last one is nearly full
-//     (8192 -> 28672, 1024 rows: 451 against 494 us; 777 rows: 442 against 362).
+// test holds the two together.  The lines come from times of both, eager calls back to back, on 76 layers from 512 x 2048 to
+// 28672 x 8192 at 129 to 2048 rows (us, the operator / dequantise and multiply; the latter is 14 us of host time at least):
+//   - cuBLAS falls off its fast kernels where an output row is no multiple of 16 bytes (9216 -> 2575, 128 rows: 20 / 125);
+//   - up to 512 rows the operator (2048 -> 2560, 400 rows: 15 / 15; 4096 -> 11008, 256 rows: 41 / 50), but for layers of many tiles
+//     of a few K blocks each above 256 rows (512 -> 28672, 512 rows: 37 / 29).  0.2 to 0.6 % slower than the better on average;
+//   - 513 to 1024 rows: small layers (1024 -> 4096, 777 rows: 13 / 17), all but shallow ones up to seven batch tiles of 128 rows
+//     (8192 -> 28672, 777 rows: 406 / 401; 11008 -> 1024, 777 rows: 28 / 34), narrow deep ones (16384 -> 1024, 1024 rows: 39 / 45).
+//     2 % slower than the better on average, 36 % at most (896 -> 6448, 520 rows: 12 / 17);
+//   - above, the matrix product at cuBLAS's rate outweighs the weights' round trip (8192 -> 28672, 2048 rows: 1094 / 919).
 bool uses_fused_kernel(int64_t rows, int64_t out_features, int64_t in_features, int64_t group_size) {
     if (rows <= 64) return true;
     if (group_size % 32 != 0) return true;
     if (group_size > 128 || in_features % 128 != 0) return false;      // the operator has no tensor-core kernel for these
-    if (out_features % 8 != 0) return true;
-    const int64_t weights = out_features * in_features;
-    const bool shallow = in_features < 1024 && out_features >= 8192;   // many tiles of a few K blocks each
-    if (rows <= 256) return rows <= 128 || !shallow;
-    if (rows <= 512) return weights <= 9 << 19 || (weights >= 32 << 20 && !shallow);
-    if (rows <= 1024 && in_features >= 5120 && (weights <= 6 << 20 || (in_features >= 8192 && weights <= 48 << 20))) return true;
-    return group_size == 128 && rows <= 1024 && (256 - rows % 256) % 256 < 64 && weights >= 64 << 20;
+    if (out_features % 8 != 0 || rows <= 256) return true;
+    if (rows > 1024 || out_features > 20 * in_features) return false;
+    if (rows <= 512 || out_features * in_features <= 4 << 20) return true;
+    return (in_features >= 2048 && rows <= 896) || in_features >= 8 * out_features;
 }
 
 // A tensor nobody has subclassed, wrapped or asked to track gradients of, backward or forward.

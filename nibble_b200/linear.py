@@ -30,17 +30,13 @@ def takes_operator(rows: int, out_features: int, in_features: int, group_size: i
         return True      # (the dequantise operator needs group_size % 32 == 0; the fused one does not)
     if group_size > 128 or in_features % 128:
         return False     # the operator has no tensor-core kernel for these
-    if out_features % 8:
+    if out_features % 8 or rows <= 256:
         return True
-    weights = out_features * in_features
-    shallow = in_features < 1024 and out_features >= 8192
-    if rows <= 256:
-        return rows <= 128 or not shallow
-    if rows <= 512:
-        return weights <= 9 << 19 or (weights >= 32 << 20 and not shallow)
-    if rows <= 1024 and in_features >= 5120 and (weights <= 6 << 20 or (in_features >= 8192 and weights <= 48 << 20)):
+    if rows > 1024 or out_features > 20 * in_features:
+        return False
+    if rows <= 512 or out_features * in_features <= 4 << 20:
         return True
-    return group_size == 128 and rows <= 1024 and (256 - rows % 256) % 256 < 64 and weights >= 64 << 20
+    return (in_features >= 2048 and rows <= 896) or in_features >= 8 * out_features
 
 
 # The coarse rule for activations whose arithmetic has to stay visible as torch operators (below), where speed is not the point:
