@@ -3,6 +3,8 @@
 // include/w4a16_b200.h.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "kernels.h"
 
 namespace w4a16 {
@@ -38,36 +40,33 @@ bool small_group_streams(const void* x, const void* packed, const void* scales, 
 
 namespace {
 
-// Whether a fast-path call with FP16 output goes to the tcgen05 GEMM rather than the streaming kernel.
-// From 65 rows on always, up to 8 rows never.  Between 9 and 64 rows the streaming kernel still wins on small layers, but its cost
-// grows with the batch and with K (every CTA stages batch x K activations, K is split ever further and the partial
-// sums travel through memory) while the GEMM's does not.  Both sides of the comparison are fits to measurements
-// on B200: the GEMM takes about 0.6 us per 128-wide K step of a round of 148 weight tiles whatever the batch; the
-// streaming kernel about 5 us plus (8 + 1.5 * K/1024) us per 1e9 multiply-adds of the batch padded to 32 or 64
-// rows.  Layers of fewer than 32 weight tiles leave most SMs of the GEMM idle and stay on the streaming kernel.
+// Ranges of K that CTAs would share a 128 x 256 tile in: up to four where half the SMs or more would idle, of 1024 and more.  Part
+// of the line below and of the workspace query; the kernels share tiles in ways of their own.
+int k_ranges(int64_t M, int64_t N, int64_t K) {
+    const int64_t tiles = (M + 255) / 256 * ((N + 127) / 128);
+    int64_t ranges = tiles > 0 ? std::min<int64_t>(4, 148 / tiles) : 1;
+    ranges = std::max<int64_t>(1, std::min<int64_t>(ranges, K / (K >= 4096 ? 1024 : 2048)));
+    const int64_t width = ((K + ranges - 1) / ranges + 255) / 256 * 256;
+    return static_cast<int>((K + width - 1) / width);
+}
+
+// Whether a fast-path call with FP16 output goes to a GEMM rather than the streaming kernel.  From 65 rows on always, up to 8
+// rows never; between, by the costs of both: the GEMM with weights in shared memory about 0.6 us per 128-wide K step of a round of
+// 148 weight tiles, the streaming kernel about 5 us plus (8 + 1.5 * K/1024) us per 1e9 multiply-adds of the padded batch.
 bool routes_to_tcgen05(int64_t M, int64_t N, int64_t K, uint32_t flags) {
     if (flags & (W4A16_FLAG_OUTPUT_F32 | W4A16_FLAG_NO_TCGEN05 | W4A16_FLAG_FORCE_GENERIC)) return false;
     if ((flags & W4A16_FLAG_FORCE_TCGEN05) || M >= w4a16::kTcgen05MinRows) return true;
     if (M <= 8) return false;
-    if (N < 4096) {
-        // Narrow layers: the fits below do not hold (few row tiles, so the streaming kernel leans on K splits whose
-        // partial sums and repeated activation staging grow with the batch).  Measured: with K = 5632, N = 2048 the
-        // GEMM, sharing K between CTAs, takes 14-15 us at 24..64 rows where the streaming kernel takes 22-42 us;
-        // with K = 2048 the streaming kernel wins throughout.  So: from 17 rows on, when a fourth of K is what fits the
-        // streaming kernel's shared memory (K of 4992 and more) and the layer has at least eight weight tiles.
-        // (with N = 1024 and K = 8192 the streaming kernel is still ahead at 17..32 rows, 14-15 us against 18 us,
-        // and behind from 33 on, 24 us against 19 us)
-        return M > 16 && N >= 1024 && K >= 4992 && (N >= 2048 || M > 32);
-    }
+    // Narrow layers, which those costs do not describe: from 17 rows on, when a fourth of K is what fits the streaming kernel's
+    // shared memory and the layer has eight weight tiles (from 33 rows on below N = 2048).  5632 -> 2048, 32 rows: 16.0 / 10.8.
+    if (N < 4096) return M > 16 && N >= 1024 && K >= 4992 && (N >= 2048 || M > 32);
     const double padded = M <= 16 ? 16.0 : M <= 32 ? 32.0 : 64.0;
     const double giga_macs = padded * static_cast<double>(K) * static_cast<double>(N) * 1e-9;
     const double streaming_us = 5.0 + giga_macs * (8.0 + 1.5 * static_cast<double>(K) / 1024.0);
     const int64_t rounds = ((N + 127) / 128 + 147) / 148;
-    // (a layer of few tiles shares the K of a tile between CTAs and pays a second small launch for the sum)
-    const int splits = w4a16::tcgen05_k_splits(M, N, K, nullptr);
-    const double gemm_us = 3.5 + 0.6 * static_cast<double>(rounds) * static_cast<double>(K) / (128.0 * splits) +
-                           (splits > 1 ? 3.0 : 0.0);
-    // 9..16 rows are close to the streaming kernel's best case: only a clear win moves them (K = 28672: 94 -> 71 us)
+    const int ranges = k_ranges(M, N, K);
+    const double gemm_us = 3.5 + 0.6 * static_cast<double>(rounds) * static_cast<double>(K) / (128.0 * ranges) + (ranges > 1 ? 3.0 : 0.0);
+    // 9..16 rows are close to the streaming kernel's best case: only a clear win moves them
     return gemm_us < (M <= 16 ? 0.85 : 1.0) * streaming_us;
 }
 
@@ -159,7 +158,7 @@ size_t w4a16_linear_workspace_bytes_flags(int64_t M, int64_t N, int64_t K, uint3
     if (M <= 0 || N <= 0 || K <= 0 || K % w4a16::kGroupFast != 0 || (flags & W4A16_FLAG_FORCE_GENERIC)) return 0;
     size_t wanted;
     if (routes_to_tcgen05(M, N, K, flags)) {
-        wanted = w4a16::tcgen05_workspace_bytes(M, N, K);     // K of layers of few tiles, in the kernel that has it from memory
+        wanted = w4a16::linear_workspace_bytes_for(M, N, k_ranges(M, N, K));
     } else {
         // a layer of few row tiles and long K may always be split, if only by w4a16_linear_f16_config
         const int splits = w4a16::choose_linear_config(M, N, K, w4a16::kMaxKSplits).k_splits;
@@ -178,8 +177,7 @@ size_t w4a16_linear_scratch_bytes(int64_t M, int64_t N, int64_t K, int64_t group
     if (flags & W4A16_FLAG_FORCE_GENERIC) return 0;
     const bool small_group = group_size != w4a16::kGroupFast;
     if (small_group ? small_group_routes_to_gemm(M, flags) : routes_to_tcgen05(M, N, K, flags)) {
-        return small_group || w4a16::gemm_from_tensor_memory(M, N, K) ? w4a16::gemm_scratch_bytes(M, N, K)
-                                                                      : w4a16::tcgen05_workspace_bytes(M, N, K);
+        return small_group || w4a16::gemm_from_tensor_memory(M, N, K) ? w4a16::gemm_scratch_bytes(M, N, K) : 0;
     }
     auto streaming = [&](int64_t rows) {
         return w4a16::linear_workspace_bytes_for(

@@ -135,9 +135,9 @@ def test_batch_too_large_for_the_streaming_kernel_without_scratch_takes_the_gemm
     (32, 8192, 4096),      # a medium batch on the forced GEMM: 32 tiles, four ranges
 ])
 def test_gemm_splits_k_when_the_layer_has_few_tiles(m, k, n):
-    """With a workspace the GEMM shares the K of an output tile between CTAs (FP32 partial sums, added in order by a
-    second kernel); without one it runs unsplit.  Both agree with the oracle, and the workspace's counter prefix,
-    which the streaming kernel relies on, is left at zero."""
+    """Layers of few tiles, whose K the GEMM shares between CTAs (inside clusters, so that a workspace changes nothing):
+    with the workspace the query names, with none and with one too small.  All agree with the oracle, and the workspace's
+    counter prefix, which the streaming kernel relies on, is left at zero."""
     lib = _native.core()
     flags = _native.FLAG_FORCE_TCGEN05
     need = lib.w4a16_linear_workspace_bytes_flags(m, n, k, flags)
@@ -267,4 +267,33 @@ def test_both_gemms_beyond_512_rows(m, k, n):
         y = capi_linear(x, packed, scales, workspace=workspace)
         torch.testing.assert_close(y.float(), want, rtol=2e-3, atol=2e-3)
         assert torch.equal(y, capi_linear(x, packed, scales, workspace=workspace))
+    assert _device_status() == 0
+
+
+@pytest.mark.parametrize(("m", "k", "n"), [
+    # 128-wide stages: 75 to 148 tiles of 128 channels, up to 128 rows; one stage, odd counts that half use the last copy of codes
+    (65, 128, 9600), (128, 384, 9601), (96, 640, 18944), (100, 896, 12345), (128, 1024, 9473), (66, 1024, 18943),
+    # 64-wide stages: more tiles than one round of the other kernel, K below 4096
+    (513, 384, 16385), (700, 640, 12000), (1100, 896, 9001), (1025, 1152, 9216), (2049, 2048, 2500), (2500, 3968, 1930),
+])
+def test_gemm_from_shared_memory(m, k, n):
+    """The calls that still take the kernel with its weights in shared memory: odd stage counts, ragged channels and batches,
+    both stage widths, with and without a bias; one launch, no scratch."""
+    from nibble_b200 import dequantize_cuda
+
+    lib = _native.core()
+    assert lib.w4a16_linear_scratch_bytes(m, n, k, 128, 0) == 0
+    _device_status()
+    torch.manual_seed(m + k)
+    packed, scales = quantize_and_pack_weights(torch.randn((n, k), device="cuda") * 0.02, 128)
+    x = torch.randn((m, k), device="cuda").half()
+    want = x.float() @ dequantize_cuda(packed, scales, 128).float().t()
+    before = lib.w4a16_launch_count()
+    y = capi_linear(x, packed, scales)
+    assert lib.w4a16_launch_count() == before + 1
+    torch.testing.assert_close(y.float(), want, rtol=2e-3, atol=2e-3)
+    for _ in range(10):
+        assert torch.equal(capi_linear(x, packed, scales), y)
+    bias = torch.randn((n,), device="cuda").half()
+    assert torch.equal(torch.ops.w4a16.linear_bias(x, packed, scales, bias, 128), y + bias)
     assert _device_status() == 0
