@@ -50,9 +50,17 @@ int k_ranges(int64_t M, int64_t N, int64_t K) {
     return static_cast<int>((K + width - 1) / width);
 }
 
-// Whether a fast-path call with FP16 output goes to a GEMM rather than the streaming kernel.  From 65 rows on always, up to 8
-// rows never; between, by the costs of both: the GEMM with weights in shared memory about 0.6 us per 128-wide K step of a round of
-// 148 weight tiles, the streaming kernel about 5 us plus (8 + 1.5 * K/1024) us per 1e9 multiply-adds of the padded batch.
+// Whether a fast-path call with FP16 output goes to a GEMM rather than the streaming kernel: from 65 rows on always, up to 8 rows
+// never.  Between 9 and 64 the line decides the arithmetic as well as the time: the streaming kernel multiplies exact codes and
+// scales its FP32 sums, the GEMM rounds each weight to FP16 first.  So the line stays where it was drawn, and no batch that has
+// exact weights loses them to a faster kernel.  It was drawn from the cost of the GEMM with weights in shared memory (0.6 us per
+// 128-wide K step of a round of 148 tiles, 3 us for sharing K) against the streaming kernel's (5 us plus 8 + 1.5 * K/1024 us
+// per 1e9 multiply-adds of the batch padded to 32 or 64 rows) -- these are the constants below; nearly every call it sends on
+// now runs the faster GEMM of linear_gemm.cu.
+// Measured on 23 layers at nine batches (us, streaming / that GEMM): beyond the line the GEMM is never slower by more than 5 % (14336 ->
+// 4096, 9 rows: 17.9 / 18.9) and up to six times as fast (8192 -> 28672, 64 rows: 251 / 47); on this side of it exact weights are
+// faster on small layers (2048 x 2048, 32 rows: 7.2 / 7.9) and cost up to twice the time on others (8192 -> 28672, 16 rows:
+// 70 / 41; 3072 -> 8192, 32 rows: 24.9 / 11.7).
 bool routes_to_tcgen05(int64_t M, int64_t N, int64_t K, uint32_t flags) {
     if (flags & (W4A16_FLAG_OUTPUT_F32 | W4A16_FLAG_NO_TCGEN05 | W4A16_FLAG_FORCE_GENERIC)) return false;
     if ((flags & W4A16_FLAG_FORCE_TCGEN05) || M >= w4a16::kTcgen05MinRows) return true;
