@@ -291,6 +291,13 @@ w4a16_linear_config choose_batch(int64_t M, int64_t tiles, int chunks, int unrol
     const size_t reduction = static_cast<size_t>(nt) * 8192;
     w4a16_linear_config best{};
     double best_time = 1e30;
+    int fitting = 0;                // the fewest splits whose slice of x fits
+    // Up to eight rows on large layers (two row tiles per SM and more), where the model is least sure of splits.  Slower than the
+    // fastest of sixteen shapes, on average over 2 to 8 rows: K that fits unsplit (140 shapes), never split 0.5 %, by the model 1.2
+    // (5632 -> 16384, 8 rows: 15.9 / 18.8 us); K that only fits four ways (19), always four 0 %, by the model 4.3 (28672 -> 8192, 8
+    // rows: 40.1 / 42.8); K that fits two ways (306 shapes of 10752 to 20480 -> 4864 to 20480), by the model with four ways a fifth
+    // dearer 1.4 %, as it is 3.3, always two 6.5 (20480 -> 10240, 4 rows: 39.3 / 39.3 / 45.2).
+    const bool large = nt == 1 && tiles >= 2 * static_cast<int64_t>(sms);
     best.k_warps = 8;
     best.k_splits = 1;
     for (int splits = 1; splits <= std::min(max_splits, kMaxKSplits) && splits <= chunks; splits *= 2) {
@@ -312,17 +319,17 @@ w4a16_linear_config choose_batch(int64_t M, int64_t tiles, int chunks, int unrol
             const double steps = 0.5 * (((per_split + kw - 1) / kw + unroll - 1) / unroll * unroll);
             double tile = steps * std::max(cost.step_chain, cost.step_issue * active) + cost.tile_end;
             if (splits > 1) tile += cost.split + cost.split_per_row * rows * splits + cost.split_per_cta * splits;
-            const double time = waves * (cost.start + cost.stage_per_8_rows * rows / 8.0 +
-                                         cost.stage_per_kb * rows * per_split * 0.25 * active + rounds * tile);
+            double time = waves * (cost.start + cost.stage_per_8_rows * rows / 8.0 +
+                                   cost.stage_per_kb * rows * per_split * 0.25 * active + rounds * tile);
+            if (large && fitting == 2 && splits == 4) time *= 1.2;
             if (time < best_time) {
                 best_time = time;
                 best.k_warps = kw;
                 best.k_splits = splits;
             }
         }
-        // With three row tiles per SM the stream of weights is what bounds a batch of up to eight rows, which the model does not
-        // know: K is then split only as far as it takes to fit (28672 -> 8192, 8 rows: four ways 40 us, eight 43).
-        if (nt == 1 && tiles >= 3 * sms && best_time < 1e30) break;
+        if (fitting == 0 && best_time < 1e30) fitting = splits;
+        if (large && fitting != 0 && fitting != 2) break;
     }
     // Nothing fits shared memory: the most splits, for the launch to refuse (and its caller to take another kernel).
     if (best_time == 1e30) {
