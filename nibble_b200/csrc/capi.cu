@@ -196,20 +196,16 @@ size_t w4a16_linear_scratch_bytes(int64_t M, int64_t N, int64_t K, int64_t group
     return whole > rest ? whole : rest;
 }
 
-int w4a16_linear_f16(const void* x, const void* packed, const void* scales, void* y, int64_t M, int64_t N,
-                     int64_t K, int64_t group_size, void* workspace, size_t workspace_bytes, uint32_t flags,
-                     w4a16_stream_t stream) {
-    return w4a16_linear_f16_bias(x, packed, scales, nullptr, y, M, N, K, group_size, workspace, workspace_bytes, flags, stream);
-}
-
-int w4a16_linear_f16_bias(const void* x, const void* packed, const void* scales, const void* bias, void* y, int64_t M, int64_t N,
-                          int64_t K, int64_t group_size, void* workspace, size_t workspace_bytes, uint32_t flags,
-                          w4a16_stream_t stream) {
+// w4a16_linear_f16_bias, and w4a16_linear_f16_input without a transform.
+static int linear_f16(const void* x, const void* packed, const void* scales, const void* bias, void* y, int64_t M, int64_t N, int64_t K,
+                      int64_t group_size, void* workspace, size_t workspace_bytes, uint32_t flags, bool among_transforms,
+                      w4a16_stream_t stream) {
     const int status = validate_linear(x, packed, scales, y, M, N, K, group_size);
     if (status != W4A16_OK || M == 0 || N == 0) return status;
     w4a16::LinearProblem p{static_cast<const __half*>(x), static_cast<const uint8_t*>(packed),
                            static_cast<const __half*>(scales), y, M, N, K, group_size,
                            workspace, workspace_bytes};
+    p.among_transforms = among_transforms;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const bool out_f32 = (flags & W4A16_FLAG_OUTPUT_F32) != 0;
     p.bias = static_cast<const __half*>(bias);
@@ -240,11 +236,23 @@ int w4a16_linear_f16_bias(const void* x, const void* packed, const void* scales,
     return W4A16_OK;
 }
 
+int w4a16_linear_f16(const void* x, const void* packed, const void* scales, void* y, int64_t M, int64_t N,
+                     int64_t K, int64_t group_size, void* workspace, size_t workspace_bytes, uint32_t flags,
+                     w4a16_stream_t stream) {
+    return linear_f16(x, packed, scales, nullptr, y, M, N, K, group_size, workspace, workspace_bytes, flags, false, stream);
+}
+
+int w4a16_linear_f16_bias(const void* x, const void* packed, const void* scales, const void* bias, void* y, int64_t M, int64_t N,
+                          int64_t K, int64_t group_size, void* workspace, size_t workspace_bytes, uint32_t flags,
+                          w4a16_stream_t stream) {
+    return linear_f16(x, packed, scales, bias, y, M, N, K, group_size, workspace, workspace_bytes, flags, false, stream);
+}
+
 int w4a16_linear_f16_input(const void* x, const void* packed, const void* scales, void* y, int64_t M, int64_t N,
                            int64_t K, int64_t group_size, void* workspace, size_t workspace_bytes, uint32_t flags,
                            const w4a16_input_transform* transform, w4a16_stream_t stream) {
     if (transform == nullptr || transform->kind == W4A16_INPUT_PLAIN) {
-        return w4a16_linear_f16(x, packed, scales, y, M, N, K, group_size, workspace, workspace_bytes, flags, stream);
+        return linear_f16(x, packed, scales, nullptr, y, M, N, K, group_size, workspace, workspace_bytes, flags, true, stream);
     }
     const int status = validate_linear(x, packed, scales, y, M, N, K, group_size);
     if (status != W4A16_OK || M == 0 || N == 0) return status;
@@ -252,6 +260,7 @@ int w4a16_linear_f16_input(const void* x, const void* packed, const void* scales
     w4a16::LinearProblem p{static_cast<const __half*>(x), static_cast<const uint8_t*>(packed),
                            static_cast<const __half*>(scales), y, M, N, K, group_size,
                            workspace, workspace_bytes, nullptr, transform};
+    p.among_transforms = true;
     int max_splits = 1;
     if (workspace != nullptr && aligned16(workspace)) {
         for (int splits = w4a16::kMaxKSplits; splits > 1; splits >>= 1) {

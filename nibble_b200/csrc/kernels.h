@@ -32,6 +32,9 @@ struct LinearProblem {
     const w4a16_peer_source* source = nullptr;  // x is another sharded layer's published result
     int64_t x_ld = 0;                           // elements between batch rows of x (0: K)
     const __half* bias = nullptr;               // [N], added to the FP16 result (FP16 output only)
+    // The call came through the entry point with input transforms: it gets the build that its neighbours in a chain get, since a
+    // second one only adds code to fetch (a decode step of 22 blocks: one build 516.5 us, the other 519.0, both mixed 524.5).
+    bool among_transforms = false;
 };
 
 // Scale groups the streaming kernel is built for (K a multiple of 128 all the same).

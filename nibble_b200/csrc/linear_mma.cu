@@ -634,6 +634,8 @@ int launch_linear_mma(const LinearProblem& prob, const w4a16_linear_config& cfg_
     if (prob.peers != nullptr || prob.source != nullptr) {
         if (variant.fn_exchange == nullptr) return W4A16_ERR_BAD_CONFIG;
         kernel = variant.fn_exchange;
+    } else if (early_weights && prob.bias == nullptr && !prob.among_transforms && variant.fn_early != nullptr) {
+        kernel = variant.fn_early;
     }
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess) return W4A16_ERR_LAUNCH;

@@ -10,6 +10,7 @@ namespace w4a16 {
 struct Variant {
     const void* fn;
     const void* fn_exchange;   // the build with the tensor-parallel paths; null where it is not instantiated
+    const void* fn_early;      // the build for early weights and no bias; null where it is not instantiated
     int red_bytes;     // shared memory for the cross-warp reduction
     int stage_bytes;   // shared memory of one pipeline stage
     int stages;
@@ -49,6 +50,15 @@ linear_mma_exchange_kernel(const MmaParams p) {
     linear_mma_body<NT, XB, TILES, KW, U, STAGES, kGroup, kFeatExchange>(p, smem, hooks);
 }
 
+// The same kernel for a single row whose weights are in place, without a bias.
+template <int KW, int U, int STAGES>
+__global__ void __launch_bounds__(kThreads, min_ctas_per_sm<1, 1>())
+linear_mma_early_kernel(const MmaParams p) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    KernelHooks hooks;
+    linear_mma_body<1, 1, 1, KW, U, STAGES, kGroup, kFeatEarly>(p, smem, hooks);
+}
+
 template <int NT, int XB, int TILES, int KW, int U, int STAGES, int GROUP>
 Variant variant_of() {
     constexpr int RW = kWarpsPerCta / KW;
@@ -57,7 +67,9 @@ Variant variant_of() {
     if constexpr (TILES == 1 && GROUP == kGroup) {   // sharded layers always run one 16-row tile per warp
         exchange = reinterpret_cast<const void*>(&linear_mma_exchange_kernel<NT, XB, TILES, KW, U, STAGES>);
     }
-    return {reinterpret_cast<const void*>(&linear_mma_kernel<NT, XB, TILES, KW, U, STAGES, GROUP>), exchange, red,
+    const void* early = nullptr;
+    if constexpr (XB == 1 && TILES == 1 && GROUP == kGroup) early = reinterpret_cast<const void*>(&linear_mma_early_kernel<KW, U, STAGES>);
+    return {reinterpret_cast<const void*>(&linear_mma_kernel<NT, XB, TILES, KW, U, STAGES, GROUP>), exchange, early, red,
             stage_bytes<TILES, U, GROUP>(), STAGES, XB};
 }
 

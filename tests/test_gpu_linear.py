@@ -386,3 +386,24 @@ def test_captured_graphs_do_not_depend_on_each_others_replays(m, k, n):
             assert torch.equal(linear_cuda(x, packed, scales, 128), want)
         torch.cuda.synchronize()
     assert torch.equal(linear_cuda(x, packed, scales, 128), want)
+
+
+@pytest.mark.parametrize(("k", "n"), [(128, 5), (384, 77), (2048, 2048), (2048, 5632), (5632, 2047), (28672, 512), (16384, 130)])
+def test_single_row_with_early_weights_gives_the_same_bits(k, n, monkeypatch):
+    """The build for single rows whose weights are in place against the general one, through the C ABI and the module's operator
+    with and without a bias, in a chain in which each call's input is the output of an earlier one."""
+    x, packed, scales = _random_case(1, k, n, seed=k + n, std=0.02)
+    ws = new_workspace(1, n, k)
+    plain = capi_linear(x, packed, scales, workspace=ws)
+    check_against_oracle(plain, x, packed, scales)
+    bias = torch.randn((n,), device="cuda").half()
+    monkeypatch.setenv("W4A16_PDL", "1")
+    for _ in range(4):
+        assert torch.equal(capi_linear(x, packed, scales, workspace=ws, flags=_native.FLAG_PROGRAMMATIC_LAUNCH), plain)
+        assert torch.equal(linear_cuda(x, packed, scales, 128), plain)
+        assert torch.equal(torch.ops.w4a16.linear_bias(x, packed, scales, bias, 128), plain + bias)
+    if n >= 128:
+        back_packed, back_scales = packed[:128, : n // 128 * 64].contiguous(), scales[:128, : max(1, n // 128)].contiguous()
+        if back_packed.shape[1] * 2 == n // 128 * 128 and back_scales.shape[1] == n // 128:
+            chained = linear_cuda(linear_cuda(x, packed, scales, 128)[:, : n // 128 * 128].contiguous(), back_packed, back_scales, 128)
+            assert torch.equal(chained, capi_linear(plain[:, : n // 128 * 128].contiguous(), back_packed, back_scales))
