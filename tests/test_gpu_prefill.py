@@ -249,7 +249,7 @@ def test_gemm_results_do_not_depend_on_timing(m, k, n, gs):
     (512, 1024, 9600), (513, 1024, 9600),      # 4 and 5 batch tiles; from 513 rows on the tiles of one round decide: 5 x 38
     (777, 1024, 5376), (777, 1024, 5377),      # 147 and 154 tiles
     (1024, 2048, 8192), (1025, 2048, 8192), (1024, 1920, 8192),
-    (2048, 8064, 4000), (2048, 8192, 4000),
+    (2048, 3968, 4000), (2048, 4096, 4000), (2048, 4096, 4700),      # 256, 256 and 304 tiles
     (5000, 4096, 1000), (3000, 256, 130),
 ])
 def test_both_gemms_beyond_512_rows(m, k, n):
@@ -273,8 +273,8 @@ def test_both_gemms_beyond_512_rows(m, k, n):
 @pytest.mark.parametrize(("m", "k", "n"), [
     # 128-wide stages: 75 to 148 tiles of 128 channels, up to 128 rows; one stage, odd counts that half use the last copy of codes
     (65, 128, 9600), (128, 384, 9601), (96, 640, 18944), (100, 896, 12345), (128, 1024, 9473), (66, 1024, 18943),
-    # 64-wide stages: more tiles than one round of the other kernel, K below 8192
-    (513, 384, 16385), (700, 640, 12000), (1100, 896, 9001), (1025, 1152, 9216), (2049, 2048, 2500), (2500, 3968, 1930), (1200, 5632, 4900),
+    # 64-wide stages: more tiles than one round of the other kernel (two, from K = 4096 on)
+    (513, 384, 16385), (700, 640, 12000), (1100, 896, 9001), (1025, 1152, 9216), (2049, 2048, 2500), (2500, 3968, 1930), (2000, 5632, 4900),
 ])
 def test_gemm_from_shared_memory(m, k, n):
     """The calls that still take the kernel with its weights in shared memory: odd stage counts, ragged channels and batches,
