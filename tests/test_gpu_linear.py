@@ -407,3 +407,39 @@ def test_single_row_with_early_weights_gives_the_same_bits(k, n, monkeypatch):
         if back_packed.shape[1] * 2 == n // 128 * 128 and back_scales.shape[1] == n // 128:
             chained = linear_cuda(linear_cuda(x, packed, scales, 128)[:, : n // 128 * 128].contiguous(), back_packed, back_scales, 128)
             assert torch.equal(chained, capi_linear(plain[:, : n // 128 * 128].contiguous(), back_packed, back_scales))
+
+
+def test_captured_calls_of_growing_needs_share_one_graph():
+    """Within a capture a call that needs more replaces the graph's buffer, on each of two streams; the next capture and eager
+    calls start afresh."""
+    shapes = [(1, 28672, 8192), (12, 8192, 4096), (128, 8192, 28672), (2, 14336, 4096)]
+    data, want = [], []
+    torch.manual_seed(11)
+    for m, k, n in shapes:
+        assert _native.core().w4a16_linear_scratch_bytes(m, n, k, 128, 0) > 0
+        packed = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda")
+        scales = (torch.rand((n, k // 128), device="cuda") * 0.01 + 1e-3).half()
+        data.append((torch.randn((m, k), device="cuda").half(), packed, scales, 128))
+        want.append(linear_cuda(*data[-1]))
+    torch.cuda.synchronize()
+    main, side = torch.cuda.Stream(), torch.cuda.Stream()
+    graphs = []
+    for _ in range(3):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=main):
+            side.wait_stream(main)
+            outputs = [linear_cuda(*case) for case in data]
+            with torch.cuda.stream(side):
+                outputs += [linear_cuda(*case) for case in reversed(data)]
+            main.wait_stream(side)
+        graphs.append((graph, outputs))
+    for graph, outputs in (graphs[2], graphs[0], graphs[1], graphs[2]):
+        for y in outputs:
+            y.fill_(float("nan"))
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, expected) for y, expected in zip(outputs, want + want[::-1]))
+        with torch.cuda.stream(main):
+            assert all(torch.equal(linear_cuda(*case), expected) for case, expected in zip(data, want))
+        torch.cuda.synchronize()
