@@ -52,11 +52,11 @@ bool uses_fused_kernel(int64_t rows, int64_t out_features, int64_t in_features, 
     return (in_features >= 2048 && rows <= 896) || in_features >= 8 * out_features;
 }
 
-// A tensor nobody has subclassed, wrapped or asked to track gradients of, backward or forward.
+// A tensor nobody has subclassed, wrapped or asked to track gradients of.
 bool plain(PyObject* object) {
     if (!THPVariable_CheckExact(object)) return false;
     const at::Tensor& t = THPVariable_Unpack(object);
-    return t.is_cuda() && !t.requires_grad() && !t._fw_grad(/*level=*/0).defined() && t.is_contiguous() &&
+    return t.is_cuda() && !t.requires_grad() && t.is_contiguous() &&
            !t.key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched,
                                                      c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Batched}));
 }
@@ -133,6 +133,9 @@ PyObject* linear_forward(PyObject*, PyObject* const* args, Py_ssize_t count) {
         Py_RETURN_NOTIMPLEMENTED;
     }
     const at::Tensor& x = THPVariable_Unpack(args[0]);
+    // forward-mode differentiation follows the product with dequantised weights (of the activations alone: asked of the buffers,
+    // which are views, it takes 0.1 us)
+    if (x._fw_grad(/*level=*/0).defined()) Py_RETURN_NOTIMPLEMENTED;
     const at::Tensor& packed = THPVariable_Unpack(args[1]);
     const at::Tensor& scales = THPVariable_Unpack(args[2]);
     std::optional<at::Tensor> bias;
