@@ -368,11 +368,11 @@ int w4a16_decode_step_f16(void* plan, const w4a16_decode_plan_info* info, w4a16_
  * splits K and so never needs scratch.
  *
  * Same arguments and results as w4a16_linear_f16 without the workspace pair.  It allocates and frees
- * nothing.  Calls that need no scratch (other group sizes, misaligned pointers, batches that go to the
- * tcgen05 GEMM) are simply forwarded.  Problems whose split-K scratch, as
- * w4a16_linear_workspace_bytes_flags reports it, exceeds the array return W4A16_ERR_TOO_LARGE and launch
- * nothing.  All calls on a device share the one array: calls that may overlap on the GPU (several
- * streams, parallel graph branches) race; calls ordered on one stream do not.  The first call on
+ * nothing.  Calls that share nothing through scratch (most; w4a16_linear_scratch_bytes) are simply
+ * forwarded, and so are those of the GEMMs whose need exceeds the array, which run without.  Other
+ * problems whose need exceeds it return W4A16_ERR_TOO_LARGE and launch nothing.  All calls on a device
+ * share the one array: calls that may overlap on the GPU (several streams, parallel graph branches)
+ * race; calls ordered on one stream do not.  The first call on
  * each device resolves the array's address and should be made outside stream capture.
  */
 int w4a16_linear_f16_static_scratch(const void* x, const void* packed, const void* scales, void* y,

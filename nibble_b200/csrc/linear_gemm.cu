@@ -1,5 +1,5 @@
 // W4A16 linear for prompts and medium batches on the 5th-generation tensor cores: the weights are dequantised straight into
-// tensor memory (TMEM) and enter the MMA from there, and the K blocks of all output tiles are dealt out evenly to the SMs.
+// tensor memory (TMEM) and enter the MMA from there, and the K blocks of output tiles are shared between SMs where that pays.
 //
 //   D[2 x 128 x BN] (TMEM, FP32)  +=  A[2 x 128 x 128] (TMEM: FP16 weights)  x  B[BN x 128] (shared memory: rows of x)
 //
@@ -8,8 +8,10 @@
 // What bounds it.  A K block of 256 weight rows is 32768 weights: 620 issue slots of each SM quarter to unpack (sixteen
 // instructions per word of eight codes), 8 clocks of MMA per batch row, 16 MMAs to issue at about 40 clocks each, and 16 KB
 // of codes plus 256 bytes per batch row out of L2, which gives an SM some 50 bytes per clock.  Hence 256 rows: with 128, the x
-// tile of a 128-row batch alone took the whole of that.  Measured: 1160 clocks a block up to 64 batch rows (the chain of
-// waits, unpacking and stores of the three dequantiser groups; two groups: 1420), 1420 at 128 rows (the MMAs' 1024).
+// tile of a 128-row batch alone took the whole of that.  Measured from the time against K, weights from HBM (K from 2048 to 16384):
+// 0.8 to 1.0 us a block at 64 batch rows (the chain of waits, unpacking and stores of the three dequantiser groups; two groups
+// took a quarter more), 1.1 to 1.3 us at 128, of which the MMAs are 0.55; and 7 to 8 us of start, exchange and end beside them, a
+// tenth to a third of a call: tensor pipe active 41 % of the time (128 rows, 8192 -> 28672).
 //
 // linear_tcgen05.cu writes the FP16 tile to shared memory instead; the store, a proxy fence and the space that takes make it
 // 1.2 to 1.9 times slower here.
