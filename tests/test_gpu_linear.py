@@ -443,3 +443,28 @@ def test_captured_calls_of_growing_needs_share_one_graph():
         with torch.cuda.stream(main):
             assert all(torch.equal(linear_cuda(*case), expected) for case, expected in zip(data, want))
         torch.cuda.synchronize()
+
+
+def test_one_workspace_serves_calls_that_share_tiles_through_it():
+    """Streaming splits of several shapes and the GEMM's equal runs, back to back through one workspace: each uses it (the exact
+    query says so), none leaves anything where another keeps its counters."""
+    lib = _native.core()
+    ws = torch.zeros(40 << 20, dtype=torch.uint8, device="cuda")
+    torch.manual_seed(5)
+    shapes = [(1, 28672, 8192), (1, 16384, 512), (6, 14336, 4096), (128, 8192, 28672), (1, 16384, 320), (12, 8192, 4096),
+              (40, 8192, 28672), (1, 28672, 8192), (2, 28672, 2560)]
+    calls = []
+    for m, k, n in shapes:
+        need = lib.w4a16_linear_scratch_bytes(m, n, k, 128, 0)
+        assert 0 < need <= ws.numel(), (m, k, n)
+        packed = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda")
+        scales = (torch.rand((n, k // 128), device="cuda") * 0.002 + 0.001).half()
+        x = torch.randn((m, k), device="cuda").half()
+        calls.append((capi_linear(x, packed, scales, workspace=ws), x, packed, scales))
+    torch.cuda.synchronize()
+    for y, x, packed, scales in calls:
+        n = packed.shape[0]
+        assert not torch.isnan(y).any()
+        rows = np.unique(np.concatenate([np.arange(0, n, max(1, n // 50)), np.arange(n - 20, n)]))
+        check_against_oracle(y, x, packed, scales, rows=rows, fp16_weights=x.shape[0] > 16)
+    assert int(ws[: 256 * 1024].sum()) == 0, "arrival counters must be back at zero"
