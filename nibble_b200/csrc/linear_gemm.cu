@@ -79,24 +79,22 @@ struct GemmParams {
     int x_slots, code_slots; // blocks of x and of codes in flight
     int slots;               // blocks of weights in TMEM
     int cluster;             // CTAs that share a tile (1: runs)
-    int tiles;
-    int units;               // tiles x k_blocks
+    int run, longer;         // units (tile, K block) of a CTA's run, or its tiles where runs are whole tiles; the first `longer` CTAs
+                             // take one more
 };
 
-// CTA c takes units first_unit(c) .. first_unit(c + 1) - 1.
+// CTA c takes units first_unit(c) .. first_unit(c + 1) - 1.  The host has divided: a 64-bit division here took each CTA a
+// microsecond at its start, and the search for a unit's owner several while a tile's parts waited (8192 -> 28672, 128 rows: 64.0
+// -> 60.4 us; 8192 x 8192, 512 rows: 61.7 -> 57.8).
 __device__ __forceinline__ int first_unit(const GemmParams& p, int c) {
     if (p.cluster > 1) return c / p.cluster * p.k_blocks + p.k_blocks * (c % p.cluster) / p.cluster;
-    const int whole = p.partial != nullptr ? p.units : p.tiles;
-    const int first = static_cast<int>(static_cast<long long>(whole) * c / static_cast<int>(gridDim.x));
+    const int first = c * p.run + min(c, p.longer);
     return p.partial != nullptr ? first : first * p.k_blocks;
 }
-// The CTA whose run holds unit u (runs are never empty).
+// The CTA whose run holds unit u, where runs may cut tiles (they are never empty).
 __device__ __forceinline__ int owner_of(const GemmParams& p, int u) {
-    const int grid = static_cast<int>(gridDim.x);
-    int c = static_cast<int>(static_cast<long long>(u) * grid / p.units);
-    while (c + 1 < grid && first_unit(p, c + 1) <= u) ++c;
-    while (c > 0 && first_unit(p, c) > u) --c;
-    return c;
+    const unsigned unit = u, in_longer = static_cast<unsigned>(p.longer) * (p.run + 1);
+    return unit < in_longer ? unit / (p.run + 1) : p.longer + (unit - in_longer) / p.run;
 }
 
 // Which CTAs hold parts of a tile, and where the first of them keeps it (the others: part 0, they start inside the tile).
@@ -805,8 +803,9 @@ int launch_linear_gemm(const LinearProblem& prob, cudaStream_t stream) {
     params.slots = g.bn <= 64 ? 3 : 2;
     params.cluster = g.cluster;
     params.m_tiles = g.m_tiles;
-    params.tiles = static_cast<int>(g.tiles);
-    params.units = static_cast<int>(g.tiles) * g.k_blocks;
+    const long long pieces = params.partial != nullptr ? g.tiles * g.k_blocks : g.tiles;
+    params.run = static_cast<int>(pieces / g.grid);
+    params.longer = static_cast<int>(pieces % g.grid);
 
     const void* kernel = gemm_kernel(prob.group);
     cudaLaunchConfig_t launch = {};
