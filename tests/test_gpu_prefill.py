@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 import torch
 
-from capi_helpers import capi_linear, check_against_oracle, new_workspace
+from capi_helpers import capi_dequantize, capi_linear, check_against_oracle, new_workspace
 from nibble_b200 import _native, quantize_and_pack_weights
 from oracle import w4a16_oracle as oracle
 
@@ -296,4 +296,27 @@ def test_gemm_from_shared_memory(m, k, n):
         assert torch.equal(capi_linear(x, packed, scales), y)
     bias = torch.randn((n,), device="cuda").half()
     assert torch.equal(torch.ops.w4a16.linear_bias(x, packed, scales, bias, 128), y + bias)
+    assert _device_status() == 0
+
+
+@pytest.mark.parametrize("gs", [128, 64, 32])
+def test_gemm_weights_are_rounded_products_for_any_scale(gs):
+    """Single ones as activations read the weights of the GEMM out: half(code * scale) whatever the scale, either side of the line
+    where warps of small scales take an FMA on (code + 8) * 2^-20 (its largest scale is 65504 / 2^20, FP16 bits 0x2BFF)."""
+    k, n = 512, 300
+    g = torch.Generator().manual_seed(gs)
+    packed = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, generator=g).cuda()
+    bits = torch.randint(1, 0x2BFF, (n, k // gs), generator=g)                       # subnormal scales among them
+    edges = torch.tensor([0x0001, 0x03FF, 0x0400, 0x2BFE, 0x2BFF, 0x2C00, 0x3C00, 0x6B00, 0x0000, 0xABFF, 0xAC00, 0x8001])
+    bits[64:128] = edges[torch.randint(0, len(edges), (64, k // gs), generator=g)]   # mixed in two warps of a tile
+    bits[128:192] = torch.where(bits[128:192] % 2 == 0, 0x2BFF, 0xABFF)              # on the line, in all of them
+    scales = bits.to(torch.int16).view(torch.float16).cuda()
+    weights = capi_dequantize(packed, scales, gs)
+    flags = _native.FLAG_FORCE_TCGEN05
+    _device_status()
+    for first in range(0, k, 128):
+        x = torch.zeros((128, k), dtype=torch.float16, device="cuda")
+        x[torch.arange(128), first + torch.arange(128)] = 1.0
+        y = capi_linear(x, packed, scales, gs, flags=flags)
+        torch.testing.assert_close(y, weights[:, first:first + 128].t(), rtol=0, atol=0)
     assert _device_status() == 0
