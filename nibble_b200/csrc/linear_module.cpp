@@ -34,22 +34,23 @@ c10::TypedOperatorHandle<Signature> operator_handle(const char* name) {
 // Whether a batch goes to the fused operator, or is multiplied by dequantised FP16 weights (same arithmetic from 65 rows
 // on: weights rounded to FP16, FP32 sums).  linear.py states the same rule (takes_operator) for the calls that stay in Python; a
 // test holds the two together.  The lines come from times of both, eager calls back to back, on 76 layers from 512 x 2048 to
-// 28672 x 8192 at 129 to 2048 rows (us, the operator / dequantise and multiply; the latter is 14 us of host time at least):
+// 28672 x 8192 up to 512 rows (us, the operator / dequantise and multiply; the latter is 14 us of host time at least):
 //   - cuBLAS falls off its fast kernels where an output row is no multiple of 16 bytes (9216 -> 2575, 128 rows: 20 / 125);
 //   - up to 512 rows the operator (2048 -> 2560, 400 rows: 15 / 15; 4096 -> 11008, 256 rows: 41 / 50), but for layers of many tiles
 //     of a few K blocks each above 256 rows (512 -> 28672, 512 rows: 37 / 29).  0.2 to 0.6 % slower than the better on average;
-//   - 513 to 1024 rows: small layers (1024 -> 4096, 777 rows: 13 / 17), all but shallow ones up to seven batch tiles of 128 rows
-//     (8192 -> 28672, 777 rows: 406 / 401; 11008 -> 1024, 777 rows: 28 / 34), narrow deep ones (16384 -> 1024, 1024 rows: 39 / 45).
-//     2 % slower than the better on average, 36 % at most (896 -> 6448, 520 rows: 12 / 17);
-//   - above, the matrix product at cuBLAS's rate outweighs the weights' round trip (8192 -> 28672, 2048 rows: 1094 / 919).
+//   - 513 to 2048 rows: layers whose 256 x 128 tiles fit one round of SMs (1024 -> 4096, 1024 rows: 12 / 18; 2048 -> 2048, 2048 rows:
+//     18 / 23), and to 1024 rows all with K >= 2048 (8192 -> 28672: 777 rows 355 / 431, 1024 rows 429 / 559; 2048 -> 28672, 777 rows:
+//     112 / 108, the worst), measured on 30 layers with 30 ms of calls each, so that the clocks are those of a long run;
+//   - above, the matrix product at cuBLAS's rate outweighs the weights' round trip, or is level with the operator on one box and a
+//     tenth faster on the next (8192 -> 28672, 2048 rows: 900 / 930, 984 / 896).
 bool uses_fused_kernel(int64_t rows, int64_t out_features, int64_t in_features, int64_t group_size) {
     if (rows <= 64) return true;
     if (group_size % 32 != 0) return true;
     if (group_size > 128 || in_features % 128 != 0) return false;      // the operator has no tensor-core kernel for these
     if (out_features % 8 != 0 || rows <= 256) return true;
-    if (rows > 1024 || out_features > 20 * in_features) return false;
-    if (rows <= 512 || out_features * in_features <= 4 << 20) return true;
-    return (in_features >= 2048 && rows <= 896) || in_features >= 8 * out_features;
+    if (rows <= 512) return out_features <= 20 * in_features;
+    if (rows > 2048) return false;
+    return (out_features + 255) / 256 * ((rows + 127) / 128) <= 148 || (rows <= 1024 && in_features >= 2048);
 }
 
 // A tensor nobody has subclassed, wrapped or asked to track gradients of.
