@@ -124,18 +124,18 @@ int launch_streaming(const w4a16::LinearProblem& p, bool small_group, uint32_t f
 //   - up to 512 rows the first (8192 -> 28672: 128 rows 66 / 88, 384 rows 195 / 219), but for batches up to 128 rows on a
 //     short K whose 128-row tiles just fit one round of SMs: nothing to share, and the second starts faster (K = 512 to 1024, N from
 //     9728 to 18944: the first 10 to 25 % slower; 1024 -> 12928, 128 rows: 12.6 / 10.9);
-//   - above, from the times of both on 114 layers from 512 x 512 to 28672 x 8192 at eleven batches of 520 to 3000 rows: the first
-//     where its tiles fit one round (4096 -> 1024, 1536 rows: 21.9 / 32.5), or K is 3072 and more (8192 -> 28672, 2048 rows: 859 /
-//     942), or 2048 and more up to 1024 rows (2048 -> 14336, 777 rows: 53 / 66); elsewhere a 256-row batch tile reads x half as
-//     often (2048 -> 28672, 1536 rows: 199 / 181).  On average 0.6 % slower than the better of the two, and 0.8 % on 63 layers at
-//     2500 to 16384 rows.
+//   - above, from the times of both on 117 layers from 512 x 256 to 28672 x 8192 at eleven batches of 513 to 8192 rows: the first
+//     where its tiles fit one round (28 % less on average; 4096 -> 256, 2048 rows: 19 / 36), two with a long K (28672 -> 4096, 1536
+//     rows: 338 / 422), or K is 2048 and more up to 1024 rows (8192 -> 28672, 777 rows: 369 / 433); elsewhere a 256-row batch tile
+//     reads x half as often (1024 -> 28672, 1536 rows: 126 / 100; 8192 -> 28672, 2048 rows: 954 / 887).  On average 0.4 to 0.6 %
+//     slower than the better of the two, never more than 17 %.
 bool w4a16::gemm_from_tensor_memory(int64_t M, int64_t N, int64_t K) {
     if (M <= 512) {
         const int64_t tiles = (N + 127) / 128;
         return !(M <= 128 && K <= 1024 && tiles > 74 && tiles <= 148);
     }
     const int64_t tiles = (N + 255) / 256 * ((M + 127) / 128);
-    return tiles <= 148 || K >= (M <= 1024 ? 2048 : 3072);
+    return tiles <= 148 || (tiles <= 296 && K >= 4096) || (M <= 1024 && K >= 2048);
 }
 
 bool w4a16::linear_routes_to_tcgen05(int64_t M, int64_t N, int64_t K, uint32_t flags) {
