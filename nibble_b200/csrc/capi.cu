@@ -78,9 +78,40 @@ bool routes_to_tcgen05(int64_t M, int64_t N, int64_t K, uint32_t flags) {
     return gemm_us < (M <= 16 ? 0.85 : 1.0) * streaming_us;
 }
 
+// Which GEMM takes a call.  us, in the order below:
+//   - kPair, pairs of SMs with whole tiles of 256 weight rows x up to 256 batch rows, where its time by the two models is the
+//     shorter one: 8192 -> 28672, 2048 rows 740 to 800 / 910 to 1060 / -; 8192 x 8192, 512 rows 59 / 67 / -; 1024 -> 8192, 128 rows
+//     0.67 of the second.  Up to 128 rows, one batch tile of the second, only in one round of pairs: in two they are level
+//     (8192 -> 28672, 96 rows: 63 / 55);
+//   - kTensorMemory, single SMs with up to 128 batch rows a tile, K of few tiles shared, up to 512 rows, and above where its tiles
+//     fit a round, two with K >= 4096, or K >= 2048 up to 1024 rows: beyond, the first is the faster one whatever the models say
+//     (157 calls, at most 1 % slower);
+//   - kSharedMemory, 128 x up to 128 with the weights in shared memory, which starts faster: up to 128 rows with K <= 1024 where
+//     its tiles just fit a round (512 -> 18944, 65 rows: 7.4 / - / 7.0).
+enum class Gemm { kPair, kTensorMemory, kSharedMemory };
+Gemm gemm_for(int64_t M, int64_t N, int64_t K, int64_t group) {
+    if (M <= 64 || M > INT32_MAX || N > INT32_MAX || K > INT32_MAX) {
+        // (M <= 64: 9 to 64 rows, and whatever a flag sends)
+        return group == w4a16::kGroupFast && M <= 128 && K <= 1024 && (N + 127) / 128 > 74 && (N + 127) / 128 <= 148 ? Gemm::kSharedMemory
+                                                                                                                      : Gemm::kTensorMemory;
+    }
+    if (M <= 128) {
+        const int64_t tiles = (N + 127) / 128;
+        if (group == w4a16::kGroupFast && K <= 1024 && tiles > 74 && tiles <= 148) return Gemm::kSharedMemory;
+        return w4a16::gemm_pair_rounds(M, N) == 1 && w4a16::gemm_pair_time(M, N, K) < w4a16::gemm_time(M, N, K) ? Gemm::kPair
+                                                                                                              : Gemm::kTensorMemory;
+    }
+    const int64_t tiles = (N + 255) / 256 * ((M + 127) / 128);
+    const bool few = M <= 512 || tiles <= 148 || (tiles <= 296 && K >= 4096) || (M <= 1024 && K >= 2048);
+    return few && w4a16::gemm_time(M, N, K) <= w4a16::gemm_pair_time(M, N, K) ? Gemm::kTensorMemory : Gemm::kPair;
+}
+
 int launch_gemm(const w4a16::LinearProblem& p, cudaStream_t stream) {
-    const bool tensor_memory = p.group != w4a16::kGroupFast || w4a16::gemm_from_tensor_memory(p.M, p.N, p.K);
-    return tensor_memory ? w4a16::launch_linear_gemm(p, stream) : w4a16::launch_linear_tcgen05(p, stream);
+    switch (gemm_for(p.M, p.N, p.K, p.group)) {
+        case Gemm::kPair: return w4a16::launch_linear_gemm_pair(p, stream);
+        case Gemm::kTensorMemory: return w4a16::launch_linear_gemm(p, stream);
+        default: return w4a16::launch_linear_tcgen05(p, stream);
+    }
 }
 
 // Whether a call with 64- or 32-wide groups goes to the GEMM, which rounds each weight to FP16.  Only where the caller has said
@@ -118,25 +149,6 @@ int launch_streaming(const w4a16::LinearProblem& p, bool small_group, uint32_t f
 }
 
 }  // namespace
-
-// Which GEMM takes a call: weights in tensor memory (256 weight rows x up to 128 batch rows a tile, K of few tiles shared), or in
-// shared memory (128 x up to 256).  us, the first / the second:
-//   - up to 512 rows the first (8192 -> 28672: 128 rows 66 / 88, 384 rows 195 / 219), but for batches up to 128 rows on a
-//     short K whose 128-row tiles just fit one round of SMs: nothing to share, and the second starts faster (K = 512 to 1024, N from
-//     9728 to 18944: the first 10 to 25 % slower; 1024 -> 12928, 128 rows: 12.6 / 10.9);
-//   - above, from the times of both on 117 layers from 512 x 256 to 28672 x 8192 at eleven batches of 513 to 8192 rows: the first
-//     where its tiles fit one round (28 % less on average; 4096 -> 256, 2048 rows: 19 / 36), two with a long K (28672 -> 4096, 1536
-//     rows: 338 / 422), or K is 2048 and more up to 1024 rows (8192 -> 28672, 777 rows: 369 / 433); elsewhere a 256-row batch tile
-//     reads x half as often (1024 -> 28672, 1536 rows: 126 / 100; 8192 -> 28672, 2048 rows: 954 / 887).  On average 0.4 to 0.6 %
-//     slower than the better of the two, never more than 17 %.
-bool w4a16::gemm_from_tensor_memory(int64_t M, int64_t N, int64_t K) {
-    if (M <= 512) {
-        const int64_t tiles = (N + 127) / 128;
-        return !(M <= 128 && K <= 1024 && tiles > 74 && tiles <= 148);
-    }
-    const int64_t tiles = (N + 255) / 256 * ((M + 127) / 128);
-    return tiles <= 148 || (tiles <= 296 && K >= 4096) || (M <= 1024 && K >= 2048);
-}
 
 bool w4a16::linear_routes_to_tcgen05(int64_t M, int64_t N, int64_t K, uint32_t flags) {
     return routes_to_tcgen05(M, N, K, flags);
@@ -186,7 +198,7 @@ size_t w4a16_linear_scratch_bytes(int64_t M, int64_t N, int64_t K, int64_t group
     if (flags & W4A16_FLAG_FORCE_GENERIC) return 0;
     const bool small_group = group_size != w4a16::kGroupFast;
     if (small_group ? small_group_routes_to_gemm(M, flags) : routes_to_tcgen05(M, N, K, flags)) {
-        return small_group || w4a16::gemm_from_tensor_memory(M, N, K) ? w4a16::gemm_scratch_bytes(M, N, K) : 0;
+        return gemm_for(M, N, K, group_size) == Gemm::kTensorMemory ? w4a16::gemm_scratch_bytes(M, N, K) : 0;
     }
     auto streaming = [&](int64_t rows) {
         return w4a16::linear_workspace_bytes_for(

@@ -63,8 +63,12 @@ int launch_linear_tcgen05(const LinearProblem& p, cudaStream_t stream);
 int launch_linear_gemm(const LinearProblem& p, cudaStream_t stream);
 // Bytes of workspace that launch_linear_gemm uses on the current device: counters and parts of tiles that equal runs cut, or 0.
 size_t gemm_scratch_bytes(int64_t M, int64_t N, int64_t K);
-// Which of the two takes a call with 128-wide groups.
-bool gemm_from_tensor_memory(int64_t M, int64_t N, int64_t K);
+// The same on pairs of SMs, up to 256 batch rows a tile (linear_gemm_pair.cu); no workspace.
+int launch_linear_gemm_pair(const LinearProblem& p, cudaStream_t stream);
+// Times of the last two by their models (us), for the choice between them, and rounds of pairs.
+double gemm_time(int64_t M, int64_t N, int64_t K);
+double gemm_pair_time(int64_t M, int64_t N, int64_t K);
+int gemm_pair_rounds(int64_t M, int64_t N);
 // Status word of these kernels (non-zero: a bounded barrier wait gave up); reading clears it and synchronises.
 int read_tcgen05_status(unsigned* value);
 constexpr int kTcgen05MinRows = 65;     // from here on every fast-path call with FP16 output takes the GEMM

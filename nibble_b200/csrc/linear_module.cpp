@@ -33,24 +33,23 @@ c10::TypedOperatorHandle<Signature> operator_handle(const char* name) {
 
 // Whether a batch goes to the fused operator, or is multiplied by dequantised FP16 weights (same arithmetic from 65 rows
 // on: weights rounded to FP16, FP32 sums).  linear.py states the same rule (takes_operator) for the calls that stay in Python; a
-// test holds the two together.  The lines come from times of both, eager calls back to back, on 76 layers from 512 x 2048 to
-// 28672 x 8192 up to 512 rows (us, the operator / dequantise and multiply; the latter is 14 us of host time at least):
+// test holds the two together.  The lines come from times of both on 34 layers from 512 x 1024 to 28672 x 8192 at 160 to 8192 rows,
+// back to back for 12 ms and more, so that the clocks are those of a long run (us, the operator / dequantise and multiply; the
+// latter is 14 us of host time at least):
 //   - cuBLAS falls off its fast kernels where an output row is no multiple of 16 bytes (9216 -> 2575, 128 rows: 20 / 125);
-//   - up to 512 rows the operator (2048 -> 2560, 400 rows: 15 / 15; 4096 -> 11008, 256 rows: 41 / 50), but for layers of many tiles
-//     of a few K blocks each above 256 rows (512 -> 28672, 512 rows: 37 / 29).  0.2 to 0.6 % slower than the better on average;
-//   - 513 to 2048 rows: layers whose 256 x 128 tiles fit one round of SMs (1024 -> 4096, 1024 rows: 12 / 18; 2048 -> 2048, 2048 rows:
-//     18 / 23), and to 1024 rows all with K >= 2048 (8192 -> 28672: 777 rows 355 / 431, 1024 rows 429 / 559; 2048 -> 28672, 777 rows:
-//     112 / 108, the worst), measured on 30 layers with 30 ms of calls each, so that the clocks are those of a long run;
-//   - above, the matrix product at cuBLAS's rate outweighs the weights' round trip, or is level with the operator on one box and a
-//     tenth faster on the next (8192 -> 28672, 2048 rows: 900 / 930, 984 / 896).
+//   - up to 512 rows the operator, never slower (8192 -> 28672, 512 rows: 201 / 374);
+//   - 513 to 1024 rows: all but shallow layers (8192 x 8192, 1024 rows: 115 / 153; 512 -> 28672, 777 rows: 1.16 times as long).
+//     0.6 % slower than the better on average;
+//   - to 4096 rows: layers with K >= 2048 (8192 -> 28672, 2048 rows: 740 to 800 / 930 to 990; 4096 x 4096: 60 / 68; 8192 -> 1024, 1536
+//     rows, the worst: 1.19 times as long) and those whose 256 x 128 tiles fit one round of SMs.  1.1 %;
+//   - above, the weights' round trip costs little beside the product (8192 -> 28672, 8192 rows: 1.02 times as long).
 bool uses_fused_kernel(int64_t rows, int64_t out_features, int64_t in_features, int64_t group_size) {
     if (rows <= 64) return true;
     if (group_size % 32 != 0) return true;
     if (group_size > 128 || in_features % 128 != 0) return false;      // the operator has no tensor-core kernel for these
     if (out_features % 8 != 0 || rows <= 256) return true;
-    if (rows <= 512) return out_features <= 20 * in_features;
-    if (rows > 2048) return false;
-    return (out_features + 255) / 256 * ((rows + 127) / 128) <= 148 || (rows <= 1024 && in_features >= 2048);
+    if (rows <= 1024) return rows <= 512 || out_features <= 20 * in_features;
+    return rows <= 4096 && (in_features >= 2048 || (out_features + 255) / 256 * ((rows + 127) / 128) <= 148);
 }
 
 // A tensor nobody has subclassed, wrapped or asked to track gradients of.

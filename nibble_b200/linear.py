@@ -32,11 +32,9 @@ def takes_operator(rows: int, out_features: int, in_features: int, group_size: i
         return False     # the operator has no tensor-core kernel for these
     if out_features % 8 or rows <= 256:
         return True
-    if rows <= 512:
-        return out_features <= 20 * in_features
-    if rows > 2048:
-        return False
-    return -(-out_features // 256) * -(-rows // 128) <= 148 or (rows <= 1024 and in_features >= 2048)
+    if rows <= 1024:
+        return rows <= 512 or out_features <= 20 * in_features
+    return rows <= 4096 and (in_features >= 2048 or -(-out_features // 256) * -(-rows // 128) <= 148)
 
 
 # The coarse rule for activations whose arithmetic has to stay visible as torch operators (below), where speed is not the point:

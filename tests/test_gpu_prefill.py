@@ -320,3 +320,37 @@ def test_gemm_weights_are_rounded_products_for_any_scale(gs):
         y = capi_linear(x, packed, scales, gs, flags=flags)
         torch.testing.assert_close(y, weights[:, first:first + 128].t(), rtol=0, atol=0)
     assert _device_status() == 0
+
+
+@pytest.mark.parametrize(("m", "k", "n", "gs"), [
+    (65, 1024, 513, 128),      # 96 rows, 48 to an SM; one channel in the last tile, none for its second SM
+    (128, 384, 300, 128),      # fewer blocks than weight slots
+    (96, 2048, 12000, 128), (200, 2048, 18900, 128),   # one tile a pair; codes and x go round their rings
+    (700, 640, 12000, 128),    # three batch tiles of 256; two tiles and more a pair: the accumulator is handed back
+    (1500, 2048, 4096, 128), (1100, 384, 9001, 128),
+    (3000, 128, 5000, 128),    # one K block a tile
+    (2050, 256, 2500, 128),
+    (1030, 896, 2000, 64), (1300, 640, 5001, 64), (2100, 384, 3100, 32),
+])
+def test_gemm_on_pairs_of_sms(m, k, n, gs):
+    """Calls that the pair kernel takes (they need no scratch), against the product with the same FP16 weights, with and without a
+    bias; the same bits again, and nothing outside the output."""
+    from nibble_b200 import dequantize_cuda
+
+    lib, flags = _native.core(), _native.FLAG_FP16_WEIGHTS
+    assert lib.w4a16_linear_scratch_bytes(m, n, k, gs, flags) == 0
+    _device_status()
+    torch.manual_seed(m + k)
+    packed, scales = quantize_and_pack_weights(torch.randn((n, k), device="cuda") * 0.02, gs)
+    x = torch.randn((m, k), device="cuda").half()
+    want = x.float() @ dequantize_cuda(packed, scales, gs).float().t()
+    before = lib.w4a16_launch_count()
+    y = capi_linear(x, packed, scales, gs, flags=flags)
+    assert lib.w4a16_launch_count() == before + 1
+    # FP32 sums in two orders, each within K * 2^-24 of the products' magnitudes, and one rounding to FP16
+    torch.testing.assert_close(y.float(), want, rtol=2e-3, atol=2e-3)
+    for _ in range(10):
+        assert torch.equal(capi_linear(x, packed, scales, gs, flags=flags), y)
+    bias = torch.randn((n,), device="cuda").half()
+    assert torch.equal(torch.ops.w4a16.linear_bias(x, packed, scales, bias, gs), y + bias)
+    assert _device_status() == 0
