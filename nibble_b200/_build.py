@@ -28,7 +28,7 @@ CORE_LIB = PKG / "libw4a16_b200.so"
 CHECKED_LIB = PKG / "libw4a16_b200_checked.so"
 TORCH_LIB = PKG / "_C.so"
 
-CUDA_SOURCES = ["capi.cu", "linear_mma.cu", "linear_mma_groups.cu", "linear_generic.cu", "dequantize.cu", "linear_static_scratch.cu", "linear_tcgen05.cu", "linear_gemm.cu", "linear_gemm_pair.cu", "quantize.cu", "decode_ops.cu", "decode_persistent.cu"]
+CUDA_SOURCES = ["capi.cu", "linear_mma.cu", "linear_mma_groups.cu", "linear_generic.cu", "dequantize.cu", "linear_static_scratch.cu", "linear_gemm.cu", "linear_gemm_pair.cu", "quantize.cu", "decode_ops.cu", "decode_persistent.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-std=c++20", "-lineinfo",

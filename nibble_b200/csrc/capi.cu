@@ -78,40 +78,23 @@ bool routes_to_tcgen05(int64_t M, int64_t N, int64_t K, uint32_t flags) {
     return gemm_us < (M <= 16 ? 0.85 : 1.0) * streaming_us;
 }
 
-// Which GEMM takes a call.  us, in the order below:
-//   - kPair, pairs of SMs with whole tiles of 256 weight rows x up to 256 batch rows, where its time by the two models is the
-//     shorter one: 8192 -> 28672, 2048 rows 740 to 800 / 910 to 1060 / -; 8192 x 8192, 512 rows 59 / 67 / -; 1024 -> 8192, 128 rows
-//     0.67 of the second.  Up to 128 rows, one batch tile of the second, only in one round of pairs: in two they are level
-//     (8192 -> 28672, 96 rows: 63 / 55);
-//   - kTensorMemory, single SMs with up to 128 batch rows a tile, K of few tiles shared, up to 512 rows, and above where its tiles
-//     fit a round, two with K >= 4096, or K >= 2048 up to 1024 rows: beyond, the first is the faster one whatever the models say
-//     (157 calls, at most 1 % slower);
-//   - kSharedMemory, 128 x up to 128 with the weights in shared memory, which starts faster: up to 128 rows with K <= 1024 where
-//     its tiles just fit a round (512 -> 18944, 65 rows: 7.4 / - / 7.0).
-enum class Gemm { kPair, kTensorMemory, kSharedMemory };
-Gemm gemm_for(int64_t M, int64_t N, int64_t K, int64_t group) {
-    if (M <= 64 || M > INT32_MAX || N > INT32_MAX || K > INT32_MAX) {
-        // (M <= 64: 9 to 64 rows, and whatever a flag sends)
-        return group == w4a16::kGroupFast && M <= 128 && K <= 1024 && (N + 127) / 128 > 74 && (N + 127) / 128 <= 148 ? Gemm::kSharedMemory
-                                                                                                                      : Gemm::kTensorMemory;
-    }
-    if (M <= 128) {
-        const int64_t tiles = (N + 127) / 128;
-        if (group == w4a16::kGroupFast && K <= 1024 && tiles > 74 && tiles <= 148) return Gemm::kSharedMemory;
-        return w4a16::gemm_pair_rounds(M, N) == 1 && w4a16::gemm_pair_time(M, N, K) < w4a16::gemm_time(M, N, K) ? Gemm::kPair
-                                                                                                              : Gemm::kTensorMemory;
-    }
+// Whether a call that goes to a GEMM takes the one on pairs of SMs, with whole tiles of 256 weight rows x up to 256 batch rows, or the
+// one on single SMs, with up to 128 batch rows a tile and the K of few tiles shared.  By their models' times (us, pairs / single SMs:
+// 8192 -> 28672, 2048 rows 740 to 800 / 910 to 1060; 8192 x 8192, 512 rows 59 / 67; 5632 -> 2048, 777 rows 30 / 24), with two lines:
+//   - up to 128 rows, one batch tile of the second kernel, only in one round of pairs: in two they are level (8192 -> 28672, 96 rows:
+//     63 / 55; in one, 1024 -> 8192, 128 rows: 7.0 / 10.4);
+//   - above 512 rows the second kernel only where its tiles fit a round, two with K >= 4096, or K >= 2048 up to 1024 rows: beyond,
+//     the first is the faster one whatever the models say (157 calls, at most 1 % slower).
+bool gemm_on_pairs(int64_t M, int64_t N, int64_t K) {
+    if (M <= 64 || M > INT32_MAX || N > INT32_MAX || K > INT32_MAX) return false;     // (9 to 64 rows, and whatever a flag sends)
+    if (M <= 128 && w4a16::gemm_pair_rounds(M, N) != 1) return false;
     const int64_t tiles = (N + 255) / 256 * ((M + 127) / 128);
-    const bool few = M <= 512 || tiles <= 148 || (tiles <= 296 && K >= 4096) || (M <= 1024 && K >= 2048);
-    return few && w4a16::gemm_time(M, N, K) <= w4a16::gemm_pair_time(M, N, K) ? Gemm::kTensorMemory : Gemm::kPair;
+    if (M > 512 && tiles > 148 && !(tiles <= 296 && K >= 4096) && !(M <= 1024 && K >= 2048)) return true;
+    return w4a16::gemm_pair_time(M, N, K) < w4a16::gemm_time(M, N, K);
 }
 
 int launch_gemm(const w4a16::LinearProblem& p, cudaStream_t stream) {
-    switch (gemm_for(p.M, p.N, p.K, p.group)) {
-        case Gemm::kPair: return w4a16::launch_linear_gemm_pair(p, stream);
-        case Gemm::kTensorMemory: return w4a16::launch_linear_gemm(p, stream);
-        default: return w4a16::launch_linear_tcgen05(p, stream);
-    }
+    return gemm_on_pairs(p.M, p.N, p.K) ? w4a16::launch_linear_gemm_pair(p, stream) : w4a16::launch_linear_gemm(p, stream);
 }
 
 // Whether a call with 64- or 32-wide groups goes to the GEMM, which rounds each weight to FP16.  Only where the caller has said
@@ -198,7 +181,7 @@ size_t w4a16_linear_scratch_bytes(int64_t M, int64_t N, int64_t K, int64_t group
     if (flags & W4A16_FLAG_FORCE_GENERIC) return 0;
     const bool small_group = group_size != w4a16::kGroupFast;
     if (small_group ? small_group_routes_to_gemm(M, flags) : routes_to_tcgen05(M, N, K, flags)) {
-        return gemm_for(M, N, K, group_size) == Gemm::kTensorMemory ? w4a16::gemm_scratch_bytes(M, N, K) : 0;
+        return gemm_on_pairs(M, N, K) ? 0 : w4a16::gemm_scratch_bytes(M, N, K);
     }
     auto streaming = [&](int64_t rows) {
         return w4a16::linear_workspace_bytes_for(

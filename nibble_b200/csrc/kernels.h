@@ -57,9 +57,7 @@ int launch_linear_mma(const LinearProblem& p, const w4a16_linear_config& cfg, bo
 // Bounds-check word of the streaming kernel; W4A16_ERR_BAD_CONFIG in builds without -DW4A16_BOUNDS_CHECK.
 int read_bounds_check(unsigned* site, unsigned* count);
 
-// Prefill-sized batches: dequantisation fused into a tcgen05 GEMM (group == 128, aligned x / packed).
-int launch_linear_tcgen05(const LinearProblem& p, cudaStream_t stream);
-// The same with the weights in tensor memory (linear_gemm.cu); groups of 64 and 32 too, aligned x / packed.
+// Batches from medium size on: the weights dequantised into tensor memory (linear_gemm.cu); is_stream_group(group), aligned x / packed.
 int launch_linear_gemm(const LinearProblem& p, cudaStream_t stream);
 // Bytes of workspace that launch_linear_gemm uses on the current device: counters and parts of tiles that equal runs cut, or 0.
 size_t gemm_scratch_bytes(int64_t M, int64_t N, int64_t K);

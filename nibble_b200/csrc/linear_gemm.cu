@@ -13,8 +13,8 @@
 // took a quarter more), 1.1 to 1.3 us at 128, of which the MMAs are 0.55; and 7 to 8 us of start, exchange and end beside them, a
 // tenth to a third of a call: tensor pipe active 41 % of the time (128 rows, 8192 -> 28672).
 //
-// linear_tcgen05.cu writes the FP16 tile to shared memory instead; the store, a proxy fence and the space that takes make it
-// 1.2 to 1.9 times slower here.
+// (A GEMM with the FP16 tile in shared memory, since given up, was 1.2 to 1.9 times slower by the store, a proxy
+// fence and the space that takes.)
 //
 // Roles of a CTA's 32 warps, one CTA per SM:
 //   warp 0        loads x (TMA), one K block per ring slot
@@ -39,6 +39,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "gemm_weights.cuh"
@@ -49,6 +50,9 @@
 
 namespace w4a16 {
 namespace {
+
+// Set when a bounded wait inside a tensor-core kernel gives up (which barrier: low byte).
+__device__ unsigned g_tcgen05_status = 0;
 
 constexpr int kHalfRows = 128;           // output channels of one MMA (TMEM lanes)
 constexpr int kRows = 2 * kHalfRows;     // ... and of a tile
@@ -764,6 +768,29 @@ GemmPlan plan_on(const GemmDevice& dev, int64_t M, int64_t N, int64_t K) {
 }
 
 }  // namespace
+
+// The status word's device address, looked up once per device.
+unsigned* tcgen05_status_address() {
+    static std::atomic<unsigned*> cached[kMaxDevices] = {};
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices) return nullptr;
+    unsigned* address = cached[device].load(std::memory_order_relaxed);
+    if (address == nullptr) {
+        void* found = nullptr;
+        if (cudaGetSymbolAddress(&found, g_tcgen05_status) != cudaSuccess) return nullptr;
+        address = static_cast<unsigned*>(found);
+        cached[device].store(address, std::memory_order_relaxed);
+    }
+    return address;
+}
+
+// Reads (and clears) the status word of the tensor-core kernels.  Synchronises the device.
+int read_tcgen05_status(unsigned* value) {
+    unsigned zero = 0;
+    if (cudaMemcpyFromSymbol(value, g_tcgen05_status, sizeof(unsigned)) != cudaSuccess) return W4A16_ERR_LAUNCH;
+    if (cudaMemcpyToSymbol(g_tcgen05_status, &zero, sizeof(unsigned)) != cudaSuccess) return W4A16_ERR_LAUNCH;
+    return W4A16_OK;
+}
 
 // The plan for the current device, or where there is none, for a B200.
 static GemmPlan plan_here(int64_t M, int64_t N, int64_t K) {

@@ -10,7 +10,7 @@
 namespace w4a16 {
 
 // Status word of the tensor-core kernels: set when a bounded wait gives up (which barrier: low byte).  One per library,
-// defined in linear_tcgen05.cu; kernels of other files get its address as a parameter.
+// defined in linear_gemm.cu; kernels of other files get its address as a parameter.
 unsigned* tcgen05_status_address();
 
 namespace {
