@@ -6,7 +6,7 @@
 // Weights are half(code * scale), accumulated in FP32 over K: the arithmetic of dequantise-then-matmul.
 //
 // What bounds it.  At 256 batch rows the MMAs: 1021 of 1024 clocks a K block measured over a tile, and with that the power limit
-// (8192 -> 28672, 2048 rows in long runs: 740 to 800 us; dequantise and cuBLAS 930 to 990, linear_gemm.cu 910 to 1060).  Against
+// (8192 -> 28672, 2048 rows in long runs: 730 to 740 us; dequantise and cuBLAS 930 to 990, linear_gemm.cu 910 to 1060).  Against
 // linear_gemm.cu a weight is dequantised half as often and a row of x is brought to half as many SMs, for the same MMAs; with a
 // row of x in every SM, 256 batch rows would take 64 bytes a clock out of L2, more than it gives.  At small batches the chain of
 // waits, unpacking and stores of the four dequantiser groups: 0.4 us a block.
@@ -20,9 +20,15 @@
 // The second CTA's dequantisers arrive at the first one's barrier themselves: a warp that waited there and passed the word on, with
 // the fence at cluster scope that a single arrival for all of them needs, took 0.7 us a block.
 //
-// A pair takes a run of whole tiles.  Tiles cut between pairs through a workspace, as linear_gemm.cu cuts them, were built as well:
-// 0.07 % faster over 442 shapes, each by the better of the two.  There is room for one accumulator beside the weights, so the
-// MMAs wait for a tile's drain, 3300 clocks of 69000 at K = 8192; with the dequantisers' help 2600, which no call showed.
+// A pair takes every 74th tile, whole.  So at any time the pairs work on neighbours: 9 batch tiles (kBand) by about 8 of N, whose x
+// and weights come out of HBM once and are shared in L2.  When a pair took neighbouring tiles itself, the 74 read 74 different tiles
+// of weights at a time, each again for every batch tile: 1.23 GB out of HBM at 2048 rows of 8192 -> 28672 instead of 0.17, which the
+// power limit turned into time (in runs of 0.15 s 794 -> 737 us; 4096 rows 1618 -> 1463; 8192 rows of 8192 x 8192 927 -> 849;
+// without bands the last two 1517 and 928; bands of 5 as these; 600 and 1024 rows unchanged).
+//
+// Tiles cut between pairs through a workspace, as linear_gemm.cu cuts them, were built as well: 0.07 % faster over 442 shapes, each
+// by the better of the two.  There is room for one accumulator beside the weights, so the MMAs wait for a tile's drain, 3300 clocks
+// of 69000 at K = 8192; with the dequantisers' help 2600, which no call showed.
 //
 // Every wait is bounded; one that gives up sets the status word and the CTA still runs to its end.
 #include <cuda.h>
@@ -58,6 +64,7 @@ constexpr int kShares = kDrainWarps / 4;                // warps that drain a qu
 constexpr int kThreads = (kFirstDequantWarp + kDequantGroups * kGroupWarps) * 32;
 constexpr int kBarrierBytes = 512;
 constexpr int kPairs = 74;               // of a B200
+constexpr int kBand = 9;                 // batch tiles side by side: 74 pairs then work on about as many tiles of N
 constexpr int kSmem = 194 * 1024;        // as in linear_gemm.cu: leaves the L1 that keeps a tile's scales
 
 struct PairParams {
@@ -69,10 +76,19 @@ struct PairParams {
     int k_blocks;            // of one tile
     int bn, m_tiles;
     int x_slots, code_slots;
-    int run, longer;         // tiles of a pair's run; the first `longer` pairs take one more
+    int tiles;
+    int band, band_tiles;    // batch tiles side by side, and tiles of that many batch tiles and all of N
 };
 
-__device__ __forceinline__ int first_tile(const PairParams& p, int pair) { return pair * p.run + min(pair, p.longer); }
+// Where a tile is.  Pair i takes tiles i, i + pairs, ...: at any time the pairs work on neighbours.
+struct Place {
+    int n0, m0;
+};
+__device__ __forceinline__ Place place_of(const PairParams& p, int tile) {
+    const int band = tile / p.band_tiles, in_band = tile - band * p.band_tiles;
+    const int width = max(1, min(p.band, p.m_tiles - band * p.band)), n = in_band / width;       // (1 for a tile past the end)
+    return {n * kTileRows, (band * p.band + in_band - n * width) * p.bn};
+}
 
 __device__ __forceinline__ unsigned first_cta_address(unsigned local) {
     unsigned remote;
@@ -127,8 +143,8 @@ linear_gemm_pair_kernel(const PairParams p, const __grid_constant__ CUtensorMap 
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int pair = static_cast<int>(blockIdx.x) >> 1, rank = static_cast<int>(blockIdx.x) & 1;
-    const int tile_begin = first_tile(p, pair), tile_end = first_tile(p, pair + 1);
-    const int blocks = (tile_end - tile_begin) * p.k_blocks;
+    const int pairs = static_cast<int>(gridDim.x) >> 1;
+    const int blocks = (p.tiles - pair + pairs - 1) / pairs * p.k_blocks;
 
     if (tid == 0) {
         for (int r = 0; r < kRing; ++r) {
@@ -154,7 +170,7 @@ linear_gemm_pair_kernel(const PairParams p, const __grid_constant__ CUtensorMap 
         const int ahead = lane / p.k_blocks;
         asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];"
                      ::"l"(reinterpret_cast<uint64_t>(&w_map)), "r"((lane - ahead * p.k_blocks) * (kBlockK / 2)),
-                       "r"((tile_begin + ahead) / p.m_tiles * kTileRows + rank * kRows)
+                       "r"(place_of(p, pair + ahead * pairs).n0 + rank * kRows)
                      : "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -170,7 +186,8 @@ linear_gemm_pair_kernel(const PairParams p, const __grid_constant__ CUtensorMap 
     const unsigned first_full = first_cta_address(full_bar(0));
     if (warp == 0) {                                   // ---- this CTA's half of x
         bool healthy = true;
-        int xs = 0, tile = tile_begin, kb = 0;
+        int xs = 0, tile = pair, kb = 0;
+        int m0 = place_of(p, tile).m0 + rank * (p.bn / 2);
         for (unsigned it = 0; it < static_cast<unsigned>(blocks); ++it) {
             const unsigned r = it % kRing;
             if (it >= static_cast<unsigned>(p.x_slots)) {
@@ -180,7 +197,7 @@ linear_gemm_pair_kernel(const PairParams p, const __grid_constant__ CUtensorMap 
             }
             if (!healthy) break;
             if (issuer) {
-                const int k = kb * kBlockK, m0 = tile % p.m_tiles * p.bn + rank * (p.bn / 2);
+                const int k = kb * kBlockK;
                 if (rank == 0) mbar_arrive_expect_tx(full_bar(r), 4 * x_half_bytes);
                 tma_load_pair(x_slot(xs), &x_map, k, m0, first_full + r * 8);
                 tma_load_pair(x_slot(xs) + x_half_bytes, &x_map, k + 64, m0, first_full + r * 8);
@@ -189,12 +206,14 @@ linear_gemm_pair_kernel(const PairParams p, const __grid_constant__ CUtensorMap 
             if (++xs == p.x_slots) xs = 0;
             if (++kb == p.k_blocks) {
                 kb = 0;
-                ++tile;
+                tile += pairs;
+                m0 = place_of(p, tile).m0 + rank * (p.bn / 2);
             }
         }
     } else if (warp == 1) {                            // ---- packed codes
         bool healthy = true;
-        int c = 0, tile = tile_begin, kb = 0;
+        int c = 0, tile = pair, kb = 0;
+        int n0 = place_of(p, tile).n0 + rank * kRows;
         unsigned round = 0;
         for (int it = 0; it < blocks; ++it) {
             if (round > 0) {
@@ -204,7 +223,7 @@ linear_gemm_pair_kernel(const PairParams p, const __grid_constant__ CUtensorMap 
             if (!healthy) break;
             if (issuer) {
                 mbar_arrive_expect_tx(codes_bar(c), kCodeBytes);
-                tma_load_2d(code_slot(c), &w_map, kb * (kBlockK / 2), tile / p.m_tiles * kTileRows + rank * kRows, codes_bar(c));
+                tma_load_2d(code_slot(c), &w_map, kb * (kBlockK / 2), n0, codes_bar(c));
             }
             __syncwarp();
             if (++c == p.code_slots) {
@@ -213,7 +232,8 @@ linear_gemm_pair_kernel(const PairParams p, const __grid_constant__ CUtensorMap 
             }
             if (++kb == p.k_blocks) {
                 kb = 0;
-                ++tile;
+                tile += pairs;
+                n0 = place_of(p, tile).n0 + rank * kRows;
             }
         }
     } else if (warp == 2 && rank == 0) {               // ---- the pair's MMAs
@@ -258,11 +278,11 @@ linear_gemm_pair_kernel(const PairParams p, const __grid_constant__ CUtensorMap 
         const unsigned lane_base = tmem + (static_cast<unsigned>((warp & 3) * 32) << 16) + kWeightColumn;
         uint32_t next_scale[kScales] = {};             // (a register each: packed in pairs they would be waited for at once)
         // Where the scales of the group's next block are: walked along, a division per block showed.
-        int next_tile = tile_begin + group / p.k_blocks, next_kb = group % p.k_blocks;
+        int next_tile = pair + group / p.k_blocks * pairs, next_kb = group % p.k_blocks;
         int left = blocks - group;                     // blocks of the run from that one on
         const __half* scale_row = nullptr;
         auto point_at_row = [&]() {                    // rows past N hold zero codes
-            scale_row = p.scales + static_cast<size_t>(min(next_tile / p.m_tiles * kTileRows + rank * kRows + r, p.N - 1)) * groups_per_row;
+            scale_row = p.scales + static_cast<size_t>(min(place_of(p, next_tile).n0 + rank * kRows + r, p.N - 1)) * groups_per_row;
         };
         auto fetch_scales = [&]() {
             if (left > 0) {
@@ -275,15 +295,15 @@ linear_gemm_pair_kernel(const PairParams p, const __grid_constant__ CUtensorMap 
             if (next_kb >= p.k_blocks) {
                 do {
                     next_kb -= p.k_blocks;
-                    ++next_tile;
+                    next_tile += pairs;
                 } while (next_kb >= p.k_blocks);
-                point_at_row();
+                if (left > 0) point_at_row();
             }
         };
         // A wait that gives up is recorded and not repeated; the loop goes on with whatever is there, so the warps stay together.
         bool healthy = true;
         unsigned c = group % p.code_slots, code_round = group / p.code_slots;
-        point_at_row();
+        if (left > 0) point_at_row();
         fetch_scales();
         for (unsigned it = group; it < static_cast<unsigned>(blocks); it += kDequantGroups) {
             uint32_t scale2[kScales], scale_2_20[kScales], minus_8_scale[kScales];
@@ -364,8 +384,8 @@ linear_gemm_pair_kernel(const PairParams p, const __grid_constant__ CUtensorMap 
     } else if (warp >= kFirstDrainWarp) {              // ---- drain
         const int row = (warp & 3) * 32 + lane;
         const int share = warp / 4 - kFirstDrainWarp / 4;                  // of a quarter of the rows: every other 16 columns
-        auto emit = [&](int tile, int col, const uint32_t (&sum)[16]) {
-            const int n = tile / p.m_tiles * kTileRows + rank * kRows + row, m = tile % p.m_tiles * p.bn + col;
+        auto emit = [&](const Place& at, int col, const uint32_t (&sum)[16]) {
+            const int n = at.n0 + rank * kRows + row, m = at.m0 + col;
             if (n >= p.N) return;
             char* out = reinterpret_cast<char*>(p.y + static_cast<size_t>(m) * p.N + n);
             const unsigned stride = static_cast<unsigned>(p.N) * 2u;
@@ -384,18 +404,20 @@ linear_gemm_pair_kernel(const PairParams p, const __grid_constant__ CUtensorMap 
             }
         };
         bool healthy = true;
-        for (int tile = tile_begin; tile < tile_end; ++tile) {
-            if (healthy) healthy = mbar_wait(acc_full_bar, (tile - tile_begin) & 1, 0x30u, p.status);
+        unsigned done = 0;
+        for (int tile = pair; tile < p.tiles; tile += pairs, ++done) {
+            const Place at = place_of(p, tile);
+            if (healthy) healthy = mbar_wait(acc_full_bar, done & 1, 0x30u, p.status);
             __syncwarp();
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (int col = share * 16; col < p.bn; col += kShares * 16) {
                 uint32_t v[16];
                 tmem_load16(tmem + (static_cast<unsigned>((warp & 3) * 32) << 16) + col, v);
-                emit(tile, col, v);
+                emit(at, col, v);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0 && tile + 1 < tile_end) mbar_arrive_remote(first_cta_address(acc_free_bar));
+            if (lane == 0 && tile + pairs < p.tiles) mbar_arrive_remote(first_cta_address(acc_free_bar));
         }
     }
 
@@ -498,8 +520,10 @@ int launch_linear_gemm_pair(const LinearProblem& prob, cudaStream_t stream) {
     if (params.status == nullptr) return W4A16_ERR_LAUNCH;
     params.M = static_cast<int>(prob.M);
     params.N = static_cast<int>(prob.N);
-    params.run = static_cast<int>(g.tiles / grid);
-    params.longer = static_cast<int>(g.tiles % grid);
+    params.tiles = static_cast<int>(g.tiles);
+    const int bands = (g.m_tiles + kBand - 1) / kBand;
+    params.band = (g.m_tiles + bands - 1) / bands;
+    params.band_tiles = static_cast<int>(g.tiles / g.m_tiles) * params.band;
     // 256 batch rows: 4 blocks of x and 8 of codes.
     const int x_bytes = params.bn * 128;
     const int room = kSmem - kBarrierBytes - 1024;

@@ -330,6 +330,7 @@ def test_gemm_weights_are_rounded_products_for_any_scale(gs):
     (1500, 2048, 4096, 128), (1100, 384, 9001, 128),
     (3000, 128, 5000, 128),    # one K block a tile
     (2050, 256, 2500, 128),
+    (2600, 256, 2300, 128), (4900, 128, 1030, 128),    # bands of 6 and 5, of 7, 7 and 6 batch tiles
     (1030, 896, 2000, 64), (1300, 640, 5001, 64), (2100, 384, 3100, 32),
 ])
 def test_gemm_on_pairs_of_sms(m, k, n, gs):
