@@ -79,7 +79,7 @@ typedef struct w4a16_linear_config {
  *
  * Fast path when group_size == 128 and x, packed are 16-byte aligned: M <= 8 runs the mma.sync
  * streaming kernel, M >= 65 (and 9..64 on layers of N >= 4096 where a cost model built from measurements
- * favours it) a tcgen05 GEMM whose producer warps dequantise into the operand tiles
+ * favours it) a tcgen05 GEMM whose producer warps dequantise into tensor memory
  * (no FP16 weight matrix in memory; weights enter the product as half(code * scale), the arithmetic of
  * the reference's dequantise-then-matmul prefill route, w4a16/linear.py:132-152).
  * group_size 64 and 32 run the streaming kernel (from 65 rows on in launches of 64 rows, or as the GEMM with

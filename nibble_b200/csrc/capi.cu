@@ -80,7 +80,7 @@ bool routes_to_tcgen05(int64_t M, int64_t N, int64_t K, uint32_t flags) {
 
 // Whether a call that goes to a GEMM takes the one on pairs of SMs, with whole tiles of 256 weight rows x up to 256 batch rows, or the
 // one on single SMs, with up to 128 batch rows a tile and the K of few tiles shared.  By their models' times (us, pairs / single SMs:
-// 8192 -> 28672, 2048 rows 740 to 800 / 910 to 1060; 8192 x 8192, 512 rows 59 / 67; 5632 -> 2048, 777 rows 30 / 24), with two lines:
+// 8192 -> 28672, 2048 rows 730 to 740 / 910 to 1060; 8192 x 8192, 512 rows 59 / 67; 5632 -> 2048, 777 rows 30 / 24), with two lines:
 //   - up to 128 rows, one batch tile of the second kernel, only in one round of pairs: in two they are level (8192 -> 28672, 96 rows:
 //     63 / 55; in one, 1024 -> 8192, 128 rows: 7.0 / 10.4);
 //   - above 512 rows the second kernel only where its tiles fit a round, two with K >= 4096, or K >= 2048 up to 1024 rows: beyond,

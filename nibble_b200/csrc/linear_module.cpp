@@ -40,7 +40,7 @@ c10::TypedOperatorHandle<Signature> operator_handle(const char* name) {
 //   - up to 512 rows the operator, never slower (8192 -> 28672, 512 rows: 201 / 374);
 //   - 513 to 1024 rows: all but shallow layers (8192 x 8192, 1024 rows: 115 / 153; 512 -> 28672, 777 rows: 1.16 times as long).
 //     0.6 % slower than the better on average;
-//   - to 4096 rows: layers with K >= 2048 (8192 -> 28672, 2048 rows: 740 to 800 / 930 to 990; 4096 x 4096: 60 / 68; 8192 -> 1024, 1536
+//   - to 4096 rows: layers with K >= 2048 (8192 -> 28672, 2048 rows: 730 to 740 / 930 to 990; 4096 x 4096: 60 / 68; 8192 -> 1024, 1536
 //     rows, the worst: 1.19 times as long) and those whose 256 x 128 tiles fit one round of SMs.  1.1 %;
 //   - above, the weights' round trip costs little beside the product (8192 -> 28672, 8192 rows: 1.02 times as long).
 bool uses_fused_kernel(int64_t rows, int64_t out_features, int64_t in_features, int64_t group_size) {
