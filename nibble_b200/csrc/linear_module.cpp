@@ -42,7 +42,8 @@ c10::TypedOperatorHandle<Signature> operator_handle(const char* name) {
 //     0.6 % slower than the better on average;
 //   - to 4096 rows: layers with K >= 2048 (8192 -> 28672, 2048 rows: 730 to 740 / 930 to 990; 4096 x 4096: 60 / 68; 8192 -> 1024, 1536
 //     rows, the worst: 1.19 times as long) and those whose 256 x 128 tiles fit one round of SMs.  1.1 %;
-//   - above, the weights' round trip costs little beside the product (8192 -> 28672, 8192 rows: 1.02 times as long).
+//   - above, the weights' round trip costs little beside the product (16384 rows: level, 0.88 to 1.09 times as long).  At 5000 and 8192
+//     rows layers with K and N >= 4096 would gain (8192 -> 28672: 0.94 and 0.96 times as long), shallower ones lose up to 5 %.
 bool uses_fused_kernel(int64_t rows, int64_t out_features, int64_t in_features, int64_t group_size) {
     if (rows <= 64) return true;
     if (group_size % 32 != 0) return true;
