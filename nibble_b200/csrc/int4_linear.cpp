@@ -7,6 +7,7 @@
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/library.h>
 
@@ -104,6 +105,30 @@ void check_status(int status, const char* what) {
     TORCH_CHECK(status == W4A16_OK, what, " failed: ", w4a16_status_string(status));
 }
 
+bool aligned16(const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
+
+// Whether the tensor-core kernels take calls of this K and group but not these addresses: a view at an odd offset, a row slice of a
+// larger scale matrix.  (Packed weights at an odd address are out: the dequantiser does not take them either.)
+bool declined_for_alignment(const at::Tensor& activations, const at::Tensor& packed_weights, const at::Tensor& scales, int64_t k,
+                            int64_t group_size) {
+    if ((group_size != 128 && group_size != 64 && group_size != 32) || k == 0 || k % 128 != 0 || !aligned16(packed_weights)) return false;
+    return !aligned16(activations) || (group_size != 128 && !aligned16(scales));
+}
+
+at::Tensor dequantize_cuda_impl(const at::Tensor& packed_weights, const at::Tensor& scales, int64_t group_size);
+
+// The product with dequantised FP16 weights, as the module forms it.  Nothing here takes part in autograd or is cast by autocast:
+// the operator's result is FP16 whatever the context.
+at::Tensor dequantize_and_multiply(const at::Tensor& activations, const at::Tensor& packed_weights, const at::Tensor& scales,
+                                   const at::Tensor* bias, int64_t group_size, int64_t m, at::IntArrayRef shape) {
+    const at::AutoDispatchBelowADInplaceOrView below;
+    const c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::DispatchKey::AutocastCUDA);
+    const at::Tensor weights = dequantize_cuda_impl(packed_weights, scales, group_size);
+    at::Tensor out = at::mm(activations.view({m, weights.size(1)}), weights.t());
+    if (bias != nullptr) out.add_(*bias);
+    return out.view(shape);
+}
+
 // `activations` is [..., K] when `any_rank` (the module's call), else [M, K]; the result keeps its leading dimensions.
 at::Tensor linear_impl(const at::Tensor& activations, const at::Tensor& packed_weights, const at::Tensor& scales,
                        const at::Tensor* bias, int64_t group_size, bool out_f32, bool any_rank) {
@@ -145,11 +170,21 @@ at::Tensor linear_impl(const at::Tensor& activations, const at::Tensor& packed_w
     int64_t m = 1;
     for (size_t i = 0; i + 1 < shape.size(); ++i) m *= shape[i];
     shape.back() = n;
-    at::Tensor output = at::detail::empty_cuda(shape, out_f32 ? at::kFloat : at::kHalf, activations.device(), c10::nullopt);
-    if (m == 0 || n == 0) return output;
+    const auto new_output = [&] {
+        return at::detail::empty_cuda(shape, out_f32 ? at::kFloat : at::kHalf, activations.device(), c10::nullopt);
+    };
+    if (m == 0 || n == 0) return new_output();
 
-    const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
     const EnvironmentChoices choices = environment_choices();
+    // The module's large batches are the product with dequantised FP16 weights whichever kernel forms it, so where the tensor-core
+    // kernels decline the addresses this one does: the generic kernel, which takes any, is no match (4096 x 4096, activations at
+    // an odd offset, 65 / 777 / 2048 rows: 400 / 4030 / 10460 us with it, 90 / 300 / 640 this way).
+    if (any_rank && m > 64 && !(choices.flags & W4A16_FLAG_FORCE_GENERIC) &&
+        declined_for_alignment(activations, packed_weights, scales, k, group_size)) {
+        return dequantize_and_multiply(activations, packed_weights, scales, bias, group_size, m, shape);
+    }
+    at::Tensor output = new_output();
+    const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
     // (the module's large batches are the product with dequantised FP16 weights, whichever kernel forms it)
     const uint32_t flags = choices.flags | (out_f32 ? W4A16_FLAG_OUTPUT_F32 : 0u) | (any_rank ? W4A16_FLAG_FP16_WEIGHTS : 0u);
     const int forced_tiles = choices.row_tiles;

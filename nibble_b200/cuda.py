@@ -145,7 +145,8 @@ def linear_bias_cuda(
     """What ``QuantizedLinear`` calls: activations of any rank ``[..., K]``, the FP16 bias added inside the kernel.
 
     Not part of the reference's surface.  Unlike ``linear_cuda`` it lets batches of 65 rows and more round each weight to FP16
-    whatever the group size, as the product with dequantised weights does.
+    whatever the group size, as the product with dequantised weights does; where the tensor-core kernels decline the addresses of
+    the activations or scales, such batches are that product.
     """
     _require_extension()
     return torch.ops.w4a16.linear_bias(activations, packed_weights, scales, bias, group_size)

@@ -245,6 +245,44 @@ def test_every_way_into_the_module_takes_the_native_route(rows, n, k, gs):
     assert torch.equal(torch.compile(layer, backend="aot_eager", fullgraph=True, dynamic=False)(x), want)
 
 
+@pytest.mark.parametrize(("k", "n"), [(1024, 264), (2048, 77)])
+@pytest.mark.parametrize("gs", [128, 64])
+@pytest.mark.parametrize("rows", [65, 777, 2048])
+def test_large_batches_at_odd_addresses_are_the_product_with_dequantised_weights(rows, gs, k, n):
+    """Activations, or scales of 64-wide groups, that the tensor-core kernels decline for their alignment: the dequantiser and a
+    matrix product, with its very bits, whichever way the call comes in; no generic kernel, which takes up to sixteen times as long."""
+    from nibble_b200 import _native
+
+    count = _native.core().w4a16_launch_count
+    torch.manual_seed(rows + n)
+    packed = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda")
+    spread = (torch.rand((n * (k // gs) + 1,), device="cuda") * 0.01 + 1e-3).half()
+    row = torch.randn((rows * k + 1,), device="cuda").half()
+    bias = torch.randn((n,), device="cuda").half()
+    for shift_x, shift_scales in ((1, 0), (0, 1), (1, 1)):
+        scales = spread[shift_scales:shift_scales + n * (k // gs)].view(n, k // gs)
+        x = row[shift_x:shift_x + rows * k].view(1, rows, k)
+        assert x.is_contiguous() and x.data_ptr() % 16 == 2 * shift_x and scales.data_ptr() % 16 == 2 * shift_scales
+        product = torch.mm(x[0], torch.ops.w4a16.dequantize(packed, scales, gs).t())
+        declined = shift_x or gs != 128
+        for b in (None, bias):
+            layer = QuantizedLinear(packed, scales, gs, bias=b)
+            want = product if b is None else product + b
+            before = count()
+            got = layer(x)
+            assert count() == before + 1 and got.shape == (1, rows, n)
+            with _Passing():
+                assert torch.equal(layer(x), got)
+            if declined:
+                assert torch.equal(got[0], want)
+                with torch.autocast("cuda", dtype=torch.bfloat16):
+                    assert torch.equal(torch.ops.w4a16.linear_bias(x, packed, scales, b, gs), got)
+            else:
+                torch.testing.assert_close(got[0], want, rtol=2e-3, atol=2e-3)
+    torch._dynamo.reset()
+    assert torch.equal(torch.compile(layer, backend="aot_eager", fullgraph=True, dynamic=False)(x), got)
+
+
 @pytest.mark.parametrize("rows", [4, 100])
 def test_transforms_follow_the_product_with_dequantised_weights(rows):
     """Forward-mode differentiation and vmap see the matrix product where the module forms one."""
