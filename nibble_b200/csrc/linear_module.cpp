@@ -47,7 +47,9 @@ c10::TypedOperatorHandle<Signature> operator_handle(const char* name) {
 bool uses_fused_kernel(int64_t rows, int64_t out_features, int64_t in_features, int64_t group_size) {
     if (rows <= 64) return true;
     if (group_size % 32 != 0) return true;
-    if (group_size > 128 || in_features % 128 != 0) return false;      // the operator has no tensor-core kernel for these
+    if ((group_size != 128 && group_size != 64 && group_size != 32) || in_features % 128 != 0) {
+        return false;      // the operator has no tensor-core kernel for these (3072 -> 4096 in groups of 96, 65 / 2048 rows: 294 / 7917 us)
+    }
     if (out_features % 8 != 0 || rows <= 256) return true;
     if (rows <= 1024) return rows <= 512 || out_features <= 20 * in_features;
     return rows <= 4096 && (in_features >= 2048 || (out_features + 255) / 256 * ((rows + 127) / 128) <= 148);

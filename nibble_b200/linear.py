@@ -28,7 +28,7 @@ def takes_operator(rows: int, out_features: int, in_features: int, group_size: i
     """
     if rows <= FUSED_MAX_ROWS or group_size % 32:
         return True      # (the dequantise operator needs group_size % 32 == 0; the fused one does not)
-    if group_size > 128 or in_features % 128:
+    if group_size not in (128, 64, 32) or in_features % 128:
         return False     # the operator has no tensor-core kernel for these
     if out_features % 8 or rows <= 256:
         return True

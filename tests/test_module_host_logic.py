@@ -114,6 +114,20 @@ def test_python_and_native_forward_state_one_rule():
     assert {True, False} == set(verdicts.values())
 
 
+def test_large_batches_go_to_the_operator_only_where_it_has_a_tensor_core_kernel():
+    """Groups of 96 divide K like those of 128 can, but no tensor-core kernel takes them: their large batches are the product with
+    dequantised weights, as those of 160 and 256 are, whatever the rows and the layer."""
+    from nibble_b200 import _native
+    from nibble_b200.linear import takes_operator
+
+    native = _native.load_torch_ops().uses_fused_kernel
+    for group in (96, 160, 192, 256):
+        for rows in (65, 256, 512, 1024, 2048, 4096, 5000):
+            for n in (1000, 1001, 4096):
+                assert not takes_operator(rows, n, 1920 * 4, group) and not native(rows, n, 1920 * 4, group)
+        assert takes_operator(64, 1000, 1920 * 4, group) and native(64, 1000, 1920 * 4, group)
+
+
 def test_group_size_without_dequantize_kernel_stays_fused(oracle_backend):
     layer = _layer(fused=False)  # group_size 4 is not a multiple of 32
     layer(ACTIVATIONS)
