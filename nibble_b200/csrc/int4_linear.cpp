@@ -107,12 +107,22 @@ void check_status(int status, const char* what) {
 
 bool aligned16(const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
 
-// Whether the tensor-core kernels take calls of this K and group but not these addresses: a view at an odd offset, a row slice of a
-// larger scale matrix.  (Packed weights at an odd address are out: the dequantiser does not take them either.)
-bool declined_for_alignment(const at::Tensor& activations, const at::Tensor& packed_weights, const at::Tensor& scales, int64_t k,
-                            int64_t group_size) {
-    if ((group_size != 128 && group_size != 64 && group_size != 32) || k == 0 || k % 128 != 0 || !aligned16(packed_weights)) return false;
+// Whether the tensor-core kernels take calls of this K and group, and the dequantiser these weights.
+bool has_tensor_core_kernel(const at::Tensor& packed_weights, int64_t k, int64_t group_size) {
+    return (group_size == 128 || group_size == 64 || group_size == 32) && k > 0 && k % 128 == 0 && aligned16(packed_weights);
+}
+
+// Whether such a call has addresses that those kernels do not take: a view at an odd offset, a row slice of a larger scale matrix.
+bool declined_for_alignment(const at::Tensor& activations, const at::Tensor& scales, int64_t group_size) {
     return !aligned16(activations) || (group_size != 128 && !aligned16(scales));
+}
+
+// Whether a variable of the environment that names a kernel is heeded by the module's call: as far as small and medium batches go,
+// which these kernels are for, and one of them refuses larger ones.
+bool heeds_named_kernel(int64_t m, int64_t n, int64_t k) {
+    if (m <= 256 || n % 8 != 0) return true;
+    if (m > 1024 || n > 20 * k) return false;
+    return m <= 512 || n * k <= 4 << 20 || (k >= 2048 && m <= 896) || k >= 8 * n;
 }
 
 at::Tensor dequantize_cuda_impl(const at::Tensor& packed_weights, const at::Tensor& scales, int64_t group_size);
@@ -178,10 +188,14 @@ at::Tensor linear_impl(const at::Tensor& activations, const at::Tensor& packed_w
     const EnvironmentChoices choices = environment_choices();
     // The module's large batches are the product with dequantised FP16 weights whichever kernel forms it, so where the tensor-core
     // kernels decline the addresses this one does: the generic kernel, which takes any, is no match (4096 x 4096, activations at
-    // an odd offset, 65 / 777 / 2048 rows: 400 / 4030 / 10460 us with it, 90 / 300 / 640 this way).
-    if (any_rank && m > 64 && !(choices.flags & W4A16_FLAG_FORCE_GENERIC) &&
-        declined_for_alignment(activations, packed_weights, scales, k, group_size)) {
-        return dequantize_and_multiply(activations, packed_weights, scales, bias, group_size, m, shape);
+    // an odd offset, 65 / 777 / 2048 rows: 400 / 4030 / 10460 us with it, 90 / 300 / 640 this way).  The same for batches beyond
+    // those that a variable's kernel is meant for (8192 -> 4096, 2048 rows, W4A16_DECODE=generic: 20990 us; W4A16_ROWS_PER_WARP: refused).
+    if (any_rank && m > 64 && has_tensor_core_kernel(packed_weights, k, group_size)) {
+        const bool generic = (choices.flags & W4A16_FLAG_FORCE_GENERIC) != 0;
+        const bool named = generic || (choices.row_tiles != 0 && bias == nullptr && group_size == 128);
+        if ((named && !heeds_named_kernel(m, n, k)) || (!generic && declined_for_alignment(activations, scales, group_size))) {
+            return dequantize_and_multiply(activations, packed_weights, scales, bias, group_size, m, shape);
+        }
     }
     at::Tensor output = new_output();
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();

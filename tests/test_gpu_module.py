@@ -283,6 +283,27 @@ def test_large_batches_at_odd_addresses_are_the_product_with_dequantised_weights
     assert torch.equal(torch.compile(layer, backend="aot_eager", fullgraph=True, dynamic=False)(x), got)
 
 
+@pytest.mark.parametrize(("variable", "value"), [("W4A16_DECODE", "generic"), ("W4A16_ROWS_PER_WARP", "2"), ("W4A16_ROWS_PER_WARP", "4")])
+@pytest.mark.parametrize(("rows", "k", "n"), [(1025, 2048, 264), (2048, 8192, 1000), (1000, 1024, 4200), (300, 512, 10248)])
+def test_variables_that_name_a_kernel_leave_large_batches_alone(variable, value, rows, k, n, monkeypatch):
+    """They are for small and medium batches: beyond, the module's product is the one with dequantised weights, by its bits, where
+    one of the kernels needs thirty times as long and the other refuses the call."""
+    torch.manual_seed(rows)
+    packed = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda")
+    scales = (torch.rand((n, k // 128), device="cuda") * 0.01 + 1e-3).half()
+    layer = QuantizedLinear(packed, scales, 128)
+    x = torch.randn((rows, k), device="cuda").half()
+    want = torch.mm(x, torch.ops.w4a16.dequantize(packed, scales, 128).t())
+    monkeypatch.setenv(variable, value)
+    assert torch.equal(layer(x), want)
+    if value == "generic":                                   # on this side it is heeded: exact weights, another product's bits
+        few = x[:100]
+        product = torch.mm(few, torch.ops.w4a16.dequantize(packed, scales, 128).t())
+        got = layer(few)
+        assert not torch.equal(got, product)
+        torch.testing.assert_close(got, product, rtol=1e-2, atol=1e-2 * float(product.abs().max()))
+
+
 @pytest.mark.parametrize("rows", [4, 100])
 def test_transforms_follow_the_product_with_dequantised_weights(rows):
     """Forward-mode differentiation and vmap see the matrix product where the module forms one."""
