@@ -16,6 +16,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 
+#include <algorithm>
 #include <optional>
 #include <tuple>
 
@@ -31,17 +32,37 @@ c10::TypedOperatorHandle<Signature> operator_handle(const char* name) {
     return c10::Dispatcher::singleton().findSchemaOrThrow(name, "").typed<Signature>();
 }
 
+// Whether the operator is the faster way for 897 to 4096 rows, by models of both (us).  Their constants are fitted to the times of both
+// on 259 calls with 897 to 4096 rows on layers of 512 to 28416 -> 256 to 20992, in runs of 14 ms: choosing by them is 0.9 % slower
+// than the better way on average.  By the depth of the layer alone (K >= 2048 to the operator) it was 2.9 %, and narrow layers, which
+// leave half of the SMs without a tile, took up to 1.6 times as long (7296 -> 384, 3072 rows: 31 / 20; 8192 -> 1024, 1536 rows: 33 / 27).
+bool operator_is_faster(int64_t rows, int64_t out_features, int64_t in_features) {
+    const int64_t k_blocks = in_features / 128, n_tiles = (out_features + 255) / 256;
+    const int64_t tiles = n_tiles * ((rows + 127) / 128), pair_tiles = n_tiles * ((rows + 255) / 256);
+    // whole rounds of pairs of SMs; or clusters of up to eight SMs that share a tile, or all SMs in equal runs
+    double by_operator = 2.5 + static_cast<double>((pair_tiles + 73) / 74) * (2.0 + 0.84 * static_cast<double>(k_blocks));
+    double single = by_operator;
+    if (tiles <= 148) {
+        const int64_t sharing = tiles > 74 ? 1 : tiles > 44 ? 2 : std::min<int64_t>(8, 132 / tiles);
+        single = (sharing > 1 ? 10.0 : 6.5) + 0.8 * static_cast<double>((k_blocks + sharing - 1) / sharing);
+    } else if ((tiles <= 296 && in_features >= 4096) || (rows <= 1024 && in_features >= 2048)) {
+        single = 20.0 + static_cast<double>(tiles * k_blocks) / 148.0;
+    }
+    if (single < by_operator) by_operator = single;
+    const double weights = static_cast<double>(out_features) * static_cast<double>(in_features);
+    const double by_product = 7.0 + weights / 1.75e6 + static_cast<double>(rows) * weights / 6.1e8;
+    return by_operator < (by_product > 15.5 ? by_product : 15.5);      // (two launches and their operators: 15.5 us of host time)
+}
+
 // Whether a batch goes to the fused operator, or is multiplied by dequantised FP16 weights (same arithmetic from 65 rows
 // on: weights rounded to FP16, FP32 sums).  linear.py states the same rule (takes_operator) for the calls that stay in Python; a
 // test holds the two together.  The lines come from times of both on 34 layers from 512 x 1024 to 28672 x 8192 at 160 to 8192 rows,
-// back to back for 12 ms and more, so that the clocks are those of a long run (us, the operator / dequantise and multiply; the
-// latter is 14 us of host time at least):
+// back to back for 12 ms and more, so that the clocks are those of a long run (us, the operator / dequantise and multiply):
 //   - cuBLAS falls off its fast kernels where an output row is no multiple of 16 bytes (9216 -> 2575, 128 rows: 20 / 125);
 //   - up to 512 rows the operator, never slower (8192 -> 28672, 512 rows: 201 / 374);
-//   - 513 to 1024 rows: all but shallow layers (8192 x 8192, 1024 rows: 115 / 153; 512 -> 28672, 777 rows: 1.16 times as long).
-//     0.6 % slower than the better on average;
-//   - to 4096 rows: layers with K >= 2048 (8192 -> 28672, 2048 rows: 730 to 740 / 930 to 990; 4096 x 4096: 60 / 68; 8192 -> 1024, 1536
-//     rows, the worst: 1.19 times as long) and those whose 256 x 128 tiles fit one round of SMs.  1.1 %;
+//   - 513 to 896 rows: all but shallow layers (8320 -> 6400, 702 rows: 65 / 85; 512 -> 28672, 777 rows: 1.16 times as long);
+//   - to 1024 rows: of those the small or narrow ones (3456 -> 256, 1024 rows: 13.8 / 15.6), and else
+//   - to 4096 rows: where the models above say so (8192 -> 28672, 2048 rows: 730 to 740 / 930 to 990);
 //   - above, the weights' round trip costs little beside the product (16384 rows: level, 0.88 to 1.09 times as long).  At 5000 and 8192
 //     rows layers with K and N >= 4096 would gain (8192 -> 28672: 0.94 and 0.96 times as long), shallower ones lose up to 5 %.
 bool uses_fused_kernel(int64_t rows, int64_t out_features, int64_t in_features, int64_t group_size) {
@@ -50,9 +71,14 @@ bool uses_fused_kernel(int64_t rows, int64_t out_features, int64_t in_features, 
     if ((group_size != 128 && group_size != 64 && group_size != 32) || in_features % 128 != 0) {
         return false;      // the operator has no tensor-core kernel for these (3072 -> 4096 in groups of 96, 65 / 2048 rows: 294 / 7917 us)
     }
-    if (out_features % 8 != 0 || rows <= 256) return true;
-    if (rows <= 1024) return rows <= 512 || out_features <= 20 * in_features;
-    return rows <= 4096 && (in_features >= 2048 || (out_features + 255) / 256 * ((rows + 127) / 128) <= 148);
+    if (out_features % 8 != 0 || rows <= 512) return true;
+    if (rows <= 1024) {
+        if (out_features > 20 * in_features) return false;
+        if (rows <= 896 || out_features * in_features <= 4 << 20 || in_features >= 8 * out_features) return true;
+        return operator_is_faster(rows, out_features, in_features);
+    }
+    if (rows > 4096 || (in_features < 2048 && (out_features + 255) / 256 * ((rows + 127) / 128) > 148)) return false;
+    return operator_is_faster(rows, out_features, in_features);
 }
 
 // A tensor nobody has subclassed, wrapped or asked to track gradients of.

@@ -30,11 +30,35 @@ def takes_operator(rows: int, out_features: int, in_features: int, group_size: i
         return True      # (the dequantise operator needs group_size % 32 == 0; the fused one does not)
     if group_size not in (128, 64, 32) or in_features % 128:
         return False     # the operator has no tensor-core kernel for these
-    if out_features % 8 or rows <= 256:
+    if out_features % 8 or rows <= 512:
         return True
     if rows <= 1024:
-        return rows <= 512 or out_features <= 20 * in_features
-    return rows <= 4096 and (in_features >= 2048 or -(-out_features // 256) * -(-rows // 128) <= 148)
+        if out_features > 20 * in_features:
+            return False
+        if rows <= 896 or out_features * in_features <= 4 << 20 or in_features >= 8 * out_features:
+            return True
+        return _operator_is_faster(rows, out_features, in_features)
+    if rows > 4096 or (in_features < 2048 and -(-out_features // 256) * -(-rows // 128) > 148):
+        return False
+    return _operator_is_faster(rows, out_features, in_features)
+
+
+def _operator_is_faster(rows: int, out_features: int, in_features: int) -> bool:
+    """For 897 to 4096 rows, by models of both ways (csrc/linear_module.cpp: operator_is_faster, which says where they come from)."""
+    k_blocks, n_tiles = in_features // 128, -(-out_features // 256)
+    tiles, pair_tiles = n_tiles * -(-rows // 128), n_tiles * -(-rows // 256)
+    by_operator = 2.5 + (pair_tiles + 73) // 74 * (2.0 + 0.84 * k_blocks)
+    single = by_operator
+    if tiles <= 148:
+        sharing = 1 if tiles > 74 else 2 if tiles > 44 else 8 if tiles <= 16 else 132 // tiles
+        single = (10.0 if sharing > 1 else 6.5) + 0.8 * -(-k_blocks // sharing)
+    elif (tiles <= 296 and in_features >= 4096) or (rows <= 1024 and in_features >= 2048):
+        single = 20.0 + tiles * k_blocks / 148.0
+    if single < by_operator:
+        by_operator = single
+    weights = out_features * in_features
+    by_product = 7.0 + weights / 1.75e6 + rows * weights / 6.1e8
+    return by_operator < by_product or by_operator < 15.5
 
 
 # The coarse rule for activations whose arithmetic has to stay visible as torch operators (below), where speed is not the point:
