@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import pathlib
+import re
 import shutil
 import subprocess
 
@@ -52,3 +53,19 @@ def test_no_launcher_keeps_a_failure():
     """std::call_once would: its one outcome stands for the life of the process."""
     for source in CSRC.glob("*.cu"):
         assert "call_once" not in source.read_text(), source.name
+
+
+def test_arrivals_at_another_cta_are_ordered_for_it():
+    """An arrival at a barrier in another CTA's shared memory, and the waits on a barrier that receives such arrivals, name the cluster
+    as their scope: the default, the CTA, orders nothing between two of them."""
+    arrivals = [(path.name, line.strip()) for path in sorted(CSRC.glob("*.cu*")) for line in path.read_text().splitlines()
+                if re.search(r'"\s*mbarrier\.arrive\S*shared::cluster', line)]
+    assert arrivals
+    for where, line in arrivals:
+        assert re.search(r"mbarrier\.arrive\.(release|relaxed)\.cluster\.shared::cluster", line), (where, line)
+    pair = (CSRC / "linear_gemm_pair.cu").read_text()
+    calls = re.sub(r"void mbar_arrive_remote\(", "", pair)
+    assert set(re.findall(r"mbar_arrive_remote\((?:first_cta_address\()?(\w+)", calls)) == {"first_full", "acc_free_bar"}
+    for barrier in ("full_bar", "acc_free_bar"):              # (first_full: the first CTA's full_bar(0))
+        waits = re.findall(r"mbar_(?:wait|test)(\S*?)\((?=%s\b)" % barrier, pair)
+        assert waits and set(waits) == {"<true>"}, barrier
