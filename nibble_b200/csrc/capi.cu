@@ -79,22 +79,24 @@ bool routes_to_tcgen05(int64_t M, int64_t N, int64_t K, uint32_t flags) {
 }
 
 // Whether a call that goes to a GEMM takes the one on pairs of SMs, with whole tiles of 256 weight rows x up to 256 batch rows, or the
-// one on single SMs, with up to 128 batch rows a tile and the K of few tiles shared.  By their models' times (us, pairs / single SMs:
+// one on single SMs, with up to 128 batch rows a tile and the K of few tiles shared, which for some layers takes a workspace.  By their
+// models' times for what either would do (us, pairs / single SMs:
 // 8192 -> 28672, 2048 rows 730 to 740 / 910 to 1060; 8192 x 8192, 512 rows 59 / 67; 5632 -> 2048, 777 rows 30 / 24), with two lines:
 //   - up to 128 rows, one batch tile of the second kernel, only in one round of pairs: in two they are level (8192 -> 28672, 96 rows:
 //     63 / 55; in one, 1024 -> 8192, 128 rows: 7.0 / 10.4);
 //   - above 512 rows the second kernel only where its tiles fit a round, two with K >= 4096, or K >= 2048 up to 1024 rows: beyond,
 //     the first is the faster one whatever the models say (157 calls, at most 1 % slower).
-bool gemm_on_pairs(int64_t M, int64_t N, int64_t K) {
+bool gemm_on_pairs(int64_t M, int64_t N, int64_t K, size_t workspace_bytes) {
     if (M <= 64 || M > INT32_MAX || N > INT32_MAX || K > INT32_MAX) return false;     // (9 to 64 rows, and whatever a flag sends)
     if (M <= 128 && w4a16::gemm_pair_rounds(M, N) != 1) return false;
     const int64_t tiles = (N + 255) / 256 * ((M + 127) / 128);
     if (M > 512 && tiles > 148 && !(tiles <= 296 && K >= 4096) && !(M <= 1024 && K >= 2048)) return true;
-    return w4a16::gemm_pair_time(M, N, K) < w4a16::gemm_time(M, N, K);
+    return w4a16::gemm_pair_time(M, N, K) < w4a16::gemm_time(M, N, K, workspace_bytes);
 }
 
 int launch_gemm(const w4a16::LinearProblem& p, cudaStream_t stream) {
-    return gemm_on_pairs(p.M, p.N, p.K) ? w4a16::launch_linear_gemm_pair(p, stream) : w4a16::launch_linear_gemm(p, stream);
+    const bool pairs = gemm_on_pairs(p.M, p.N, p.K, w4a16::usable_workspace(p));
+    return pairs ? w4a16::launch_linear_gemm_pair(p, stream) : w4a16::launch_linear_gemm(p, stream);
 }
 
 // Whether a call with 64- or 32-wide groups goes to the GEMM, which rounds each weight to FP16.  Only where the caller has said
@@ -181,7 +183,7 @@ size_t w4a16_linear_scratch_bytes(int64_t M, int64_t N, int64_t K, int64_t group
     if (flags & W4A16_FLAG_FORCE_GENERIC) return 0;
     const bool small_group = group_size != w4a16::kGroupFast;
     if (small_group ? small_group_routes_to_gemm(M, flags) : routes_to_tcgen05(M, N, K, flags)) {
-        return gemm_on_pairs(M, N, K) ? 0 : w4a16::gemm_scratch_bytes(M, N, K);
+        return gemm_on_pairs(M, N, K, SIZE_MAX) ? 0 : w4a16::gemm_scratch_bytes(M, N, K);
     }
     auto streaming = [&](int64_t rows) {
         return w4a16::linear_workspace_bytes_for(

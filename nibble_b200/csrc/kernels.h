@@ -37,6 +37,11 @@ struct LinearProblem {
     bool among_transforms = false;
 };
 
+// Bytes of workspace that a call may share tiles through.
+inline size_t usable_workspace(const LinearProblem& p) {
+    return p.workspace != nullptr && reinterpret_cast<uintptr_t>(p.workspace) % 16 == 0 ? p.workspace_bytes : 0;
+}
+
 // Scale groups the streaming kernel is built for (K a multiple of 128 all the same).
 constexpr bool is_stream_group(int64_t group) { return group == 128 || group == 64 || group == 32; }
 
@@ -63,8 +68,8 @@ int launch_linear_gemm(const LinearProblem& p, cudaStream_t stream);
 size_t gemm_scratch_bytes(int64_t M, int64_t N, int64_t K);
 // The same on pairs of SMs, up to 256 batch rows a tile (linear_gemm_pair.cu); no workspace.
 int launch_linear_gemm_pair(const LinearProblem& p, cudaStream_t stream);
-// Times of the last two by their models (us), for the choice between them, and rounds of pairs.
-double gemm_time(int64_t M, int64_t N, int64_t K);
+// Times of the last two by their models (us), for the choice between them, the first's with this much workspace; and rounds of pairs.
+double gemm_time(int64_t M, int64_t N, int64_t K, size_t workspace_bytes);
 double gemm_pair_time(int64_t M, int64_t N, int64_t K);
 int gemm_pair_rounds(int64_t M, int64_t N);
 // Status word of these kernels (non-zero: a bounded barrier wait gave up); reading clears it and synchronises.

@@ -663,6 +663,7 @@ struct GemmPlan {
     int grid;                // of the runs (cluster == 1)
     bool cut;                // runs may hold parts of tiles
     double time;             // us, by the model that chose them
+    double whole_time;       // ... of runs of whole tiles
 };
 
 // `clusters[s]`: clusters of s CTAs that run at once (0 where unknown or none).
@@ -684,6 +685,7 @@ GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, const int* clusters
     g.grid = static_cast<int>(std::min<long long>(sms, g.tiles));
     const double rounds = static_cast<double>((g.tiles + sms - 1) / sms);
     double best = rounds * g.k_blocks * block + ends + (rounds - 1.0) * next_tile;
+    g.whole_time = best;
     for (int s = 2; s <= kMaxCluster && s <= g.k_blocks; ++s) {
         if (clusters == nullptr || clusters[s] <= 0 || g.tiles * s > INT32_MAX) continue;
         const long long waves = (g.tiles + clusters[s] - 1) / clusters[s];
@@ -763,8 +765,16 @@ int current_device(const GemmDevice** dev) {
     return devices.get(device, [device](GemmDevice& d) { return learn_device(device, d); }, dev);
 }
 
-GemmPlan plan_on(const GemmDevice& dev, int64_t M, int64_t N, int64_t K) {
-    return plan_gemm(M, N, K, std::min(dev.sms, 148), dev.clusters);
+// What a call with this much workspace does: runs that may not cut tiles are whole ones.
+GemmPlan plan_on(const GemmDevice& dev, int64_t M, int64_t N, int64_t K, size_t workspace_bytes) {
+    const int sms = std::min(dev.sms, 148);
+    GemmPlan g = plan_gemm(M, N, K, sms, dev.clusters);
+    if (g.cut && workspace_bytes < linear_counter_bytes(M, N) + gemm_partial_bytes(g)) {
+        g.cut = false;
+        g.grid = static_cast<int>(std::min<long long>(sms, g.tiles));
+        g.time = g.whole_time;
+    }
+    return g;
 }
 
 }  // namespace
@@ -793,23 +803,23 @@ int read_tcgen05_status(unsigned* value) {
 }
 
 // The plan for the current device, or where there is none, for a B200.
-static GemmPlan plan_here(int64_t M, int64_t N, int64_t K) {
+static GemmPlan plan_here(int64_t M, int64_t N, int64_t K, size_t workspace_bytes) {
     static const GemmDevice b200;
     const GemmDevice* dev = nullptr;
     if (current_device(&dev) != W4A16_OK) {
         (void)cudaGetLastError();
         dev = &b200;
     }
-    return plan_on(*dev, M, N, K);
+    return plan_on(*dev, M, N, K, workspace_bytes);
 }
 
 size_t gemm_scratch_bytes(int64_t M, int64_t N, int64_t K) {
     if (M > INT32_MAX || N > INT32_MAX || K > INT32_MAX) return 0;
-    const GemmPlan g = plan_here(M, N, K);
+    const GemmPlan g = plan_here(M, N, K, SIZE_MAX);
     return g.cut ? linear_counter_bytes(M, N) + gemm_partial_bytes(g) : 0;
 }
 
-double gemm_time(int64_t M, int64_t N, int64_t K) { return plan_here(M, N, K).time; }
+double gemm_time(int64_t M, int64_t N, int64_t K, size_t workspace_bytes) { return plan_here(M, N, K, workspace_bytes).time; }
 
 int launch_linear_gemm(const LinearProblem& prob, cudaStream_t stream) {
     if (prob.K % kBlockK != 0 || prob.K <= 0 || !is_stream_group(prob.group)) return W4A16_ERR_BAD_CONFIG;
@@ -820,14 +830,9 @@ int launch_linear_gemm(const LinearProblem& prob, cudaStream_t stream) {
     const GemmDevice* dev = nullptr;
     const int known = current_device(&dev);
     if (known != W4A16_OK) return known;
-    GemmPlan g = plan_on(*dev, prob.M, prob.N, prob.K);
+    const GemmPlan g = plan_on(*dev, prob.M, prob.N, prob.K, usable_workspace(prob));
     if (g.tiles * g.k_blocks > INT32_MAX) return W4A16_ERR_TOO_LARGE;
     const size_t counters = linear_counter_bytes(prob.M, prob.N);
-    if (g.cut && (prob.workspace == nullptr || reinterpret_cast<uintptr_t>(prob.workspace) % 16 != 0 ||
-                  prob.workspace_bytes < counters + gemm_partial_bytes(g))) {
-        g.cut = false;
-        g.grid = static_cast<int>(std::min<long long>(dev->sms, g.tiles));
-    }
     CUtensorMap x_map, w_map;
     if (!encode_rows(&x_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, prob.x, prob.M, prob.K * 2, 128, g.bn, CU_TENSOR_MAP_SWIZZLE_128B,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||

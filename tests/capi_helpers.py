@@ -51,6 +51,17 @@ def capi_linear(x, packed, scales, group_size=128, *, workspace=None, flags=0, c
     return y
 
 
+def kernels_of(call) -> list[str]:
+    """Names of the device functions that ``call()`` launches, in order."""
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as profile:
+        call()
+        torch.cuda.synchronize()
+    names = [event.name for event in profile.events() if event.device_type == torch.autograd.DeviceType.CUDA]
+    assert names, "the profiler saw nothing"
+    return names
+
+
 def capi_dequantize(packed, scales, group_size=128, expect=0):
     n, k = packed.shape[0], packed.shape[1] * 2
     w = torch.empty((n, k), dtype=torch.float16, device=packed.device)

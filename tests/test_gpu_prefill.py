@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 import torch
 
-from capi_helpers import capi_dequantize, capi_linear, check_against_oracle, new_workspace
+from capi_helpers import capi_dequantize, capi_linear, check_against_oracle, kernels_of, new_workspace
 from nibble_b200 import _native, quantize_and_pack_weights
 from oracle import w4a16_oracle as oracle
 
@@ -354,4 +354,33 @@ def test_gemm_on_pairs_of_sms(m, k, n, gs):
         assert torch.equal(capi_linear(x, packed, scales, gs, flags=flags), y)
     bias = torch.randn((n,), device="cuda").half()
     assert torch.equal(torch.ops.w4a16.linear_bias(x, packed, scales, bias, gs), y + bias)
+    assert _device_status() == 0
+
+
+def _gemm_of(call) -> str:
+    """Which GEMM one call takes: "single" SMs or "pair"."""
+    names = [name for name in kernels_of(call) if "linear_" in name]
+    assert len(names) == 1, names
+    assert "linear_gemm_kernel" in names[0] or "linear_gemm_pair_kernel" in names[0], names
+    return "pair" if "linear_gemm_pair_kernel" in names[0] else "single"
+
+
+@pytest.mark.parametrize(("m", "k", "n"), [(300, 8192, 28672), (384, 4096, 14336)])
+def test_the_gemm_is_chosen_by_what_the_workspace_allows(m, k, n):
+    """Equal runs that cut tiles are what makes single SMs the faster way for these layers: a call without room for the parts
+    takes pairs, whatever the room would have allowed."""
+    lib = _native.core()
+    need = lib.w4a16_linear_scratch_bytes(m, n, k, 128, 0)
+    assert need > 4 << 20
+    torch.manual_seed(m)
+    packed = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda")
+    scales = (torch.rand((n, k // 128), device="cuda") * 0.01 + 1e-3).half()
+    x = torch.randn((m, k), device="cuda").half()
+    workspace = torch.zeros(need + 16, dtype=torch.uint8, device="cuda")
+    results = {}
+    for name, given in (("enough", workspace[:need]), ("too small", workspace[:need - 1]), ("misaligned", workspace[8:need + 8]), ("none", None)):
+        results[name] = capi_linear(x, packed, scales, workspace=given)
+        assert _gemm_of(lambda: capi_linear(x, packed, scales, workspace=given)) == ("single" if name == "enough" else "pair"), name
+    assert torch.equal(results["too small"], results["none"]) and torch.equal(results["misaligned"], results["none"])
+    torch.testing.assert_close(results["enough"], results["none"], rtol=2e-3, atol=1e-2)
     assert _device_status() == 0
