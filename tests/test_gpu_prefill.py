@@ -1,5 +1,4 @@
-"""-m gpu: prefill-sized batches (M >= 65) take the tcgen05 GEMM with the dequantisation fused into its
-producer warps.  Checked against the oracle on the same packed codes, against the mma.sync kernel,
+"""-m gpu: prefill-sized batches (M >= 65) take one of the two tcgen05 GEMMs that dequantise into tensor memory.  Checked against the oracle on the same packed codes, against the mma.sync kernel,
 and for a clean device status word (no barrier wait gave up)."""
 from __future__ import annotations
 
@@ -20,6 +19,14 @@ def _device_status() -> int:
     value = ctypes.c_uint32(123)
     assert _native.core().w4a16_device_status(ctypes.byref(value)) == 0
     return value.value
+
+
+def _gemm_of(call) -> str:
+    """Which GEMM one call takes: "single" SMs or "pair"."""
+    names = [name for name in kernels_of(call) if "linear_" in name]
+    assert len(names) == 1, names
+    assert "linear_gemm_kernel" in names[0] or "linear_gemm_pair_kernel" in names[0], names
+    return "pair" if "linear_gemm_pair_kernel" in names[0] else "single"
 
 
 def _case(m, k, n, seed):
@@ -51,10 +58,10 @@ def test_tcgen05_path_matches_oracle(m, k, n):
 
 
 @pytest.mark.parametrize(("m", "k", "n"), [
-    (600, 512, 8192),      # 3 x 64 tiles: more tiles than SMs, every CTA reuses an accumulator buffer
-    (1024, 256, 16384),    # 512 tiles: at least three per CTA, both accumulator buffers recycled
+    (600, 512, 8192),      # pairs of SMs, 3 x 32 tiles: two for some
+    (1024, 256, 16384),    # 256 tiles: at least three a pair
     (257, 1024, 1000),     # two ragged batch tiles, ragged last weight slab
-    (2048, 2048, 640),     # 8 batch tiles walked in groups
+    (2048, 2048, 640),     # single SMs, 16 batch tiles
 ])
 def test_tcgen05_many_tiles(m, k, n):
     _device_status()
@@ -70,17 +77,16 @@ def test_tcgen05_many_tiles(m, k, n):
 
 
 @pytest.mark.parametrize(("m", "k", "n"), [
-    (17, 384, 128),       # three 128-wide stages: the last copy of codes of a tile is half used
-    (40, 640, 256),       # five stages, two tiles
-    (64, 1152, 384),      # nine stages
-    (128, 896, 200),      # seven stages, 128-row batch tile (three operand stages, three working groups)
-    (130, 640, 128),      # 64-wide stages (batch tile above 128 rows), ten of them: a half-used last copy
-    (256, 384, 256),      # six 64-wide stages
-    (200, 128, 128),      # two 64-wide stages: half a copy in all
+    (17, 384, 128),       # single SMs: three blocks, one for each group of dequantisers
+    (40, 640, 256),       # five
+    (64, 1152, 384),      # nine, two tiles
+    (128, 896, 200),      # pairs of SMs: seven, for four groups
+    (130, 640, 128),      # five; one SM of the pair has no channel
+    (256, 384, 256),      # single SMs, two batch tiles
+    (200, 128, 128),      # one block
 ])
-def test_forced_gemm_on_odd_stage_counts(m, k, n):
-    """Stage counts that do not fill the last copy of codes, for both stage widths, through the flag that
-    sends any batch to the GEMM."""
+def test_forced_gemm_on_odd_block_counts(m, k, n):
+    """K blocks that do not come out even among the groups of dequantisers, through the flag that sends any batch to a GEMM."""
     _device_status()
     x, packed, scales = _case(m, k, n, seed=m * 7 + k)
     y = capi_linear(x, packed, scales, flags=_native.FLAG_FORCE_TCGEN05)
@@ -127,12 +133,12 @@ def test_batch_too_large_for_the_streaming_kernel_without_scratch_takes_the_gemm
 
 
 @pytest.mark.parametrize(("m", "k", "n"), [
-    (65, 4096, 256),       # 2 tiles: four K ranges of 1024 (ranges are not made shorter than that)
-    (65, 4096, 250),       # the same with M x N not a multiple of four: the element-wise sum kernel
-    (128, 4096, 1024),     # 8 tiles: four ranges
-    (100, 4352, 640),      # 5 tiles, K = 17 x 256: three ranges of 1280 and one of 512
-    (300, 8192, 512),      # two batch tiles (64-wide stages), 8 tiles in all: four ranges of 2048
-    (32, 8192, 4096),      # a medium batch on the forced GEMM: 32 tiles, four ranges
+    (65, 4096, 256),       # 1 tile: eight CTAs share its 32 blocks
+    (65, 4096, 250),       # the same, ragged channels
+    (128, 4096, 1024),     # 4 tiles
+    (100, 4352, 640),      # 3 tiles of 34 blocks: shares of four and five
+    (300, 8192, 512),      # three batch tiles, 6 tiles in all
+    (32, 8192, 4096),      # a medium batch on the forced GEMM: 16 tiles
 ])
 def test_gemm_splits_k_when_the_layer_has_few_tiles(m, k, n):
     """Layers of few tiles, whose K the GEMM shares between CTAs (inside clusters, so that a workspace changes nothing):
@@ -164,11 +170,13 @@ def test_all_nibble_values_and_repeatability(golden):
     packed = torch.from_numpy(data["packed"]).cuda()
     scales = torch.from_numpy(data["scales"]).cuda()
     x = torch.randn((96, 1024), generator=torch.Generator().manual_seed(5)).half().cuda()
-    first = capi_linear(x, packed, scales)
-    second = capi_linear(x, packed, scales)
-    assert torch.equal(first, second)
-    assert _device_status() == 0
-    check_against_oracle(first, x, packed, scales, fp16_weights=True)
+    for rows, gemm in ((96, "pair"), (64, "single")):
+        some = x[:rows]
+        first = capi_linear(some, packed, scales, flags=_native.FLAG_FORCE_TCGEN05)
+        assert _gemm_of(lambda: capi_linear(some, packed, scales, flags=_native.FLAG_FORCE_TCGEN05)) == gemm
+        assert torch.equal(capi_linear(some, packed, scales, flags=_native.FLAG_FORCE_TCGEN05), first)
+        assert _device_status() == 0
+        check_against_oracle(first, some, packed, scales, fp16_weights=True)
 
 
 @pytest.mark.parametrize(("m", "k", "n", "gs"), [
@@ -176,13 +184,13 @@ def test_all_nibble_values_and_repeatability(golden):
     (65, 4096, 1900, 128),     # batch tile above 64 rows: two weight slots
     (128, 8192, 28672, 128),   # equal runs that cut tiles, two segments each
     (40, 8192, 28672, 128),    # ... with three weight slots
-    (100, 5632, 12345, 128),   # ... on ragged channels
-    (130, 512, 40000, 128),    # runs of several whole tiles, two batch tiles
-    (512, 1024, 5000, 128),
+    (100, 5632, 19001, 128),   # ... on ragged channels
+    (300, 512, 20000, 128),    # runs of several whole tiles, three batch tiles
+    (777, 1024, 5376, 128),    # 147 whole tiles
     (128, 4096, 3000, 64), (300, 8192, 1000, 32), (77, 2048, 32000, 32),
 ])
-def test_gemm_from_tensor_memory(m, k, n, gs):
-    """Every way the GEMM shares tiles, with and without a workspace, against the product with the same FP16 weights."""
+def test_gemm_on_single_sms(m, k, n, gs):
+    """Every way this GEMM shares tiles, with and without a workspace, against the product with the same FP16 weights."""
     from nibble_b200 import dequantize_cuda
 
     _device_status()
@@ -192,6 +200,7 @@ def test_gemm_from_tensor_memory(m, k, n, gs):
     want = x.float() @ dequantize_cuda(packed, scales, gs).float().t()
     ws = torch.zeros(40 << 20, dtype=torch.uint8, device="cuda")
     for workspace in (ws, ws, None):
+        assert _gemm_of(lambda: capi_linear(x, packed, scales, gs, workspace=workspace, flags=_native.FLAG_FORCE_TCGEN05)) == "single"
         y = capi_linear(x, packed, scales, gs, workspace=workspace, flags=_native.FLAG_FORCE_TCGEN05)
         torch.testing.assert_close(y.float(), want, rtol=2e-3, atol=2e-3)
         assert torch.equal(y, capi_linear(x, packed, scales, gs, workspace=workspace, flags=_native.FLAG_FORCE_TCGEN05))
@@ -223,8 +232,11 @@ def test_scratch_query_is_exact_for_equal_runs(m, k, n, gs):
 
 
 @pytest.mark.parametrize("gs", [128, 64, 32])
-@pytest.mark.parametrize(("m", "k", "n"), [(128, 8192, 28672), (64, 8192, 16384), (100, 28672, 8192), (300, 5632, 12345)])
-def test_gemm_results_do_not_depend_on_timing(m, k, n, gs):
+@pytest.mark.parametrize(("m", "k", "n", "gemm"), [
+    (128, 8192, 28672, "single"), (64, 8192, 16384, "single"), (100, 28672, 8192, "single"), (300, 5632, 12345, "single"),
+    (2048, 8192, 28672, "pair"), (512, 2048, 5000, "pair"), (700, 640, 12000, "pair"),
+])
+def test_gemm_results_do_not_depend_on_timing(m, k, n, gemm, gs):
     """Forty calls, with other work in front of some of them, give the bits of the first: a slot of codes refilled while a
     dequantiser still reads it shows as a few wrong output channels in one call out of many."""
     torch.manual_seed(m + gs)
@@ -234,6 +246,7 @@ def test_gemm_results_do_not_depend_on_timing(m, k, n, gs):
     flags = _native.FLAG_FORCE_TCGEN05
     for workspace in (None, torch.zeros(40 << 20, dtype=torch.uint8, device="cuda")):
         first = capi_linear(x, packed, scales, gs, workspace=workspace, flags=flags)
+        assert _gemm_of(lambda: capi_linear(x, packed, scales, gs, workspace=workspace, flags=flags)) == gemm
         different = 0
         for call in range(40):
             if call % 4 == 3:
@@ -245,16 +258,17 @@ def test_gemm_results_do_not_depend_on_timing(m, k, n, gs):
     assert _device_status() == 0
 
 
-@pytest.mark.parametrize(("m", "k", "n"), [
-    (512, 1024, 9600), (513, 1024, 9600),      # 4 and 5 batch tiles; from 513 rows on the tiles of one round decide: 5 x 38
-    (777, 1024, 5376), (777, 1024, 5377),      # 147 and 154 tiles
-    (1024, 2048, 8192), (1025, 2048, 8192), (1024, 1920, 8192),
-    (2048, 3968, 4000), (2048, 4096, 4000), (2048, 4096, 4700),      # 256, 256 and 304 tiles
-    (5000, 4096, 1000), (3000, 256, 130),
+@pytest.mark.parametrize(("m", "k", "n", "gemm"), [
+    (64, 2048, 18944, None), (128, 2048, 18944, "pair"), (128, 2048, 18945, "single"),          # 74 and 75 tiles of pairs
+    (777, 1024, 5376, "single"), (777, 1024, 5377, "pair"),                                     # 147 and 154 of single SMs
+    (1024, 2048, 9728, "single"), (1025, 2048, 9728, "pair"), (1024, 1920, 9728, "pair"),
+    (2500, 3968, 1930, "pair"), (2500, 4096, 1930, "single"),                                   # 160
+    (2048, 4096, 4700, "pair"),                                                                 # 304
+    (2048, 4096, 4000, "pair"), (5000, 4096, 1000, "single"), (3000, 256, 130, "single"),       # by their models
 ])
-def test_both_gemms_beyond_512_rows(m, k, n):
-    """Either side of every line between the two GEMMs: the product with the same FP16 weights, the same bits again, and
-    nothing outside the output."""
+def test_either_side_of_the_lines_between_the_gemms(m, k, n, gemm):
+    """The kernel that each side of each line names runs there, and gives the product with the same FP16 weights, the same bits again,
+    and nothing outside the output."""
     from nibble_b200 import dequantize_cuda
 
     _device_status()
@@ -265,20 +279,19 @@ def test_both_gemms_beyond_512_rows(m, k, n):
     need = _native.core().w4a16_linear_scratch_bytes(m, n, k, 128, 0)
     for workspace in (None, torch.zeros(max(need, 16), dtype=torch.uint8, device="cuda")):
         y = capi_linear(x, packed, scales, workspace=workspace)
+        if gemm is not None and (workspace is not None or need == 0):      # (64 rows stream or not by a line of their own)
+            assert _gemm_of(lambda: capi_linear(x, packed, scales, workspace=workspace)) == gemm
         torch.testing.assert_close(y.float(), want, rtol=2e-3, atol=2e-3)
         assert torch.equal(y, capi_linear(x, packed, scales, workspace=workspace))
     assert _device_status() == 0
 
 
 @pytest.mark.parametrize(("m", "k", "n"), [
-    # 128-wide stages: 75 to 148 tiles of 128 channels, up to 128 rows; one stage, odd counts that half use the last copy of codes
     (65, 128, 9600), (128, 384, 9601), (96, 640, 18944), (100, 896, 12345), (128, 1024, 9473), (66, 1024, 18943),
-    # 64-wide stages: more tiles than one round of the other kernel (two, from K = 4096 on)
     (513, 384, 16385), (700, 640, 12000), (1100, 896, 9001), (1025, 1152, 9216), (2049, 2048, 2500), (2500, 3968, 1930), (2000, 5632, 4900),
 ])
-def test_gemm_from_shared_memory(m, k, n):
-    """The calls that still take the kernel with its weights in shared memory: odd stage counts, ragged channels and batches,
-    both stage widths, with and without a bias; one launch, no scratch."""
+def test_gemms_on_ragged_layers(m, k, n):
+    """Odd numbers of K blocks, ragged channels and batches, with and without a bias; one launch, no scratch."""
     from nibble_b200 import dequantize_cuda
 
     lib = _native.core()
@@ -301,7 +314,7 @@ def test_gemm_from_shared_memory(m, k, n):
 
 @pytest.mark.parametrize("gs", [128, 64, 32])
 def test_gemm_weights_are_rounded_products_for_any_scale(gs):
-    """Single ones as activations read the weights of the GEMM out: half(code * scale) whatever the scale, either side of the line
+    """Single ones as activations read the weights of both GEMMs out: half(code * scale) whatever the scale, either side of the line
     where warps of small scales take an FMA on (code + 8) * 2^-20 (its largest scale is 65504 / 2^20, FP16 bits 0x2BFF)."""
     k, n = 512, 300
     g = torch.Generator().manual_seed(gs)
@@ -314,11 +327,13 @@ def test_gemm_weights_are_rounded_products_for_any_scale(gs):
     weights = capi_dequantize(packed, scales, gs)
     flags = _native.FLAG_FORCE_TCGEN05
     _device_status()
-    for first in range(0, k, 128):
-        x = torch.zeros((128, k), dtype=torch.float16, device="cuda")
-        x[torch.arange(128), first + torch.arange(128)] = 1.0
-        y = capi_linear(x, packed, scales, gs, flags=flags)
-        torch.testing.assert_close(y, weights[:, first:first + 128].t(), rtol=0, atol=0)
+    for rows, gemm in ((128, "pair"), (64, "single")):
+        for first in range(0, k, rows):
+            x = torch.zeros((rows, k), dtype=torch.float16, device="cuda")
+            x[torch.arange(rows), first + torch.arange(rows)] = 1.0
+            y = capi_linear(x, packed, scales, gs, flags=flags)
+            torch.testing.assert_close(y, weights[:, first:first + rows].t(), rtol=0, atol=0)
+        assert _gemm_of(lambda: capi_linear(x, packed, scales, gs, flags=flags)) == gemm
     assert _device_status() == 0
 
 
@@ -348,6 +363,7 @@ def test_gemm_on_pairs_of_sms(m, k, n, gs):
     before = lib.w4a16_launch_count()
     y = capi_linear(x, packed, scales, gs, flags=flags)
     assert lib.w4a16_launch_count() == before + 1
+    assert _gemm_of(lambda: capi_linear(x, packed, scales, gs, flags=flags)) == "pair"
     # FP32 sums in two orders, each within K * 2^-24 of the products' magnitudes, and one rounding to FP16
     torch.testing.assert_close(y.float(), want, rtol=2e-3, atol=2e-3)
     for _ in range(10):
@@ -355,14 +371,6 @@ def test_gemm_on_pairs_of_sms(m, k, n, gs):
     bias = torch.randn((n,), device="cuda").half()
     assert torch.equal(torch.ops.w4a16.linear_bias(x, packed, scales, bias, gs), y + bias)
     assert _device_status() == 0
-
-
-def _gemm_of(call) -> str:
-    """Which GEMM one call takes: "single" SMs or "pair"."""
-    names = [name for name in kernels_of(call) if "linear_" in name]
-    assert len(names) == 1, names
-    assert "linear_gemm_kernel" in names[0] or "linear_gemm_pair_kernel" in names[0], names
-    return "pair" if "linear_gemm_pair_kernel" in names[0] else "single"
 
 
 @pytest.mark.parametrize(("m", "k", "n"), [(300, 8192, 28672), (384, 4096, 14336)])

@@ -105,7 +105,7 @@ def test_python_and_native_forward_state_one_rule():
 
     native = _native.load_torch_ops().uses_fused_kernel
     rows = [1, 64, 65, 128, 129, 192, 193, 255, 256, 257, 448, 449, 511, 512, 513, 640, 704, 705, 768, 769, 960, 961, 1023, 1024,
-            1025, 1216, 2048, 5000, 896, 897]
+            1025, 1216, 1536, 2048, 3072, 4095, 4096, 4097, 5000, 896, 897]
     sizes = [8, 100, 256, 1000, 1024, 1152, 2048, 2304, 3072, 4096, 5003, 5120, 5632, 6144, 8064, 8192, 11008, 12928, 16384, 28672, 32000]
     inner = [64, 96, 128, 384, 512, 896, 1024, 1152, 2048, 3072, 4096, 4992, 5120, 5632, 8064, 8192, 11008, 14336, 16384, 28672]
     verdicts = {(r, n, k, g): takes_operator(r, n, k, g)
