@@ -93,16 +93,7 @@ __device__ __forceinline__ uint64_t operand_desc(unsigned smem_address) {
     return desc;
 }
 
-// D (TMEM) += A (shared memory) x B (shared memory), or A from TMEM.
-__device__ __forceinline__ void umma_f16(unsigned tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t instr_desc,
-                                         uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(instr_desc), "r"(accumulate)
-        : "memory");
-}
+// D (TMEM) += A (TMEM) x B (shared memory).
 __device__ __forceinline__ void umma_f16_tmem_a(unsigned tmem_d, unsigned tmem_a, uint64_t b_desc, uint32_t instr_desc,
                                                 uint32_t accumulate) {
     asm volatile(
