@@ -41,7 +41,8 @@ bool small_group_streams(const void* x, const void* packed, const void* scales, 
 namespace {
 
 // Ranges of K that CTAs would share a 128 x 256 tile in: up to four where half the SMs or more would idle, of 1024 and more.  Part
-// of the line below and of the workspace query; the kernels share tiles in ways of their own.
+// of the line below; and of the workspace query, whose answer also serves explicit launch shapes that split K.  The GEMMs share tiles
+// in ways of their own, which w4a16_linear_scratch_bytes knows.
 int k_ranges(int64_t M, int64_t N, int64_t K) {
     const int64_t tiles = (M + 255) / 256 * ((N + 127) / 128);
     int64_t ranges = tiles > 0 ? std::min<int64_t>(4, 148 / tiles) : 1;
@@ -55,8 +56,8 @@ int k_ranges(int64_t M, int64_t N, int64_t K) {
 // scales its FP32 sums, the GEMM rounds each weight to FP16 first.  So the line stays where it was drawn, and no batch that has
 // exact weights loses them to a faster kernel.  It was drawn from the cost of the GEMM with weights in shared memory (0.6 us per
 // 128-wide K step of a round of 148 tiles, 3 us for sharing K) against the streaming kernel's (5 us plus 8 + 1.5 * K/1024 us
-// per 1e9 multiply-adds of the batch padded to 32 or 64 rows) -- these are the constants below; nearly every call it sends on
-// now runs the faster GEMM of linear_gemm.cu.
+// per 1e9 multiply-adds of the batch padded to 32 or 64 rows) -- these are the constants below; the calls it sends on run the
+// faster GEMM of linear_gemm.cu.
 // Measured on 23 layers at nine batches (us, streaming / that GEMM): beyond the line the GEMM is never slower by more than 5 % (14336 ->
 // 4096, 9 rows: 17.9 / 18.9) and up to six times as fast (8192 -> 28672, 64 rows: 251 / 47); on this side of it exact weights are
 // faster on small layers (2048 x 2048, 32 rows: 7.2 / 7.9) and cost up to twice the time on others (8192 -> 28672, 16 rows:
@@ -82,7 +83,7 @@ bool routes_to_tcgen05(int64_t M, int64_t N, int64_t K, uint32_t flags) {
 // one on single SMs, with up to 128 batch rows a tile and the K of few tiles shared, which for some layers takes a workspace.  By their
 // models' times for what either would do (us, pairs / single SMs:
 // 8192 -> 28672, 2048 rows 730 to 740 / 910 to 1060; 8192 x 8192, 512 rows 59 / 67; 5632 -> 2048, 777 rows 30 / 24), with two lines:
-//   - up to 128 rows, one batch tile of the second kernel, only in one round of pairs: in two they are level (8192 -> 28672, 96 rows:
+//   - up to 128 rows, one batch tile of the second kernel, only in one round of pairs: in two it loses (8192 -> 28672, 96 rows:
 //     63 / 55; in one, 1024 -> 8192, 128 rows: 7.0 / 10.4);
 //   - above 512 rows the second kernel only where its tiles fit a round, two with K >= 4096, or K >= 2048 up to 1024 rows: beyond,
 //     the first is the faster one whatever the models say (157 calls, at most 1 % slower).

@@ -77,6 +77,7 @@ at::Tensor workspace_for(const at::Device& device, cudaStream_t stream, int64_t 
 //                        for compatibility and means 2.  Anything else is an error, as in the reference
 //                        (csrc/int4_linear_kernel.cu:481-491).
 //   W4A16_DECODE         "generic" forces the generic kernel
+// (The module heeds the first two as far as heeds_named_kernel says.)
 //   W4A16_PDL            "1": weights may be read before the kernel in front has finished
 struct EnvironmentChoices {
     int row_tiles = 0;      // 0: not forced

@@ -8,10 +8,10 @@
 // What bounds it.  A K block of 256 weight rows is 32768 weights: 500 issue slots of each SM quarter to unpack (thirteen
 // instructions per word of eight codes), 8 clocks of MMA per batch row, 16 MMAs to issue at about 40 clocks each, and 16 KB
 // of codes plus 256 bytes per batch row out of L2, which gives an SM some 50 bytes per clock.  Hence 256 rows: with 128, the x
-// tile of a 128-row batch alone took the whole of that.  Measured from the time against K, weights from HBM (K from 2048 to 16384):
-// 0.8 to 1.0 us a block at 64 batch rows (the chain of waits, unpacking and stores of the three dequantiser groups; two groups
-// took a quarter more), 1.1 to 1.3 us at 128, of which the MMAs are 0.55; and 7 to 8 us of start, exchange and end beside them, a
-// tenth to a third of a call: tensor pipe active 41 % of the time (128 rows, 8192 -> 28672).
+// tile of a 128-row batch alone took the whole of that.  Measured from the time against K (one tile a CTA, 37888 channels, K from 2048 to
+// 16384, calls back to back): a block at 64 batch rows 0.56 us while the weights stay in L2, 0.71 to 0.97 out of HBM (the chain of waits,
+// unpacking and stores of the three dequantiser groups; two groups took a quarter more), at 128 rows 0.69, and 0.89 to 1.17, of which
+// the MMAs are 0.55; and 5 to 11 us of start and end beside them: tensor pipe active 48 % of the time (128 rows, 8192 -> 28672).
 //
 // (A GEMM with the FP16 tile in shared memory, since given up, was 1.2 to 1.9 times slower by the store, a proxy
 // fence and the space that takes.)

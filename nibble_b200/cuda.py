@@ -146,7 +146,8 @@ def linear_bias_cuda(
 
     Not part of the reference's surface.  Unlike ``linear_cuda`` it lets batches of 65 rows and more round each weight to FP16
     whatever the group size, as the product with dequantised weights does; where the tensor-core kernels decline the addresses of
-    the activations or scales, such batches are that product.
+    the activations or scales, such batches are that product, and so are those beyond what a kernel named by ``W4A16_DECODE`` or
+    ``W4A16_ROWS_PER_WARP`` is meant for.
     """
     _require_extension()
     return torch.ops.w4a16.linear_bias(activations, packed_weights, scales, bias, group_size)
