@@ -33,9 +33,10 @@ c10::TypedOperatorHandle<Signature> operator_handle(const char* name) {
 }
 
 // Whether the operator is the faster way for 897 to 4096 rows, by models of both (us).  Their constants are fitted to the times of both
-// on 259 calls with 897 to 4096 rows on layers of 512 to 28416 -> 256 to 20992, in runs of 14 ms: choosing by them is 0.9 % slower
-// than the better way on average.  By the depth of the layer alone (K >= 2048 to the operator) it was 2.9 %, and narrow layers, which
-// leave half of the SMs without a tile, took up to 1.6 times as long (7296 -> 384, 3072 rows: 31 / 20; 8192 -> 1024, 1536 rows: 33 / 27).
+// on 259 calls on layers of 512 to 28416 -> 256 to 20992, in runs of 14 ms.  On 700 other calls (by which the term for few tiles was
+// set) choosing by them is 0.8 % slower than the better way on average, and more than 3 % slower than the product on 24.  By the depth
+// of the layer alone (K >= 2048 to the operator) it was 2.1 % and 142, and narrow layers, which leave half of the SMs without a tile,
+// took up to 1.6 times as long (7296 -> 384, 3072 rows: 31 / 20; 8192 -> 1024, 1536 rows: 33 / 27).
 bool operator_is_faster(int64_t rows, int64_t out_features, int64_t in_features) {
     const int64_t k_blocks = in_features / 128, n_tiles = (out_features + 255) / 256;
     const int64_t tiles = n_tiles * ((rows + 127) / 128), pair_tiles = n_tiles * ((rows + 255) / 256);
@@ -50,7 +51,8 @@ bool operator_is_faster(int64_t rows, int64_t out_features, int64_t in_features)
     }
     if (single < by_operator) by_operator = single;
     const double weights = static_cast<double>(out_features) * static_cast<double>(in_features);
-    const double by_product = 7.0 + weights / 1.75e6 + static_cast<double>(rows) * weights / 6.1e8;
+    double by_product = 7.0 + weights / 1.75e6 + static_cast<double>(rows) * weights / 6.1e8;
+    if (tiles <= 33) by_product += 0.04 * static_cast<double>(k_blocks);      // cuBLAS is short of tiles too (17792 -> 256, 1792 rows: 24 / 33)
     return by_operator < (by_product > 15.5 ? by_product : 15.5);      // (two launches and their operators: 15.5 us of host time)
 }
 

@@ -58,6 +58,8 @@ def _operator_is_faster(rows: int, out_features: int, in_features: int) -> bool:
         by_operator = single
     weights = out_features * in_features
     by_product = 7.0 + weights / 1.75e6 + rows * weights / 6.1e8
+    if tiles <= 33:
+        by_product += 0.04 * k_blocks
     return by_operator < by_product or by_operator < 15.5
 
 

@@ -138,7 +138,7 @@ def test_narrow_layers_of_many_rows_go_to_the_product():
                        (1536, 8192, 1024), (1536, 4096, 1024), (1024, 5376, 1536), (2816, 12672, 384)):
         assert not takes_operator(rows, n, k, 128) and not native(rows, n, k, 128)
     for rows, k, n in ((2048, 8192, 28672), (2048, 14336, 4096), (2155, 6272, 2048), (1063, 24832, 3584), (2048, 5632, 2048), (4096, 8192, 1024),
-                       (960, 8192, 8192), (1280, 512, 768), (1024, 8192, 1024)):
+                       (960, 8192, 8192), (1280, 512, 768), (1024, 8192, 1024), (1792, 17792, 256), (1187, 10240, 512)):
         assert takes_operator(rows, n, k, 128) and native(rows, n, k, 128)
 
 
